@@ -272,11 +272,16 @@ int rptc_embed_mailbox(const void *table, const uint64_t *slots, uint32_t *steps
  * shift-register walk from state 0 minimises sum_i pos_weight[i] * (samples[i] - alphabet[state_i])^2, and that
  * minimum (loss[rows]).  alphabet fp32 [2^L], 4 <= L <= 16.  First-minimum tie breaks and unfused fp32 arithmetic, as
  * in the reference.  workspace: rptc_viterbi_workspace_bytes(rows, n, L) bytes of device memory, 256-byte aligned
- * (two cost arrays and one survivor byte per position, row and state prefix: 16 KiB per row and position at L = 16). */
+ * (two survivor bits per position, row and state prefix: 4 KiB per row and position at L = 16).
+ * rptc_viterbi_encode_banked: the rows are `banks` equal groups of consecutive rows with one alphabet each,
+ * alphabets fp32 [banks][2^L] (quantize_hf.py:135-150), all of them in one launch. */
 int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L);
 int rptc_viterbi_encode(const float *alphabet, const float *pos_weight, const float *samples, int64_t ld_samples, int64_t rows,
                         int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss, void *workspace, int64_t workspace_bytes,
                         rptc_stream_t stream);
+int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks, const float *pos_weight, const float *samples,
+                               int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
+                               void *workspace, int64_t workspace_bytes, rptc_stream_t stream);
 
 /* --- tensor-parallel decode: output transform + all-reduce + residual add in one kernel over NVLink peer
  * memory (no reference counterpart; the reference has no distributed code) ---

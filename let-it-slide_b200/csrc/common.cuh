@@ -40,11 +40,11 @@ struct SmemOptIn {
     bool done[kMaxDevices] = {};
 };
 template <typename Kernel>
-inline int allow_max_smem(Kernel kern, SmemOptIn &seen) {
+inline int allow_max_smem(Kernel kern, SmemOptIn &seen, int bytes = 227 * 1024) {
     const int dev = current_device();
     if (dev < 0) return cuda_fail(cudaErrorInvalidDevice);
     if (!seen.done[dev]) {
-        RPTC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        RPTC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         seen.done[dev] = true;
     }
     return RPTC_OK;

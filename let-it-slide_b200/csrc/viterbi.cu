@@ -2,94 +2,316 @@
 // whose shift-register walk  s = ((s << 2) | q) & (2^L - 1),  s_start = 0,  minimises
 //   sum_i pos_weight[i] * (samples[i] - alphabet[s_i])^2           (rptc.py:13-71, diagonal corrections).
 //
-// Dynamic programme over the 2^L states, one launch per position for a batch of rows:
-//   best[p]   = min over d = 0..3 of rho[(d << (L-2)) | p]          (first minimum, like jnp.argmin: rptc.py:27-30)
-//   rho'[4p+q] = best[p] + w * (x - alphabet[4p+q])^2                (rptc.py:52)
-// Thread p reads its four predecessors (four coalesced streams), records the winning d in back[i][row][p] and
-// writes the four successor costs with one 16-byte store.  rho ping-pongs between two buffers that stay in L2 for
-// batches up to ~128 rows; the survivors are walked backwards by one thread per row (rptc.py:62-68).
-// The arithmetic is spelled with round-to-nearest intrinsics so that no multiply-add is contracted: costs, and
+// Dynamic programme over the 2^L states (M = 2^L, P = M / 4, Q = M / 16).  The textbook step keeps the cost rho of every
+// state; here only the quarter as many values best[p] = min over d of rho[d P + p] exist, because a cost is used nowhere
+// else (rptc.py:27-30,52):
+//   best'[p'] = min over d = 0..3 of  best[d Q + (p' >> 2)] + w * (x - alphabet[d P + p'])^2      (first minimum)
+// A row's 2^14 values at L = 16 are 64 KiB: they stay in shared memory (two buffers) for the whole row, and the whole
+// row is ONE piece of work of a persistent launch instead of one launch per position.  A thread owns G groups of four
+// consecutive p', so a group needs four values of best and gives four, and its 16 alphabet entries, which no position
+// changes, stay in registers.  At L = 16 the 65,536 entries are as large as a register file, so a cluster of two CTAs
+// shares a row: each CTA makes half of the p', and stores each result where it will be read, its own or its
+// partner's shared memory.  Two rows alternate in a CTA there, so that a row's barrier passes under the other's work.
+// Bound: the arithmetic (four unfused operations per state and the minima; fp32 pairs halve the issue slots of the
+// former).  Against one launch per position with the costs in L2 (1024 x 1024 samples, L = 16, 32 alphabets):
+// see the table in the design notes of this kernel's test.
+// The winners d leave as two bits each, four to a byte, and a warp per row walks them backwards (rptc.py:62-68), three
+// positions per trip to memory.
+// The arithmetic is spelled with round-to-nearest instructions so that no multiply-add is contracted: costs, and
 // therefore ties and paths, are those of the fp32 reference.
 #include "common.cuh"
 
 namespace rptc {
 
-__global__ void viterbi_init_kernel(float *__restrict__ rho, int64_t M) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < M) rho[(int64_t)blockIdx.y * M + s] = s == 0 ? 0.f : INFINITY;       // initial state is zero (rptc.py:57-58)
+struct ViterbiParams {
+    const float *alphabets;        // [banks][M]
+    const float *pos_weight;       // [n]
+    const float *samples;          // [rows][ld_samples]
+    int64_t ld_samples;
+    uint8_t *back;                 // [rows][n][Q]: winners of position i (i >= 1), prefix 4b + j in bits 2j, 2j+1 of byte b
+    int32_t *final_state;          // [rows]
+    float *loss;                   // [rows]
+    int32_t n, L;
+    int32_t rows_per_bank, items_per_bank, n_items;
+};
+
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 
-__global__ void __launch_bounds__(256) viterbi_step_kernel(const float *__restrict__ rho, float *__restrict__ rho_next,
-                                                           uint8_t *__restrict__ back, const float4 *__restrict__ alphabet,
-                                                           const float *__restrict__ samples, int64_t ld_samples,
-                                                           const float *__restrict__ pos_weight, int64_t index, int64_t P) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
-    if (p >= P) return;
-    const float *r = rho + row * 4 * P;
-    const float c0 = r[p], c1 = r[P + p], c2 = r[2 * P + p], c3 = r[3 * P + p];
-    float best = c0;
-    int d = 0;
-    if (c1 < best) best = c1, d = 1;
-    if (c2 < best) best = c2, d = 2;
-    if (c3 < best) best = c3, d = 3;
-    back[row * P + p] = (uint8_t)d;
-    const float x = samples[row * ld_samples + index], w = pos_weight[index];
-    const float4 a = alphabet[p];
-    auto cost = [&](float e) {
-        const float diff = __fsub_rn(x, e);
-        return __fadd_rn(best, __fmul_rn(w, __fmul_rn(diff, diff)));
-    };
-    reinterpret_cast<float4 *>(rho_next + row * 4 * P)[p] = make_float4(cost(a.x), cost(a.y), cost(a.z), cost(a.w));
+// First minimum of four as (value, index): the index of the first of c0..c3 that equals the minimum.
+__device__ __forceinline__ float first_min(float c0, float c1, float c2, float c3, uint32_t &bits, int shift) {
+    const float m01 = fminf(c0, c1), m = fminf(m01, fminf(c2, c3));
+    const bool hi = m01 != m;
+    const bool lo = (hi ? c2 : c0) != m;
+    if (hi) bits |= 2u << shift;
+    if (lo) bits |= 1u << shift;
+    return m;
 }
 
-// First minimum of each row of rho -> (loss, final state).
-__global__ void __launch_bounds__(1024) viterbi_argmin_kernel(const float *__restrict__ rho, int64_t M, float *__restrict__ loss,
-                                                              int32_t *__restrict__ final_state) {
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    const float *r = rho + (int64_t)blockIdx.x * M;
-    float best = INFINITY;
-    int at = 0x7FFFFFFF;
-    for (int64_t s = threadIdx.x; s < M; s += 1024) {
-        const float v = r[s];
-        if (v < best || (v == best && s < at)) best = v, at = (int)s;
-    }
-    auto better = [](float v, int i, float bvv, int bii) { return v < bvv || (v == bvv && i < bii); };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Orders (cost, state) pairs: smaller cost first, then the smaller state (rptc.py:59, the first minimum).
+__device__ __forceinline__ unsigned long long cost_key(float v, uint32_t state) {
+    uint32_t u = __float_as_uint(v + 0.f);                      // -0 counts as +0
+    u ^= (u >> 31) ? 0xFFFFFFFFu : 0x80000000u;
+    return ((unsigned long long)u << 32) | state;
+}
+
+// CL CTAs share a row, a thread owns G groups of four prefixes, R rows alternate in a CTA.
+template <int CL, int G, int R>
+__global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiParams p) {
+    extern __shared__ __align__(16) float best_sm[];            // [R][2][P / CL]
+    __shared__ unsigned long long red[33];
+    const int t = threadIdx.x;
+    const int M = 1 << p.L, P = M >> 2, Q = M >> 4;
+    const int QC = Q / CL, PC = P / CL;                         // this CTA's share of a quarter, of all prefixes
+    uint32_t rank = 0;
+    if (CL == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const bool active = G * t < QC;                             // small L: fewer groups than a warp has lanes
+    const int kk = active ? G * t : 0;                          // first group, within this CTA
+    const int k = (int)rank * QC + kk;                          // and overall
+    // Where this thread's 4 G results go: prefix i = 4 k is read as best[d Q + k'] with d = i / Q, k' = i % Q, by the CTA
+    // that owns group k'.  4 G results never straddle two readers (CL == 2 has QC = 2048).
+    const int out_d = 4 * k / Q, out_k = 4 * k - out_d * Q;
+    const uint32_t out_rank = CL == 2 ? (uint32_t)(out_k / QC) : 0u;
+    const uint32_t out_off = CL == 2 ? 4u * (uint32_t)(out_d * QC + out_k - (int)out_rank * QC) : 16u * (uint32_t)k;
+    const uint32_t s0 = smem_addr(best_sm);
+    uint32_t out_base = s0;
+    if (CL == 2) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out_base) : "r"(s0), "r"(out_rank));
+
+    auto arrive = [] { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); };
+    auto wait = [] { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };
+
+    for (int item = blockIdx.x / CL; item < p.n_items; item += gridDim.x / CL) {
+        const int bank = item / p.items_per_bank, j = item - bank * p.items_per_bank;
+        const int row0 = bank * p.rows_per_bank + j * R;
+        const int n_rows = R == 1 ? 1 : min(R, p.rows_per_bank - j * R);
+        f32x2 na[G][4][2];                                      // alphabet entries, negated: x - e = x + (-e)
+        {
+            const float4 *alpha = reinterpret_cast<const float4 *>(p.alphabets + (int64_t)bank * M);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const int oi = __shfl_xor_sync(0xFFFFFFFFu, at, o);
-        if (better(ov, oi, best, at)) best = ov, at = oi;
-    }
-    if (lane == 0) bv[warp] = best, bi[warp] = at;
-    __syncthreads();
-    if (warp == 0) {
-        best = bv[lane], at = bi[lane];
+            for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            const int oi = __shfl_xor_sync(0xFFFFFFFFu, at, o);
-            if (better(ov, oi, best, at)) best = ov, at = oi;
+                for (int d = 0; d < 4; ++d) {
+                    const float4 a = __ldg(alpha + d * Q + k + g);
+                    na[g][d][0] = pack2(-a.x, -a.y);
+                    na[g][d][1] = pack2(-a.z, -a.w);
+                }
         }
-        if (lane == 0) {
-            loss[blockIdx.x] = best;
-            final_state[blockIdx.x] = at == 0x7FFFFFFF ? 0 : at;
+        // before the first position only the state 0 is possible (rptc.py:57-58)
+        for (int i = t; i < R * PC; i += blockDim.x) {
+            const int r = i / PC, o = i - r * PC;
+            best_sm[2 * r * PC + o] = (o == 0 && rank == 0) ? 0.f : INFINITY;
         }
+        if (CL == 2) {
+            arrive();
+            wait();
+            if (R == 2) arrive();
+        } else {
+            __syncthreads();
+        }
+        const float *xp[R];
+        uint8_t *bp[R];
+        float xn[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = row0 + (r < n_rows ? r : 0);
+            xp[r] = p.samples + (int64_t)row * p.ld_samples;
+            bp[r] = p.back + (int64_t)row * p.n * Q + k;
+            xn[r] = __ldg(xp[r]);
+        }
+        float wn = __ldg(p.pos_weight);
+
+        // the four predecessors' values of this thread's groups
+        auto load_best = [&](int r, int cur, float (&b)[4][G]) {
+            const float *src = best_sm + (2 * r + cur) * PC + kk;
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                if (G == 2) {
+                    const float2 v = *reinterpret_cast<const float2 *>(src + d * QC);
+                    b[d][0] = v.x, b[d][G - 1] = v.y;
+                } else {
+                    b[d][0] = src[d * QC];
+                }
+            }
+        };
+        // costs of the states d P + 4 (k + g) + 2 h + {0, 1}
+        auto costs = [&](const float (&b)[4][G], int g, int h, f32x2 x2, f32x2 w2, float (&lo)[4], float (&hi)[4]) {
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                const f32x2 diff = add2(x2, na[g][d][h]);
+                unpack2(add2(pack2(b[d][g], b[d][g]), mul2(w2, mul2(diff, diff))), lo[d], hi[d]);
+            }
+        };
+        auto step = [&](int r, int cur, float x, float w) {
+            float b[4][G];
+            load_best(r, cur, b);
+            const f32x2 x2 = pack2(x, x), w2 = pack2(w, w);
+            const uint32_t dst = out_base + 4u * (uint32_t)((2 * r + (cur ^ 1)) * PC) + out_off;
+            uint32_t bits = 0;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                float m[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float lo[4], hi[4];
+                    costs(b, g, h, x2, w2, lo, hi);
+                    m[2 * h] = first_min(lo[0], lo[1], lo[2], lo[3], bits, 8 * g + 4 * h);
+                    m[2 * h + 1] = first_min(hi[0], hi[1], hi[2], hi[3], bits, 8 * g + 4 * h + 2);
+                }
+                if (active) {
+                    if (CL == 2)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+                    else
+                        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+                }
+            }
+            bp[r] += Q;
+            if (active) {
+                if (G == 2) *reinterpret_cast<uint16_t *>(bp[r]) = (uint16_t)bits;
+                else *bp[r] = (uint8_t)bits;
+            }
+        };
+        int cur = 0;
+#pragma unroll 1
+        for (int i = 0; i + 1 < p.n; ++i) {
+            const float w = wn;
+            wn = __ldg(p.pos_weight + i + 1);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float x = xn[r];
+                xn[r] = __ldg(xp[r] + i + 1);
+                if (r < n_rows) step(r, cur, x, w);
+                if (CL == 2) {
+                    // With two rows the barrier entered here is the one left after the OTHER row's next step.
+                    if (R == 2) wait(), arrive();
+                    else arrive(), wait();
+                }
+            }
+            if (CL == 1) __syncthreads();
+            cur ^= 1;
+        }
+        if (CL == 2 && R == 2) wait();
+        // the last position: the cheapest of all states, first minimum
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            unsigned long long key = ~0ull;
+            if (r < n_rows && active) {
+                float b[4][G];
+                load_best(r, cur, b);
+                const f32x2 x2 = pack2(xn[r], xn[r]), w2 = pack2(wn, wn);
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float lo[4], hi[4];
+                        costs(b, g, h, x2, w2, lo, hi);
+#pragma unroll
+                        for (int d = 0; d < 4; ++d) {
+                            const uint32_t s = (uint32_t)(d * P + 4 * (k + g) + 2 * h);
+                            key = min(key, min(cost_key(lo[d], s), cost_key(hi[d], s + 1)));
+                        }
+                    }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) key = min(key, __shfl_xor_sync(0xFFFFFFFFu, key, o));
+            __syncthreads();                                    // `red` is free
+            if ((t & 31) == 0) red[t >> 5] = key;
+            __syncthreads();
+            if (t < 32) {
+                key = t < (int)(blockDim.x + 31) / 32 ? red[t] : ~0ull;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) key = min(key, __shfl_xor_sync(0xFFFFFFFFu, key, o));
+            }
+            if (CL == 2) {
+                if (t == 0 && rank == 1) {
+                    uint32_t dst;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(smem_addr(&red[32])));
+                    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(dst), "l"(key) : "memory");
+                }
+                __syncwarp();
+                arrive();
+                wait();
+                if (t == 0 && rank == 0) key = min(key, red[32]);
+            }
+            if (t == 0 && rank == 0 && r < n_rows) {
+                const uint32_t u = (uint32_t)(key >> 32);
+                p.loss[row0 + r] = __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+                p.final_state[row0 + r] = (int32_t)(key & 0xFFFFFFFFu);
+            }
+            __syncwarp();
+            if (CL == 2) arrive(), wait();                      // red[32] has been read; at the end, nobody leaves early
+        }
+        if (CL == 1) __syncthreads();                           // the buffers are free for the next row
     }
 }
 
-// One thread per row walks the survivors from the last position to the first.
-__global__ void viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state, int64_t rows,
-                                         int64_t n, int64_t P, int L, int32_t *__restrict__ symbols, int64_t ld_sym) {
-    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per row walks the winners from the last position to the first.  A position's winner is needed to know which
+// winner of the position before it to read, but with two bits each there are only four (sixteen) candidates one (two)
+// positions on: lanes 0, 1-4 and 5-20 fetch all of them at once, and the walk takes three positions per trip to memory.
+__global__ void __launch_bounds__(128) viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state,
+                                                                int64_t rows, int64_t n, int L, int32_t *__restrict__ symbols,
+                                                                int64_t ld_sym) {
+    const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (row >= rows) return;
+    const int64_t Q = int64_t(1) << (L - 4);
+    const uint8_t *b = back + row * n * Q;
+    const int level = lane == 0 ? 0 : lane < 5 ? 1 : 2;
+    const uint32_t d1 = level == 0 ? 0u : level == 1 ? (uint32_t)lane - 1u : (uint32_t)(lane - 5) >> 2, d2 = (uint32_t)(lane - 5) & 3u;
+    auto before = [&](uint32_t s, uint32_t d) { return (d << (L - 2)) | (s >> 2); };      // the state that reached s by winner d
     uint32_t state = (uint32_t)final_state[row];
-    for (int64_t i = n - 1; i >= 0; --i) {
-        symbols[row * ld_sym + i] = (int32_t)(state & 3u);
-        const uint32_t prefix = state >> 2;
-        state = ((uint32_t)back[(i * rows + row) * P + prefix] << (L - 2)) | prefix;
+    for (int64_t i = n - 1; i >= 0; i -= 3) {
+        uint32_t s = state;
+        if (level >= 1) s = before(s, d1);
+        if (level >= 2) s = before(s, d2);
+        const int64_t at = i - level;
+        uint32_t d = 0;                                         // before position 1 there is only the start state
+        if (lane < 21 && at >= 1) d = ((uint32_t)__ldg(b + at * Q + (s >> 4)) >> (2 * ((s >> 2) & 3u))) & 3u;
+        const uint32_t w0 = __shfl_sync(0xFFFFFFFFu, d, 0);
+        const uint32_t w1 = __shfl_sync(0xFFFFFFFFu, d, 1 + (int)w0);
+        const uint32_t w2 = __shfl_sync(0xFFFFFFFFu, d, 5 + 4 * (int)w0 + (int)w1);
+        const uint32_t s1 = before(state, w0), s2 = before(s1, w1);
+        const uint32_t mine = lane == 0 ? state : lane == 1 ? s1 : s2;
+        if (lane < 3 && i - lane >= 0) symbols[row * ld_sym + i - lane] = (int32_t)(mine & 3u);
+        state = before(s2, w2);
     }
+}
+
+template <int CL, int G, int R>
+static int launch_forward(const ViterbiParams &p, int threads, int slots, cudaStream_t stream) {
+    static SmemOptIn opted;
+    auto kern = viterbi_forward_kernel<CL, G, R>;
+    if (int e = allow_max_smem(kern, opted, 128 * 1024)) return e;
+    const int64_t items = p.n_items;
+    const int clusters = (int)(items < slots ? items : slots);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * CL));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)R * 2 * ((size_t(1) << p.L) / 4 / CL) * sizeof(float);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    RPTC_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+    return RPTC_OK;
 }
 
 }  // namespace rptc
@@ -98,35 +320,68 @@ using namespace rptc;
 
 extern "C" int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L) {
     if (rows <= 0 || n <= 0 || L < 4 || L > 16) return -1;
-    const int64_t M = int64_t(1) << L;
-    return 2 * rows * M * 4 + n * rows * (M / 4) + rows * 4 + 256;
+    const int64_t back = rows * n * (int64_t(1) << (L - 4));
+    return (back + 255) / 256 * 256 + rows * 4;
+}
+
+extern "C" int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks, const float *pos_weight, const float *samples,
+                                          int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
+                                          void *workspace, int64_t workspace_bytes, rptc_stream_t stream) {
+    if (!alphabets || !pos_weight || !samples || !symbols || !loss || !workspace) return RPTC_ERR_ARG;
+    if (L < 4 || L > 16) return RPTC_ERR_UNSUPPORTED;
+    if (rows <= 0 || rows > 65535 || n <= 0 || banks <= 0 || rows % banks || ld_samples < n || ld_sym < n) return RPTC_ERR_SHAPE;
+    if (n > (int64_t(1) << 30)) return RPTC_ERR_TOO_LARGE;
+    if (workspace_bytes < rptc_viterbi_workspace_bytes(rows, n, L)) return RPTC_ERR_TOO_LARGE;
+    if ((reinterpret_cast<uintptr_t>(alphabets) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255)) return RPTC_ERR_ALIGN;
+    if (int e = rptc_check_device()) return e;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    ViterbiParams p;
+    p.alphabets = alphabets;
+    p.pos_weight = pos_weight;
+    p.samples = samples;
+    p.ld_samples = ld_samples;
+    p.back = static_cast<uint8_t *>(workspace);
+    const int64_t back_bytes = (rows * n * (int64_t(1) << (L - 4)) + 255) / 256 * 256;
+    p.final_state = reinterpret_cast<int32_t *>(p.back + back_bytes);
+    p.loss = loss;
+    p.n = (int32_t)n;
+    p.L = L;
+    p.rows_per_bank = (int32_t)(rows / banks);
+    auto rows_at_once = [&](int r) {
+        p.items_per_bank = (p.rows_per_bank + r - 1) / r;
+        p.n_items = (int32_t)(banks * p.items_per_bank);
+    };
+    // Threads per CTA: a quarter of 2^(L-2) prefixes in groups of four, two groups a thread from L = 10 on (below, one warp
+    // has lanes to spare).  At L = 15 and 16 one CTA of 1024 threads fills an SM; two rows then alternate in it unless
+    // that would leave SMs idle (fewer pairs of rows than places for them).  Smaller L run one row per CTA and as many
+    // CTAs as fit (64 registers a thread).
+    const int groups = 1 << (L - 4), sms = num_sms();
+    int e;
+    rows_at_once(2);
+    if (L == 16) {
+        const int places = sms / 2;
+        if (p.n_items >= places) {
+            e = launch_forward<2, 2, 2>(p, 1024, places, s);
+        } else {
+            rows_at_once(1);
+            e = launch_forward<2, 2, 1>(p, 1024, places, s);
+        }
+    } else if (L == 15 && p.n_items >= sms) {
+        e = launch_forward<1, 2, 2>(p, 1024, sms, s);
+    } else {
+        rows_at_once(1);
+        if (L >= 10) e = launch_forward<1, 2, 1>(p, groups / 2, sms * (L == 15 ? 1 : L == 10 ? 32 : 2048 / groups), s);
+        else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
+    }
+    if (e) return e;
+    viterbi_backtrack_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym);
+    RPTC_CUDA(cudaGetLastError());
+    return RPTC_OK;
 }
 
 extern "C" int rptc_viterbi_encode(const float *alphabet, const float *pos_weight, const float *samples, int64_t ld_samples,
                                    int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss, void *workspace,
                                    int64_t workspace_bytes, rptc_stream_t stream) {
-    if (!alphabet || !pos_weight || !samples || !symbols || !loss || !workspace) return RPTC_ERR_ARG;
-    if (L < 4 || L > 16) return RPTC_ERR_UNSUPPORTED;
-    if (rows <= 0 || rows > 65535 || n <= 0 || ld_samples < n || ld_sym < n) return RPTC_ERR_SHAPE;
-    if (workspace_bytes < rptc_viterbi_workspace_bytes(rows, n, L)) return RPTC_ERR_TOO_LARGE;
-    if ((reinterpret_cast<uintptr_t>(alphabet) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255)) return RPTC_ERR_ALIGN;
-    if (int e = rptc_check_device()) return e;
-    const int64_t M = int64_t(1) << L, P = M / 4;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    float *rho_a = static_cast<float *>(workspace), *rho_b = rho_a + rows * M;
-    uint8_t *back = reinterpret_cast<uint8_t *>(rho_b + rows * M);
-    int32_t *final_state = reinterpret_cast<int32_t *>(back + n * rows * P + ((256 - (n * rows * P) % 256) % 256));
-    viterbi_init_kernel<<<dim3((unsigned)((M + 255) / 256), (unsigned)rows), 256, 0, s>>>(rho_a, M);
-    const dim3 grid((unsigned)((P + 255) / 256), (unsigned)rows);
-    for (int64_t i = 0; i < n; ++i) {
-        viterbi_step_kernel<<<grid, 256, 0, s>>>(rho_a, rho_b, back + i * rows * P, reinterpret_cast<const float4 *>(alphabet), samples,
-                                                 ld_samples, pos_weight, i, P);
-        float *t = rho_a;
-        rho_a = rho_b;
-        rho_b = t;
-    }
-    viterbi_argmin_kernel<<<(unsigned)rows, 1024, 0, s>>>(rho_a, M, loss, final_state);
-    viterbi_backtrack_kernel<<<(unsigned)((rows + 63) / 64), 64, 0, s>>>(back, final_state, rows, n, P, L, symbols, ld_sym);
-    RPTC_CUDA(cudaGetLastError());
-    return RPTC_OK;
+    return rptc_viterbi_encode_banked(alphabet, 1, pos_weight, samples, ld_samples, rows, n, L, symbols, ld_sym, loss, workspace,
+                                      workspace_bytes, stream);
 }

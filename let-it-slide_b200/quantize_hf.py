@@ -64,18 +64,24 @@ def factorize(W: torch.Tensor):
     return biases_out, biases_in, scales_out, scales_in, normalized
 
 
-def megabatch_alphabet(megabatch: torch.Tensor, shift_register_size: int) -> torch.Tensor:
-    """2^L evenly spaced quantiles of a bank's values, by linear interpolation of the sorted sample
-    (quantize_hf.py:136-140).  Interpolated in float64 and rounded to fp32."""
+def megabatch_alphabets(megabatches: torch.Tensor, shift_register_size: int) -> torch.Tensor:
+    """2^L evenly spaced quantiles of each bank's values, megabatches [banks, values] -> fp32 [banks, 2^L], by linear
+    interpolation of the sorted sample (quantize_hf.py:136-140).  Interpolated in float64 and rounded to fp32."""
     M = 1 << shift_register_size
-    fp = torch.sort(megabatch.reshape(-1).to(torch.float64)).values
-    N = fp.numel()
+    fp = torch.sort(megabatches, dim=1).values
+    N = fp.shape[1]
     x = (2 * torch.arange(M, dtype=torch.float64, device=fp.device) + 1) / 2 / M
     pos = x * N - 0.5                                  # position of x on the sample grid xp[j] = (2j+1)/(2N)
     lo = pos.floor().clamp(0, N - 1).to(torch.int64)
     hi = (lo + 1).clamp(max=N - 1)
     frac = (pos - lo.to(torch.float64)).clamp(0, 1)
-    return (fp[lo] + (fp[hi] - fp[lo]) * frac).to(torch.float32)
+    f_lo, f_hi = fp[:, lo].to(torch.float64), fp[:, hi].to(torch.float64)
+    return (f_lo + (f_hi - f_lo) * frac).to(torch.float32)
+
+
+def megabatch_alphabet(megabatch: torch.Tensor, shift_register_size: int) -> torch.Tensor:
+    """`megabatch_alphabets` of one bank: fp32 [2^L]."""
+    return megabatch_alphabets(megabatch.reshape(1, -1), shift_register_size)[0]
 
 
 def seeded_permute(seed: int) -> Callable[[torch.Tensor], torch.Tensor]:
@@ -94,16 +100,18 @@ def round_weights(permute, weights: torch.Tensor, importance: torch.Tensor, shif
     assert m % (num_banks * batch_size) == 0, (m, num_banks, batch_size)
     per_bank = m // num_banks
     pos_weight = importance.to(torch.float32) ** 2           # sum(corrections[index]**2) of a diagonal matrix (rptc.py:21)
+    quantiles = megabatch_alphabets(weights.reshape(num_banks, -1), shift_register_size)
+    alphabets = torch.stack([permute(alphabet) for alphabet in quantiles])
+    if weights.is_cuda and alphabets.dtype == torch.float32 and 4 <= shift_register_size <= 16:
+        # the CUDA encoder takes all banks at once: a bank has too few rows to fill the GPU
+        return ops.viterbi_encode_banked(alphabets, pos_weight, weights)[0], alphabets
     symbols = torch.empty((m, n), dtype=torch.int32, device=weights.device)
-    alphabets = []
-    for b in range(num_banks):
+    for b, alphabet in enumerate(alphabets):
         rows = slice(b * per_bank, (b + 1) * per_bank)
-        alphabet = permute(megabatch_alphabet(weights[rows], shift_register_size))
-        alphabets.append(alphabet)
         for r0 in range(rows.start, rows.stop, batch_size):
             q, _ = quantize_rows(alphabet, pos_weight, weights[r0:r0 + batch_size].to(torch.float32))
             symbols[r0:r0 + batch_size] = q
-    return symbols, torch.stack(alphabets)
+    return symbols, alphabets
 
 
 def evaluate_layer(H: torch.Tensor, W: torch.Tensor, recon: torch.Tensor):

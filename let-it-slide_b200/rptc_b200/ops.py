@@ -330,26 +330,40 @@ def next_token(logits: torch.Tensor, next_ids: torch.Tensor, ids: torch.Tensor |
 
 def viterbi_encode(alphabet: torch.Tensor, pos_weight: torch.Tensor, samples: torch.Tensor, workspace_limit: int = 12 << 30):
     """Code-A trellis encoder on the GPU (rptc_viterbi_encode): samples fp32 [rows, n] -> (symbols int32 [rows, n],
-    loss fp32 [rows]).  Rows go through in batches sized so that the survivor memory stays under `workspace_limit`."""
-    M = alphabet.numel()
+    loss fp32 [rows])."""
+    return viterbi_encode_banked(alphabet[None, :], pos_weight, samples, workspace_limit)
+
+
+def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, samples: torch.Tensor, workspace_limit: int = 12 << 30):
+    """The same for `alphabets` [banks, 2^L] whose banks own equal groups of consecutive rows of `samples`
+    (rptc_viterbi_encode_banked).  Rows go through in batches sized so that the survivor memory stays under
+    `workspace_limit`: whole banks while one fits, else parts of a bank."""
+    banks, M = alphabets.shape
     L = M.bit_length() - 1
     if M != 1 << L:
         raise RuntimeError("the alphabet must have 2^L entries")
-    alphabet = alphabet.to(torch.float32).contiguous()
+    alphabets = alphabets.to(torch.float32).contiguous()
     pos_weight = pos_weight.to(torch.float32).contiguous()
     samples = samples.to(torch.float32).contiguous()
     rows, n = samples.shape
+    if rows % banks:
+        raise RuntimeError("the banks must hold equally many rows")
     symbols = torch.empty((rows, n), dtype=torch.int32, device=samples.device)
     loss = torch.empty(rows, dtype=torch.float32, device=samples.device)
-    per_row = lib().rptc_viterbi_workspace_bytes(1, n, L)
-    batch = max(1, min(rows, 128, workspace_limit // per_row))
+    fit = max(1, min(65535, workspace_limit // lib().rptc_viterbi_workspace_bytes(1, n, L)))      # rows at once
+    per_bank = rows // banks
+    step = min(rows, fit // per_bank * per_bank if fit >= per_bank else fit)
     with torch.cuda.device(samples.device):
-        need = lib().rptc_viterbi_workspace_bytes(batch, n, L)
+        need = lib().rptc_viterbi_workspace_bytes(step, n, L)
         ws = torch.empty(need, dtype=torch.uint8, device=samples.device)
-        for r0 in range(0, rows, batch):
-            r = min(batch, rows - r0)
-            check(lib().rptc_viterbi_encode(ptr(alphabet), ptr(pos_weight), ptr(samples[r0:]), n, r, n, L, ptr(symbols[r0:]), n,
-                                            ptr(loss[r0:]), ptr(ws), need, stream_ptr()), "rptc_viterbi_encode")
+        r0 = 0
+        while r0 < rows:
+            bank, inside = divmod(r0, per_bank)
+            r = min(step, rows - r0) if step >= per_bank else min(step, per_bank - inside)
+            check(lib().rptc_viterbi_encode_banked(ptr(alphabets[bank:]), max(1, r // per_bank), ptr(pos_weight), ptr(samples[r0:]), n, r, n, L,
+                                                   ptr(symbols[r0:]), n, ptr(loss[r0:]), ptr(ws), need, stream_ptr()),
+                  "rptc_viterbi_encode_banked")
+            r0 += r
     return symbols, loss
 
 

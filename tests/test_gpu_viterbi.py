@@ -81,3 +81,25 @@ def _states(sym: torch.Tensor, L: int) -> torch.Tensor:
         state = ((state << 2) | sym[:, i].long()) & ((1 << L) - 1)
         out[:, i] = state
     return out
+
+
+@pytest.mark.parametrize("L,n,banks,per_bank", [(5, 7, 2, 3), (9, 33, 1, 2), (10, 12, 3, 1), (13, 21, 2, 5), (14, 9, 1, 3), (15, 1, 1, 2), (15, 12, 2, 2),
+                                                (15, 5, 100, 3), (16, 11, 1, 1), (16, 2, 2, 3), (16, 6, 51, 3)])
+def test_banked_encoder_at_the_edges_of_its_variants(L, n, banks, per_bank):
+    """One and two rows per CTA, one CTA and a pair of CTAs per row, banks with a row left over."""
+    import rptc
+    from rptc_b200 import ops
+    g = torch.Generator().manual_seed(L * 100 + n)
+    alphabets = (torch.randn(banks, 1 << L, generator=g) * 64).round() / 64          # equal entries: ties
+    samples = torch.randn(banks * per_bank, n, generator=g)
+    weights = 0.5 + torch.rand(n, generator=g)
+    sym, loss = ops.viterbi_encode_banked(alphabets.cuda(), weights.cuda(), samples.cuda())
+    for b in range(banks):
+        rows = slice(b * per_bank, (b + 1) * per_bank)
+        want_sym, want_loss = rptc.quantize_rows(alphabets[b], weights, samples[rows])
+        assert torch.equal(sym[rows].cpu(), want_sym), b
+        torch.testing.assert_close(loss[rows].cpu(), want_loss, rtol=1e-6, atol=0)
+    # a workspace that holds two rows only: parts of banks
+    again, _ = ops.viterbi_encode_banked(alphabets[:2].cuda(), weights.cuda(), samples[: min(banks, 2) * per_bank].cuda(),
+                                         workspace_limit=2 * (n << (L - 4)) + 1024)
+    assert torch.equal(again, sym[: again.shape[0]])
