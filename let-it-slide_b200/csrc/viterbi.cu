@@ -10,11 +10,11 @@
 // row is ONE piece of work of a persistent launch instead of one launch per position.  A thread owns G groups of four
 // consecutive p', so a group needs four values of best and gives four, and its 16 alphabet entries, which no position
 // changes, stay in registers.  At L = 16 the 65,536 entries are as large as a register file, so a cluster of two CTAs
-// shares a row: each CTA makes half of the p', and stores each result where it will be read, its own or its
-// partner's shared memory.  Two rows alternate in a CTA there, so that a row's barrier passes under the other's work.
-// Bound: the arithmetic (four unfused operations per state and the minima; fp32 pairs halve the issue slots of the
-// former).  Against one launch per position with the costs in L2 (1024 x 1024 samples, L = 16, 32 alphabets):
-// see the table in the design notes of this kernel's test.
+// shares a row: each CTA makes half of the p' and sends the half of its results that its partner reads by one bulk copy.  Two rows alternate in a CTA there, so that a row's values travel under the other's work.
+// Bound: instruction issue (four unfused operations per state and the minima; pairs of fp32 values take half the issue
+// slots for the former).  1024 x 1024 samples, L = 16: 603 ms with one launch per position and batch of eight rows and
+// the costs in L2; 23.1 ms with cluster barriers between positions (their release waits for the winners' stores); 30.8 ms
+// with st.async into the partner; 16.3 ms as it is (issue slots 76 % used).  L = 15: 7.2 ms.
 // The winners d leave as two bits each, four to a byte, and a warp per row walks them backwards (rptc.py:62-68), three
 // positions per trip to memory.
 // The arithmetic is spelled with round-to-nearest instructions so that no multiply-add is contracted: costs, and
@@ -33,6 +33,7 @@ struct ViterbiParams {
     float *loss;                   // [rows]
     int32_t n, L;
     int32_t rows_per_bank, items_per_bank, n_items;
+    unsigned int *status;
 };
 
 using f32x2 = unsigned long long;
@@ -53,14 +54,26 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return d;
 }
 
-// First minimum of four as (value, index): the index of the first of c0..c3 that equals the minimum.
-__device__ __forceinline__ float first_min(float c0, float c1, float c2, float c3, uint32_t &bits, int shift) {
+// First minimum of four: returns the value and adds its index (the first of c0..c3 that equals it) to `bits`, a float
+// that counts in units of 1 from 2^23, so that its low bits are the number added up.  The two additions go to the
+// multiply-add pipe: the half-rate pipe of the minima, comparisons and logic is the busier one.
+__device__ __forceinline__ float first_min(float c0, float c1, float c2, float c3, float &bits, int shift) {
     const float m01 = fminf(c0, c1), m = fminf(m01, fminf(c2, c3));
-    const bool hi = m01 != m;
-    const bool lo = (hi ? c2 : c0) != m;
-    if (hi) bits |= 2u << shift;
-    if (lo) bits |= 1u << shift;
+    asm("{\n\t.reg .pred hi, lo;\n\t.reg .f32 v;\n\t"
+        "setp.neu.f32 hi, %1, %2;\n\t"
+        "selp.f32 v, %3, %4, hi;\n\t"
+        "setp.neu.f32 lo, v, %2;\n\t"
+        "@hi add.rn.f32 %0, %0, %5;\n\t"
+        "@lo add.rn.f32 %0, %0, %6;\n\t}"
+        : "+f"(bits)
+        : "f"(m01), "f"(m), "f"(c2), "f"(c0), "f"((float)(2 << shift)), "f"((float)(1 << shift)));
     return m;
+}
+// Shared memory of this CTA -> shared memory of a CTA of the cluster, counted in bytes on a barrier over there.
+__device__ __forceinline__ void bulk_s2s(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes),
+                 "r"(bar)
+                 : "memory");
 }
 
 // Orders (cost, state) pairs: smaller cost first, then the smaller state (rptc.py:59, the first minimum).
@@ -73,24 +86,47 @@ __device__ __forceinline__ unsigned long long cost_key(float v, uint32_t state) 
 // CL CTAs share a row, a thread owns G groups of four prefixes, R rows alternate in a CTA.
 template <int CL, int G, int R>
 __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiParams p) {
-    extern __shared__ __align__(16) float best_sm[];            // [R][2][P / CL]
+    extern __shared__ __align__(128) float best_sm[];           // per row and buffer: P / CL values, and with CL == 2 half as many to send
     __shared__ unsigned long long red[33];
+    __shared__ __align__(8) unsigned long long full_bar[R][2];  // CL == 2
+    __shared__ uint32_t warps_done[R];
     const int t = threadIdx.x;
     const int M = 1 << p.L, P = M >> 2, Q = M >> 4;
     const int QC = Q / CL, PC = P / CL;                         // this CTA's share of a quarter, of all prefixes
+    const int slab = CL == 2 ? PC + PC / 2 : PC;                // floats per row and buffer
     uint32_t rank = 0;
     if (CL == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool active = G * t < QC;                             // small L: fewer groups than a warp has lanes
     const int kk = active ? G * t : 0;                          // first group, within this CTA
     const int k = (int)rank * QC + kk;                          // and overall
     // Where this thread's 4 G results go: prefix i = 4 k is read as best[d Q + k'] with d = i / Q, k' = i % Q, by the CTA
-    // that owns group k'.  4 G results never straddle two readers (CL == 2 has QC = 2048).
-    const int out_d = 4 * k / Q, out_k = 4 * k - out_d * Q;
-    const uint32_t out_rank = CL == 2 ? (uint32_t)(out_k / QC) : 0u;
-    const uint32_t out_off = CL == 2 ? 4u * (uint32_t)(out_d * QC + out_k - (int)out_rank * QC) : 16u * (uint32_t)k;
+    // that owns group k'.  4 G results never straddle two readers (CL == 2 has QC = 2048).  What the partner reads is
+    // put down behind this CTA's own values, in the order in which the partner holds it (quarters 2 rank, 2 rank + 1).
+    uint32_t out_off = 16u * (uint32_t)k;
+    if (CL == 2) {
+        const int d = 4 * k / Q, o = 4 * k - d * Q, reader = o / QC;
+        out_off = 4u * (uint32_t)((reader == (int)rank ? d * QC : PC + (d - 2 * (int)rank) * QC) + o - reader * QC);
+    }
     const uint32_t s0 = smem_addr(best_sm);
-    uint32_t out_base = s0;
-    if (CL == 2) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out_base) : "r"(s0), "r"(out_rank));
+    // CL == 2, per row: `full` of a buffer completes when this CTA's warps have all put down their values of a position
+    // and the partner's half has landed.  The warp that finishes a position last sends this CTA's half.  So a completed
+    // `full` also says that both CTAs have finished with the buffer that the next results go to, and that what was sent
+    // from the other buffer has arrived.  Nothing here needs a fence at cluster scope, which would wait for the winners
+    // on their way to global memory.  Once a wait has run out no other is tried: the kernel goes on to its end with
+    // what it has.
+    const uint32_t full0 = smem_addr(full_bar);
+    uint32_t peer_s0 = s0, peer_full0 = full0;
+    uint32_t full_phase = 0;                                    // bit 2 r + buffer
+    bool ok = true;
+    if (CL == 2) {
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer_full0) : "r"(full0), "r"(rank ^ 1u));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer_s0) : "r"(s0), "r"(rank ^ 1u));
+        if (t == 0) {
+            for (int i = 0; i < 2 * R; ++i) mbar_init(full0 + 8 * i, 1);
+            for (int i = 0; i < R; ++i) warps_done[i] = 0;
+            mbar_fence_init();
+        }
+    }
 
     auto arrive = [] { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); };
     auto wait = [] { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };
@@ -114,12 +150,11 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
         // before the first position only the state 0 is possible (rptc.py:57-58)
         for (int i = t; i < R * PC; i += blockDim.x) {
             const int r = i / PC, o = i - r * PC;
-            best_sm[2 * r * PC + o] = (o == 0 && rank == 0) ? 0.f : INFINITY;
+            best_sm[2 * r * slab + o] = (o == 0 && rank == 0) ? 0.f : INFINITY;
         }
         if (CL == 2) {
             arrive();
             wait();
-            if (R == 2) arrive();
         } else {
             __syncthreads();
         }
@@ -137,7 +172,7 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
 
         // the four predecessors' values of this thread's groups
         auto load_best = [&](int r, int cur, float (&b)[4][G]) {
-            const float *src = best_sm + (2 * r + cur) * PC + kk;
+            const float *src = best_sm + (2 * r + cur) * slab + kk;
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
                 if (G == 2) {
@@ -156,12 +191,18 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
                 unpack2(add2(pack2(b[d][g], b[d][g]), mul2(w2, mul2(diff, diff))), lo[d], hi[d]);
             }
         };
-        auto step = [&](int r, int cur, float x, float w) {
+        auto step = [&](int r, int i, int cur, float x, float w) {
+            const int nxt = cur ^ 1;
+            if (CL == 2 && i > 0) {
+                const uint32_t at = 2 * r + cur;
+                if (ok) ok = mbar_wait(full0 + 8 * at, (full_phase >> at) & 1u, p.status);
+                full_phase ^= 1u << at;
+            }
             float b[4][G];
             load_best(r, cur, b);
             const f32x2 x2 = pack2(x, x), w2 = pack2(w, w);
-            const uint32_t dst = out_base + 4u * (uint32_t)((2 * r + (cur ^ 1)) * PC) + out_off;
-            uint32_t bits = 0;
+            const uint32_t to = 4u * (uint32_t)((2 * r + nxt) * slab), dst = s0 + to + out_off;
+            float bits = 8388608.f;                             // 2^23
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 float m[4];
@@ -172,17 +213,27 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
                     m[2 * h] = first_min(lo[0], lo[1], lo[2], lo[3], bits, 8 * g + 4 * h);
                     m[2 * h + 1] = first_min(hi[0], hi[1], hi[2], hi[3], bits, 8 * g + 4 * h + 2);
                 }
-                if (active) {
-                    if (CL == 2)
-                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
-                    else
-                        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+                if (active)
+                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+            }
+            if (CL == 2) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the copy engine reads what was put down
+                __syncwarp();
+                if ((t & 31) == 0) {
+                    uint32_t before;
+                    asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_addr(&warps_done[r])) : "memory");
+                    if ((before & 31u) == 31u) {                // 32 warps: this was the last one
+                        const uint32_t half = 2u * (uint32_t)PC;
+                        mbar_expect_tx(full0 + 8 * (2 * r + nxt), half);
+                        bulk_s2s(peer_s0 + to + rank * half, s0 + to + 2u * half, half, peer_full0 + 8u * (uint32_t)(2 * r + nxt));
+                    }
                 }
+                __syncwarp();
             }
             bp[r] += Q;
             if (active) {
-                if (G == 2) *reinterpret_cast<uint16_t *>(bp[r]) = (uint16_t)bits;
-                else *bp[r] = (uint8_t)bits;
+                if (G == 2) *reinterpret_cast<uint16_t *>(bp[r]) = (uint16_t)__float_as_uint(bits);
+                else *bp[r] = (uint8_t)__float_as_uint(bits);
             }
         };
         int cur = 0;
@@ -194,21 +245,20 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
             for (int r = 0; r < R; ++r) {
                 const float x = xn[r];
                 xn[r] = __ldg(xp[r] + i + 1);
-                if (r < n_rows) step(r, cur, x, w);
-                if (CL == 2) {
-                    // With two rows the barrier entered here is the one left after the OTHER row's next step.
-                    if (R == 2) wait(), arrive();
-                    else arrive(), wait();
-                }
+                if (r < n_rows) step(r, i, cur, x, w);
             }
             if (CL == 1) __syncthreads();
             cur ^= 1;
         }
-        if (CL == 2 && R == 2) wait();
         // the last position: the cheapest of all states, first minimum
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             unsigned long long key = ~0ull;
+            if (CL == 2 && r < n_rows && p.n > 1) {
+                const uint32_t at = 2 * r + cur;
+                if (ok) ok = mbar_wait(full0 + 8 * at, (full_phase >> at) & 1u, p.status);
+                full_phase ^= 1u << at;
+            }
             if (r < n_rows && active) {
                 float b[4][G];
                 load_best(r, cur, b);
@@ -295,13 +345,13 @@ template <int CL, int G, int R>
 static int launch_forward(const ViterbiParams &p, int threads, int slots, cudaStream_t stream) {
     static SmemOptIn opted;
     auto kern = viterbi_forward_kernel<CL, G, R>;
-    if (int e = allow_max_smem(kern, opted, 128 * 1024)) return e;
+    if (int e = allow_max_smem(kern, opted, 192 * 1024)) return e;
     const int64_t items = p.n_items;
     const int clusters = (int)(items < slots ? items : slots);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * CL));
     cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)R * 2 * ((size_t(1) << p.L) / 4 / CL) * sizeof(float);
+    cfg.dynamicSmemBytes = (size_t)R * 2 * ((size_t(1) << p.L) / 4 / CL) * (CL == 2 ? 6 : 4);      // with CL == 2, half as much again to send
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -347,6 +397,8 @@ extern "C" int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks,
     p.n = (int32_t)n;
     p.L = L;
     p.rows_per_bank = (int32_t)(rows / banks);
+    p.status = device_status_word();
+    if (!p.status) return RPTC_ERR_CUDA;
     auto rows_at_once = [&](int r) {
         p.items_per_bank = (p.rows_per_bank + r - 1) / r;
         p.n_items = (int32_t)(banks * p.items_per_bank);
