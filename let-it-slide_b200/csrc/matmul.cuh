@@ -1,0 +1,25 @@
+// The fused matrix products as the library's own entry points call them (host side): the checks of arguments are done,
+// and the rows of W may come in banks that each have a lookup table of their own.
+#pragma once
+#include "common.cuh"
+
+namespace rptc {
+
+// W is `banks` groups of `m` rows (m a multiple of 32, TILED codes one bank after the other); bank b decodes through
+// lut + b * lut_stride.
+struct Banks {
+    int32_t banks = 1;
+    int64_t lut_stride = 0;      // fp16 elements
+};
+
+// Columns of y per bank: a bank's rows rounded up to whole tiles.
+int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, int32_t banks, const rptc_format &f);
+// y[t][bank * gemm_bank_columns + row] = fp16(sum_c x[t][c] W[bank][row][c]); columns beyond a bank's m rows hold no
+// result.  Shapes and alignments as rptc_gemm's, with m % 32 == 0 where banks > 1.
+int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
+                int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
+// acc[b][bank * m + row] += sum_c W[bank][row][c] x[b][c] for one to eight activation rows (a power of two of them).
+int gemv_banked(const void *codes, const void *lut, const __half *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int batch,
+                const Banks &banks, const rptc_format &f, cudaStream_t stream);
+
+}  // namespace rptc

@@ -132,3 +132,10 @@ def test_two_sm_kernel_passes_the_identity_cases():
     r = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-x", "-k", "identity or llama_shapes"],
                        env=env, capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("m,n,tokens", [(128, 448, 9), (256, 1024, 128), (384, 2112, 129), (4096, 1088, 100), (256, 4160, 257), (1152, 4032, 640)])
+def test_gemm_tiles_and_splits(code, K, L, S, m, n, tokens):
+    """One and two token halves, tiles past the last row, and a reduction shared by one, two and four CTAs (uneven parts)."""
+    _run(code, K, L, S, m, n, tokens, seed=m + n + tokens)
