@@ -26,11 +26,9 @@
 // makes room for the third activation stage beside two 32 KiB weight stages.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and
 // returns (TMEM is still released).
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include "common.cuh"
 #include "matmul.cuh"
+#include "tc_ptx.cuh"
 
 namespace rptc {
 
@@ -83,50 +81,6 @@ __device__ __forceinline__ GemmBars gemm_bars(uint32_t base) {
 template <int CODE>
 struct GemmDecode {
     static constexpr int kCode = CODE == RPTC_CODE_HASH ? kCodeHashPacked : CODE;
-};
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(bar)
-                 : "memory");
-}
-// Tile of shared memory -> global through the tensor map (clipped at the tensor's bounds), tracked by the thread's bulk group.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y, uint32_t src) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T, kind::f16, cta_group::1
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// K-major operand tile, 128-byte swizzle, 8-row groups 1024 bytes apart; `addr` + 32 bytes per K = 16 step.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
-// fp32 accumulate, fp16 A and B, both K-major, M = 128
-constexpr uint32_t instr_desc(int n_rows) { return (1u << 4) | ((uint32_t)(n_rows >> 3) << 17) | ((uint32_t)(128 >> 4) << 24); }
-
-// Position in a ring of `n` stages without a division per step.
-struct RingPos {
-    int s;
-    uint32_t phase;
-    __device__ __forceinline__ void advance(int n) {
-        if (++s == n) s = 0, phase ^= 1u;
-    }
-    __device__ __forceinline__ void advance_by(int k, int n) {
-        for (int i = 0; i < k; ++i) advance(n);
-    }
 };
 
 // `window` in the functions below: bits to OR onto every planned shared-memory offset (0 outside a cluster; inside one,
@@ -467,13 +421,12 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_tiled_fn() {
     return fn;
 }
 
-// fp16 [rows][cols] with `ld` elements between rows, in swizzled boxes of 64 columns x 128 rows.
-static int encode_map(CUtensorMap &map, const void *base, int64_t cols, int64_t rows, int64_t ld) {
+int encode_map(CUtensorMap &map, const void *base, int64_t cols, int64_t rows, int64_t ld, int box_rows) {
     auto encode = encode_tiled_fn();
     if (!encode) return RPTC_ERR_CUDA;
     const cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64, 128}, estride[2] = {1, 1};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, estride[2] = {1, 1};
     const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dim, stride, box, estride,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -587,12 +540,16 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
     return true;
 }
 
-// Microseconds of one 64-column step of a tile, and of a CTA around its steps (start, table, epilogue; the exchange of
-// partial sums on top where a tile is shared).  Measured; what matters is their ratio.
+// Microseconds of one 64-column step of a tile, and of a CTA around its steps (start, table, epilogue, and where a tile is
+// shared the exchange of partial sums).  Measured on 4096 rows x 4096 and 11008 columns; what matters is their ratio.
 static double step_us(int rows, int halves, int code) {
-    if (code == RPTC_CODE_LUT) return rows == 256 ? 1.05 : 0.62;
-    if (halves == 2) return rows == 256 ? 0.80 : 0.60;
-    return rows == 256 ? 0.55 : 0.40;
+    if (code == RPTC_CODE_LUT) return rows == 256 ? 1.43 : halves == 2 ? 0.92 : 0.77;
+    if (halves == 2) return rows == 256 ? 0.61 : 0.56;
+    return rows == 256 ? 0.58 : 0.44;
+}
+static double around_us(int rows, int halves, int split) {
+    const double tile = rows / 256.0 * halves;               // in wide tiles of one half
+    return 5.0 + 1.5 * tile + (split > 1 ? 1.5 + 1.3 * tile * (split == 4 ? 2.0 : 1.0) : 0.0);
 }
 
 // Clusters of `split` CTAs that fit the device at once (one CTA per SM, and a cluster stays within one group of SMs, so
@@ -641,7 +598,7 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, int32_t bank
             for (int split = 1; split <= rows / 64 && (split == 1 || steps >= 8 * split); split *= 2) {
                 const int64_t places = cluster_places(split);
                 const int64_t waves = (tiles + places - 1) / places;
-                const double us = waves * ((double)((steps + split - 1) / split) * step_us(rows, halves, f.code) + (split > 1 ? 9.0 : 6.0));
+                const double us = waves * ((double)((steps + split - 1) / split) * step_us(rows, halves, f.code) + around_us(rows, halves, split));
                 if (!best.rows || us < best_us) best = {rows, halves, split}, best_us = us;
             }
         }
@@ -661,8 +618,8 @@ int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, co
     if (!g.rows || !plan_gemm(p, g, f)) return RPTC_ERR_UNSUPPORTED;
     p.tiles_per_bank = (int32_t)((m + g.rows - 1) / g.rows);
     CUtensorMap map, ymap;
-    if (int e = encode_map(map, x, n, tokens, ld_x)) return e;
-    if (int e = encode_map(ymap, y, banks.banks == 1 ? m : (int64_t)banks.banks * p.tiles_per_bank * g.rows, tokens, ld_y)) return e;
+    if (int e = encode_map(map, x, n, tokens, ld_x, 128)) return e;
+    if (int e = encode_map(ymap, y, banks.banks == 1 ? m : (int64_t)banks.banks * p.tiles_per_bank * g.rows, tokens, ld_y, 128)) return e;
     p.codes = static_cast<const uint4 *>(codes);
     p.lut = static_cast<const __half *>(lut);
     p.carry_in = carry_in;

@@ -18,6 +18,7 @@
 // Other layouts (and the reference-quirk modes) take a plain 128-bit-load path in the same kernel.
 #include "common.cuh"
 #include "fwht.cuh"
+#include "matmul.cuh"
 
 namespace rptc {
 
@@ -973,6 +974,8 @@ extern "C" int rptc_gemv(const void *codes, const void *lut, const uint32_t *car
                          rptc_stream_t stream) {
     if (int e = validate_gemv_args(codes, lut, x, ld_x, acc, ld_acc, m, n, batch, x_order, fmt)) return e;
     if (int e = rptc_check_device()) return e;
+    if (batch > 2 && x_order == RPTC_XORDER_NATURAL && gemv_few_takes(n, batch, *fmt, x, ld_x))
+        return gemv_few(codes, lut, carry_in, x, ld_x, acc, ld_acc, m, n, batch, Banks(), *fmt, static_cast<cudaStream_t>(stream));
     // batches beyond eight, or not a power of two, run as a short sequence of launches (8 + 8, 4 + 1, ...)
     int done = 0;
     while (done < batch) {

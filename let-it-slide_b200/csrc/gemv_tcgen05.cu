@@ -1,0 +1,374 @@
+// Fused RPTC decode + matrix product for a few activation rows on the sm_100a tensor cores:
+//   acc[t][row] += sum_c x[t][c] * W[row][c]        x: [tokens][n] fp16, tokens up to a few hundred, W decoded on the fly
+//
+// The decoded weights never touch shared memory: they are the A operand of tcgen05.mma and go from the registers they are
+// decoded into straight to tensor memory (tcgen05.st; M = 128 weight rows in the 128 lanes), and the activations are the B
+// operand (N = tokens rounded up to 16, K-major in shared memory, brought in by TMA).  What is left for shared memory are
+// the table lookups, so that the cost of a step is that of its decode whatever the number of tokens -- the fused GEMM,
+// which decodes into shared memory, pays 32 KiB of stores and 48 KiB of operand reads per 256 rows x 64 columns, and the
+// mma.sync kernels repeat the decode for every eight activation rows.
+//
+// A tile is RB x 128 weight rows (RB = 1, 2, 4); a step is 64 columns of it.  The tiles' steps, laid end to end, are cut
+// into equal ranges, one per CTA of a persistent grid; a CTA's range meets a tile in one segment.  Sixteen producer warps
+// form four groups of four (a warp reaches the 32 tensor-memory lanes of its number modulo four): a group owns one of the
+// RB row blocks and one of 4 / RB equal parts of a segment's steps, so that it walks along its rows and keeps the 16 bits
+// of history.  A thread owns a row: its code bits arrive through a private ring of asynchronous copies, four steps ahead.
+// One lane of warp 16 loads the activations and one of warp 17 issues the MMAs, both taking the groups' steps in turn:
+// position j of part 0, 1, ...  A segment's sums are added to the caller's fp32 accumulator with atomics.
+// Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and returns.
+#include "common.cuh"
+#include "matmul.cuh"
+#include "tc_ptx.cuh"
+
+namespace rptc {
+
+constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * 18;
+constexpr int kFewAhead = 4;                         // steps of a thread's code bits in flight
+constexpr uint32_t kFewBars = 0x400, kFewHistory = 0x800, kFewCodes = 0x2800, kFewTop = 0x38800;
+constexpr int kFewMaxXStages = 8;
+constexpr int kFewACols = 32 * 4;                    // tensor-memory columns of the decoded weights: 64 fp16 per group and lane
+constexpr int kFewTmemCols = 512;
+
+struct FewParams {
+    const uint4 *codes;
+    const __half *lut;
+    const uint32_t *carry_in;
+    float *acc;
+    int64_t ld_acc;
+    int64_t m, lut_stride;                           // rows of a bank, fp16 elements from one bank's table to the next
+    int32_t n_steps, n_units;                        // 64-column steps, 128-bit units per row
+    int32_t tokens, n_cols;                          // activation rows, rounded up to 16
+    int32_t tiles, ctas;                             // per bank
+    int32_t L, S;
+    uint32_t lut_addr, x_addr;
+    int32_t n_xstages;
+    unsigned int *status;
+};
+
+// A segment: the steps [s0, s1) of one tile, and the part of them that one group takes.
+struct FewSegment {
+    int32_t tile, s0, s1;
+    uint32_t end;                                    // where the next segment starts in the CTA's range
+    __device__ __forceinline__ FewSegment(uint32_t pos, uint32_t range_end, int32_t n_steps) {
+        tile = (int32_t)(pos / (uint32_t)n_steps);
+        s0 = (int32_t)(pos - (uint32_t)tile * (uint32_t)n_steps);
+        s1 = min(n_steps, s0 + (int32_t)(range_end - pos));
+        end = pos + (uint32_t)(s1 - s0);
+    }
+    template <int PARTS>
+    __device__ __forceinline__ int32_t part_begin(int part) const { return s0 + (s1 - s0) * part / PARTS; }
+};
+
+template <int CODE, int K, int RB>
+__global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
+    constexpr int UPS = K / 2;                       // 128-bit units per step
+    constexpr int PARTS = 4 / RB;
+    constexpr int NW = 4 * UPS;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (smem_addr(smem_raw) > kFewBars) {            // the dynamic area starts later than the plan says
+        if (tid == 0) atomicExch(p.status, kStatusSmemPlan);
+        return;
+    }
+    const uint32_t full_x = kFewBars, empty_x = full_x + 8 * kFewMaxXStages, full_a = empty_x + 8 * kFewMaxXStages, empty_a = full_a + 32,
+                   sums = empty_a + 32, drained = sums + 8, table_bar = drained + 8, tmem_slot = table_bar + 8;
+    const int bank = blockIdx.x / p.ctas;
+    const uint32_t cta = blockIdx.x - bank * p.ctas;
+    // this CTA's range of the bank's steps
+    const uint32_t total = (uint32_t)p.tiles * (uint32_t)p.n_steps;
+    const uint32_t per = total / p.ctas, extra = total - per * p.ctas;
+    const uint32_t c0 = cta * per + min(cta, extra), c1 = c0 + per + (cta < extra ? 1u : 0u);
+
+    if (tid == 0) {
+        for (int i = 0; i < kFewMaxXStages; ++i) mbar_init(full_x + 8 * i, 1), mbar_init(empty_x + 8 * i, 1);
+        for (int g = 0; g < 4; ++g) mbar_init(full_a + 8 * g, 4), mbar_init(empty_a + 8 * g, 1);
+        mbar_init(sums, 1);
+        mbar_init(drained, kFewWarps);
+        mbar_init(table_bar, 1);
+        mbar_fence_init();
+        if (CODE == RPTC_CODE_LUT) {                 // a plain image of the codebook: one bulk copy
+            mbar_expect_tx(table_bar, 2u << p.L);
+            bulk_g2s(p.lut_addr, p.lut + (int64_t)bank * p.lut_stride, 2u << p.L, table_bar);
+        }
+    }
+    if (warp == kFewMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(kFewTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    bool ok = true;
+
+    // ---- a producer's code bits: private ring of copies ----
+    const int group = warp >> 2, block = group % RB, part = group / RB;
+    const int64_t lane_row = block * 128 + (warp & 3) * 32 + lane;       // row inside the tile
+    const uint32_t ring = kFewCodes + (uint32_t)warp * (kFewAhead * UPS * 512) + 16u * lane, hist = kFewHistory + 4u * tid;
+    const uint4 *bank_codes = p.codes + (int64_t)bank * p.m * p.n_units;
+    uint32_t f_next = c0, f_slot = 0;                                     // fetch cursor: next segment, ring slot
+    int32_t f_s = 0, f_b = 0;                                             // steps left of the part at hand
+    bool f_fresh = false, f_valid = false;
+    const uint4 *f_src = nullptr;
+    int64_t f_row = 0;
+    auto fetch = [&]() {
+        while (f_s == f_b && f_next < c1) {                               // the next segment in which this part has steps
+            const FewSegment g(f_next, c1, p.n_steps);
+            f_next = g.end;
+            f_s = g.part_begin<PARTS>(part), f_b = g.part_begin<PARTS>(part + 1);
+            f_fresh = true;
+            f_row = (int64_t)g.tile * (RB * 128) + lane_row;
+            f_valid = f_row < p.m;                                        // of a whole warp: m is a multiple of 32
+            f_src = bank_codes + ((f_row >> 5) * (int64_t)p.n_units + (int64_t)f_s * UPS) * 32 + (f_row & 31);
+        }
+        if (f_s < f_b) {
+            if (f_valid) {
+#pragma unroll
+                for (int q = 0; q < UPS; ++q) cp_async16(ring + (f_slot * UPS + q) * 512u, f_src + q * 32);
+                if (f_fresh) {
+                    const uint32_t dst = hist + 2048u * f_slot;
+                    if (f_s == 0) {
+                        const uint32_t v = p.carry_in ? __ldg(p.carry_in + f_row) : 0u;
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
+                    } else {
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(reinterpret_cast<const uint32_t *>(f_src - 32) + 3) : "memory");
+                    }
+                }
+            }
+            f_fresh = false;
+            f_src += UPS * 32;
+            ++f_s;
+        }
+        cp_async_commit();                            // an empty group when nothing is left keeps the count constant
+        if (++f_slot == kFewAhead) f_slot = 0;
+    };
+    if (warp < kFewWarps) {
+#pragma unroll 1
+        for (int i = 0; i < kFewAhead; ++i) fetch();
+    }
+    if (CODE != RPTC_CODE_LUT) lut_fill<CODE>(p.lut_addr, p.lut + (int64_t)bank * p.lut_stride, p.L, p.S);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_allow_next_grid();
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+    const uint32_t a_cols = tmem + (kFewTmemCols - kFewACols);
+
+    if (warp < kFewWarps) {
+        // ================= decode =================
+        const Lut<CODE> lut = lut_view<CODE>(p.lut_addr, p.L, p.S);
+        if (CODE == RPTC_CODE_LUT) ok = mbar_wait(table_bar, 0, p.status);
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        uint32_t a_phase = 1u, seg_phase = 0u, slot = 0;
+        for (uint32_t pos = c0; pos < c1 && ok;) {
+            const FewSegment g(pos, c1, p.n_steps);
+            pos = g.end;
+            const int64_t row = (int64_t)g.tile * (RB * 128) + lane_row;
+            const bool valid = row < p.m;
+            const int32_t len = g.part_begin<PARTS>(part + 1) - g.part_begin<PARTS>(part);
+            uint32_t prevw = 0;
+#pragma unroll 1
+            for (int32_t i = 0; i < len && ok; ++i) {
+                cp_async_wait<kFewAhead - 1>();      // this step's words have landed
+                uint32_t R[2 * NW], out[32];
+                if (valid) {
+                    if (i == 0) prevw = lds32(hist + 2048u * slot);
+#pragma unroll
+                    for (int q = 0; q < UPS; ++q) {
+                        const uint4 v = lds128(ring + (slot * UPS + q) * 512u);
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            R[8 * q + 2 * k] = __funnelshift_l(w[k], prevw, 16);
+                            R[8 * q + 2 * k + 1] = w[k];
+                            prevw = w[k];
+                        }
+                    }
+                }
+                fetch();
+                if (++slot == kFewAhead) slot = 0;
+                if (valid) {
+#pragma unroll
+                    for (int pi = 0; pi < 32; pi += 4) {
+                        uint32_t four[4];
+                        decode_quad_bits<CODE, K>(R, lut, pi, four);
+                        out[pi] = four[0], out[pi + 1] = four[1], out[pi + 2] = four[2], out[pi + 3] = four[3];
+                    }
+                }
+                ok = mbar_wait(empty_a + 8 * group, a_phase, p.status);      // the MMAs have read the group's last step
+                a_phase ^= 1u;
+                if (ok && valid) {                   // rows past the end: whatever the lanes hold stays in rows nobody reads
+                    tc_fence_after();
+                    tmem_store32(a_cols + 32u * (uint32_t)group + lanes, out);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_a + 8 * group);
+            }
+            // ---- the segment's sums: this thread's row, eight tokens at a time, the parts in turn ----
+            if (ok) ok = mbar_wait(sums, seg_phase, p.status);
+            seg_phase ^= 1u;
+            tc_fence_after();
+            if (ok && valid) {
+                float *dst = p.acc + (int64_t)bank * p.m + row;
+#pragma unroll 1
+                for (int t0 = 8 * part; t0 < p.tokens; t0 += 8 * PARTS) {
+                    uint32_t v[8];
+                    tmem_load8(tmem + lanes + (uint32_t)(block * p.n_cols + t0), v);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (t0 + e < p.tokens) atomicAdd(dst + (int64_t)(t0 + e) * p.ld_acc, __uint_as_float(v[e]));
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(drained);
+        }
+        cp_async_wait<0>();
+    } else if (warp == kFewTmaWarp) {
+        // ================= activations =================
+        pdl_wait_prior_grids();
+        if (lane == 0) {
+            RingPos px = {0, 1u};
+            const uint32_t bytes = 128u * (uint32_t)p.n_cols;
+            for (uint32_t pos = c0; pos < c1 && ok;) {
+                const FewSegment g(pos, c1, p.n_steps);
+                pos = g.end;
+                const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
+                for (int32_t j = 0; j < rounds && ok; ++j)
+                    for (int q = 0; q < PARTS && ok; ++q) {
+                        const int32_t s = g.part_begin<PARTS>(q) + j;
+                        if (s >= g.part_begin<PARTS>(q + 1)) continue;
+                        ok = mbar_wait(empty_x + 8 * px.s, px.phase, p.status);
+                        if (!ok) break;
+                        mbar_expect_tx(full_x + 8 * px.s, bytes);
+                        tma_load_2d(p.x_addr + (uint32_t)px.s * bytes, &x_map, s * 64, 0, full_x + 8 * px.s);
+                        px.advance(p.n_xstages);
+                    }
+            }
+        }
+    } else if (lane == 0) {
+        // ================= MMA issue =================
+        RingPos px = {0, 0u};
+        uint32_t a_phases = 0u, seg = 0;             // bit g: parity of group g's next step
+        const uint32_t bytes = 128u * (uint32_t)p.n_cols, idesc = instr_desc(p.n_cols);
+        for (uint32_t pos = c0; pos < c1 && ok; ++seg) {
+            const FewSegment g(pos, c1, p.n_steps);
+            pos = g.end;
+            if (seg > 0) ok = mbar_wait(drained, (seg - 1) & 1u, p.status);      // the last segment's sums have been taken
+            tc_fence_after();
+            const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
+            uint32_t accumulate = 0u;
+            for (int32_t j = 0; j < rounds && ok; ++j)
+                for (int q = 0; q < PARTS && ok; ++q) {
+                    if (g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
+                    ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status);
+                    const uint32_t xb = p.x_addr + (uint32_t)px.s * bytes;
+#pragma unroll
+                    for (int b = 0; b < RB; ++b) {
+                        const int grp = q * RB + b;
+                        if (ok) ok = mbar_wait(full_a + 8 * grp, (a_phases >> grp) & 1u, p.status);
+                        if (!ok) break;
+                        a_phases ^= 1u << grp;
+                        tc_fence_after();
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tc_mma_f16_ta(tmem + (uint32_t)(b * p.n_cols), a_cols + (uint32_t)(32 * grp + 8 * k), umma_desc_sw128(xb + 32u * k), idesc,
+                                          accumulate | (uint32_t)k);
+                        tc_commit(empty_a + 8 * grp);
+                    }
+                    accumulate = 1u;
+                    tc_commit(empty_x + 8 * px.s);
+                    px.advance(p.n_xstages);
+                }
+            if (ok) tc_commit(sums);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kFewMmaWarp) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kFewTmemCols) : "memory");
+    }
+}
+
+template <int CODE, int K, int RB>
+static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t stream) {
+    static SmemOptIn opted;
+    auto kern = gemv_few_kernel<CODE, K, RB>;
+    if (int e = allow_max_smem(kern, opted)) return e;
+    return launch(kern, dim3(grid), dim3(kFewThreads), kFewTop, stream, p, map);
+}
+
+template <int CODE, int K>
+static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t s) {
+    switch (rb) {
+        case 1: return launch_few<CODE, K, 1>(p, map, grid, s);
+        case 2: return launch_few<CODE, K, 2>(p, map, grid, s);
+    }
+    return launch_few<CODE, K, 4>(p, map, grid, s);
+}
+
+// Row blocks per tile.  More of them read the activations from L2 fewer times, fewer cut the work finer.
+static int few_row_blocks(int n_cols) { return n_cols <= 32 ? 1 : n_cols <= 96 ? 2 : 2; }
+
+// Where the table and the activation ring go; false when two stages do not fit.
+static bool few_plan(FewParams &p, const rptc_format &f) {
+    const uint32_t codes_end = kFewCodes + kFewWarps * kFewAhead * (f.K / 2) * 512;
+    uint32_t free;
+    if (f.code == RPTC_CODE_HASH) {
+        p.lut_addr = kHashLutWindow;
+        free = kHashLutWindow + kHashLutBytes;
+    } else {
+        p.lut_addr = codes_end;
+        free = (codes_end + (f.code == RPTC_CODE_LUT ? (2u << f.L) : (128u << f.S)) + 1023u) & ~1023u;
+    }
+    if (free >= kFewTop) return false;
+    p.x_addr = free;
+    p.n_xstages = (int32_t)((kFewTop - free) / (128u * (uint32_t)p.n_cols));
+    if (p.n_xstages > kFewMaxXStages) p.n_xstages = kFewMaxXStages;
+    return p.n_xstages >= 2;
+}
+
+bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x) {
+    FewParams p;
+    p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
+    return f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE && (f.K == 2 || f.K == 4) && n % 64 == 0 && tokens <= kFewMaxTokens &&
+           few_row_blocks(p.n_cols) * p.n_cols <= kFewTmemCols - kFewACols && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % 8 == 0 &&
+           few_plan(p, f);
+}
+
+int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
+             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s) {
+    FewParams p;
+    p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
+    if (!few_plan(p, f)) return RPTC_ERR_UNSUPPORTED;
+    const int rb = few_row_blocks(p.n_cols);
+    CUtensorMap map;
+    if (int e = encode_map(map, x, n, tokens, ld_x, p.n_cols)) return e;
+    p.codes = static_cast<const uint4 *>(codes);
+    p.lut = static_cast<const __half *>(lut);
+    p.carry_in = carry_in;
+    p.acc = acc;
+    p.ld_acc = ld_acc;
+    p.m = m;
+    p.lut_stride = banks.lut_stride;
+    p.n_steps = (int32_t)(n / 64);
+    p.n_units = (int32_t)(n * f.K / 128);
+    p.tokens = (int32_t)tokens;
+    p.tiles = (int32_t)((m + rb * 128 - 1) / (rb * 128));
+    if ((int64_t)p.tiles * p.n_steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
+    // one bank's table per CTA: the SMs are dealt out to the banks
+    p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
+    if ((int64_t)p.ctas > (int64_t)p.tiles * p.n_steps) p.ctas = p.tiles * p.n_steps;
+    p.L = f.L;
+    p.S = f.S;
+    p.status = device_status_word();
+    if (!p.status) return RPTC_ERR_CUDA;
+    const unsigned grid = (unsigned)(banks.banks * p.ctas);
+    switch (f.code) {
+        case RPTC_CODE_LUT: return f.K == 2 ? launch_few_rb<RPTC_CODE_LUT, 2>(rb, p, map, grid, s) : launch_few_rb<RPTC_CODE_LUT, 4>(rb, p, map, grid, s);
+        case RPTC_CODE_HASH: return launch_few_rb<RPTC_CODE_HASH, 2>(rb, p, map, grid, s);
+        case RPTC_CODE_LITE: return f.K == 2 ? launch_few_rb<RPTC_CODE_LITE, 2>(rb, p, map, grid, s) : launch_few_rb<RPTC_CODE_LITE, 4>(rb, p, map, grid, s);
+    }
+    return RPTC_ERR_UNSUPPORTED;
+}
+
+}  // namespace rptc

@@ -132,3 +132,21 @@ def test_gemv_full_size_linearity(m, n):
     err_s = (ysum.double() - ref_s).abs()
     tol_s = GEMV_HFMA2_TOL * dense.double().norm(dim=1)[None, :] * xs.double().norm() + 2.0**-11 * ref_s.abs() + 1e-4
     assert bool((err_s <= tol_s).all()), f"batch 1 max err/tol {(err_s / tol_s).max().item():.3f}"
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("m,n,batch", [(32, 64, 3), (32, 128, 16), (128, 64 * 149, 17), (160, 320, 33), (1056, 2112, 5), (4096, 1088, 64), (384, 4160, 48)])
+def test_gemv_few_rows_at_tile_and_range_edges(code, K, L, S, m, n, batch):
+    """Rows past a tile's end, ranges that start inside a tile, parts of a segment without a step, one to four groups of 16 tokens."""
+    from rptc_b200 import Format, ops
+    g = torch.Generator(device="cuda").manual_seed(m + n + batch)
+    fmt = Format(code, K, L, S, o.LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, K, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn((batch, n), dtype=torch.float16, device="cuda", generator=g)
+    dense = ops.decompress(codes, lut, m, n, fmt).double()
+    exact = x.double() @ dense.t()
+    y = ops.gemv(codes, lut, x, m, n, fmt)
+    torch.cuda.synchronize()
+    ops.device_status()
+    check_product(y.float().cpu().numpy(), exact.cpu().numpy(), dense.norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(), GEMV_FP32_TOL)
