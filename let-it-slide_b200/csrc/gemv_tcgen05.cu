@@ -1,5 +1,5 @@
 // Fused RPTC decode + matrix product for a few activation rows on the sm_100a tensor cores:
-//   acc[t][row] += sum_c x[t][c] * W[row][c]        x: [tokens][n] fp16, tokens up to a few hundred, W decoded on the fly
+//   acc[t][row] += sum_c x[t][c] * W[row][c]        x: [tokens][n] fp16, up to 96 tokens, W decoded on the fly
 //
 // The decoded weights never touch shared memory: they are the A operand of tcgen05.mma and go from the registers they are
 // decoded into straight to tensor memory (tcgen05.st; M = 128 weight rows in the 128 lanes), and the activations are the B
@@ -13,8 +13,10 @@
 // form four groups of four (a warp reaches the 32 tensor-memory lanes of its number modulo four): a group owns one of the
 // RB row blocks and one of 4 / RB equal parts of a segment's steps, so that it walks along its rows and keeps the 16 bits
 // of history.  A thread owns a row: its code bits arrive through a private ring of asynchronous copies, four steps ahead.
-// One lane of warp 16 loads the activations and one of warp 17 issues the MMAs, both taking the groups' steps in turn:
-// position j of part 0, 1, ...  A segment's sums are added to the caller's fp32 accumulator with atomics.
+// One lane of warp 16 loads the activations, taking the parts' steps in turn: position j of part 0, 1, ...  Each group has
+// an MMA warp and an accumulator of its own: issuing a step (two waits, four MMAs, two commits) takes one thread about
+// 600 clocks, as long as a group takes to decode it, so that one issuer for all four groups held the kernel to a
+// quarter of the speed.  A segment's sums are added to the caller's fp32 accumulator with atomics.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and returns.
 #include "common.cuh"
 #include "matmul.cuh"
@@ -22,7 +24,8 @@
 
 namespace rptc {
 
-constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * 18;
+static_assert(4 * kFewMaxTokens <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
+constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * (kFewMmaWarp + 4);
 constexpr int kFewAhead = 4;                         // steps of a thread's code bits in flight
 constexpr uint32_t kFewBars = 0x400, kFewHistory = 0x800, kFewCodes = 0x2800, kFewTop = 0x38800;
 constexpr int kFewMaxXStages = 8;
@@ -80,9 +83,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
     const uint32_t c0 = cta * per + min(cta, extra), c1 = c0 + per + (cta < extra ? 1u : 0u);
 
     if (tid == 0) {
-        for (int i = 0; i < kFewMaxXStages; ++i) mbar_init(full_x + 8 * i, 1), mbar_init(empty_x + 8 * i, 1);
+        for (int i = 0; i < kFewMaxXStages; ++i) mbar_init(full_x + 8 * i, 1), mbar_init(empty_x + 8 * i, RB);
         for (int g = 0; g < 4; ++g) mbar_init(full_a + 8 * g, 4), mbar_init(empty_a + 8 * g, 1);
-        mbar_init(sums, 1);
+        mbar_init(sums, 4);
         mbar_init(drained, kFewWarps);
         mbar_init(table_bar, 1);
         mbar_fence_init();
@@ -99,44 +102,50 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
 
     // ---- a producer's code bits: private ring of copies ----
     const int group = warp >> 2, block = group % RB, part = group / RB;
-    const int64_t lane_row = block * 128 + (warp & 3) * 32 + lane;       // row inside the tile
+    const int32_t lane_row = block * 128 + (warp & 3) * 32 + lane;       // row inside the tile
     const uint32_t ring = kFewCodes + (uint32_t)warp * (kFewAhead * UPS * 512) + 16u * lane, hist = kFewHistory + 4u * tid;
     const uint4 *bank_codes = p.codes + (int64_t)bank * p.m * p.n_units;
-    uint32_t f_next = c0, f_slot = 0;                                     // fetch cursor: next segment, ring slot
-    int32_t f_s = 0, f_b = 0;                                             // steps left of the part at hand
-    bool f_fresh = false, f_valid = false;
+    // rows past the bank's end decode its last block of 32 rows; their sums are not used
+    auto row_in_bank = [&](int32_t tile) { return min((int64_t)tile * (RB * 128) + lane_row, p.m - 32 + lane); };
+    uint32_t f_next = c0, slot = 0;                                       // fetch cursor: next segment; ring slot (of the fetch and of the decode)
+    int32_t f_left = 0;                                                   // steps left of the part at hand
     const uint4 *f_src = nullptr;
-    int64_t f_row = 0;
-    auto fetch = [&]() {
-        while (f_s == f_b && f_next < c1) {                               // the next segment in which this part has steps
+    auto copy_step = [&]() {
+#pragma unroll
+        for (int q = 0; q < UPS; ++q) cp_async16(ring + (slot * UPS + q) * 512u, f_src + q * 32);
+        f_src += UPS * 32;
+        --f_left;
+    };
+    auto fetch_any = [&]() {                                              // one step into `slot`, if any is left
+        bool fresh = false;
+        int32_t s = 0;
+        int64_t row = 0;
+        while (f_left == 0 && f_next < c1) {                              // the next segment in which this part has steps
             const FewSegment g(f_next, c1, p.n_steps);
             f_next = g.end;
-            f_s = g.part_begin<PARTS>(part), f_b = g.part_begin<PARTS>(part + 1);
-            f_fresh = true;
-            f_row = (int64_t)g.tile * (RB * 128) + lane_row;
-            f_valid = f_row < p.m;                                        // of a whole warp: m is a multiple of 32
-            f_src = bank_codes + ((f_row >> 5) * (int64_t)p.n_units + (int64_t)f_s * UPS) * 32 + (f_row & 31);
+            s = g.part_begin<PARTS>(part);
+            f_left = g.part_begin<PARTS>(part + 1) - s;
+            fresh = true;
+            row = row_in_bank(g.tile);
+            f_src = bank_codes + ((row >> 5) * (int64_t)p.n_units + (int64_t)s * UPS) * 32 + (row & 31);
         }
-        if (f_s < f_b) {
-            if (f_valid) {
-#pragma unroll
-                for (int q = 0; q < UPS; ++q) cp_async16(ring + (f_slot * UPS + q) * 512u, f_src + q * 32);
-                if (f_fresh) {
-                    const uint32_t dst = hist + 2048u * f_slot;
-                    if (f_s == 0) {
-                        const uint32_t v = p.carry_in ? __ldg(p.carry_in + f_row) : 0u;
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
-                    } else {
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(reinterpret_cast<const uint32_t *>(f_src - 32) + 3) : "memory");
-                    }
-                }
+        if (f_left == 0) return;
+        if (fresh) {
+            const uint32_t dst = hist + 2048u * slot;
+            if (s == 0) {
+                const uint32_t v = p.carry_in ? __ldg(p.carry_in + row) : 0u;
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
+            } else {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(reinterpret_cast<const uint32_t *>(f_src - 32) + 3) : "memory");
             }
-            f_fresh = false;
-            f_src += UPS * 32;
-            ++f_s;
         }
-        cp_async_commit();                            // an empty group when nothing is left keeps the count constant
-        if (++f_slot == kFewAhead) f_slot = 0;
+        copy_step();
+    };
+    auto fetch = [&]() {
+        if (f_left > 0) copy_step();
+        else fetch_any();
+        cp_async_commit();                                                // an empty group when nothing is left keeps the count constant
+        slot = (slot + 1) % kFewAhead;
     };
     if (warp < kFewWarps) {
 #pragma unroll 1
@@ -149,6 +158,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
     pdl_allow_next_grid();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+    tmem = __shfl_sync(0xFFFFFFFFu, tmem, 0);                             // the same in all lanes, and known to be
     const uint32_t a_cols = tmem + (kFewTmemCols - kFewACols);
 
     if (warp < kFewWarps) {
@@ -156,48 +166,40 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
         const Lut<CODE> lut = lut_view<CODE>(p.lut_addr, p.L, p.S);
         if (CODE == RPTC_CODE_LUT) ok = mbar_wait(table_bar, 0, p.status);
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-        uint32_t a_phase = 1u, seg_phase = 0u, slot = 0;
+        uint32_t a_phase = 1u, seg_phase = 0u;
         for (uint32_t pos = c0; pos < c1 && ok;) {
             const FewSegment g(pos, c1, p.n_steps);
             pos = g.end;
             const int64_t row = (int64_t)g.tile * (RB * 128) + lane_row;
-            const bool valid = row < p.m;
             const int32_t len = g.part_begin<PARTS>(part + 1) - g.part_begin<PARTS>(part);
             uint32_t prevw = 0;
 #pragma unroll 1
             for (int32_t i = 0; i < len && ok; ++i) {
                 cp_async_wait<kFewAhead - 1>();      // this step's words have landed
                 uint32_t R[2 * NW], out[32];
-                if (valid) {
-                    if (i == 0) prevw = lds32(hist + 2048u * slot);
+                if (i == 0) prevw = lds32(hist + 2048u * slot);
 #pragma unroll
-                    for (int q = 0; q < UPS; ++q) {
-                        const uint4 v = lds128(ring + (slot * UPS + q) * 512u);
-                        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                for (int q = 0; q < UPS; ++q) {
+                    const uint4 v = lds128(ring + (slot * UPS + q) * 512u);
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            R[8 * q + 2 * k] = __funnelshift_l(w[k], prevw, 16);
-                            R[8 * q + 2 * k + 1] = w[k];
-                            prevw = w[k];
-                        }
+                    for (int k = 0; k < 4; ++k) {
+                        R[8 * q + 2 * k] = __funnelshift_l(w[k], prevw, 16);
+                        R[8 * q + 2 * k + 1] = w[k];
+                        prevw = w[k];
                     }
                 }
-                fetch();
-                if (++slot == kFewAhead) slot = 0;
-                if (valid) {
+                fetch();                             // the words are in registers: the slot takes the step kFewAhead further on
 #pragma unroll
-                    for (int pi = 0; pi < 32; pi += 4) {
-                        uint32_t four[4];
-                        decode_quad_bits<CODE, K>(R, lut, pi, four);
-                        out[pi] = four[0], out[pi + 1] = four[1], out[pi + 2] = four[2], out[pi + 3] = four[3];
-                    }
+                for (int pi = 0; pi < 32; pi += 4) {
+                    uint32_t four[4];
+                    decode_quad_bits<CODE, K>(R, lut, pi, four);
+                    out[pi] = four[0], out[pi + 1] = four[1], out[pi + 2] = four[2], out[pi + 3] = four[3];
                 }
                 ok = mbar_wait(empty_a + 8 * group, a_phase, p.status);      // the MMAs have read the group's last step
                 a_phase ^= 1u;
-                if (ok && valid) {                   // rows past the end: whatever the lanes hold stays in rows nobody reads
-                    tc_fence_after();
-                    tmem_store32(a_cols + 32u * (uint32_t)group + lanes, out);
-                }
+                tc_fence_after();
+                tmem_store32(a_cols + 32u * (uint32_t)group + lanes, out);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_a + 8 * group);
@@ -206,15 +208,22 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
             if (ok) ok = mbar_wait(sums, seg_phase, p.status);
             seg_phase ^= 1u;
             tc_fence_after();
-            if (ok && valid) {
+            if (ok && row < p.m) {                   // of a whole warp: m is a multiple of 32
                 float *dst = p.acc + (int64_t)bank * p.m + row;
 #pragma unroll 1
                 for (int t0 = 8 * part; t0 < p.tokens; t0 += 8 * PARTS) {
-                    uint32_t v[8];
-                    tmem_load8(tmem + lanes + (uint32_t)(block * p.n_cols + t0), v);
+                    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+                    for (int a = 0; a < PARTS; ++a) {
+                        if (g.part_begin<PARTS>(a) == g.part_begin<PARTS>(a + 1)) continue;      // no step of this segment
+                        uint32_t v[8];
+                        tmem_load8(tmem + lanes + (uint32_t)((a * RB + block) * p.n_cols + t0), v);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) sum[e] += __uint_as_float(v[e]);
+                    }
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        if (t0 + e < p.tokens) atomicAdd(dst + (int64_t)(t0 + e) * p.ld_acc, __uint_as_float(v[e]));
+                        if (t0 + e < p.tokens) atomicAdd(dst + (int64_t)(t0 + e) * p.ld_acc, sum[e]);
                 }
             }
             tc_fence_before();
@@ -244,11 +253,13 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
                     }
             }
         }
-    } else if (lane == 0) {
-        // ================= MMA issue =================
+    } else {
+        // ================= MMA issue for one group: the whole warp waits, one lane issues =================
+        const int grp = __shfl_sync(0xFFFFFFFFu, warp, 0) - kFewMmaWarp, mine = grp / RB;
         RingPos px = {0, 0u};
-        uint32_t a_phases = 0u, seg = 0;             // bit g: parity of group g's next step
+        uint32_t a_phase = 0u, seg = 0;
         const uint32_t bytes = 128u * (uint32_t)p.n_cols, idesc = instr_desc(p.n_cols);
+        const uint32_t d_tmem = tmem + (uint32_t)(grp * p.n_cols), a_tmem = a_cols + 32u * (uint32_t)grp;
         for (uint32_t pos = c0; pos < c1 && ok; ++seg) {
             const FewSegment g(pos, c1, p.n_steps);
             pos = g.end;
@@ -257,28 +268,35 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
             const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
             uint32_t accumulate = 0u;
             for (int32_t j = 0; j < rounds && ok; ++j)
-                for (int q = 0; q < PARTS && ok; ++q) {
+#pragma unroll
+                for (int q = 0; q < PARTS; ++q) {
                     if (g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
-                    ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status);
-                    const uint32_t xb = p.x_addr + (uint32_t)px.s * bytes;
+                    if (q == mine && ok) {
+                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * grp, a_phase, p.status);
+                        a_phase ^= 1u;
+                        if (ok) {
+                            tc_fence_after();
+                            const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)px.s * bytes);
+                            if (elect_one()) {
 #pragma unroll
-                    for (int b = 0; b < RB; ++b) {
-                        const int grp = q * RB + b;
-                        if (ok) ok = mbar_wait(full_a + 8 * grp, (a_phases >> grp) & 1u, p.status);
-                        if (!ok) break;
-                        a_phases ^= 1u << grp;
-                        tc_fence_after();
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc_mma_f16_ta(tmem + (uint32_t)(b * p.n_cols), a_cols + (uint32_t)(32 * grp + 8 * k), umma_desc_sw128(xb + 32u * k), idesc,
-                                          accumulate | (uint32_t)k);
-                        tc_commit(empty_a + 8 * grp);
+                                for (int k = 0; k < 4; ++k)      // + 32 bytes of shared memory, + 8 columns of tensor memory
+                                    tc_mma_f16_ta(d_tmem, a_tmem + 8u * k, xb + 2u * k, idesc, accumulate | (uint32_t)k);
+                                tc_commit(empty_a + 8 * grp);
+                                tc_commit(empty_x + 8 * px.s);
+                            }
+                            __syncwarp();
+                            accumulate = 1u;
+                        }
                     }
-                    accumulate = 1u;
-                    tc_commit(empty_x + 8 * px.s);
                     px.advance(p.n_xstages);
                 }
-            if (ok) tc_commit(sums);
+            if (ok) {
+                if (elect_one()) {
+                    if (accumulate) tc_commit(sums);
+                    else mbar_arrive(sums);          // no step of this segment
+                }
+                __syncwarp();
+            }
         }
     }
     tc_fence_before();
@@ -307,7 +325,7 @@ static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, uns
 }
 
 // Row blocks per tile.  More of them read the activations from L2 fewer times, fewer cut the work finer.
-static int few_row_blocks(int n_cols) { return n_cols <= 32 ? 1 : n_cols <= 96 ? 2 : 2; }
+static int few_row_blocks(int n_cols) { return n_cols <= 32 ? 1 : 2; }
 
 // Where the table and the activation ring go; false when two stages do not fit.
 static bool few_plan(FewParams &p, const rptc_format &f) {
@@ -331,7 +349,7 @@ bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void 
     FewParams p;
     p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
     return f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE && (f.K == 2 || f.K == 4) && n % 64 == 0 && tokens <= kFewMaxTokens &&
-           few_row_blocks(p.n_cols) * p.n_cols <= kFewTmemCols - kFewACols && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % 8 == 0 &&
+           (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % 8 == 0 &&
            few_plan(p, f);
 }
 

@@ -19,7 +19,7 @@ int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, int32_t banks, c
 int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
                 int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
 // acc[b][bank * m + row] += sum_c W[bank][row][c] x[b][c], up to kFewMaxTokens activation rows, where gemv_few_takes says so.
-constexpr int64_t kFewMaxTokens = 192;
+constexpr int64_t kFewMaxTokens = 96;
 bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x);
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);

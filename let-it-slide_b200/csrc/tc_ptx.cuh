@@ -71,6 +71,13 @@ __device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // Position in a ring of `n` stages without a division per step.
 struct RingPos {
     int s;
