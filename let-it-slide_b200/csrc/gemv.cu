@@ -1,21 +1,18 @@
-// Fused RPTC decode + matvec for decode batches 1..8 on sm_100a.
+// Fused RPTC decode + matvec for one or two activation rows on sm_100a (more of them: gemv_tcgen05.cu).
 //
 // Work decomposition.  Rows are taken 32 at a time (a "row block": lane l owns row 32*rb + l) and a
 // row's stream is cut into 128-bit units.  The (row block, unit) grid is flattened row-block-major
-// and cut into equal contiguous ranges, one per warp of a persistent grid of one 512-thread CTA per
-// SM, so that every SM gets the same number of units whatever m and n are.  In the native TILED
+// and cut into equal contiguous ranges over a persistent grid of one 512-thread CTA per SM, so that
+// every SM gets the same number of units whatever m and n are.  In the native TILED
 // layout that flattened order is the memory order: a warp's range is one linear stream of 512-byte
-// units.  Lane 0 of each warp streams it into a private shared-memory ring with 1-D bulk (TMA)
-// copies of two units each, completing on mbarriers, several units ahead; every lane then takes its
-// own 128 bits with one conflict-free LDS.128.  The 16-bit shift-register windows are rebuilt in
-// registers with funnel shifts, hashed / looked up in a bank-replicated shared-memory table, and
-// multiplied into half2 accumulators that are flushed to fp32 every unit.  A warp walks along its
-// rows, so the 16 bits of history a unit needs are simply the last word of the unit before it (one
-// extra 32-bit load at the start of a run).  Partial row sums are added to the fp32 accumulator in
-// global memory with atomics.
+// units.  The 16-bit shift-register windows are rebuilt in registers with funnel shifts and hashed /
+// looked up in a shared-memory table.  A warp walks along its rows, so the 16 bits of history a unit
+// needs are simply the last word of the unit before it (one extra 32-bit load at the start of a run).
+// Partial row sums are added to the fp32 accumulator in global memory with atomics.  W may come in
+// banks of rows with a table each: the CTAs are then dealt out to the banks.
 //
-// Activations are staged once per CTA in shared memory and read back as warp-broadcast LDS.128.
-// Other layouts (and the reference-quirk modes) take a plain 128-bit-load path in the same kernel.
+// Activations are staged once per CTA in shared memory.  Other layouts (and the reference-quirk modes)
+// take a plain 128-bit-load path in a kernel of their own.
 #include "common.cuh"
 #include "fwht.cuh"
 #include "matmul.cuh"
@@ -31,12 +28,11 @@ namespace rptc {
 constexpr int kGemvThreads = RPTC_GEMV_THREADS;
 constexpr int kGemvWarps = kGemvThreads / 32;
 constexpr int kStages = RPTC_GEMV_STAGES;        // ring depth per warp
-constexpr int kStageUnits = 2;                   // units per bulk copy
+constexpr int kStageUnits = 2;                   // units per stage: one of each row block of a granule
 constexpr uint32_t kUnitBytes = 512;             // 32 rows x 128 bits
 constexpr uint32_t kStageBytes = kStageUnits * kUnitBytes;
-constexpr uint32_t kBarBytes = 1024;             // kGemvWarps * kStages * 8 <= 1024
+constexpr uint32_t kBarBytes = 1024;             // the barrier of the table's bulk copy; the ring starts behind it
 constexpr uint32_t kRingBytes = kGemvWarps * kStages * kStageBytes;
-static_assert(kGemvWarps * kStages * 8 <= kBarBytes, "barrier area too small");
 static_assert(kBarBytes + kRingBytes + 1024 <= kHashLutWindow, "ring must fit below the HASH table window");
 
 struct GemvParams {
@@ -58,6 +54,9 @@ struct GemvParams {
     SwigluParams sw;
     float *clear;
     int64_t clear_count;
+    // gemv_rows_kernel, MODE 0: CTAs per bank of rows, fp16 elements from one bank's table to the next
+    int32_t ctas;
+    int64_t lut_stride;
 };
 
 // Source pair of stream pair s under the fused reference kernel's x staging (inference.cu:216-221,249).
@@ -245,8 +244,26 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
         if (threadIdx.x == 0) atomicExch(p.status, kStatusSmemPlan);
         return;
     }
+    // the bank this CTA works on, and its number among the bank's CTAs
+    const uint32_t bank = MODE == 0 ? blockIdx.x / (uint32_t)p.ctas : 0u, n_ctas = MODE == 0 ? (uint32_t)p.ctas : gridDim.x;
+    const uint32_t cta = blockIdx.x - bank * n_ctas;
+    const __half *table = p.lut + (MODE == 0 ? (int64_t)bank * p.lut_stride : 0);
+    const uint4 *codes = p.codes + (MODE == 0 ? (int64_t)bank * p.m * p.n_units : 0);
+    float *acc = p.acc + (MODE == 0 ? (int64_t)bank * p.m : 0);
     // ---- prologue: nothing here depends on the kernels before this one ----
-    const LutPending lut_pending = lut_fill_begin<CODE>(lut_tab, p.lut, p.L, p.S);
+    // The table code's codebook (128 KiB at L = 16) is a plain image: one bulk copy, awaited in front of the main loop.
+    LutPending lut_pending;
+    if (CODE == RPTC_CODE_LUT) {
+        if (threadIdx.x == 0) {
+            mbar_init(s0, 1);
+            mbar_fence_init();
+            mbar_expect_tx(s0, 2u << p.L);
+            bulk_g2s(lut_tab, table, 2u << p.L, s0);
+        }
+        lut_pending.deferred = false;
+    } else {
+        lut_pending = lut_fill_begin<CODE>(lut_tab, table, p.L, p.S);
+    }
     const Lut<CODE> lut = lut_view<CODE>(lut_tab, p.L, p.S);
     pdl_allow_next_grid();
 
@@ -265,9 +282,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
         // inside the CTA (again by at most one).  The warps that carry one granule more are thereby spread over all SMs
         // -- and over the four schedulers of each -- instead of filling the first CTAs of the grid.
         const uint32_t T = n_rbp * (uint32_t)nu;
-        const uint32_t cta_per = T / gridDim.x, cta_extra = T - cta_per * gridDim.x;
-        const uint32_t cta_g0 = blockIdx.x * cta_per + min((uint32_t)blockIdx.x, cta_extra);
-        const uint32_t cta_n = cta_per + (blockIdx.x < cta_extra ? 1u : 0u);
+        const uint32_t cta_per = T / n_ctas, cta_extra = T - cta_per * n_ctas;
+        const uint32_t cta_g0 = cta * cta_per + min(cta, cta_extra);
+        const uint32_t cta_n = cta_per + (cta < cta_extra ? 1u : 0u);
         const uint32_t w_per = cta_n / kGemvWarps, w_extra = cta_n - w_per * kGemvWarps;
         const uint32_t g0 = cta_g0 + (uint32_t)warp * w_per + min((uint32_t)warp, w_extra);
         const uint32_t count = w_per + ((uint32_t)warp < w_extra ? 1u : 0u);
@@ -290,7 +307,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
                 c.rbp = gi / (uint32_t)nu;
                 c.u = (int32_t)(gi - c.rbp * (uint32_t)nu);
             }
-            c.ptr = p.codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)(useg0 + c.u) << 5) + lane;
+            c.ptr = codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)(useg0 + c.u) << 5) + lane;
             return c;
         };
         auto advance = [&](Cursor &c) {      // to the next granule in this kernel's order
@@ -303,12 +320,12 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
                         c.rbp = 0;
                         c.u += (int32_t)UPB;
                     }
-                    c.ptr = p.codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)c.u << 5) + lane;
+                    c.ptr = codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)c.u << 5) + lane;
                 }
             } else if (c.u == nu) {
                 c.u = 0;
                 ++c.rbp;
-                c.ptr = p.codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)useg0 << 5) + lane;
+                c.ptr = codes + (int64_t)(2 * c.rbp) * rb_stride + ((int64_t)useg0 << 5) + lane;
             }
         };
         Cursor fc = cursor_at(count ? g0 : 0u);      // fetch cursor
@@ -370,7 +387,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
                 n.u = 0;
                 ++n.rbp;
             }
-            n.ptr = p.codes + (int64_t)(2 * n.rbp) * rb_stride + ((int64_t)(useg0 + n.u) << 5) + lane;
+            n.ptr = codes + (int64_t)(2 * n.rbp) * rb_stride + ((int64_t)(useg0 + n.u) << 5) + lane;
             return n;
         };
         uint32_t prev_a = 0u, prev_b = 0u, next_prev_a = 0u, next_prev_b = 0u;
@@ -471,6 +488,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
         }
         late_prologue();      // threads that loaded nothing, other paths
         __syncthreads();
+        if (CODE == RPTC_CODE_LUT && useg0 == 0 && !mbar_wait(s0, 0, p.status)) {
+            cp_async_wait<0>();
+            break;
+        }
 
         // ---- main loop: one granule per step ----
         const uint32_t x_base = xs + (uint32_t)(g >> 2) * x_batch_stride;
@@ -479,7 +500,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
             if (out_batch < BATCH) {
                 const int64_t row_a = ((int64_t)rbp << 6) + out_row;
                 const bool has_b = 2 * rbp + 1 < n_rb;
-                float *dst = p.acc + (int64_t)out_batch * p.ld_acc + row_a;
+                float *dst = acc + (int64_t)out_batch * p.ld_acc + row_a;
                 atomicAdd(dst, c0[0] + c1[0]);
                 atomicAdd(dst + 1, c0[1] + c1[1]);
                 if (has_b) {
@@ -543,283 +564,6 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
     if (!waited_prior) pdl_wait_prior_grids();
 }
 
-// ---- batch 4 and 8: word per lane, up to eight activation rows as the B operand -----------------------------------
-// Same granules and work split as gemv_rows_kernel, with the codes brought in by bulk copies into a per-warp ring.  The
-// products run on mma.sync m16n8k16 (fp16 in, fp32 accumulate) with the decoded weights as the A operand:
-//  * lane (g = lane/4, t = lane%4) decodes WORD t of rows g, g+8, g+16, g+24 of the 32-row tile (the tile is
-//    read as four conflict-free 32-bit loads instead of one 128-bit load per row); the 16 stream bits before a
-//    word come from lane t-1 (same unit) or, for t == 0, from lane t+3's word of the unit before -- one shuffle;
-//  * a word holds PW = 16/K weight pairs.  MMA i of a word takes pairs 2i, 2i+1 of rows g / g+8 as a0..a3, so
-//    the k index of a product is (t, pair, element) -- a permutation of the unit's columns that the B operand
-//    follows by reading the activations of columns [t*2*PW, (t+1)*2*PW) of the unit for lane t, batch row g;
-//  * the accumulator fragment of a lane is rows g, g+8 x batch columns 2t, 2t+1: after a run, lanes with
-//    2t < BATCH add their sums to the caller's accumulator.
-// Per 64 weights a lane issues 4 word loads, 12 window instructions, 4 per pair for the lookup, 8 MMAs and 2
-// activation loads; there is no fp16 partial sum, and BATCH up to 8 costs only the shared memory for x.
-template <int CODE, int K, int BATCH>
-__global__ void __launch_bounds__(kGemvThreads, 1) gemv_mma_kernel(const GemvParams p) {
-    constexpr int WPU = 128 / K;
-    constexpr int PAIRS = WPU / 2;
-    constexpr int PW = 16 / K;                 // weight pairs in a 32-bit word
-    constexpr uint32_t kXPad = 16;             // bytes between activation rows beyond their length: spreads rows over banks
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t4 = lane & 3;
-    const uint32_t s0 = smem_addr(smem_raw);
-    const uint32_t bars = s0 + (uint32_t)warp * kStages * 8u;
-    const uint32_t ring = s0 + kBarBytes + (uint32_t)warp * kStages * kStageBytes;
-    uint32_t lut_tab, xs;
-    if (CODE == RPTC_CODE_HASH) {
-        lut_tab = kHashLutWindow;
-        xs = kHashLutWindow + kHashLutBytes;
-    } else {
-        lut_tab = s0 + kBarBytes + kRingBytes;
-        xs = lut_tab + lut_bytes<CODE>(p.L, p.S);
-    }
-    if (CODE == RPTC_CODE_HASH && s0 + kBarBytes + kRingBytes > kHashLutWindow) {
-        if (threadIdx.x == 0) atomicExch(p.status, kStatusSmemPlan);
-        return;
-    }
-    // ---- prologue: nothing here depends on the kernels before this one ----
-    const LutPending lut_pending = lut_fill_begin<CODE>(lut_tab, p.lut, p.L, p.S);
-    if (lane == 0) {
-#pragma unroll
-        for (int s = 0; s < kStages; ++s) mbar_init(bars + 8u * s, 1);
-        mbar_fence_init();
-    }
-    __syncwarp();
-    const Lut<CODE> lut = lut_view<CODE>(lut_tab, p.L, p.S);
-    pdl_allow_next_grid();
-
-    const uint32_t n_rb = (uint32_t)(p.m >> 5), n_rbp = (n_rb + 1) >> 1;
-    const uint32_t x_batch_stride = (uint32_t)p.seg_units * WPU * 2u + kXPad;
-    const int64_t rb_stride = (int64_t)p.n_units << 5;        // 128-bit units between row blocks of the TILED layout
-    const int halo_src = (lane & ~3) | ((t4 + 3) & 3);
-    uint32_t slot = 0, phase = 0;
-    bool ok = true, waited_prior = false;
-
-    for (int32_t useg0 = 0; useg0 < p.n_units; useg0 += p.seg_units) {
-        const int32_t nu = min(p.seg_units, p.n_units - useg0);
-        // two-level even split: contiguous ranges per CTA, then per warp (see gemv_rows_kernel)
-        const uint32_t T = n_rbp * (uint32_t)nu;
-        const uint32_t cta_per = T / gridDim.x, cta_extra = T - cta_per * gridDim.x;
-        const uint32_t cta_g0 = blockIdx.x * cta_per + min((uint32_t)blockIdx.x, cta_extra);
-        const uint32_t cta_n = cta_per + (blockIdx.x < cta_extra ? 1u : 0u);
-        const uint32_t w_per = cta_n / kGemvWarps, w_extra = cta_n - w_per * kGemvWarps;
-        const uint32_t g0 = cta_g0 + (uint32_t)warp * w_per + min((uint32_t)warp, w_extra);
-        const uint32_t count = w_per + ((uint32_t)warp < w_extra ? 1u : 0u);
-        const uint32_t rbp0 = count ? g0 / (uint32_t)nu : 0u;
-        const int32_t u0 = count ? (int32_t)(g0 - rbp0 * (uint32_t)nu) : 0;
-
-        // fetch cursor (lane 0)
-        uint32_t frbp = rbp0;
-        int32_t fu = u0;
-        const uint4 *fptr = p.codes + (int64_t)(2 * rbp0) * rb_stride + ((int64_t)(useg0 + u0) << 5);
-        auto issue_stage = [&](uint32_t at_slot) {
-            const bool has_b = 2 * frbp + 1 < n_rb;
-            const uint32_t bar = bars + 8u * at_slot, dst = ring + at_slot * kStageBytes;
-            mbar_expect_tx(bar, has_b ? 2 * kUnitBytes : kUnitBytes);
-            bulk_g2s(dst, fptr, kUnitBytes, bar);
-            if (has_b) bulk_g2s(dst + kUnitBytes, fptr + rb_stride, kUnitBytes, bar);
-            fptr += 32;
-            if (++fu == nu) {
-                fu = 0;
-                ++frbp;
-                fptr = p.codes + (int64_t)(2 * frbp) * rb_stride + ((int64_t)useg0 << 5);
-            }
-        };
-        uint32_t to_issue = count;
-        {
-            const uint32_t ahead = min(count, (uint32_t)kStages);
-            if (lane == 0) {
-                uint32_t sl = slot;
-                for (uint32_t k = 0; k < ahead; ++k) {
-                    issue_stage(sl);
-                    if (++sl == kStages) sl = 0;
-                }
-            }
-            to_issue -= ahead;
-        }
-
-        // Word 3 of the unit in front of a run, rows g + 8j of both blocks: part of the weights, so the first run's are
-        // fetched here, before anything that depends on the grid in front.
-        auto load_history = [&](uint32_t rbpx, int32_t ug, uint32_t (&pa)[4], uint32_t (&pb)[4]) {
-            const int64_t row0 = (int64_t)rbpx << 6;
-            const bool has_b = 2 * rbpx + 1 < n_rb;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t r = row0 + g + 8 * j;
-                if (ug == 0) {
-                    pa[j] = p.carry_in ? __ldg(p.carry_in + r) : 0u;
-                    pb[j] = (p.carry_in && has_b) ? __ldg(p.carry_in + r + 32) : 0u;
-                } else {
-                    const uint32_t *last = reinterpret_cast<const uint32_t *>(p.codes + (int64_t)(2 * rbpx) * rb_stride +
-                                                                               ((int64_t)(ug - 1) << 5) + (g + 8 * j)) + 3;
-                    pa[j] = __ldg(last);
-                    pb[j] = has_b ? __ldg(last + 4 * rb_stride) : 0u;
-                }
-            }
-        };
-        uint32_t first_pa[4] = {0u, 0u, 0u, 0u}, first_pb[4] = {0u, 0u, 0u, 0u};
-        if (count) load_history(rbp0, useg0 + u0, first_pa, first_pb);
-
-        // ---- activations of this column segment -> shared memory ----
-        if (!waited_prior) {
-            pdl_wait_prior_grids();
-            waited_prior = true;
-            // the codebook loads were issued before the wait
-            lut_fill_end<CODE>(lut_tab, lut_pending, p.S);
-        }
-        if (useg0 > 0) __syncthreads();
-        {
-        const int64_t col0 = (int64_t)useg0 * WPU;
-        const int pairs = nu * PAIRS;
-        if (p.x_order == RPTC_XORDER_NATURAL && ((p.ld_x | col0) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0) {
-            const int vecs = pairs >> 2;
-#pragma unroll 1
-            for (int b = 0; b < BATCH; ++b) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (int64_t)b * p.ld_x + col0);
-                const uint32_t dst = xs + (uint32_t)b * x_batch_stride;
-                for (int i0 = threadIdx.x; i0 < vecs; i0 += 4 * kGemvThreads) {
-                    uint4 v[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (i0 + k * kGemvThreads < vecs) v[k] = ld_ordered_u128(src + i0 + k * kGemvThreads);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (i0 + k * kGemvThreads < vecs)
-                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * (i0 + k * kGemvThreads)),
-                                         "r"(v[k].x), "r"(v[k].y), "r"(v[k].z), "r"(v[k].w)
-                                         : "memory");
-                }
-            }
-        } else {
-            for (int i = threadIdx.x; i < BATCH * pairs; i += kGemvThreads) {
-                const int b = i / pairs, s = i - b * pairs;
-                int64_t src = (col0 >> 1) + s;
-                if (p.x_order == RPTC_XORDER_K2_LEGACY) src = k2_legacy_pair(src, p.n);
-                const uint32_t v = ld_ordered_u32(reinterpret_cast<const uint32_t *>(p.x + (int64_t)b * p.ld_x) + src);
-                asm volatile("st.shared.u32 [%0], %1;" ::"r"(xs + (uint32_t)b * x_batch_stride + 4u * s), "r"(v) : "memory");
-            }
-        }
-        }
-        __syncthreads();
-
-        // ---- main loop: runs of consecutive units inside one pair of row blocks ----
-        // this lane's activations: batch row g (any valid row when g >= BATCH: those columns of D are not used)
-        const uint32_t x_lane = xs + (uint32_t)(g < BATCH ? g : 0) * x_batch_stride + (uint32_t)t4 * (PW * 4u);
-        uint32_t rbp = rbp0;
-        int32_t u = u0;
-        uint32_t k = 0;
-        while (k < count && ok) {
-            const uint32_t run = min(count - k, (uint32_t)(nu - u));
-            const int64_t row0 = (int64_t)rbp << 6;               // first row of block a; block b starts 32 later
-            const bool has_b = 2 * rbp + 1 < n_rb;
-            // word 3 of the unit before the run, rows g + 8j of both blocks (lanes t == 3 hand it to lanes t == 0)
-            uint32_t pa[4], pb[4];
-            if (k == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) pa[j] = first_pa[j], pb[j] = first_pb[j];
-            } else {
-                load_history(rbp, useg0 + u, pa, pb);
-            }
-            float ca[2][4], cb[2][4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) ca[h][i] = cb[h][i] = 0.f;
-            uint32_t xu = x_lane + (uint32_t)u * (WPU * 2u);
-#pragma unroll 1
-            for (uint32_t jj = 0; jj < run; ++jj) {
-                ok = mbar_wait(bars + 8u * slot, phase, p.status);
-                if (!ok) break;
-                const uint32_t stage_base = ring + slot * kStageBytes + 4u * lane;
-                uint32_t xr[PW];
-                if (PW == 8) {
-                    const uint4 x0 = lds128(xu), x1 = lds128(xu + 16u);
-                    xr[0] = x0.x, xr[1] = x0.y, xr[2] = x0.z, xr[3] = x0.w;
-                    xr[PW - 4] = x1.x, xr[PW - 3] = x1.y, xr[PW - 2] = x1.z, xr[PW - 1] = x1.w;
-                } else {
-                    const uint4 x0 = lds128(xu);
-                    xr[0] = x0.x, xr[1] = x0.y, xr[2] = x0.z, xr[3] = x0.w;
-                }
-#pragma unroll
-                for (int blk = 0; blk < 2; ++blk) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        w[j] = lds32(stage_base + (uint32_t)blk * kUnitBytes + 128u * j);      // block b absent: stale bytes, sums dropped
-                    uint32_t R[4][2];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint32_t &prev = blk == 0 ? pa[j] : pb[j];
-                        const uint32_t give = t4 == 3 ? prev : w[j];
-                        const uint32_t before = __shfl_sync(0xFFFFFFFFu, give, halo_src);
-                        prev = w[j];
-                        R[j][0] = __funnelshift_l(w[j], before, 16);
-                        R[j][1] = w[j];
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                        for (int i = 0; i < PW / 2; ++i) {
-                            const uint32_t a0 = (decode_pair_bits<CODE, K>(R[2 * h], lut, 2 * i));
-                            const uint32_t a1 = (decode_pair_bits<CODE, K>(R[2 * h + 1], lut, 2 * i));
-                            const uint32_t a2 = (decode_pair_bits<CODE, K>(R[2 * h], lut, 2 * i + 1));
-                            const uint32_t a3 = (decode_pair_bits<CODE, K>(R[2 * h + 1], lut, 2 * i + 1));
-                            mma_16816(blk == 0 ? ca[h] : cb[h], a0, a1, a2, a3, xr[2 * i], xr[2 * i + 1]);
-                        }
-                    }
-                }
-                xu += WPU * 2u;
-                __syncwarp();                     // every lane has taken its words: the slot can be refilled
-                if (to_issue) {
-                    if (lane == 0) issue_stage(slot);
-                    --to_issue;
-                }
-                if (++slot == kStages) {
-                    slot = 0;
-                    phase ^= 1u;
-                }
-            }
-            // c[h][0..1]: row g + 16h, batch columns 2t, 2t+1;  c[h][2..3]: row g + 16h + 8
-            if (2 * t4 < BATCH) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int col = 2 * t4 + (e & 1);
-                        if (col < BATCH) {
-                            const int64_t r = row0 + g + 16 * h + 8 * (e >> 1);
-                            atomicAdd(p.acc + (int64_t)col * p.ld_acc + r, ca[h][e]);
-                            if (has_b) atomicAdd(p.acc + (int64_t)col * p.ld_acc + r + 32, cb[h][e]);
-                        }
-                    }
-                }
-            }
-            k += run;
-            u += (int32_t)run;
-            if (u == nu) {
-                u = 0;
-                ++rbp;
-            }
-        }
-        if (!ok) {
-            // After a failed wait: give the copies still in flight a bounded chance to land before
-            // the shared memory they target is released, then stop.
-            for (int s = 0; s < kStages; ++s) {
-                mbar_wait(bars + 8u * slot, phase, p.status);
-                if (++slot == kStages) {
-                    slot = 0;
-                    phase ^= 1u;
-                }
-            }
-            break;
-        }
-    }
-    if (!waited_prior) pdl_wait_prior_grids();
-}
-
 __global__ void gemv_finish_kernel(float *__restrict__ acc, int64_t ld_acc, __half *__restrict__ y, int64_t ld_y,
                                    int64_t m, int batch, float scale, int accumulate, int clear) {
     pdl_allow_next_grid();
@@ -845,42 +589,32 @@ static int launch_gemv(const GemvParams &p, size_t smem, cudaStream_t stream) {
     return launch(kern, dim3(num_sms()), dim3(kGemvThreads), smem, stream, p);
 }
 
-template <int CODE, int K, int BATCH>
-static int launch_gemv_mma(const GemvParams &p, size_t smem, cudaStream_t stream) {
-    static SmemOptIn opted;
-    auto kern = gemv_mma_kernel<CODE, K, BATCH>;
-    if (int e = allow_max_smem(kern, opted)) return e;
-    return launch(kern, dim3(num_sms()), dim3(kGemvThreads), smem, stream, p);
-}
-
 template <int CODE, int K, int BATCH, int MODE>
-static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t stream) {
+static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t stream, int grid = num_sms()) {
     static SmemOptIn opted;
     auto kern = gemv_rows_kernel<CODE, K, BATCH, MODE>;
     if (int e = allow_max_smem(kern, opted)) return e;
-    return launch(kern, dim3(num_sms()), dim3(kGemvThreads), smem, stream, p);
+    return launch(kern, dim3(grid), dim3(kGemvThreads), smem, stream, p);
 }
 
 template <int CODE, int K>
-static int dispatch(const GemvParams &p, int batch, bool tiled, size_t smem, cudaStream_t stream) {
+static int dispatch(const GemvParams &p, int batch, bool tiled, size_t smem, int grid, cudaStream_t stream) {
     if (!tiled) return batch == 1 && !p.in.h_in ? launch_gemv<CODE, K>(p, smem, stream) : RPTC_ERR_UNSUPPORTED;
     if (p.in.h_in) {
         if (batch > 2) return RPTC_ERR_UNSUPPORTED;
         return batch == 1 ? launch_gemv_rows<CODE, K, 1, 1>(p, smem, stream) : launch_gemv_rows<CODE, K, 2, 1>(p, smem, stream);
     }
     switch (batch) {
-        case 1: return launch_gemv_rows<CODE, K, 1, 0>(p, smem, stream);
-        case 2: return launch_gemv_rows<CODE, K, 2, 0>(p, smem, stream);
-        case 4: return launch_gemv_mma<CODE, K, 4>(p, smem, stream);
-        case 8: return launch_gemv_mma<CODE, K, 8>(p, smem, stream);
+        case 1: return launch_gemv_rows<CODE, K, 1, 0>(p, smem, stream, grid);
+        case 2: return launch_gemv_rows<CODE, K, 2, 0>(p, smem, stream, grid);
     }
     return RPTC_ERR_ARG;
 }
 
-// One launch for batch in {1,2,4,8}.
+// One launch for batch in {1,2}.
 static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in, const __half *x, int64_t ld_x, float *acc,
                     int64_t ld_acc, int64_t m, int64_t n, int batch, int x_order, const rptc_format &f, cudaStream_t stream,
-                    const rptc_gemv_input *in = nullptr) {
+                    const rptc_gemv_input *in = nullptr, const Banks &banks = Banks()) {
     const int K = f.K;
     const int wpu = 128 / K;
     GemvParams p;
@@ -903,6 +637,10 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
     if (!p.status) return RPTC_ERR_CUDA;
     const bool tma = f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE;
     p.in = in ? *in : rptc_gemv_input{};
+    // one bank's table per CTA: the SMs are dealt out to the banks
+    p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
+    p.lut_stride = banks.lut_stride;
+    const int grid = banks.banks * p.ctas;
 
     // shared-memory plan (must mirror the kernel's)
     const size_t kMaxSmem = 227 * 1024 - 1024;     // leave room for the 1 KiB the system may reserve
@@ -918,7 +656,7 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
     if (seg < 1) return RPTC_ERR_TOO_LARGE;
     if (seg > p.n_units) seg = p.n_units;
     p.seg_units = (int32_t)seg;
-    size_t smem = fixed + size_t(seg) * unit_x_bytes + size_t(batch) * 16;     // the tensor-core kernel pads each row of x
+    size_t smem = fixed + size_t(seg) * unit_x_bytes;
     if (in) {
         if (seg != p.n_units) return RPTC_ERR_TOO_LARGE;                        // computed activations live in one segment
         smem += 4096 * sizeof(float) + 128;                                     // exchange buffer of the 4096-point transform
@@ -927,15 +665,15 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
 
     switch (f.code) {
         case RPTC_CODE_LUT:
-            if (K == 2) return dispatch<RPTC_CODE_LUT, 2>(p, batch, tma, smem, stream);
-            if (K == 4) return dispatch<RPTC_CODE_LUT, 4>(p, batch, tma, smem, stream);
+            if (K == 2) return dispatch<RPTC_CODE_LUT, 2>(p, batch, tma, smem, grid, stream);
+            if (K == 4) return dispatch<RPTC_CODE_LUT, 4>(p, batch, tma, smem, grid, stream);
             break;
         case RPTC_CODE_HASH:
-            if (K == 2) return dispatch<RPTC_CODE_HASH, 2>(p, batch, tma, smem, stream);
+            if (K == 2) return dispatch<RPTC_CODE_HASH, 2>(p, batch, tma, smem, grid, stream);
             break;
         case RPTC_CODE_LITE:
-            if (K == 2) return dispatch<RPTC_CODE_LITE, 2>(p, batch, tma, smem, stream);
-            if (K == 4) return dispatch<RPTC_CODE_LITE, 4>(p, batch, tma, smem, stream);
+            if (K == 2) return dispatch<RPTC_CODE_LITE, 2>(p, batch, tma, smem, grid, stream);
+            if (K == 4) return dispatch<RPTC_CODE_LITE, 4>(p, batch, tma, smem, grid, stream);
             break;
     }
     return RPTC_ERR_UNSUPPORTED;
@@ -943,11 +681,23 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
 
 int check_format(const rptc_format *f);   // api.cu
 
+int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
+                const Banks &banks, const rptc_format &f, cudaStream_t stream) {
+    if (tokens > 2 && gemv_few_takes(n, tokens, f, x, ld_x))
+        return gemv_few(codes, lut, nullptr, x, ld_x, acc, ld_acc, m, n, tokens, banks, f, stream);
+    for (int64_t t = 0; t < tokens; t += 2) {
+        const int e = gemv_one(codes, lut, nullptr, static_cast<const __half *>(x) + t * ld_x, ld_x, acc + t * ld_acc, ld_acc, m, n,
+                               tokens - t >= 2 ? 2 : 1, RPTC_XORDER_NATURAL, f, stream, nullptr, banks);
+        if (e) return e;
+    }
+    return RPTC_OK;
+}
+
 }  // namespace rptc
 
 using namespace rptc;
 
-constexpr int kMaxGemvBatch = 64;      // rows of activations per call; more than eight run as a sequence of launches
+constexpr int kMaxGemvBatch = 64;      // rows of activations per call
 
 // Every check of rptc_gemv's arguments that needs no device work, in the order the entry point reports them.
 static int validate_gemv_args(const void *codes, const void *lut, const void *x, int64_t ld_x, const float *acc, int64_t ld_acc,
@@ -974,13 +724,13 @@ extern "C" int rptc_gemv(const void *codes, const void *lut, const uint32_t *car
                          rptc_stream_t stream) {
     if (int e = validate_gemv_args(codes, lut, x, ld_x, acc, ld_acc, m, n, batch, x_order, fmt)) return e;
     if (int e = rptc_check_device()) return e;
+    // Up to two rows the lane-per-row kernel is the faster one (28672 x 8192: 28.0 against 30.6 us).
     if (batch > 2 && x_order == RPTC_XORDER_NATURAL && gemv_few_takes(n, batch, *fmt, x, ld_x))
         return gemv_few(codes, lut, carry_in, x, ld_x, acc, ld_acc, m, n, batch, Banks(), *fmt, static_cast<cudaStream_t>(stream));
-    // batches beyond eight, or not a power of two, run as a short sequence of launches (8 + 8, 4 + 1, ...)
+    // what the kernel for a few rows does not take (rows of x that are not 16-byte aligned, the legacy order): pairs of rows
     int done = 0;
     while (done < batch) {
-        int b = 8;
-        while (b > batch - done) b >>= 1;
+        const int b = batch - done >= 2 ? 2 : 1;
         int e = gemv_one(codes, lut, carry_in, static_cast<const __half *>(x) + (int64_t)done * ld_x, ld_x,
                          acc + (int64_t)done * ld_acc, ld_acc, m, n, b, x_order, *fmt, static_cast<cudaStream_t>(stream));
         if (e) return e;

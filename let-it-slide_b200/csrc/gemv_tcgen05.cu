@@ -13,7 +13,7 @@
 // form four groups of four (a warp reaches the 32 tensor-memory lanes of its number modulo four): a group owns one of the
 // RB row blocks and one of 4 / RB equal parts of a segment's steps, so that it walks along its rows and keeps the 16 bits
 // of history.  A thread owns a row: its code bits arrive through a private ring of asynchronous copies, four steps ahead.
-// One lane of warp 16 loads the activations, taking the parts' steps in turn: position j of part 0, 1, ...  Each group has
+// Warp 16 loads the activations, taking the parts' steps in turn: position j of part 0, 1, ...  Each group has
 // an MMA warp and an accumulator of its own: issuing a step (two waits, four MMAs, two commits) takes one thread about
 // 600 clocks, as long as a group takes to decode it, so that one issuer for all four groups held the kernel to a
 // quarter of the speed.  A segment's sums are added to the caller's fp32 accumulator with atomics.
@@ -234,24 +234,25 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
     } else if (warp == kFewTmaWarp) {
         // ================= activations =================
         pdl_wait_prior_grids();
-        if (lane == 0) {
-            RingPos px = {0, 1u};
-            const uint32_t bytes = 128u * (uint32_t)p.n_cols;
-            for (uint32_t pos = c0; pos < c1 && ok;) {
-                const FewSegment g(pos, c1, p.n_steps);
-                pos = g.end;
-                const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
-                for (int32_t j = 0; j < rounds && ok; ++j)
-                    for (int q = 0; q < PARTS && ok; ++q) {
-                        const int32_t s = g.part_begin<PARTS>(q) + j;
-                        if (s >= g.part_begin<PARTS>(q + 1)) continue;
-                        ok = mbar_wait(empty_x + 8 * px.s, px.phase, p.status);
-                        if (!ok) break;
+        RingPos px = {0, 1u};
+        const uint32_t bytes = 128u * (uint32_t)p.n_cols;
+        for (uint32_t pos = c0; pos < c1 && ok;) {
+            const FewSegment g(pos, c1, p.n_steps);
+            pos = g.end;
+            const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
+            for (int32_t j = 0; j < rounds && ok; ++j)
+#pragma unroll
+                for (int q = 0; q < PARTS; ++q) {
+                    const int32_t s = g.part_begin<PARTS>(q) + j;
+                    if (s >= g.part_begin<PARTS>(q + 1) || !ok) continue;
+                    ok = mbar_wait(empty_x + 8 * px.s, px.phase, p.status);
+                    if (ok && elect_one()) {
                         mbar_expect_tx(full_x + 8 * px.s, bytes);
                         tma_load_2d(p.x_addr + (uint32_t)px.s * bytes, &x_map, s * 64, 0, full_x + 8 * px.s);
-                        px.advance(p.n_xstages);
                     }
-            }
+                    __syncwarp();
+                    px.advance(p.n_xstages);
+                }
         }
     } else {
         // ================= MMA issue for one group: the whole warp waits, one lane issues =================
@@ -324,8 +325,19 @@ static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, uns
     return launch_few<CODE, K, 4>(p, map, grid, s);
 }
 
-// Row blocks per tile.  More of them read the activations from L2 fewer times, fewer cut the work finer.
-static int few_row_blocks(int n_cols) { return n_cols <= 32 ? 1 : 2; }
+// Row blocks per tile.  With four of them a step of activations is loaded, waited for and handed back once per 512 rows;
+// the relative times of a 128-row block are measured (28672 x 8192, 8 tokens: 31.0 us with four, 33.9 with two, 47.0
+// with one).  A bank that is not a whole number of tiles leaves groups without rows: count the blocks that are walked.
+static int few_row_blocks(int64_t m) {
+    const int64_t blocks = (m + 127) / 128;
+    int best = 4;
+    double best_cost = 0;
+    for (int rb = 4; rb >= 1; rb >>= 1) {
+        const double cost = (double)((blocks + rb - 1) / rb * rb) * (rb == 4 ? 1.0 : rb == 2 ? 1.1 : 1.5);
+        if (rb == 4 || cost < best_cost) best = rb, best_cost = cost;
+    }
+    return best;
+}
 
 // Where the table and the activation ring go; false when two stages do not fit.
 static bool few_plan(FewParams &p, const rptc_format &f) {
@@ -358,7 +370,7 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
     FewParams p;
     p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
     if (!few_plan(p, f)) return RPTC_ERR_UNSUPPORTED;
-    const int rb = few_row_blocks(p.n_cols);
+    const int rb = few_row_blocks(m);
     CUtensorMap map;
     if (int e = encode_map(map, x, n, tokens, ld_x, p.n_cols)) return e;
     p.codes = static_cast<const uint4 *>(codes);

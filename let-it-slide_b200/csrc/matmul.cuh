@@ -23,5 +23,9 @@ constexpr int64_t kFewMaxTokens = 96;
 bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x);
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
+// The same for any number of activation rows (TILED codes, no quirk, no carry): gemv_few where it takes them, else the
+// lane-per-row kernel for one or two rows at a time.
+int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
+                const Banks &banks, const rptc_format &f, cudaStream_t stream);
 
 }  // namespace rptc

@@ -170,11 +170,8 @@ class RPTCLlama:
                 and self.cfg.head_dim == 128 and self.blocks[0].qkv.block_out >= 128 and self.fused_tp)
 
     def _extra_launches(self) -> int:
-        """Launches beyond one per matvec: a fused matvec takes up to eight activation rows per launch (8 + 8 at sixteen
-        rows, 4 + 1 at five), and so does the output head."""
-        q, r = divmod(self.rows, 8)
-        per_matvec = q + bin(r).count("1") - 1
-        return 4 * per_matvec * len(self.blocks) + (self.rows - 1) // 8
+        """Launches beyond one per matvec: the output head takes up to eight activation rows per launch."""
+        return (self.rows - 1) // 8
 
     def step_eager(self) -> None:
         if self._glueable():
