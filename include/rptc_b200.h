@@ -205,6 +205,41 @@ int rptc_swiglu_hadamard_f16(const void *gate_up, int64_t ld_in, void *out, int6
                              const void *signs_in, int64_t rows, int64_t n, int block, float scale_out, float scale_in,
                              rptc_stream_t stream);
 
+/* --- whole layers in one call (no reference counterpart: the reference has no layer objects) ---
+ * The kernels of a call follow one another by programmatic dependent launch whatever rptc_set_pdl says.  Codes, tables,
+ * scales and signs must be complete before the kernels that the stream already holds start to run out (they are read
+ * early); activations may come from the kernel right in front.  Workspace: caller-owned device memory, 256-byte aligned,
+ * of *_workspace_bytes for that number of rows; it holds nothing between calls. */
+/* y = s_out * H( scale * W( H( s_in * x ) ) ), Hadamard blocks block_in / block_out (rptc_hadamard's rules); without
+ * signs (both NULL) y = scale * W x, where more than 64 rows need scale == 1.  x fp16 [rows][n], y fp16 [rows][m].
+ * TILED layout, K = 2 or 4; more than 64 rows need m % 128 == 0 and n % 64 == 0. */
+typedef struct rptc_linear {
+    const void *codes, *lut;
+    const uint32_t *carry_in;            /* or NULL */
+    const void *signs_in, *signs_out;    /* fp16 [n], [m], or both NULL */
+    int64_t m, n;
+    int32_t block_in, block_out;
+    float scale;
+    rptc_format fmt;
+} rptc_linear;
+int64_t rptc_linear_workspace_bytes(const rptc_linear *layer, int64_t rows);
+int rptc_linear_forward(const rptc_linear *layer, const void *x, void *y, int64_t rows, void *workspace, int64_t workspace_bytes,
+                        rptc_stream_t stream);
+/* The layer quantize_hf.py stores (quantize_hf.py:77-117,120-156,166): y = scales_out * W (scales_in * x) +
+ * biases_out * sum(x) + <biases_in, x> (+ bias), W = `banks` banks of m / banks rows with an alphabet each (code LUT, K = 2,
+ * fp16 [banks][2^L]), a bank's codes padded to bank_blocks blocks of 32 rows (TILED).  x and y of `dtype` 0 = fp16,
+ * 1 = bf16, 2 = fp32, [tokens][n] and [tokens][m]; n % 64 == 0.  Biases and scales fp32. */
+typedef struct rptc_packed {
+    const void *codes, *alphabets;
+    const float *biases_out, *biases_in, *scales_out, *scales_in;
+    const float *bias;                   /* [m] or NULL */
+    int64_t m, n;
+    int32_t banks, bank_blocks, L;
+} rptc_packed;
+int64_t rptc_packed_workspace_bytes(const rptc_packed *layer, int64_t tokens);
+int rptc_packed_forward(const rptc_packed *layer, const void *x, int dtype, void *y, int64_t tokens, void *workspace,
+                        int64_t workspace_bytes, rptc_stream_t stream);
+
 /* --- the non-quantised pieces of a Llama-architecture decode step (no reference counterpart: the
  * reference evaluates models through Hugging Face transformers, quantize_hf.py:230-236) --- */
 

@@ -22,6 +22,8 @@ struct HadParams {
     int32_t in_is_f32, transpose, clear_in;
     float scale;
     int64_t n;
+    float *clear;               // optional fp32 range that this launch zeroes (its own, not the input)
+    int64_t clear_count;        // a multiple of 4
 };
 
 __global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
@@ -30,6 +32,12 @@ __global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
     pdl_wait_prior_grids();
     const int t = threadIdx.x;
     const int64_t row = blockIdx.y;
+    if (p.clear) {
+        float4 *z = reinterpret_cast<float4 *>(p.clear);
+        const int64_t step = (int64_t)gridDim.x * gridDim.y * blockDim.x;
+        for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + t; 4 * i < p.clear_count; i += step)
+            z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const int64_t col = (int64_t)blockIdx.x * p.chunk + 8 * t;
     if (col >= p.n) return;     // only with blocks <= 256 (whole warps leave; such blocks need no CTA barrier)
     float v[8];
@@ -144,9 +152,10 @@ static float hadamard_norm(int block) {
 
 using namespace rptc;
 
-extern "C" int rptc_hadamard(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs,
-                             const void *residual, int64_t ld_res, int64_t rows, int64_t n, int block, int transpose,
-                             float scale, int clear_in, rptc_stream_t stream) {
+namespace rptc {
+int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
+                       int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
+                       int64_t clear_count, cudaStream_t stream) {
     if (!in || !out) return RPTC_ERR_ARG;
     if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
     if (rows <= 0 || n <= 0 || (n % block) || ld_in < n || ld_out < n || (residual && ld_res < n)) return RPTC_ERR_SHAPE;
@@ -174,15 +183,25 @@ extern "C" int rptc_hadamard(const void *in, int in_is_f32, int64_t ld_in, void 
     p.clear_in = clear_in;
     p.scale = scale * hadamard_norm(block);
     p.n = n;
+    p.clear = clear_count > 0 ? clear : nullptr;
+    p.clear_count = clear_count;
     if (block <= 256 && n > 256) {
         // small blocks: a warp per 256 columns, eight warps per CTA, so that many-row inputs do not become
         // hundreds of thousands of one-warp CTAs
         p.chunk = 2048;
         return launch(hadamard_kernel, dim3((unsigned)((n + 2047) / 2048), (unsigned)rows), dim3(256), 0,
-                      static_cast<cudaStream_t>(stream), p);
+                      stream, p);
     }
     return launch(hadamard_kernel, dim3((unsigned)(n / chunk), (unsigned)rows), dim3(chunk / 8), 0,
-                  static_cast<cudaStream_t>(stream), p);
+                  stream, p);
+}
+}  // namespace rptc
+
+extern "C" int rptc_hadamard(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs,
+                             const void *residual, int64_t ld_res, int64_t rows, int64_t n, int block, int transpose,
+                             float scale, int clear_in, rptc_stream_t stream) {
+    return hadamard_and_clear(in, in_is_f32, ld_in, out, ld_out, signs, residual, ld_res, rows, n, block, transpose, scale, clear_in, nullptr, 0,
+                              static_cast<cudaStream_t>(stream));
 }
 
 static int swiglu_launch(float *acc, const void *in16, int64_t ld_in, void *out, int64_t ld_out, const void *signs_out,

@@ -7,7 +7,7 @@ namespace rptc {
 // whatever the source layout is.
 __global__ void repack_kernel(const uint4 *__restrict__ src, UnitStrides ss, uint4 *__restrict__ dst, int dst_layout,
                               int64_t m, int64_t n_units) {
-    pdl_allow_next_grid();
+    // No early start for the kernel behind: the matrix products read packed codes before their dependency wait.
     pdl_wait_prior_grids();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m * n_units) return;

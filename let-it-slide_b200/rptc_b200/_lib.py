@@ -63,6 +63,20 @@ class GemvInput(ctypes.Structure):
                 ("w_norm", ctypes.c_void_p), ("clear", ctypes.c_void_p), ("clear_count", ctypes.c_int64)]
 
 
+class Linear(ctypes.Structure):
+    """Mirror of `rptc_linear`."""
+    _fields_ = [("codes", ctypes.c_void_p), ("lut", ctypes.c_void_p), ("carry_in", ctypes.c_void_p), ("signs_in", ctypes.c_void_p),
+                ("signs_out", ctypes.c_void_p), ("m", ctypes.c_int64), ("n", ctypes.c_int64), ("block_in", ctypes.c_int32),
+                ("block_out", ctypes.c_int32), ("scale", ctypes.c_float), ("fmt", Format)]
+
+
+class Packed(ctypes.Structure):
+    """Mirror of `rptc_packed`."""
+    _fields_ = [("codes", ctypes.c_void_p), ("alphabets", ctypes.c_void_p), ("biases_out", ctypes.c_void_p), ("biases_in", ctypes.c_void_p),
+                ("scales_out", ctypes.c_void_p), ("scales_in", ctypes.c_void_p), ("bias", ctypes.c_void_p), ("m", ctypes.c_int64),
+                ("n", ctypes.c_int64), ("banks", ctypes.c_int32), ("bank_blocks", ctypes.c_int32), ("L", ctypes.c_int32)]
+
+
 _lib = None
 
 _SIGS = {
@@ -140,6 +154,12 @@ _SIGS = {
     "rptc_viterbi_encode_banked": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                                   ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.c_void_p, ctypes.c_int64,
                                                   ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]),
+    "rptc_linear_workspace_bytes": (ctypes.c_int64, [ctypes.POINTER(Linear), ctypes.c_int64]),
+    "rptc_linear_forward": (ctypes.c_int, [ctypes.POINTER(Linear), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                           ctypes.c_int64, ctypes.c_void_p]),
+    "rptc_packed_workspace_bytes": (ctypes.c_int64, [ctypes.POINTER(Packed), ctypes.c_int64]),
+    "rptc_packed_forward": (ctypes.c_int, [ctypes.POINTER(Packed), ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int64,
+                                           ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]),
     "rptc_rope_cache_prompt": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
                                               ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_float,
                                               ctypes.c_void_p]),
@@ -175,6 +195,20 @@ def exported_symbols() -> list[str]:
 def check(status: int, where: str) -> None:
     if status != OK:
         raise RPTCError(status, where)
+
+
+def call(name: str, device: torch.device, *args) -> None:
+    """One entry point on `device` and torch's current stream there (the last argument of every such entry point).  The
+    device is switched only when it is not the current one: the context manager costs as much as a short launch."""
+    fn = getattr(_lib or lib(), name)
+    index = device.index
+    if index == torch._C._cuda_getDevice():
+        status = fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    else:
+        with torch.cuda.device(device):
+            status = fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    if status != OK:
+        raise RPTCError(status, name)
 
 
 def stream_ptr(stream: torch.cuda.Stream | None = None) -> int:

@@ -7,7 +7,7 @@ import torch
 
 from . import _lib
 from ._lib import (CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_TILED, LAYOUT_UNITMAJOR, XORDER_NATURAL,
-                   Format, check, lib, ptr, stream_ptr)
+                   Format, call, check, lib, ptr, stream_ptr)
 
 
 def _cuda_contig(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
@@ -54,8 +54,7 @@ def repack(codes: torch.Tensor, src_layout: int, dst_layout: int, m: int, n_unit
     else:
         shape = (m // 32, n_units, 32, 4)
     out = torch.empty(shape, dtype=torch.int32, device=codes.device)
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_repack(ptr(codes), src_layout, ptr(out), dst_layout, m, n_units, stream_ptr()), "rptc_repack")
+    call("rptc_repack", codes.device, ptr(codes), src_layout, ptr(out), dst_layout, m, n_units)
     return out
 
 
@@ -75,9 +74,7 @@ def decompress(codes: torch.Tensor, lut: torch.Tensor, m: int, n: int, fmt: Form
             raise RuntimeError("out must be a CUDA fp16 [m, n] tensor with unit column stride")
     if carry_in is not None:
         _cuda_contig(carry_in, "carry_in", torch.int32)
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_decompress(ptr(codes), ptr(lut), ptr(carry_in), ptr(out), out.stride(0), m, n, ctypes.byref(fmt),
-                                    stream_ptr()), "rptc_decompress")
+    call("rptc_decompress", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(out), out.stride(0), m, n, ctypes.byref(fmt))
     return out
 
 
@@ -98,10 +95,8 @@ def gemv_acc(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, acc: torch
         raise RuntimeError("codes has the wrong number of elements for m, n, K")
     if lut.numel() != fmt.lut_numel():
         raise RuntimeError(f"lut must have {fmt.lut_numel()} elements, got {lut.numel()}")
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_gemv(ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0) if x.shape[0] > 1 else max(n, x.stride(0)),
-                              ptr(acc), acc.stride(0) if acc.shape[0] > 1 else max(m, acc.stride(0)), m, n, x.shape[0],
-                              x_order, ctypes.byref(fmt), stream_ptr()), "rptc_gemv")
+    call("rptc_gemv", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0) if x.shape[0] > 1 else max(n, x.stride(0)),
+         ptr(acc), acc.stride(0) if acc.shape[0] > 1 else max(m, acc.stride(0)), m, n, x.shape[0], x_order, ctypes.byref(fmt))
 
 
 def gemv_norm_input(codes: torch.Tensor, lut: torch.Tensor, acc: torch.Tensor, m: int, n: int, fmt: Format, rows: int,
@@ -113,9 +108,8 @@ def gemv_norm_input(codes: torch.Tensor, lut: torch.Tensor, acc: torch.Tensor, m
     from ._lib import GemvInput
     d = GemvInput(ptr(prev_acc), 0 if prev_acc is None else _ld(prev_acc, n), ptr(signs_out), scale_out, eps,
                   ptr(signs_in), ptr(h_in), ptr(h_out), _ld(h_in, n), ptr(w_norm), ptr(clear), 0 if clear is None else clear.numel())
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_gemv_glued(ptr(codes), ptr(lut), ptr(carry_in), ctypes.byref(d), ptr(acc), _ld(acc, m), m, n, rows,
-                                    ctypes.byref(fmt), stream_ptr()), "rptc_gemv_glued")
+    call("rptc_gemv_glued", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ctypes.byref(d), ptr(acc), _ld(acc, m), m, n, rows,
+         ctypes.byref(fmt))
 
 
 def gemv_swiglu_input(codes: torch.Tensor, lut: torch.Tensor, acc: torch.Tensor, m: int, n: int, fmt: Format, rows: int,
@@ -123,10 +117,9 @@ def gemv_swiglu_input(codes: torch.Tensor, lut: torch.Tensor, acc: torch.Tensor,
                       block: int, clear: torch.Tensor | None = None, carry_in: torch.Tensor | None = None) -> None:
     """acc += W x with x = H(s_in * silu(g) * u), (g | u) = s_out * H(prev_acc) * scale_out, made inside the launch
     block by block (rptc_gemv_swiglu).  `clear` is zeroed by the launch."""
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_gemv_swiglu(ptr(codes), ptr(lut), ptr(carry_in), ptr(prev_acc), _ld(prev_acc, 2 * n), ptr(signs_out), scale_out,
-                                     ptr(signs_in), block, ptr(acc), _ld(acc, m), m, n, rows, ctypes.byref(fmt), ptr(clear),
-                                     0 if clear is None else clear.numel(), stream_ptr()), "rptc_gemv_swiglu")
+    call("rptc_gemv_swiglu", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(prev_acc), _ld(prev_acc, 2 * n), ptr(signs_out),
+         scale_out, ptr(signs_in), block, ptr(acc), _ld(acc, m), m, n, rows, ctypes.byref(fmt), ptr(clear),
+         0 if clear is None else clear.numel())
 
 
 def gemv_finish(acc: torch.Tensor, y: torch.Tensor, m: int, scale: float = 1.0, accumulate: bool = False,
@@ -136,10 +129,8 @@ def gemv_finish(acc: torch.Tensor, y: torch.Tensor, m: int, scale: float = 1.0, 
         acc = acc.unsqueeze(0)
     if y.dim() == 1:
         y = y.unsqueeze(0)
-    with torch.cuda.device(acc.device):
-        check(lib().rptc_gemv_finish(ptr(acc), acc.stride(0) if acc.shape[0] > 1 else max(m, acc.stride(0)), ptr(y),
-                                     y.stride(0) if y.shape[0] > 1 else max(m, y.stride(0)), m, acc.shape[0], scale,
-                                     int(accumulate), int(clear), stream_ptr()), "rptc_gemv_finish")
+    call("rptc_gemv_finish", acc.device, ptr(acc), acc.stride(0) if acc.shape[0] > 1 else max(m, acc.stride(0)), ptr(y),
+         y.stride(0) if y.shape[0] > 1 else max(m, y.stride(0)), m, acc.shape[0], scale, int(accumulate), int(clear))
 
 
 def gemv(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, m: int, n: int, fmt: Format,
@@ -162,9 +153,8 @@ def gemm(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, m: int, n: int
         raise RuntimeError("x must be a CUDA fp16 [tokens, n] tensor with unit column stride")
     if out is None:
         out = torch.empty((x.shape[0], m), dtype=torch.float16, device=x.device)
-    with torch.cuda.device(codes.device):
-        check(lib().rptc_gemm(ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0), ptr(out), out.stride(0), m, n,
-                              x.shape[0], ctypes.byref(fmt), stream_ptr()), "rptc_gemm")
+    call("rptc_gemm", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0), ptr(out), out.stride(0), m, n, x.shape[0],
+         ctypes.byref(fmt))
     return out
 
 
@@ -185,20 +175,16 @@ def hadamard(x: torch.Tensor, signs: torch.Tensor | None, block: int, transpose:
         _cuda_contig(signs, "signs", torch.float16)
     if residual is not None and residual.dim() == 1:
         residual = residual.unsqueeze(0)
-    with torch.cuda.device(x.device):
-        check(lib().rptc_hadamard(ptr(x), int(x.dtype == torch.float32), _ld(x, n), ptr(out), _ld(out, n), ptr(signs),
-                                  ptr(residual), 0 if residual is None else _ld(residual, n), rows, n, block, int(transpose),
-                                  scale, int(clear_in), stream_ptr()), "rptc_hadamard")
+    call("rptc_hadamard", x.device, ptr(x), int(x.dtype == torch.float32), _ld(x, n), ptr(out), _ld(out, n), ptr(signs), ptr(residual),
+         0 if residual is None else _ld(residual, n), rows, n, block, int(transpose), scale, int(clear_in))
     return out[0] if squeeze else out
 
 
 def swiglu_hadamard(acc: torch.Tensor, out: torch.Tensor, signs_out: torch.Tensor | None, signs_in: torch.Tensor | None,
                     n: int, block: int, scale_out: float, scale_in: float = 1.0, clear: bool = True) -> torch.Tensor:
     """Fused gated-MLP middle (rptc_swiglu_hadamard): acc fp32 [rows, 2n] -> out fp16 [rows, n]."""
-    with torch.cuda.device(acc.device):
-        check(lib().rptc_swiglu_hadamard(ptr(acc), _ld(acc, 2 * n), ptr(out), _ld(out, n), ptr(signs_out), ptr(signs_in),
-                                         acc.shape[0], n, block, scale_out, scale_in, int(clear), stream_ptr()),
-              "rptc_swiglu_hadamard")
+    call("rptc_swiglu_hadamard", acc.device, ptr(acc), _ld(acc, 2 * n), ptr(out), _ld(out, n), ptr(signs_out), ptr(signs_in),
+         acc.shape[0], n, block, scale_out, scale_in, int(clear))
     return out
 
 
@@ -206,44 +192,37 @@ def swiglu_hadamard_f16(gate_up: torch.Tensor, out: torch.Tensor, signs_out: tor
                         n: int, block: int, scale_out: float, scale_in: float = 1.0) -> torch.Tensor:
     """Fused gated-MLP middle from the fp16 output of a matrix product (rptc_swiglu_hadamard_f16):
     gate_up fp16 [rows, 2n] -> out fp16 [rows, n]."""
-    with torch.cuda.device(gate_up.device):
-        check(lib().rptc_swiglu_hadamard_f16(ptr(gate_up), _ld(gate_up, 2 * n), ptr(out), _ld(out, n), ptr(signs_out), ptr(signs_in),
-                                             gate_up.shape[0], n, block, scale_out, scale_in, stream_ptr()),
-              "rptc_swiglu_hadamard_f16")
+    call("rptc_swiglu_hadamard_f16", gate_up.device, ptr(gate_up), _ld(gate_up, 2 * n), ptr(out), _ld(out, n), ptr(signs_out),
+         ptr(signs_in), gate_up.shape[0], n, block, scale_out, scale_in)
     return out
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, eps: float) -> torch.Tensor:
     rows, n = x.shape
-    with torch.cuda.device(x.device):
-        check(lib().rptc_rmsnorm(ptr(x), _ld(x, n), ptr(w), ptr(out), _ld(out, n), rows, n, eps, stream_ptr()), "rptc_rmsnorm")
+    call("rptc_rmsnorm", x.device, ptr(x), _ld(x, n), ptr(w), ptr(out), _ld(out, n), rows, n, eps)
     return out
 
 
 def rope_cache(qkv: torch.Tensor, pos: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, hq: int, hkv: int, d: int,
                theta: float) -> None:
     rows = qkv.shape[0]
-    with torch.cuda.device(qkv.device):
-        check(lib().rptc_rope_cache(ptr(qkv), _ld(qkv, qkv.shape[1]), ptr(pos), ptr(kcache), ptr(vcache), rows, hq, hkv, d,
-                                    kcache.shape[1], theta, stream_ptr()), "rptc_rope_cache")
+    call("rptc_rope_cache", qkv.device, ptr(qkv), _ld(qkv, qkv.shape[1]), ptr(pos), ptr(kcache), ptr(vcache), rows, hq, hkv, d,
+         kcache.shape[1], theta)
 
 
 def rope_cache_prompt(qkv: torch.Tensor, rows: int, tokens: int, kcache: torch.Tensor, vcache: torch.Tensor, hq: int, hkv: int, d: int,
                       theta: float) -> None:
     """RoPE of q (in place) and k, and the cache writes of k and v, for a whole prompt (rptc_rope_cache_prompt):
     qkv fp16 [rows * tokens, (hq + 2 hkv) d]."""
-    with torch.cuda.device(qkv.device):
-        check(lib().rptc_rope_cache_prompt(ptr(qkv), _ld(qkv, qkv.shape[1]), rows, tokens, ptr(kcache), ptr(vcache), hq, hkv, d,
-                                           kcache.shape[1], theta, stream_ptr()), "rptc_rope_cache_prompt")
+    call("rptc_rope_cache_prompt", qkv.device, ptr(qkv), _ld(qkv, qkv.shape[1]), rows, tokens, ptr(kcache), ptr(vcache), hq, hkv, d,
+         kcache.shape[1], theta)
 
 
 def attn_decode(qkv: torch.Tensor, pos: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, out: torch.Tensor, hq: int,
                 hkv: int, d: int, signs_in: torch.Tensor | None = None) -> torch.Tensor:
     rows = qkv.shape[0]
-    with torch.cuda.device(qkv.device):
-        check(lib().rptc_attn_decode(ptr(qkv), _ld(qkv, qkv.shape[1]), ptr(pos), ptr(kcache), ptr(vcache), ptr(out),
-                                     _ld(out, out.shape[1]), rows, hq, hkv, d, kcache.shape[1], d ** -0.5, ptr(signs_in),
-                                     stream_ptr()), "rptc_attn_decode")
+    call("rptc_attn_decode", qkv.device, ptr(qkv), _ld(qkv, qkv.shape[1]), ptr(pos), ptr(kcache), ptr(vcache), ptr(out),
+         _ld(out, out.shape[1]), rows, hq, hkv, d, kcache.shape[1], d ** -0.5, ptr(signs_in))
     return out
 
 
@@ -253,10 +232,8 @@ def qkv_attn_decode(acc: torch.Tensor, signs_out: torch.Tensor | None, scale_out
     """Output transform of the fused qkv layer + RoPE + KV append + attention (+ per-head input transform of the
     output projection) in one launch (rptc_qkv_attn_decode)."""
     rows = acc.shape[0]
-    with torch.cuda.device(acc.device):
-        check(lib().rptc_qkv_attn_decode(ptr(acc), _ld(acc, acc.shape[1]), ptr(signs_out), scale_out, ptr(pos), ptr(kcache),
-                                         ptr(vcache), ptr(out), _ld(out, out.shape[1]), rows, heads, kv_heads, kcache.shape[1], theta,
-                                         ptr(signs_in), stream_ptr()), "rptc_qkv_attn_decode")
+    call("rptc_qkv_attn_decode", acc.device, ptr(acc), _ld(acc, acc.shape[1]), ptr(signs_out), scale_out, ptr(pos), ptr(kcache),
+         ptr(vcache), ptr(out), _ld(out, out.shape[1]), rows, heads, kv_heads, kcache.shape[1], theta, ptr(signs_in))
     return out
 
 
@@ -265,10 +242,8 @@ def finish_norm_hadamard(acc: torch.Tensor | None, signs_out: torch.Tensor | Non
                          out: torch.Tensor) -> torch.Tensor:
     """h += output transform of acc; out = input transform of rmsnorm(h) (rptc_finish_norm_hadamard)."""
     rows, n = h.shape
-    with torch.cuda.device(h.device):
-        check(lib().rptc_finish_norm_hadamard(ptr(acc), 0 if acc is None else _ld(acc, n), ptr(signs_out), scale_out, ptr(h),
-                                              _ld(h, n), ptr(w_norm), eps, ptr(signs_in), int(transform_in), ptr(out),
-                                              _ld(out, n), rows, n, stream_ptr()), "rptc_finish_norm_hadamard")
+    call("rptc_finish_norm_hadamard", h.device, ptr(acc), 0 if acc is None else _ld(acc, n), ptr(signs_out), scale_out, ptr(h), _ld(h, n),
+         ptr(w_norm), eps, ptr(signs_in), int(transform_in), ptr(out), _ld(out, n), rows, n)
     return out
 
 
@@ -276,10 +251,8 @@ def qkv_finish(acc: torch.Tensor, signs_out: torch.Tensor | None, scale: float, 
                vcache: torch.Tensor, pos: torch.Tensor, hq: int, hkv: int, block: int, theta: float) -> None:
     """Output transform of the fused qkv layer + RoPE + KV-cache append (rptc_qkv_finish)."""
     rows = acc.shape[0]
-    with torch.cuda.device(acc.device):
-        check(lib().rptc_qkv_finish(ptr(acc), _ld(acc, acc.shape[1]), ptr(signs_out), scale, ptr(q_out), _ld(q_out, q_out.shape[1]),
-                                    ptr(kcache), ptr(vcache), ptr(pos), rows, hq, hkv, kcache.shape[1], block, theta,
-                                    stream_ptr()), "rptc_qkv_finish")
+    call("rptc_qkv_finish", acc.device, ptr(acc), _ld(acc, acc.shape[1]), ptr(signs_out), scale, ptr(q_out), _ld(q_out, q_out.shape[1]),
+         ptr(kcache), ptr(vcache), ptr(pos), rows, hq, hkv, kcache.shape[1], block, theta)
 
 
 def dense_gemv(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -291,18 +264,14 @@ def dense_gemv(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None
     if out is None:
         out = torch.empty((x.shape[0], m), dtype=torch.float16, device=x.device)
     o2 = out.unsqueeze(0) if out.dim() == 1 else out
-    with torch.cuda.device(W.device):
-        for b0 in range(0, x.shape[0], 8):              # the kernel takes up to eight activation rows per launch
-            xb, ob = x[b0:b0 + 8], o2[b0:b0 + 8]
-            check(lib().rptc_dense_gemv(ptr(W), W.stride(0), ptr(xb), _ld(xb, n), ptr(ob), _ld(ob, m), m, n, xb.shape[0], stream_ptr()),
-                  "rptc_dense_gemv")
+    for b0 in range(0, x.shape[0], 8):                  # the kernel takes up to eight activation rows per launch
+        xb, ob = x[b0:b0 + 8], o2[b0:b0 + 8]
+        call("rptc_dense_gemv", W.device, ptr(W), W.stride(0), ptr(xb), _ld(xb, n), ptr(ob), _ld(ob, m), m, n, xb.shape[0])
     return out[0] if squeeze and out.dim() == 2 else out
 
 
 def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    with torch.cuda.device(table.device):
-        check(lib().rptc_embed(ptr(table), ptr(ids), ptr(out), _ld(out, table.shape[1]), ids.shape[0], table.shape[1],
-                               stream_ptr()), "rptc_embed")
+    call("rptc_embed", table.device, ptr(table), ptr(ids), ptr(out), _ld(out, table.shape[1]), ids.shape[0], table.shape[1])
     return out
 
 
@@ -312,9 +281,8 @@ def embed_mailbox(table: torch.Tensor, slots: torch.Tensor, steps_done: torch.Te
     (rptc_embed_mailbox)."""
     if not slots.is_pinned() or slots.dtype != torch.int64 or steps_done.dtype != torch.int32:
         raise RuntimeError("slots must be a pinned int64 host tensor and steps_done an int32 device tensor")
-    with torch.cuda.device(table.device):
-        check(lib().rptc_embed_mailbox(ptr(table), ptr(slots), ptr(steps_done), ptr(ids), ptr(out), _ld(out, table.shape[1]),
-                                       ids.shape[0], table.shape[1], table.shape[0], timeout_ms, stream_ptr()), "rptc_embed_mailbox")
+    call("rptc_embed_mailbox", table.device, ptr(table), ptr(slots), ptr(steps_done), ptr(ids), ptr(out), _ld(out, table.shape[1]),
+         ids.shape[0], table.shape[1], table.shape[0], timeout_ms)
 
 
 def next_token(logits: torch.Tensor, next_ids: torch.Tensor, ids: torch.Tensor | None = None, pos: torch.Tensor | None = None,
@@ -323,9 +291,8 @@ def next_token(logits: torch.Tensor, next_ids: torch.Tensor, ids: torch.Tensor |
     rows, n = logits.shape
     if next_ids.dtype != torch.int64 or (mirror is not None and (mirror.dtype != torch.int64 or not mirror.is_pinned())):
         raise RuntimeError("next_ids must be int64 and mirror a pinned int64 host tensor")
-    with torch.cuda.device(logits.device):
-        check(lib().rptc_next_token(ptr(logits), _ld(logits, n), rows, n, ptr(next_ids), ptr(ids), ptr(pos), ptr(mirror),
-                                    ptr(steps_done), stream_ptr()), "rptc_next_token")
+    call("rptc_next_token", logits.device, ptr(logits), _ld(logits, n), rows, n, ptr(next_ids), ptr(ids), ptr(pos), ptr(mirror),
+         ptr(steps_done))
 
 
 def viterbi_encode(alphabet: torch.Tensor, pos_weight: torch.Tensor, samples: torch.Tensor, workspace_limit: int = 12 << 30):

@@ -161,3 +161,23 @@ def test_packed_layer_with_banks_that_are_not_whole_row_blocks(tokens):
     want = x.double() @ layer.decoded().double().t()
     got = layer(x).double()
     assert (got - want).abs().max().item() <= 2e-3 * want.abs().max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,n,banks,L,tokens", [(256, 64, 8, 12, 1), (352, 320, 4, 14, 2), (4096, 512, 32, 16, 3), (1376, 1024, 8, 16, 96), (1376, 1024, 8, 16, 97),
+                                                (4096, 1088, 16, 16, 300)])
+def test_packed_layer_forward_over_its_products(m, n, banks, L, tokens, dtype):
+    """One to two tokens, a few, and the tiled product; banks that are and are not whole row blocks and tiles; every type."""
+    import quantize_hf as q
+    g = torch.Generator(device="cuda").manual_seed(m + tokens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    symbols = torch.randint(0, 4, (m, n), generator=g, device="cuda", dtype=torch.int32)
+    layer = q.FactorizedRPTCLinear.from_parts(symbols, rnd(banks, 1 << L), 0.1 * rnd(m), 0.1 * rnd(n), 0.5 + rnd(m).abs(), 0.5 + rnd(n).abs(), rnd(m))
+    x = rnd(tokens, n).to(dtype)
+    xs = (x.float() * layer.scales_in).half()
+    want = (xs.double() @ layer.decoded().double().t()) * layer.scales_out.double() + x.double().sum(1, keepdim=True) * layer.biases_out.double() \
+        + (x.double() @ layer.biases_in.double())[:, None] + layer.bias.double()
+    got = layer(x)
+    assert got.dtype == dtype
+    assert (got.double() - want).norm() <= (4e-3 if dtype == torch.bfloat16 else 6e-4) * want.norm()
