@@ -109,6 +109,16 @@ int rptc_repack(const void *src, int src_layout, void *dst, int dst_layout, int6
 int rptc_decompress(const void *codes, const void *lut, const uint32_t *carry_in, void *out, int64_t ld_out,
                     int64_t m, int64_t n, const rptc_format *fmt, rptc_stream_t stream);
 
+/* Symbols (int32 [rows][length], 0..3) -> out[row][i] = alphabet[state_i] rounded to fp16, state = the last L <= 16 bits of
+ * the row's symbols up to i, zero before the row (rptc.py:74-85).  alphabet [2^L] and out [rows][length] are both fp32
+ * (is_f32 = 1) or both fp16. */
+int rptc_dequantize(const void *alphabet, const int32_t *symbols, void *out, int is_f32, int64_t rows, int64_t length, int L,
+                    rptc_stream_t stream);
+/* Symbols of `bits` = 1, 2, 4 or 8 bits (int32 [rows][length]) -> ROWMAJOR words [rows][row_words], first symbol on top,
+ * zeros behind the row's end. */
+int rptc_pack_symbols(const int32_t *symbols, void *words, int64_t rows, int64_t length, int64_t row_words, int bits,
+                      rptc_stream_t stream);
+
 /* Fused decode + matvec, batch 1..64:  acc[b][row] += sum_c W[row][c] * x[b][c]   (fp32 acc).  One launch where x is
  * 16-byte aligned with ld_x % 8 == 0 and n % 64 == 0 (and for one or two rows), else one per two activation rows.
  * Replaces the kernels behind decompress_matvec_{16,20}_{6,8}_1 (inference.cu:189-277) and
@@ -161,6 +171,16 @@ int rptc_gemv_swiglu(const void *codes, const void *lut, const uint32_t *carry_i
  * accumulate = 1 gives decompress_matvec_t's `out +=` (inference_t.cu:170-171). */
 int rptc_gemv_finish(float *acc, int64_t ld_acc, void *y, int64_t ld_y, int64_t m, int batch, float scale,
                      int accumulate, int clear, rptc_stream_t stream);
+
+/* rptc_gemv + rptc_gemv_finish with the device time of both (the reference's functions return it, inference.cu:344-355):
+ * y = fp16(W x) (+ y if accumulate), batch 1.  acc is fp32 scratch [m] that is zero on entry and left zero; waits for the
+ * result.  *ms: milliseconds between events on the stream around the work. */
+int rptc_gemv_timed(const void *codes, const void *lut, const void *x, float *acc, void *y, int64_t m, int64_t n, int x_order,
+                    int accumulate, const rptc_format *fmt, float *ms, rptc_stream_t stream);
+/* Device time of whatever is launched between the two on the stream, by the calling thread (one pair of events per thread
+ * and device, kept); rptc_timer_end waits for the end. */
+int rptc_timer_begin(rptc_stream_t stream);
+int rptc_timer_end(float *ms, rptc_stream_t stream);
 
 /* The fused matvec for callers that cannot allocate device memory where they call this library (a server whose
  * memory pool owns the whole device, a plugin that must not go around its host's allocator, a process with a

@@ -130,3 +130,54 @@ extern "C" int rptc_device_status(void) {
     }
     return RPTC_OK;
 }
+
+// ---- device time of a piece of work ------------------------------------------------------------------
+namespace rptc {
+struct TimerEvents {
+    cudaEvent_t begin = nullptr, end = nullptr;
+};
+static thread_local TimerEvents g_timers[kMaxDevices];      // kept: creating a pair costs as much as a launch
+static int timer_events(TimerEvents *&t) {
+    const int dev = current_device();
+    if (dev < 0) return cuda_fail(cudaErrorNoDevice);
+    t = &g_timers[dev];
+    if (!t->begin) RPTC_CUDA(cudaEventCreate(&t->begin));
+    if (!t->end) RPTC_CUDA(cudaEventCreate(&t->end));
+    return RPTC_OK;
+}
+}  // namespace rptc
+
+extern "C" int rptc_timer_begin(rptc_stream_t stream) {
+    TimerEvents *t;
+    if (int e = rptc_check_device()) return e;
+    if (int e = timer_events(t)) return e;
+    RPTC_CUDA(cudaEventRecord(t->begin, static_cast<cudaStream_t>(stream)));
+    return RPTC_OK;
+}
+
+extern "C" int rptc_timer_end(float *ms, rptc_stream_t stream) {
+    if (!ms) return RPTC_ERR_ARG;
+    TimerEvents *t;
+    if (int e = rptc_check_device()) return e;
+    if (int e = timer_events(t)) return e;
+    RPTC_CUDA(cudaEventRecord(t->end, static_cast<cudaStream_t>(stream)));
+    RPTC_CUDA(cudaEventSynchronize(t->end));
+    RPTC_CUDA(cudaEventElapsedTime(ms, t->begin, t->end));
+    return RPTC_OK;
+}
+
+extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x, float *acc, void *y, int64_t m, int64_t n, int x_order,
+                               int accumulate, const rptc_format *fmt, float *ms, rptc_stream_t stream) {
+    if (!y || !ms) return RPTC_ERR_ARG;
+    if (int e = rptc_timer_begin(stream)) return e;
+    if (int e = rptc_gemv(codes, lut, nullptr, x, n, acc, m, m, n, 1, x_order, fmt, stream)) return e;
+    {
+        // the finish behind the product may start early: it waits for the product's sums itself
+        const bool before = pdl_enabled();
+        rptc_set_pdl(1);
+        const int e = rptc_gemv_finish(acc, m, y, m, m, 1, 1.f, accumulate, 1, stream);
+        rptc_set_pdl(before ? 1 : 0);
+        if (e) return e;
+    }
+    return rptc_timer_end(ms, stream);
+}

@@ -6,8 +6,8 @@
 `quantize` is the Viterbi encoder of rptc.py:13-71 (state = last L bits, 2 bits per step, start
 state 0, first-minimum tie break); it is the offline half: CUDA fp32 tensors take the CUDA encoder
 (csrc/viterbi.cu), anything else a torch restatement of the same recurrence.
-`dequantize` is the decoder of rptc.py:74-85 and is the hot path: it packs the symbols into the
-MSB-first bitstream the kernels read and calls the CUDA decompress kernel, so it needs CUDA tensors
+`dequantize` is the decoder of rptc.py:74-85 and is the hot path: one CUDA kernel from symbols to weights
+(csrc/dequantize.cu; packed streams have the decompress kernel), so it needs CUDA tensors
 (there is no CPU decode path in this package).  The codebook is held in fp16 on the device, as in
 the reference's kernels (inference.cu:114-117): `dequantize` returns the fp16-rounded alphabet
 entries, cast back to the alphabet's dtype.
@@ -16,7 +16,7 @@ from __future__ import annotations
 
 import torch
 
-from rptc_b200 import CODE_LUT, LAYOUT_ROWMAJOR, Format, ops
+from rptc_b200 import ops
 
 
 def quantize_rows(permuted_alphabet: torch.Tensor, weights: torch.Tensor, samples: torch.Tensor):
@@ -66,6 +66,9 @@ def pack_symbols(quantized: torch.Tensor, bits: int = 2) -> torch.Tensor:
     per = 32 // bits
     assert 32 % bits == 0
     n_words = -(-length // (4 * per)) * 4
+    if quantized.is_cuda and bits in (1, 2, 4, 8) and quantized.numel():
+        q = quantized.to(torch.int32).contiguous()
+        return ops.pack_symbols(q if q.data_ptr() % 16 == 0 else q.clone(), bits, n_words)
     sym = torch.zeros((rows, n_words * per), dtype=torch.int64, device=quantized.device)
     sym[:, :length] = quantized.to(torch.int64)
     shifts = (bits * (per - 1 - torch.arange(per, device=quantized.device))).to(torch.int64)
@@ -78,15 +81,10 @@ def dequantize(permuted_alphabet: torch.Tensor, quantized: torch.Tensor) -> torc
     if not quantized.is_cuda:
         raise RuntimeError("dequantize runs on the CUDA kernels: pass CUDA tensors")
     single = quantized.dim() == 1
-    q = quantized[None, :] if single else quantized
-    rows, length = q.shape
-    L = permuted_alphabet.shape[0].bit_length() - 1
-    pad_rows = -(-rows // 32) * 32
-    words = pack_symbols(q, 2)
-    if pad_rows != rows:
-        words = torch.cat([words, words.new_zeros((pad_rows - rows, words.shape[1]))])
-    n = words.shape[1] * 16
-    out = ops.decompress(words.contiguous(), permuted_alphabet.to(device=q.device, dtype=torch.float16).contiguous(), pad_rows, n,
-                         Format(CODE_LUT, 2, L, 0, LAYOUT_ROWMAJOR))
-    out = out[:rows, :length].to(permuted_alphabet.dtype)
+    q = (quantized[None, :] if single else quantized).to(torch.int32).contiguous()
+    # fp32 alphabets are rounded to fp16 on the way into the kernel's table; other types here
+    alphabet = permuted_alphabet.to(q.device).contiguous()
+    if alphabet.dtype != torch.float32:
+        alphabet = alphabet.to(torch.float16)
+    out = ops.dequantize(alphabet, q).to(permuted_alphabet.dtype)
     return out[0] if single else out

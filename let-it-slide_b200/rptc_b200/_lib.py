@@ -154,6 +154,15 @@ _SIGS = {
     "rptc_viterbi_encode_banked": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                                   ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.c_void_p, ctypes.c_int64,
                                                   ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]),
+    "rptc_dequantize": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64,
+                                       ctypes.c_int, ctypes.c_void_p]),
+    "rptc_pack_symbols": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int,
+                                         ctypes.c_void_p]),
+    "rptc_gemv_timed": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
+                                       ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.POINTER(Format), ctypes.POINTER(ctypes.c_float),
+                                       ctypes.c_void_p]),
+    "rptc_timer_begin": (ctypes.c_int, [ctypes.c_void_p]),
+    "rptc_timer_end": (ctypes.c_int, [ctypes.POINTER(ctypes.c_float), ctypes.c_void_p]),
     "rptc_linear_workspace_bytes": (ctypes.c_int64, [ctypes.POINTER(Linear), ctypes.c_int64]),
     "rptc_linear_forward": (ctypes.c_int, [ctypes.POINTER(Linear), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
                                            ctypes.c_int64, ctypes.c_void_p]),

@@ -78,6 +78,30 @@ def decompress(codes: torch.Tensor, lut: torch.Tensor, m: int, n: int, fmt: Form
     return out
 
 
+def dequantize(alphabet: torch.Tensor, symbols: torch.Tensor) -> torch.Tensor:
+    """2-bit symbols int32 [rows, length] -> alphabet[state], rounded to fp16, in the alphabet's dtype (fp16 or fp32)
+    (rptc_dequantize)."""
+    _cuda_contig(alphabet, "alphabet")
+    _cuda_contig(symbols, "symbols", torch.int32)
+    if alphabet.dtype not in (torch.float16, torch.float32):
+        raise RuntimeError("alphabet must be fp16 or fp32")
+    rows, length = symbols.shape
+    out = torch.empty((rows, length), dtype=alphabet.dtype, device=symbols.device)
+    if out.numel():
+        call("rptc_dequantize", symbols.device, alphabet.data_ptr(), symbols.data_ptr(), out.data_ptr(), int(alphabet.dtype == torch.float32), rows,
+             length, alphabet.numel().bit_length() - 1)
+    return out
+
+
+def pack_symbols(symbols: torch.Tensor, bits: int, row_words: int) -> torch.Tensor:
+    """Symbols int32 [rows, length] -> ROWMAJOR words int32 [rows, row_words], first symbol on top (rptc_pack_symbols)."""
+    _cuda_contig(symbols, "symbols", torch.int32)
+    rows, length = symbols.shape
+    words = torch.empty((rows, row_words), dtype=torch.int32, device=symbols.device)
+    call("rptc_pack_symbols", symbols.device, ptr(symbols), ptr(words), rows, length, row_words, bits)
+    return words
+
+
 def gemv_acc(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, acc: torch.Tensor, m: int, n: int, fmt: Format,
              x_order: int = XORDER_NATURAL, carry_in: torch.Tensor | None = None) -> None:
     """acc[b, :m] += W x[b]  (fp32 accumulator; rptc_gemv).  x: fp16 [b, n] or [n]."""

@@ -19,10 +19,13 @@ instead of the reference's kernels.  Differences, all deliberate:
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from rptc_b200 import (CODE_HASH, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_UNITMAJOR, QUIRK_K1_LANE0_SEED,
                        QUIRK_K2_LANE0_CARRY, QUIRK_NONE, XORDER_K2_LEGACY, XORDER_NATURAL, Format, ops)
+from rptc_b200._lib import call
 
 _quirks = False
 _scratch: dict[tuple[int, int, int], torch.Tensor] = {}
@@ -49,7 +52,7 @@ def _check(t: torch.Tensor, name: str, dtype: torch.dtype, dim: int | None = Non
 def _acc(device: torch.device, m: int) -> torch.Tensor:
     """fp32 accumulator of the fused matvecs, one per (device, stream, m): calls on different streams share nothing, like
     the reference's functions, which write `out` directly (inference.cu:335-342)."""
-    key = (device.index or 0, torch.cuda.current_stream(device).cuda_stream, m)
+    key = (device.index, torch._C._cuda_getCurrentRawStream(device.index), m)
     buf = _scratch.get(key)
     if buf is None:
         buf = torch.zeros((1, m), dtype=torch.float32, device=device)
@@ -57,13 +60,25 @@ def _acc(device: torch.device, m: int) -> torch.Tensor:
     return buf
 
 
-def _timed(fn) -> float:
-    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    start.record()
+def _timed(device: torch.device, fn) -> float:
+    ms = ctypes.c_float()
+    call("rptc_timer_begin", device)
     fn()
-    stop.record()
-    stop.synchronize()
-    return start.elapsed_time(stop)
+    call("rptc_timer_end", device, ms)
+    return ms.value
+
+
+def _timed_matvec(compressed, codebook, x, out, m: int, n: int, fmt: Format, x_order: int, accumulate: bool) -> float:
+    """out = (or +=) W x and the device time it took, in one native call."""
+    device, ms = out.device, ctypes.c_float()
+    acc = _acc(device, m)
+    try:
+        call("rptc_gemv_timed", device, compressed.data_ptr(), codebook.data_ptr(), x.data_ptr(), acc.data_ptr(), out.data_ptr(), m, n, x_order,
+             int(accumulate), fmt, ms)
+    except Exception:
+        _scratch.clear()      # an accumulator that was not finished is not zero
+        raise
+    return ms.value
 
 
 def matvec(decompressed: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> float:
@@ -74,7 +89,7 @@ def matvec(decompressed: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> fl
     _check(out, "out", torch.float16, 1)
     if decompressed.shape[1] != x.shape[0] or decompressed.shape[0] != out.shape[0]:
         raise RuntimeError("shapes of decompressed [m, n], x [n] and out [m] do not agree")
-    return _timed(lambda: ops.dense_gemv(decompressed, x, out=out))
+    return _timed(out.device, lambda: ops.dense_gemv(decompressed, x, out=out))
 
 
 _ones: dict[tuple[int, int], torch.Tensor] = {}
@@ -87,7 +102,7 @@ def rowsum(decompressed: torch.Tensor, out: torch.Tensor) -> float:
     key = (decompressed.device.index or 0, decompressed.shape[1])
     if key not in _ones:
         _ones[key] = torch.ones(decompressed.shape[1], dtype=torch.float16, device=decompressed.device)
-    return _timed(lambda: ops.dense_gemv(decompressed, _ones[key], out=out))
+    return _timed(out.device, lambda: ops.dense_gemv(decompressed, _ones[key], out=out))
 
 
 def decompress(compressed: torch.Tensor, codebook: torch.Tensor, out: torch.Tensor) -> float:
@@ -104,7 +119,7 @@ def decompress(compressed: torch.Tensor, codebook: torch.Tensor, out: torch.Tens
     if tuple(out.shape) != (m, n):
         raise RuntimeError("out must be [m, n]")
     fmt = Format(CODE_LUT, 2, 16, 0, LAYOUT_ROWMAJOR, QUIRK_K1_LANE0_SEED if _quirks else QUIRK_NONE)
-    return _timed(lambda: ops.decompress(compressed, codebook, m, n, fmt, out=out))
+    return _timed(out.device, lambda: ops.decompress(compressed, codebook, m, n, fmt, out=out))
 
 
 def _decompress_matvec(S: int, compressed, codebook, x, out) -> float:
@@ -126,14 +141,7 @@ def _decompress_matvec(S: int, compressed, codebook, x, out) -> float:
     if m % 32:
         raise RuntimeError("m must be a multiple of 32")
     fmt = Format(CODE_HASH, 2, 16, S, LAYOUT_CHUNKED, QUIRK_K2_LANE0_CARRY if _quirks else QUIRK_NONE)
-    acc = _acc(out.device, m)
-
-    def run():
-        acc.zero_()
-        ops.gemv_acc(compressed, codebook, x, acc, m, n, fmt, XORDER_K2_LEGACY)
-        ops.gemv_finish(acc, out, m, clear=True)
-
-    return _timed(run)
+    return _timed_matvec(compressed, codebook, x, out, m, n, fmt, XORDER_K2_LEGACY, False)
 
 
 def decompress_matvec_16_6_1(compressed, codebook, x, out) -> float:
@@ -167,14 +175,7 @@ def _decompress_matvec_t(L: int, compressed, codebook, x, out) -> float:
     if compressed.numel() != m * n // 16:
         raise RuntimeError("compressed must hold m*n/16 words")
     fmt = Format(CODE_LUT, 2, L, 0, LAYOUT_UNITMAJOR, QUIRK_NONE)
-    acc = _acc(out.device, m)
-
-    def run():
-        acc.zero_()
-        ops.gemv_acc(compressed, codebook, x, acc, m, n, fmt, XORDER_NATURAL)
-        ops.gemv_finish(acc, out, m, accumulate=True, clear=True)
-
-    return _timed(run)
+    return _timed_matvec(compressed, codebook, x, out, m, n, fmt, XORDER_NATURAL, True)
 
 
 def decompress_matvec_t_16(compressed, codebook, x, out) -> float:

@@ -85,3 +85,20 @@ def test_config0_quantize_pack_decompress_matvec():
     y = ops.gemv(codes, alphabet.half(), x, m, n, fmt).float()
     ref = x.float() @ recon.t()
     assert (y - ref).abs().max() <= 2e-3 * recon.norm(dim=1).max() * x.float().norm() + 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.float64])
+@pytest.mark.parametrize("rows,length,L", [(1, 1, 4), (3, 7, 8), (2, 256, 16), (5, 1001, 11), (1, 8193, 16), (4096, 700, 16), (2500, 1027, 14)])
+def test_dequantize_over_pieces_and_tails(rows, length, L, dtype):
+    """Rows that are and are not whole pieces of 256 symbols, aligned or not, through L2 and through the table."""
+    import rptc
+    g = torch.Generator(device="cuda").manual_seed(rows + length)
+    alphabet = torch.randn(1 << L, generator=g, device="cuda", dtype=torch.float64).to(dtype)
+    sym = torch.randint(0, 4, (rows, length), generator=g, device="cuda", dtype=torch.int32)
+    got = rptc.dequantize(alphabet, sym)
+    states = torch.zeros((rows, length), dtype=torch.int64, device="cuda")
+    for back in range((L + 1) // 2):                        # the symbols that the state's L bits come from
+        states[:, back:] |= sym[:, : length - back].long() << (2 * back)
+    assert got.dtype == dtype and torch.equal(got, alphabet.half().to(dtype)[states & ((1 << L) - 1)])
+    assert torch.equal(rptc.pack_symbols(sym, 2).cpu(), rptc.pack_symbols(sym.cpu(), 2))
