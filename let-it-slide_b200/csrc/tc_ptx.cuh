@@ -7,8 +7,9 @@
 
 namespace rptc {
 
-// fp16 [rows][cols] with `ld` elements between rows, in 128-byte-swizzled boxes of 64 columns x `box_rows` rows.
-int encode_map(CUtensorMap &map, const void *base, int64_t cols, int64_t rows, int64_t ld, int box_rows);      // gemm_tcgen05.cu
+// fp16 [rows][cols] with `ld` elements between rows, in boxes of `box_cols` columns (64: 128-byte swizzle, 32: 64-byte) x
+// `box_rows` rows.                                                                                     gemm_tcgen05.cu
+int encode_map(CUtensorMap &map, const void *base, int64_t cols, int64_t rows, int64_t ld, int box_rows, int box_cols = 64);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
