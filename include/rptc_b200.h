@@ -274,6 +274,17 @@ int rptc_rope_cache(void *qkv, int64_t ld_qkv, const int32_t *pos, void *kcache,
  * cache positions 0 .. tokens-1. */
 int rptc_rope_cache_prompt(void *qkv, int64_t ld_qkv, int64_t rows, int64_t tokens, void *kcache, void *vcache, int hq, int hkv,
                            int d, int max_pos, float theta, rptc_stream_t stream);
+/* The glue of a prompt's forward pass around the matrix products (fp16 products in, before their output transform).
+ * rptc_prompt_norm: h += s_out * H(y) * scale_out (y NULL: h as it is); out = H(s_in * rmsnorm(h) * w_norm), rows of n =
+ * 4096 or 8192 in Hadamard blocks of 4096; h in place.
+ * rptc_prompt_qkv: qkv fp16 [rows * tokens][ld] = [q | k | v heads of 128], y = s_out * H(qkv) * scale in blocks of 128; q rotated in
+ * place, rotated k and v to cache positions 0 .. tokens-1.  angles: fp32 [tokens][64][2], cosines and sines
+ * (rptc_rope_angles). */
+int rptc_prompt_norm(const void *y, int64_t ld_y, const void *signs_out, float scale_out, void *h, int64_t ld_h, const void *w_norm,
+                     float eps, const void *signs_in, void *out, int64_t ld_out, int64_t rows, int64_t n, rptc_stream_t stream);
+int rptc_prompt_qkv(void *qkv, int64_t ld, const void *signs_out, float scale, int64_t rows, int64_t tokens, void *kcache, void *vcache,
+                    int hq, int hkv, int max_pos, const void *angles, rptc_stream_t stream);
+int rptc_rope_angles(void *angles, int64_t tokens, float theta, rptc_stream_t stream);
 /* Single-query attention of each row's q heads over cache positions [0, pos[row]]; d must be 128.
  * qkv, kcache and vcache must be 16-byte aligned and ld_qkv a multiple of 8 (rows are read 16 bytes at a time).
  * signs_in (fp16 [hq*128] or NULL): when given, each head's output is also put through the input-side

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(64) rope_cache_kernel(__half *__restrict__ qkv
 __global__ void __launch_bounds__(256) rope_cache_prompt_kernel(__half *__restrict__ qkv, int64_t ld_qkv, __half *__restrict__ kcache,
                                                                __half *__restrict__ vcache, int hq, int hkv, int d, int max_pos,
                                                                RopeFreq freq) {
+    pdl_wait_prior_grids();
     const int p = blockIdx.x, row = blockIdx.y, T = gridDim.x;
     const int half_d = d / 2, i = threadIdx.x % 64, grp = threadIdx.x / 64;      // pair index, head group (4 groups)
     if (i >= half_d) return;

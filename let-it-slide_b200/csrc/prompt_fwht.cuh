@@ -1,0 +1,118 @@
+// Walsh-Hadamard building blocks for many rows (prompts): 32 values per thread, two exchanges through shared memory.
+//
+// A segment is 1024 columns for a warp (blocks of at most 256) or 4096 for a CTA of 128 threads (any block up to 4096); it
+// may hold several blocks.  Element e of a segment is at e + 8 (e >> 8) in the exchange buffer, which keeps all accesses
+// below free of bank conflicts.  Three layouts of a thread's 32 values, by the bits of e that vary inside the thread:
+//   rows     bits 0-2 and two more (warp: 8, 9; CTA: 8, 9 or 10, 11): four pieces of eight consecutive elements, loaded and
+//            stored as 16 bytes of fp16 each
+//   columns  bits 3-7
+// A transform does the stages of its own bits in each layout, in any order; stages at or above the block size are skipped.
+// Against eight values per thread with shuffles (five stages x eight values through the same pipe as shared memory) this
+// moves 2048 x 4096 in 8 us instead of 24.
+#pragma once
+#include "common.cuh"
+#include "fwht.cuh"
+
+namespace rptc {
+
+constexpr int kWarpSegFloats = 1024 + 32, kCtaSegFloats = 4096 + 128;
+
+// One butterfly stage over bit `H` of the index of v.
+template <int H>
+__device__ __forceinline__ void stage(float (&v)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        if ((i & H) == 0) {
+            const float a = v[i], b = v[i + H];
+            v[i] = a + b;
+            v[i + H] = a - b;
+        }
+}
+
+// v[8 j + i] is element i of piece j: the stages of bits 0-2, and of the two bits that number the pieces (`lo` and `lo + 1`).
+__device__ __forceinline__ void row_stages(float (&v)[32], int block_bits, int lo) {
+    if (block_bits > 0) stage<1>(v);
+    if (block_bits > 1) stage<2>(v);
+    if (block_bits > 2) stage<4>(v);
+    if (block_bits > lo) stage<8>(v);
+    if (block_bits > lo + 1) stage<16>(v);
+}
+// v[k] is element bits 3-7 = k.
+__device__ __forceinline__ void column_stages(float (&v)[32], int block_bits) {
+    if (block_bits > 3) stage<1>(v);
+    if (block_bits > 4) stage<2>(v);
+    if (block_bits > 5) stage<4>(v);
+    if (block_bits > 6) stage<8>(v);
+    if (block_bits > 7) stage<16>(v);
+}
+
+// Where a thread's pieces and columns are.  WARP segments: pieces at 8 lane + 256 j.  CTA segments (t of 128 threads): with
+// `far` pieces at 8 t + 1024 j (bits 10, 11 vary), else at 8 lane + 1024 warp + 256 j (bits 8, 9 vary).
+template <bool CTA>
+struct SegThread {
+    int lane, warp, t;
+    __device__ __forceinline__ SegThread() : lane(threadIdx.x & 31), warp(CTA ? (threadIdx.x >> 5) & 3 : 0), t(threadIdx.x & 127) {}
+    __device__ __forceinline__ int piece(int j, bool far) const {
+        if (!CTA) return 8 * lane + 256 * j;
+        return far ? 8 * t + 1024 * j : 8 * lane + 1024 * warp + 256 * j;
+    }
+    __device__ __forceinline__ int column() const {      // element of k = 0: bits 0-2 from the lane, bits 8 up from the rest
+        return (lane & 7) + 256 * ((lane >> 3) + 4 * warp);
+    }
+    static __device__ __forceinline__ int at(int e) { return e + 8 * (e >> 8); }
+    static __device__ __forceinline__ void sync() {
+        if (CTA) __syncthreads();
+        else __syncwarp();
+    }
+    // The two halves of a piece as 16-byte accesses; lanes with bit 2 set take the upper half first, so that eight lanes
+    // with a stride of 32 bytes meet all banks once.
+    __device__ __forceinline__ void put_pieces(float *buf, const float (&v)[32], bool far) const {
+        const bool swap = lane & 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 *p = reinterpret_cast<float4 *>(buf + at(piece(j, far)));
+            const float4 a = make_float4(v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]);
+            const float4 b = make_float4(v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
+            p[swap ? 1 : 0] = swap ? b : a;
+            p[swap ? 0 : 1] = swap ? a : b;
+        }
+    }
+    __device__ __forceinline__ void get_pieces(const float *buf, float (&v)[32], bool far) const {
+        const bool swap = lane & 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 *p = reinterpret_cast<const float4 *>(buf + at(piece(j, far)));
+            const float4 x = p[swap ? 1 : 0], y = p[swap ? 0 : 1];
+            const float4 a = swap ? y : x, b = swap ? x : y;
+            v[8 * j] = a.x, v[8 * j + 1] = a.y, v[8 * j + 2] = a.z, v[8 * j + 3] = a.w;
+            v[8 * j + 4] = b.x, v[8 * j + 5] = b.y, v[8 * j + 6] = b.z, v[8 * j + 7] = b.w;
+        }
+    }
+    __device__ __forceinline__ void put_columns(float *buf, const float (&v)[32]) const {
+        float *p = buf + at(column());
+#pragma unroll
+        for (int k = 0; k < 32; ++k) p[8 * k] = v[k];
+    }
+    __device__ __forceinline__ void get_columns(const float *buf, float (&v)[32]) const {
+        const float *p = buf + at(column());
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = p[8 * k];
+    }
+};
+
+__device__ __forceinline__ void unpack8_at(const uint4 &a, float *v) {
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(u32_as_half2(w[i]));
+        v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ uint4 pack8_from(const float *v) {
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = half2_as_u32(__floats2half2_rn(v[2 * i], v[2 * i + 1]));
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+}  // namespace rptc

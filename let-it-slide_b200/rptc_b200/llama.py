@@ -526,7 +526,6 @@ class RPTCLlama:
         if R != self.rows or T > cfg.max_pos:
             raise ValueError("tokens must be [rows, T] with T <= max_pos")
         D = cfg.head_dim
-        q_dim = self.heads_l * D
         h = self.embed[tokens.long()].reshape(R * T, cfg.hidden)                     # fp16 residual stream
 
         def reduce(y):
@@ -535,38 +534,77 @@ class RPTCLlama:
                 dist.all_reduce(y, group=self.tp_group)
             return y
 
-        xn = torch.empty_like(h)
-        for i, b in enumerate(self.blocks):
-            ops.rmsnorm(h, b.norm1, xn, cfg.rms_eps)
-            qkv = b.qkv(xn)
-            ops.rope_cache_prompt(qkv, R, T, self.kcache[i], self.vcache[i], self.heads_l, self.kv_heads_l, D, cfg.rope_theta)
-            q = qkv[:, :q_dim].reshape(R, T, self.heads_l, D)                        # rotated in place
-            k, v = self.kcache[i][:, :T], self.vcache[i][:, :T]
-            att = torch.nn.functional.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2),
-                                                                   is_causal=True, enable_gqa=self.heads_l != self.kv_heads_l)
-            att = att.transpose(1, 2).reshape(R * T, q_dim)
-            fused = b.o.incoherent and R * T > 8 and self.tp_world == 1       # residual and SwiGLU inside the glue kernels
-            if fused:
-                h = b.o.finish_t(b.o.product_t(b.o.transform_in(att)), residual=h)
-            else:
-                h = h + reduce(b.o(att))
-            ops.rmsnorm(h, b.norm2, xn, cfg.rms_eps)
-            if fused:
-                gu = b.gate_up.product_t(b.gate_up.transform_in(xn))                  # before gate-up's output transform
-                mlp_t = ops.swiglu_hadamard_f16(gu, torch.empty((R * T, self.ffn_l), dtype=torch.float16, device=self.device),
-                                                b.gate_up.signs_out, b.down.signs_in, self.ffn_l, b.down.block_in, b.gate_up.scale)
-                h = b.down.finish_t(b.down.product_t(mlp_t), residual=h)
-            else:
+        b0 = self.blocks[0]
+        fused = b0.o.incoherent and R * T > 8 and self.tp_world == 1              # residuals, rotation and SwiGLU inside the glue kernels
+        last = None
+        if fused:
+            lib().rptc_set_pdl(1)
+            try:
+                last = self._prefill_blocks_fused(h, R, T)
+            finally:
+                lib().rptc_set_pdl(0)
+        else:
+            xn = torch.empty_like(h)
+            for i, b in enumerate(self.blocks):
+                ops.rmsnorm(h, b.norm1, xn, cfg.rms_eps)
+                qkv = b.qkv(xn)
+                ops.rope_cache_prompt(qkv, R, T, self.kcache[i], self.vcache[i], self.heads_l, self.kv_heads_l, D, cfg.rope_theta)
+                h = h + reduce(b.o(self._prompt_attention(qkv, i, R, T)))
+                ops.rmsnorm(h, b.norm2, xn, cfg.rms_eps)
                 gu = b.gate_up(xn)
                 mlp = torch.nn.functional.silu(gu[:, : self.ffn_l]).mul_(gu[:, self.ffn_l:])      # fp32 inside, fp16 in and out
                 h = h + reduce(b.down(mlp))
-        last = h.reshape(R, T, cfg.hidden)[:, -1].contiguous()
+            last = h.reshape(R, T, cfg.hidden)[:, -1].contiguous()
         ops.rmsnorm(last, self.norm_f, self.xn, cfg.rms_eps)
         ops.dense_gemv(self.head, self.xn, out=self.logits)
         self.pos.fill_(T - 1)
         self._pos_hi = T
         ops.next_token(self.logits, self.next_ids, self.ids, self.pos, None)        # pos -> T, ids -> greedy choice
         return self.logits
+
+    def _prompt_attention(self, qkv: torch.Tensor, i: int, R: int, T: int) -> torch.Tensor:
+        """Causal attention of a prompt whose rotated q sit in the first columns of qkv and whose k and v are in the caches."""
+        D, q_dim = self.cfg.head_dim, self.heads_l * self.cfg.head_dim
+        q = qkv[:, :q_dim].view(R, T, self.heads_l, D)
+        k, v = self.kcache[i][:, :T], self.vcache[i][:, :T]
+        att = torch.nn.functional.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2),
+                                                               is_causal=True, enable_gqa=self.heads_l != self.kv_heads_l)
+        return att.transpose(1, 2).reshape(R * T, q_dim)
+
+    def _prefill_blocks_fused(self, h: torch.Tensor, R: int, T: int) -> torch.Tensor:
+        """The blocks over a prompt's residual stream h [R * T, hidden] (updated in place), with everything between two
+        matrix products in one kernel each; returns the residual stream of every row's last position."""
+        cfg = self.cfg
+        heads_of_128 = cfg.head_dim == 128 and self.blocks[0].qkv.block_out == 128
+        whole_rows = cfg.hidden in (4096, 8192)                      # the norm kernel's rows: one or two 4096-point blocks
+        xt, mlp = torch.empty_like(h), torch.empty((R * T, self.ffn_l), dtype=torch.float16, device=h.device)
+        angles = ops.rope_angles(T, cfg.rope_theta, h.device) if heads_of_128 else None
+        y, prev = None, None                                         # product whose output side is still to be added to h, its layer
+
+        def norm_into(w_norm, lin):
+            if whole_rows:
+                ops.prompt_norm(y, prev.signs_out if prev else None, prev.scale if prev else 1.0, h, w_norm, cfg.rms_eps, lin.signs_in, xt)
+                return xt
+            if prev is not None:
+                ops.hadamard(y, prev.signs_out, prev.block_out, transpose=True, scale=prev.scale, residual=h, out=h)
+            ops.rmsnorm(h, w_norm, xt, cfg.rms_eps)
+            return lin.transform_in(xt, out=xt)
+
+        for i, b in enumerate(self.blocks):
+            qkv = b.qkv.product_t(norm_into(b.norm1, b.qkv))
+            if heads_of_128:
+                ops.prompt_qkv(qkv, b.qkv.signs_out, b.qkv.scale, R, T, self.kcache[i], self.vcache[i], self.heads_l, self.kv_heads_l, angles)
+            else:
+                qkv = b.qkv.finish_t(qkv)
+                ops.rope_cache_prompt(qkv, R, T, self.kcache[i], self.vcache[i], self.heads_l, self.kv_heads_l, cfg.head_dim, cfg.rope_theta)
+            att = self._prompt_attention(qkv, i, R, T)
+            y, prev = b.o.product_t(b.o.transform_in(att, out=att)), b.o
+            gu = b.gate_up.product_t(norm_into(b.norm2, b.gate_up))
+            ops.swiglu_hadamard_f16(gu, mlp, b.gate_up.signs_out, b.down.signs_in, self.ffn_l, b.down.block_in, b.gate_up.scale)
+            y, prev = b.down.product_t(mlp), b.down
+        # only the last position of each row is read on
+        pick = lambda t: t.view(R, T, -1)[:, -1].contiguous()
+        return prev.finish_t(pick(y), residual=pick(h))
 
     def reference_logits(self, tokens: torch.Tensor, act_dtype: torch.dtype | None = None) -> torch.Tensor:
         """fp32 torch forward of the same network on `tokens` [rows, T] -> logits [rows, T, vocab].

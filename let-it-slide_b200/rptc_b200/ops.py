@@ -242,6 +242,29 @@ def rope_cache_prompt(qkv: torch.Tensor, rows: int, tokens: int, kcache: torch.T
          kcache.shape[1], theta)
 
 
+def rope_angles(tokens: int, theta: float, device) -> torch.Tensor:
+    """Cosines and sines of positions 0 .. tokens-1 for 128-wide heads, fp32 [tokens, 64, 2] (rptc_rope_angles)."""
+    out = torch.empty((tokens, 64, 2), dtype=torch.float32, device=device)
+    call("rptc_rope_angles", out.device, ptr(out), tokens, theta)
+    return out
+
+
+def prompt_norm(y: torch.Tensor | None, signs_out: torch.Tensor | None, scale_out: float, h: torch.Tensor, w_norm: torch.Tensor, eps: float,
+                signs_in: torch.Tensor | None, out: torch.Tensor) -> torch.Tensor:
+    """h += output transform of the product y; out = input transform of rmsnorm(h), many rows (rptc_prompt_norm)."""
+    rows, n = h.shape
+    call("rptc_prompt_norm", h.device, ptr(y), 0 if y is None else _ld(y, n), ptr(signs_out), scale_out, ptr(h), _ld(h, n), ptr(w_norm), eps,
+         ptr(signs_in), ptr(out), _ld(out, n), rows, n)
+    return out
+
+
+def prompt_qkv(qkv: torch.Tensor, signs_out: torch.Tensor | None, scale: float, rows: int, tokens: int, kcache: torch.Tensor,
+               vcache: torch.Tensor, hq: int, hkv: int, angles: torch.Tensor) -> None:
+    """Output transform of the fused qkv product + RoPE + cache writes for a whole prompt (rptc_prompt_qkv)."""
+    call("rptc_prompt_qkv", qkv.device, ptr(qkv), _ld(qkv, qkv.shape[1]), ptr(signs_out), scale, rows, tokens, ptr(kcache), ptr(vcache), hq, hkv,
+         kcache.shape[1], ptr(angles))
+
+
 def attn_decode(qkv: torch.Tensor, pos: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, out: torch.Tensor, hq: int,
                 hkv: int, d: int, signs_in: torch.Tensor | None = None) -> torch.Tensor:
     rows = qkv.shape[0]
