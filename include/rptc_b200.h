@@ -202,6 +202,11 @@ int rptc_gemv_f16_static(const void *codes, const void *lut, const uint32_t *car
 int rptc_gemm(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y,
               int64_t ld_y, int64_t m, int64_t n, int64_t tokens, const rptc_format *fmt, rptc_stream_t stream);
 
+/* The same with every sum taken as one chain along the reduction: a token's result is the same bits whatever the number of
+ * tokens in the call (rptc_gemm shares the reduction among several CTAs where there are few tiles). */
+int rptc_gemm_invariant(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y,
+                        int64_t ld_y, int64_t m, int64_t n, int64_t tokens, const rptc_format *fmt, rptc_stream_t stream);
+
 /* Block-diagonal randomized Hadamard transform along rows of length n (block = power of two <= 4096
  * dividing n).  No reference counterpart (incoherence processing is an extension of this build).
  *   in_is_f32 = 0: in is fp16 [rows][ld_in];  1: in is fp32 (e.g. the rptc_gemv accumulator).
@@ -312,7 +317,7 @@ int rptc_finish_norm_hadamard(float *acc, int64_t ld_acc, const void *signs_out,
 int rptc_qkv_finish(float *acc, int64_t ld_acc, const void *signs_out, float scale, void *q_out, int64_t ld_q, void *kcache,
                     void *vcache, const int32_t *pos, int64_t rows, int hq, int hkv, int max_pos, int block, float theta,
                     rptc_stream_t stream);
-/* Dense fp16 matvec y[b] = W x[b] (fp32 accumulation), batch 1..8: the output head, and the dense-bandwidth
+/* Dense fp16 matvec y[b] = W x[b] (fp32 accumulation), batch 1..16: the output head, and the dense-bandwidth
  * probe the reference's tests call `matvec` (rptc_kernels/tests/test_matvec.py:18, not exported by wrapper.cpp). */
 int rptc_dense_gemv(const void *W, int64_t ld_w, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m, int64_t n,
                     int batch, rptc_stream_t stream);

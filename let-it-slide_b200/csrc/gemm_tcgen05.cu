@@ -586,7 +586,7 @@ static int64_t cluster_places(int split) {
 // tile feeds the tensor pipe about 1.35 times faster per weight row, but there are half as many of it; sharing a tile's
 // reduction over two or four CTAs fills SMs that would be idle (4096 rows x 512 tokens are 32 wide tiles for 148 SMs)
 // at the price of the exchange.  A CTA keeps at least eight steps.
-static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, int32_t banks, const rptc_format &f) {
+static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     GemmShape best = {0, 0, 0};
     double best_us = 0;
     const int64_t steps = n / kStepCols;
@@ -594,8 +594,8 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, int32_t bank
         for (int halves = tokens > 128 ? 2 : 1; halves >= 1; --halves) {
             GemmParams probe;
             if (!plan_gemm(probe, {rows, halves, 1}, f)) continue;
-            const int64_t tiles = banks * ((m + rows - 1) / rows) * ((tokens + halves * 128 - 1) / (halves * 128));
-            for (int split = 1; split <= rows / 64 && (split == 1 || steps >= 8 * split); split *= 2) {
+            const int64_t tiles = banks.banks * ((m + rows - 1) / rows) * ((tokens + halves * 128 - 1) / (halves * 128));
+            for (int split = 1; split <= (banks.may_split ? rows / 64 : 1) && (split == 1 || steps >= 8 * split); split *= 2) {
                 const int64_t places = cluster_places(split);
                 const int64_t waves = (tiles + places - 1) / places;
                 const double us = waves * ((double)((steps + split - 1) / split) * step_us(rows, halves, f.code) + around_us(rows, halves, split));
@@ -606,14 +606,14 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, int32_t bank
     return best;
 }
 
-int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, int32_t banks, const rptc_format &f) {
+int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     const GemmShape g = choose_shape(m, n, tokens, banks, f);
     return g.rows ? (m + g.rows - 1) / g.rows * g.rows : 0;
 }
 
 int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
                 int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s) {
-    const GemmShape g = choose_shape(m, n, tokens, banks.banks, f);
+    const GemmShape g = choose_shape(m, n, tokens, banks, f);
     GemmParams p;
     if (!g.rows || !plan_gemm(p, g, f)) return RPTC_ERR_UNSUPPORTED;
     p.tiles_per_bank = (int32_t)((m + g.rows - 1) / g.rows);
@@ -654,8 +654,8 @@ int check_format(const rptc_format *f);   // api.cu
 
 using namespace rptc;
 
-extern "C" int rptc_gemm(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y,
-                         int64_t ld_y, int64_t m, int64_t n, int64_t tokens, const rptc_format *fmt, rptc_stream_t stream) {
+static int gemm_checked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
+                        int64_t n, int64_t tokens, const Banks &banks, const rptc_format *fmt, rptc_stream_t stream) {
     if (!codes || !lut || !x || !y || !fmt) return RPTC_ERR_ARG;
     if (int e = check_format(fmt)) return e;
     if (fmt->layout != RPTC_LAYOUT_TILED || fmt->quirk != RPTC_QUIRK_NONE) return RPTC_ERR_UNSUPPORTED;
@@ -666,5 +666,17 @@ extern "C" int rptc_gemm(const void *codes, const void *lut, const uint32_t *car
         (reinterpret_cast<uintptr_t>(y) & 15) || (ld_x % 8) || (ld_y % 8))
         return RPTC_ERR_ALIGN;
     if (int e = rptc_check_device()) return e;
-    return gemm_banked(codes, lut, carry_in, x, ld_x, y, ld_y, m, n, tokens, Banks(), *fmt, static_cast<cudaStream_t>(stream));
+    return gemm_banked(codes, lut, carry_in, x, ld_x, y, ld_y, m, n, tokens, banks, *fmt, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int rptc_gemm(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y,
+                         int64_t ld_y, int64_t m, int64_t n, int64_t tokens, const rptc_format *fmt, rptc_stream_t stream) {
+    return gemm_checked(codes, lut, carry_in, x, ld_x, y, ld_y, m, n, tokens, Banks(), fmt, stream);
+}
+
+extern "C" int rptc_gemm_invariant(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y,
+                                   int64_t ld_y, int64_t m, int64_t n, int64_t tokens, const rptc_format *fmt, rptc_stream_t stream) {
+    Banks banks;
+    banks.may_split = false;
+    return gemm_checked(codes, lut, carry_in, x, ld_x, y, ld_y, m, n, tokens, banks, fmt, stream);
 }

@@ -69,13 +69,6 @@ __device__ __forceinline__ int64_t k2_legacy_pair(int64_t s, int64_t n) {
     return 4 * (p % q8) + p / q8;
 }
 
-// D += A B on one 16 x 8 x 16 tile: fp16 operands, fp32 accumulation.
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // The general kernel: any layout (strided 128-bit loads straight from memory, one unit of one row block per
 // step), the reference kernels' lane-0 deviations, batch 1.  The native TILED layout takes the two kernels below.
 template <int CODE, int K>

@@ -157,11 +157,11 @@ namespace rptc {
 int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int64_t ld_out, const __half *signs, const __half *residual,
                   int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
                   cudaStream_t stream);
-int swiglu_rows(const void *gate_up, int64_t ld_in, void *out, int64_t ld_out, const void *signs_out, const void *signs_in, int64_t rows, int64_t n,
-                int block, float scale_out, float scale_in, cudaStream_t stream);
-// From this many rows on the kernels that walk down the rows are used; fewer leave most of an SM idle and the kernels with
-// eight values per thread, which have four times the warps, finish first.
-constexpr int64_t kManyRows = 32;
+// Which inputs go to the kernels that walk down the rows.  Blocks above 256 columns: from 32 rows on (2048 x 4096: 13.4 us
+// against 19.3; up to 128 rows both take 3.3).  Smaller blocks need no barrier in the kernels with eight values per thread,
+// which have more warps in flight: those stay ahead until the memory traffic is what counts (512 x 11008: 8.8 us against
+// 9.6; 2048 x 12288: 31.5 against 27.1).
+static bool many_rows(int64_t rows, int64_t n, int block) { return block > 256 ? rows >= 32 : rows * n >= (int64_t(8) << 20); }
 
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
@@ -178,7 +178,7 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
         return RPTC_ERR_ALIGN;
     if (clear_in && !in_is_f32) return RPTC_ERR_ARG;
     if (int e = rptc_check_device()) return e;
-    if (rows >= kManyRows)
+    if (many_rows(rows, n, block))
         return hadamard_rows(in, in_is_f32, ld_in, static_cast<__half *>(out), ld_out, static_cast<const __half *>(signs),
                              static_cast<const __half *>(residual), ld_res, rows, n, block, transpose, scale, clear_in, clear, clear_count, stream);
     HadParams p;
@@ -232,8 +232,6 @@ static int swiglu_launch(float *acc, const void *in16, int64_t ld_in, void *out,
         (ld_in % (acc ? 4 : 8)) || (ld_out % 8) || (n % 8))
         return RPTC_ERR_ALIGN;
     if (int e = rptc_check_device()) return e;
-    if (in16 && block <= 256 && rows >= kManyRows)
-        return swiglu_rows(in16, ld_in, out, ld_out, signs_out, signs_in, rows, n, block, scale_out, scale_in, static_cast<cudaStream_t>(stream));
     SwigluParams p;
     p.acc = acc;
     p.in16 = acc ? nullptr : static_cast<const __half *>(in16);

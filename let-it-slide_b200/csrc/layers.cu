@@ -125,7 +125,9 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
 static bool packed_plan(const rptc_packed &l, int64_t tokens, int64_t &cols) {
     const rptc_format f = {RPTC_CODE_LUT, 2, l.L, 0, RPTC_LAYOUT_TILED, RPTC_QUIRK_NONE};
     const bool few = tokens <= kFewMaxTokens;
-    cols = few ? (int64_t)l.bank_blocks * 32 : gemm_bank_columns((int64_t)l.bank_blocks * 32, l.n, tokens, l.banks, f);
+    Banks banks;
+    banks.banks = l.banks;
+    cols = few ? (int64_t)l.bank_blocks * 32 : gemm_bank_columns((int64_t)l.bank_blocks * 32, l.n, tokens, banks, f);
     return few;
 }
 

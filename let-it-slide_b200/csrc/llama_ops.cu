@@ -120,15 +120,19 @@ __global__ void __launch_bounds__(256) rope_cache_prompt_kernel(__half *__restri
     }
 }
 
-// Single-query attention over the cache: one CTA of 512 threads per (row, q head); d == 128.
+// Single-query attention over the cache: one CTA per (row, q head); d == 128.
 // One trip to memory: every warp fetches the K AND V rows of its positions (16 of each in flight, positions
-// interleaved over the 16 warps) before anything that depends on the kernel in front, then keeps a running
-// maximum / sum / weighted V sum of its own (online softmax); the 16 partial states meet in shared memory.
-// Contexts beyond 256 take further chunks of 256 positions through the same registers.
+// interleaved over the warps) before anything that depends on the kernel in front, then keeps a running
+// maximum / sum / weighted V sum of its own (online softmax); the warps' partial states meet in shared memory.
+// Longer contexts take further chunks of positions through the same registers.
 // A warp takes two positions at a time, one per half-warp: lane (half, dl) holds dims 8*dl .. 8*dl+7 of its half's
 // position (one 16-byte load per row and lane, four shuffle stages per pair of scores).
-constexpr int kAttnThreads = 512, kAttnWarps = 16, kAttnUnroll = 8;      // 8 slots x 2 positions x 16 warps = 256 positions in flight
-__global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(const __half *__restrict__ qkv, int64_t ld_qkv,
+// A CTA of 16 warps fills an SM (8 slots x 2 positions x 16 warps = 256 positions in flight).  Where there are more (row,
+// head) pairs than SMs, CTAs of 8 or 4 warps share one instead: 16 rows x 32 heads at context 130 took four waves of 16-warp
+// CTAs (24 us in the decode step) whose warps had two positions each.
+constexpr int kAttnUnroll = 8;
+template <int kAttnWarps>
+__global__ void __launch_bounds__(32 * kAttnWarps, 16 / kAttnWarps) attn_decode_kernel(const __half *__restrict__ qkv, int64_t ld_qkv,
                                                                   const int32_t *__restrict__ pos, const __half *__restrict__ kcache,
                                                                   const __half *__restrict__ vcache, __half *__restrict__ out,
                                                                   int64_t ld_out, int hq, int hkv, int max_pos, float scale,
@@ -356,8 +360,17 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(const __half 
     }
 }
 
-// Dense fp16 matvec  y[b][r] = sum_c W[r][c] x[b][c]  (fp32 accumulation), one warp per row of W, the
-// batch (<= 8) handled inside.  Used for the output head; also the dense-bandwidth probe the
+template <typename... Args>
+static int launch_attn(int heads, int64_t rows, cudaStream_t stream, Args... args) {
+    const dim3 grid((unsigned)heads, (unsigned)rows);
+    const int64_t ctas = heads * rows, sms = num_sms();
+    if (ctas <= sms) return launch(attn_decode_kernel<16>, grid, dim3(512), 0, stream, args...);
+    if (ctas <= 2 * sms) return launch(attn_decode_kernel<8>, grid, dim3(256), 0, stream, args...);
+    return launch(attn_decode_kernel<4>, grid, dim3(128), 0, stream, args...);
+}
+
+// Dense fp16 matvec  y[b][r] = sum_c W[r][c] x[b][c]  (fp32 accumulation), one warp per row of W, one or two
+// activation rows.  Used for the output head; also the dense-bandwidth probe the
 // reference's stale tests call `matvec` (rptc_kernels/tests/test_matvec.py:18).
 template <int BATCH>
 __global__ void __launch_bounds__(256) dense_gemv_kernel(const __half *__restrict__ W, int64_t ld_w, const __half *__restrict__ x,
@@ -390,6 +403,84 @@ __global__ void __launch_bounds__(256) dense_gemv_kernel(const __half *__restric
     for (int b = 0; b < BATCH; ++b) {
         const float s = warp_sum(acc[b]);
         if (lane == 0) y[(int64_t)b * ld_y + row] = __float2half_rn(s);
+    }
+}
+
+// The same for 3 to 16 activation rows, W read once: a warp takes 16 rows of W as the A operand of mma.sync m16n8k16 (HBM-bound:
+// the legacy tensor path's rate is far above what W can be read at).  The k index of a product is permuted so that a lane
+// takes 16 contiguous bytes of W and of x: lane t of a group of four holds columns 8t .. 8t + 7 of every 32.  x goes through
+// shared memory in chunks of columns; eight 128-bit loads of W are in flight per lane.  32000 x 4096, 16 rows: 2 x 144 us
+// with eight rows at a time through packed multiply-adds.
+constexpr int kDenseWarps = 16, kDenseUnroll = 4;
+constexpr uint32_t kDenseXBytes = 128 * 1024;
+template <int NT>                                             // groups of eight activation rows
+__global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_mma_kernel(const __half *__restrict__ W, int64_t ld_w, const __half *__restrict__ x,
+                                                                       int64_t ld_x, __half *__restrict__ y, int64_t ld_y, int64_t m, int n,
+                                                                       int batch, int chunk) {
+    extern __shared__ __align__(16) unsigned char dense_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t xs = smem_addr(dense_smem), x_stride = (uint32_t)chunk * 2u + 64u;      // two rows cover all banks
+    const int64_t tiles = (m + 15) / 16, per_round = (int64_t)gridDim.x * kDenseWarps;
+    pdl_allow_next_grid();
+    pdl_wait_prior_grids();
+    for (int64_t base = 0; base < tiles; base += per_round) {
+        const int64_t tile = base + (int64_t)warp * gridDim.x + blockIdx.x;
+        const bool active = tile < tiles;
+        const int64_t r0 = min(tile * 16 + g, m - 1), r1 = min(tile * 16 + g + 8, m - 1);
+        const __half *w0 = W + r0 * ld_w + 8 * t, *w1 = W + r1 * ld_w + 8 * t;
+        float c[NT][4];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+        for (int k0 = 0; k0 < n; k0 += chunk) {
+            const int len = min(chunk, n - k0), steps = (len + 31) / 32;
+            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+            uint4 a0[kDenseUnroll], a1[kDenseUnroll];
+            auto fetch = [&](int s) {
+#pragma unroll
+                for (int u = 0; u < kDenseUnroll; ++u) {
+                    const int k = 32 * (s + u) + 8 * t;
+                    const bool in = active && k < len;
+                    a0[u] = in ? ldg128_stream(w0 + k0 + 32 * (s + u)) : zero;
+                    a1[u] = in ? ldg128_stream(w1 + k0 + 32 * (s + u)) : zero;
+                }
+            };
+            fetch(0);
+            if (base + k0 > 0) __syncthreads();               // everyone is done with the chunk before
+            const int vecs = steps * 4;                       // 16-byte pieces per row, zeros past the row's end
+            for (int i = threadIdx.x; i < 8 * NT * vecs; i += 32 * kDenseWarps) {
+                const int b = i / vecs, k = (i - b * vecs) * 8;
+                const uint4 v = (b < batch && k < len) ? ld_ordered_u128(x + (int64_t)b * ld_x + k0 + k) : zero;
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(xs + (uint32_t)b * x_stride + 2u * k), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+            }
+            __syncthreads();
+            const uint32_t xl = xs + (uint32_t)g * x_stride + 16u * t;
+            for (int s = 0; s < steps; s += kDenseUnroll) {
+                uint4 b0[kDenseUnroll], b1[kDenseUnroll];
+#pragma unroll
+                for (int u = 0; u < kDenseUnroll; ++u) b0[u] = a0[u], b1[u] = a1[u];
+                if (s + kDenseUnroll < steps) fetch(s + kDenseUnroll);
+#pragma unroll
+                for (int u = 0; u < kDenseUnroll; ++u) {
+                    if (s + u >= steps) break;
+#pragma unroll
+                    for (int i = 0; i < NT; ++i) {
+                        const uint4 xv = lds128(xl + (uint32_t)(8 * i) * x_stride + 64u * (uint32_t)(s + u));
+                        mma_16816(c[i], b0[u].x, b1[u].x, b0[u].y, b1[u].y, xv.x, xv.y);
+                        mma_16816(c[i], b0[u].z, b1[u].z, b0[u].w, b1[u].w, xv.z, xv.w);
+                    }
+                }
+            }
+        }
+        if (active) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int b = 8 * i + 2 * t + (e & 1);
+                    const int64_t row = tile * 16 + g + 8 * (e >> 1);
+                    if (b < batch && row < m) y[(int64_t)b * ld_y + row] = __float2half_rn(c[i][e]);
+                }
+        }
     }
 }
 
@@ -539,7 +630,7 @@ extern "C" int rptc_attn_decode(const void *qkv, int64_t ld_qkv, const int32_t *
     if (int e = rptc_check_device()) return e;
     unsigned int *status = device_status_word();
     if (!status) return RPTC_ERR_CUDA;
-    return launch(attn_decode_kernel, dim3((unsigned)hq, (unsigned)rows), dim3(kAttnThreads), 0, static_cast<cudaStream_t>(stream),
+    return launch_attn(hq, rows, static_cast<cudaStream_t>(stream),
                   static_cast<const __half *>(qkv), ld_qkv, pos, static_cast<const __half *>(kcache), static_cast<const __half *>(vcache),
                   static_cast<__half *>(out), ld_out, hq, hkv, max_pos, scale, static_cast<const __half *>(signs_in),
                   static_cast<float *>(nullptr), (int64_t)0, static_cast<const __half *>(nullptr), 0.f, RopeFreq{0.f, 0.f},
@@ -559,7 +650,7 @@ extern "C" int rptc_qkv_attn_decode(float *acc, int64_t ld_acc, const void *sign
     if (int e = rptc_check_device()) return e;
     unsigned int *status = device_status_word();
     if (!status) return RPTC_ERR_CUDA;
-    return launch(attn_decode_kernel, dim3((unsigned)heads, (unsigned)rows), dim3(kAttnThreads), 0, static_cast<cudaStream_t>(stream),
+    return launch_attn(heads, rows, static_cast<cudaStream_t>(stream),
                   static_cast<const __half *>(nullptr), (int64_t)0, pos, static_cast<const __half *>(kcache),
                   static_cast<const __half *>(vcache), static_cast<__half *>(out), ld_out, heads, kv_heads, max_pos, 0.08838834764831845f,
                   static_cast<const __half *>(signs_in), acc, ld_acc, static_cast<const __half *>(signs_out), scale_out, rope_freq(theta, 128),
@@ -570,30 +661,30 @@ extern "C" int rptc_dense_gemv(const void *W, int64_t ld_w, const void *x, int64
                                int batch, rptc_stream_t stream) {
     if (!W || !x || !y) return RPTC_ERR_ARG;
     if (m <= 0 || n <= 0 || (n % 8) || ld_w < n || ld_x < n || ld_y < m) return RPTC_ERR_SHAPE;
-    if (batch < 1 || batch > 8) return RPTC_ERR_ARG;
+    if (batch < 1 || batch > 16) return RPTC_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(x) & 15) || (ld_w % 8) || (ld_x % 8)) return RPTC_ERR_ALIGN;
     if (int e = rptc_check_device()) return e;
-    const dim3 grid((unsigned)((m + 7) / 8)), block(256);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const __half *Wp = static_cast<const __half *>(W), *xp = static_cast<const __half *>(x);
     __half *yp = static_cast<__half *>(y);
-    int done = 0;
-    while (done < batch) {
-        int b = 8;
-        while (b > batch - done) b >>= 1;
-        int e;
-        const __half *xb = xp + (int64_t)done * ld_x;
-        __half *yb = yp + (int64_t)done * ld_y;
-        switch (b) {
-            case 8: e = launch(dense_gemv_kernel<8>, grid, block, 0, s, Wp, ld_w, xb, ld_x, yb, ld_y, m, (int)n); break;
-            case 4: e = launch(dense_gemv_kernel<4>, grid, block, 0, s, Wp, ld_w, xb, ld_x, yb, ld_y, m, (int)n); break;
-            case 2: e = launch(dense_gemv_kernel<2>, grid, block, 0, s, Wp, ld_w, xb, ld_x, yb, ld_y, m, (int)n); break;
-            default: e = launch(dense_gemv_kernel<1>, grid, block, 0, s, Wp, ld_w, xb, ld_x, yb, ld_y, m, (int)n); break;
-        }
-        if (e) return e;
-        done += b;
+    if (batch <= 2) {
+        const dim3 grid((unsigned)((m + 7) / 8)), block(256);
+        return batch == 2 ? launch(dense_gemv_kernel<2>, grid, block, 0, s, Wp, ld_w, xp, ld_x, yp, ld_y, m, (int)n)
+                          : launch(dense_gemv_kernel<1>, grid, block, 0, s, Wp, ld_w, xp, ld_x, yp, ld_y, m, (int)n);
     }
-    return RPTC_OK;
+    const int nt = batch <= 8 ? 1 : 2;
+    int64_t chunk = kDenseXBytes / (16 * nt);                          // columns of x in shared memory at once
+    if (chunk > n) chunk = (n + 63) / 64 * 64;
+    const size_t smem = (size_t)(8 * nt) * (chunk * 2 + 64);
+    const int64_t tiles = (m + 15) / 16;
+    const unsigned ctas = (unsigned)(tiles < num_sms() ? tiles : num_sms());
+    static SmemOptIn opted1, opted2;
+    if (nt == 1) {
+        if (int e = allow_max_smem(dense_mma_kernel<1>, opted1, 132 * 1024)) return e;
+        return launch(dense_mma_kernel<1>, dim3(ctas), dim3(32 * kDenseWarps), smem, s, Wp, ld_w, xp, ld_x, yp, ld_y, m, (int)n, batch, (int)chunk);
+    }
+    if (int e = allow_max_smem(dense_mma_kernel<2>, opted2, 132 * 1024)) return e;
+    return launch(dense_mma_kernel<2>, dim3(ctas), dim3(32 * kDenseWarps), smem, s, Wp, ld_w, xp, ld_x, yp, ld_y, m, (int)n, batch, (int)chunk);
 }
 
 extern "C" int rptc_embed(const void *table, const int32_t *ids, void *out, int64_t ld_out, int64_t rows, int64_t n,

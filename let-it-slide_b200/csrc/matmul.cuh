@@ -10,10 +10,11 @@ namespace rptc {
 struct Banks {
     int32_t banks = 1;
     int64_t lut_stride = 0;      // fp16 elements
+    bool may_split = true;       // false: every sum is one chain along the reduction, whatever the number of tokens
 };
 
 // Columns of y per bank: a bank's rows rounded up to whole tiles.
-int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, int32_t banks, const rptc_format &f);
+int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f);
 // y[t][bank * gemm_bank_columns + row] = fp16(sum_c x[t][c] W[bank][row][c]); columns beyond a bank's m rows hold no
 // result.  Shapes and alignments as rptc_gemm's, with m % 32 == 0 where banks > 1.
 int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,

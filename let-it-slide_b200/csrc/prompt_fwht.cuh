@@ -1,14 +1,17 @@
-// Walsh-Hadamard building blocks for many rows (prompts): 32 values per thread, two exchanges through shared memory.
+// Walsh-Hadamard building blocks for many rows (prompts): 32 values per thread, exchanges through shared memory.
 //
 // A segment is 1024 columns for a warp (blocks of at most 256) or 4096 for a CTA of 128 threads (any block up to 4096); it
 // may hold several blocks.  Element e of a segment is at e + 8 (e >> 8) in the exchange buffer, which keeps all accesses
-// below free of bank conflicts.  Three layouts of a thread's 32 values, by the bits of e that vary inside the thread:
-//   rows     bits 0-2 and two more (warp: 8, 9; CTA: 8, 9 or 10, 11): four pieces of eight consecutive elements, loaded and
-//            stored as 16 bytes of fp16 each
+// below free of bank conflicts.  The layouts of a thread's 32 values, by the bits of e that vary inside the thread:
+//   pieces   bits 0-2 and two more (warp: 8, 9; CTA: 10, 11): four pieces of eight consecutive elements, loaded and stored
+//            as 16 bytes of fp16 each
 //   columns  bits 3-7
-// A transform does the stages of its own bits in each layout, in any order; stages at or above the block size are skipped.
-// Against eight values per thread with shuffles (five stages x eight values through the same pipe as shared memory) this
-// moves 2048 x 4096 in 8 us instead of 24.
+//   far      (CTA) bits 0 and 8-11: sixteen pairs, 256 elements apart
+// A transform does the stages of bits 0-2 in pieces, 3-7 in columns, 8-11 in far: in ascending order, the order of the
+// kernels with eight values per thread, so that the results of both are the same bits.  Stages at or above the block size
+// are skipped.  A thread that has read its values in one layout may write them in the same layout without a barrier.
+// Against eight values per thread with shuffles (five stages x eight values through the same pipe as shared memory):
+// 2048 x 4096 in 13.4 us instead of 19.3.
 #pragma once
 #include "common.cuh"
 #include "fwht.cuh"
@@ -29,13 +32,11 @@ __device__ __forceinline__ void stage(float (&v)[32]) {
         }
 }
 
-// v[8 j + i] is element i of piece j: the stages of bits 0-2, and of the two bits that number the pieces (`lo` and `lo + 1`).
-__device__ __forceinline__ void row_stages(float (&v)[32], int block_bits, int lo) {
-    if (block_bits > 0) stage<1>(v);
-    if (block_bits > 1) stage<2>(v);
-    if (block_bits > 2) stage<4>(v);
-    if (block_bits > lo) stage<8>(v);
-    if (block_bits > lo + 1) stage<16>(v);
+// v[8 j + i] is element i of piece j.
+__device__ __forceinline__ void piece_stages(float (&v)[32]) {
+    stage<1>(v);                       // blocks have at least eight elements
+    stage<2>(v);
+    stage<4>(v);
 }
 // v[k] is element bits 3-7 = k.
 __device__ __forceinline__ void column_stages(float (&v)[32], int block_bits) {
@@ -45,17 +46,21 @@ __device__ __forceinline__ void column_stages(float (&v)[32], int block_bits) {
     if (block_bits > 6) stage<8>(v);
     if (block_bits > 7) stage<16>(v);
 }
+// v[2 k + e] is element e of pair k.
+__device__ __forceinline__ void far_stages(float (&v)[32], int block_bits) {
+    if (block_bits > 8) stage<2>(v);
+    if (block_bits > 9) stage<4>(v);
+    if (block_bits > 10) stage<8>(v);
+    if (block_bits > 11) stage<16>(v);
+}
 
-// Where a thread's pieces and columns are.  WARP segments: pieces at 8 lane + 256 j.  CTA segments (t of 128 threads): with
-// `far` pieces at 8 t + 1024 j (bits 10, 11 vary), else at 8 lane + 1024 warp + 256 j (bits 8, 9 vary).
+// Where a thread's values are; t of 128 threads in a CTA segment.
 template <bool CTA>
 struct SegThread {
     int lane, warp, t;
     __device__ __forceinline__ SegThread() : lane(threadIdx.x & 31), warp(CTA ? (threadIdx.x >> 5) & 3 : 0), t(threadIdx.x & 127) {}
-    __device__ __forceinline__ int piece(int j, bool far) const {
-        if (!CTA) return 8 * lane + 256 * j;
-        return far ? 8 * t + 1024 * j : 8 * lane + 1024 * warp + 256 * j;
-    }
+    __device__ __forceinline__ int piece(int j) const { return CTA ? 8 * t + 1024 * j : 8 * lane + 256 * j; }
+    __device__ __forceinline__ int pair(int k) const { return 2 * t + 256 * k; }
     __device__ __forceinline__ int column() const {      // element of k = 0: bits 0-2 from the lane, bits 8 up from the rest
         return (lane & 7) + 256 * ((lane >> 3) + 4 * warp);
     }
@@ -66,26 +71,37 @@ struct SegThread {
     }
     // The two halves of a piece as 16-byte accesses; lanes with bit 2 set take the upper half first, so that eight lanes
     // with a stride of 32 bytes meet all banks once.
-    __device__ __forceinline__ void put_pieces(float *buf, const float (&v)[32], bool far) const {
+    __device__ __forceinline__ void put_pieces(float *buf, const float (&v)[32]) const {
         const bool swap = lane & 4;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float4 *p = reinterpret_cast<float4 *>(buf + at(piece(j, far)));
+            float4 *p = reinterpret_cast<float4 *>(buf + at(piece(j)));
             const float4 a = make_float4(v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]);
             const float4 b = make_float4(v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
             p[swap ? 1 : 0] = swap ? b : a;
             p[swap ? 0 : 1] = swap ? a : b;
         }
     }
-    __device__ __forceinline__ void get_pieces(const float *buf, float (&v)[32], bool far) const {
+    __device__ __forceinline__ void get_pieces(const float *buf, float (&v)[32]) const {
         const bool swap = lane & 4;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float4 *p = reinterpret_cast<const float4 *>(buf + at(piece(j, far)));
+            const float4 *p = reinterpret_cast<const float4 *>(buf + at(piece(j)));
             const float4 x = p[swap ? 1 : 0], y = p[swap ? 0 : 1];
             const float4 a = swap ? y : x, b = swap ? x : y;
             v[8 * j] = a.x, v[8 * j + 1] = a.y, v[8 * j + 2] = a.z, v[8 * j + 3] = a.w;
             v[8 * j + 4] = b.x, v[8 * j + 5] = b.y, v[8 * j + 6] = b.z, v[8 * j + 7] = b.w;
+        }
+    }
+    __device__ __forceinline__ void put_pairs(float *buf, const float (&v)[32]) const {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) *reinterpret_cast<float2 *>(buf + at(pair(k))) = make_float2(v[2 * k], v[2 * k + 1]);
+    }
+    __device__ __forceinline__ void get_pairs(const float *buf, float (&v)[32]) const {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float2 p = *reinterpret_cast<const float2 *>(buf + at(pair(k)));
+            v[2 * k] = p.x, v[2 * k + 1] = p.y;
         }
     }
     __device__ __forceinline__ void put_columns(float *buf, const float (&v)[32]) const {

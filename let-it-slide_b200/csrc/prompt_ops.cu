@@ -2,7 +2,6 @@
 //   hadamard_rows     rptc_hadamard for many rows
 //   norm_rows         h += s_out * H(y) * scale;  xn = rmsnorm(h) * w;  out = H(s_in * xn)        (rptc_prompt_norm)
 //   qkv_rows          output transform of the fused qkv layer, rotary embedding, cache writes     (rptc_prompt_qkv)
-//   swiglu_rows       rptc_swiglu_hadamard_f16 for many rows
 // Bound: HBM / L2 (each input read once, each output written once).  A warp or CTA keeps its columns and walks down the rows,
 // so that signs and weights of its columns stay in registers.
 #include "common.cuh"
@@ -35,10 +34,14 @@ struct HadRowsParams {
     int64_t clear_count;
 };
 
-// One segment of a row per warp (blocks up to 256) or per CTA of 128 threads.
+__device__ __forceinline__ uint32_t ldcg_u32(const void *p) { return __ldcg(static_cast<const uint32_t *>(p)); }
+
+// One segment of a row per warp (blocks up to 256, results in the layout of the pieces) or per CTA of 128 threads (results in
+// the layout of the pairs).
 template <bool CTA, bool IN_F32>
 __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_kernel(const HadRowsParams p) {
     constexpr int kSeg = CTA ? 4096 : 1024, kUnits = CTA ? 1 : 8;       // segments per CTA
+    constexpr uint32_t kOnes = 0x3C003C00u;
     __shared__ __align__(16) float smem[CTA ? kCtaSegFloats : 8 * kWarpSegFloats];
     const SegThread<CTA> th;
     const int unit = CTA ? 0 : threadIdx.x >> 5;
@@ -54,18 +57,20 @@ __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_ke
     }
     if (worker >= workers) return;
     const int64_t col0 = (worker % segs) * kSeg;
-    const int lo = CTA ? 10 : 8;                             // the bits that number the pieces as loaded
-    uint4 sg[4];                                             // of the pieces as they are when the signs apply
+    // the columns of pair of values i (v[2 i], v[2 i + 1]) as loaded and as stored
+    auto col_in = [&](int i) { return col0 + th.piece(i >> 2) + 2 * (i & 3); };
+    auto col_out = [&](int i) { return CTA ? col0 + th.pair(i) : col_in(i); };
+    uint32_t sg[16];                                         // signs of the columns where they apply, two to a register
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t c = col0 + th.piece(j, !p.transpose);
-        sg[j] = (p.signs && c < p.n) ? __ldg(reinterpret_cast<const uint4 *>(p.signs + c)) : make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+    for (int i = 0; i < 16; ++i) {
+        const int64_t c = p.transpose ? col_out(i) : col_in(i);
+        sg[i] = (p.signs && c < p.n) ? __ldg(reinterpret_cast<const uint32_t *>(p.signs + c)) : kOnes;
     }
     for (int64_t row = worker / segs; row < p.rows; row += workers / segs) {
         float v[32];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int64_t c = col0 + th.piece(j, true);
+            const int64_t c = col0 + th.piece(j);
             if (IN_F32) {
                 float *src = const_cast<float *>(static_cast<const float *>(p.in)) + row * p.ld_in + c;
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
@@ -80,49 +85,56 @@ __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_ke
                 unpack8_at(raw, v + 8 * j);
             }
         }
-        uint4 res[4];
+        uint32_t res[16];
         if (p.residual) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t c = col0 + th.piece(j, false);
-                if (c < p.n) res[j] = __ldcg(reinterpret_cast<const uint4 *>(p.residual + row * p.ld_res + c));
-            }
+            for (int i = 0; i < 16; ++i)
+                if (col_out(i) < p.n) res[i] = ldcg_u32(p.residual + row * p.ld_res + col_out(i));
         }
         if (!p.transpose) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float s[8];
-                unpack8_at(sg[j], s);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[8 * j + i] *= s[i];
+            for (int i = 0; i < 16; ++i) {
+                const float2 s = __half22float2(u32_as_half2(sg[i]));
+                v[2 * i] *= s.x, v[2 * i + 1] *= s.y;
             }
         }
-        row_stages(v, p.block_bits, lo);
-        th.put_pieces(buf, v, true);
+        piece_stages(v);
+        th.put_pieces(buf, v);
         th.sync();
         th.get_columns(buf, v);
         column_stages(v, p.block_bits);
         th.put_columns(buf, v);
         th.sync();
-        th.get_pieces(buf, v, false);
         if (CTA) {
-            if (p.block_bits > 8) stage<8>(v);
-            if (p.block_bits > 9) stage<16>(v);
+            th.get_pairs(buf, v);
+            far_stages(v, p.block_bits);
+        } else {
+            th.get_pieces(buf, v);
         }
+        uint32_t o[16];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t c = col0 + th.piece(j, false);
-            if (c >= p.n) continue;
-            float s[8], r[8];
-            if (p.transpose) unpack8_at(sg[j], s);
-            if (p.residual) unpack8_at(res[j], r);
-            float o[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                o[i] = v[8 * j + i] * (p.transpose ? p.scale * s[i] : p.scale);
-                if (p.residual) o[i] += r[i];
+        for (int i = 0; i < 16; ++i) {
+            float2 s = make_float2(p.scale, p.scale);
+            if (p.transpose) {
+                const float2 f = __half22float2(u32_as_half2(sg[i]));
+                s.x *= f.x, s.y *= f.y;
             }
-            *reinterpret_cast<uint4 *>(p.out + row * p.ld_out + c) = pack8_from(o);
+            float2 w = make_float2(__fmul_rn(v[2 * i], s.x), __fmul_rn(v[2 * i + 1], s.y));
+            if (p.residual) {
+                const float2 r = __half22float2(u32_as_half2(res[i]));
+                w.x = __fadd_rn(w.x, r.x), w.y = __fadd_rn(w.y, r.y);
+            }
+            o[i] = half2_as_u32(__floats2half2_rn(w.x, w.y));
+        }
+        __half *dst = p.out + row * p.ld_out;
+        if (CTA) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (col_out(i) < p.n) *reinterpret_cast<uint32_t *>(dst + col_out(i)) = o[i];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (col0 + th.piece(j) < p.n) *reinterpret_cast<uint4 *>(dst + col0 + th.piece(j)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         }
         th.sync();                                           // the buffer is free for the next row
     }
@@ -180,106 +192,111 @@ struct NormRowsParams {
     int64_t ld_out, rows;
 };
 
-// A row of NH x 4096 elements (each 4096 one Hadamard block of both transforms) per CTA of NH x 128 threads.
+// A row of NH x 4096 elements (each 4096 one Hadamard block of both transforms) per CTA of NH x 128 threads.  The results are
+// the bits that rptc_hadamard, rptc_rmsnorm and rptc_hadamard give one after the other: same order of all sums.  (That of the
+// squares is one of 256 threads over pairs 512 elements apart: a thread here holds what two of those hold.)
 template <int NH>
 __global__ void __launch_bounds__(128 * NH, 4 / NH) norm_rows_kernel(const NormRowsParams p) {
     constexpr int n = 4096 * NH;
     __shared__ __align__(16) float smem[NH * kCtaSegFloats];
-    __shared__ float red[2][4 * NH];
+    __shared__ float red[8], carry[2][128];
     const SegThread<true> th;
-    const int part = threadIdx.x >> 7, warp = threadIdx.x >> 5;
+    const int part = threadIdx.x >> 7;
     float *buf = smem + part * kCtaSegFloats;
-    const uint4 ones = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
-    // this thread's columns after the output transform: signs of the layer in front, and weight x sign of what comes next
-    // (a sign commutes with the rounding of the normalised value)
-    uint4 so[4], ws[4];
+    const int col0 = 4096 * part;
+    // this thread's columns between the transforms: signs of the layer in front, and weight x sign of what comes next (a sign
+    // commutes with the rounding of the normalised value)
+    uint32_t so[16], ws[16];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = 4096 * part + th.piece(j, false);
-        so[j] = p.signs_out ? __ldg(reinterpret_cast<const uint4 *>(p.signs_out + c)) : ones;
-        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(p.w_norm + c)), si = p.signs_in ? __ldg(reinterpret_cast<const uint4 *>(p.signs_in + c)) : ones;
-        float a[8], b[8];
-        unpack8_at(w, a);
-        unpack8_at(si, b);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] *= b[i];
-        ws[j] = pack8_from(a);
+    for (int k = 0; k < 16; ++k) {
+        const int c = col0 + th.pair(k);
+        so[k] = p.signs_out ? __ldg(reinterpret_cast<const uint32_t *>(p.signs_out + c)) : 0x3C003C00u;
+        const float2 w = __half22float2(u32_as_half2(__ldg(reinterpret_cast<const uint32_t *>(p.w_norm + c))));
+        const float2 si = p.signs_in ? __half22float2(u32_as_half2(__ldg(reinterpret_cast<const uint32_t *>(p.signs_in + c)))) : make_float2(1.f, 1.f);
+        ws[k] = half2_as_u32(__floats2half2_rn(w.x * si.x, w.y * si.y));
     }
     pdl_allow_next_grid();
     pdl_wait_prior_grids();
     const float hn = 0.015625f;                              // 1 / sqrt(4096)
-    int turn = 0;
-    for (int64_t row = blockIdx.x; row < p.rows; row += gridDim.x, turn ^= 1) {
-        uint4 hr[4];
-        __half *hrow = p.h + row * p.ld_h + 4096 * part;
+    for (int64_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
+        uint32_t hr[16];
+        __half *hrow = p.h + row * p.ld_h + col0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) hr[j] = __ldcg(reinterpret_cast<const uint4 *>(hrow + th.piece(j, false)));
+        for (int k = 0; k < 16; ++k) hr[k] = ldcg_u32(hrow + th.pair(k));
         float v[32];
         if (p.y) {
-            const __half *yrow = p.y + row * p.ld_y + 4096 * part;
+            const __half *yrow = p.y + row * p.ld_y + col0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) unpack8_at(__ldcg(reinterpret_cast<const uint4 *>(yrow + th.piece(j, true))), v + 8 * j);
-            row_stages(v, 12, 10);
-            th.put_pieces(buf, v, true);
+            for (int j = 0; j < 4; ++j) unpack8_at(__ldcg(reinterpret_cast<const uint4 *>(yrow + th.piece(j))), v + 8 * j);
+            piece_stages(v);
+            th.put_pieces(buf, v);
             __syncthreads();
             th.get_columns(buf, v);
             column_stages(v, 12);
             th.put_columns(buf, v);
             __syncthreads();
-            th.get_pieces(buf, v, false);
-            stage<8>(v);
-            stage<16>(v);
+            th.get_pairs(buf, v);
+            far_stages(v, 12);
             const float sc = p.scale_out * hn;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float s[8], r[8];
-                unpack8_at(so[j], s);
-                unpack8_at(hr[j], r);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[8 * j + i] = r[i] + v[8 * j + i] * sc * s[i];
-                const uint4 o = pack8_from(v + 8 * j);
-                *reinterpret_cast<uint4 *>(hrow + th.piece(j, false)) = o;
-                unpack8_at(o, v + 8 * j);                     // go on from the rounded residual stream, as a reader of h would
+            for (int k = 0; k < 16; ++k) {
+                const float2 s = __half22float2(u32_as_half2(so[k])), r = __half22float2(u32_as_half2(hr[k]));
+                const float a = __fadd_rn(__fmul_rn(v[2 * k], sc * s.x), r.x), b = __fadd_rn(__fmul_rn(v[2 * k + 1], sc * s.y), r.y);
+                hr[k] = half2_as_u32(__floats2half2_rn(a, b));
+                *reinterpret_cast<uint32_t *>(hrow + th.pair(k)) = hr[k];
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) unpack8_at(hr[j], v + 8 * j);
         }
-        float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) ss += v[i] * v[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-        if (th.lane == 0) red[turn][warp] = ss;
-        __syncthreads();                                      // also: everyone is done with the exchange buffer
-        ss = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4 * NH; ++i) ss += red[turn][i];
-        const float inv = rsqrtf(ss / n + p.eps);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float w[8];
-            unpack8_at(ws[j], w);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[8 * j + i] = __half2float(__float2half_rn(v[8 * j + i] * inv * w[i]));
+        for (int k = 0; k < 16; ++k) {                        // go on from the rounded residual stream, as a reader of h would
+            const float2 f = __half22float2(u32_as_half2(hr[k]));
+            v[2 * k] = f.x, v[2 * k + 1] = f.y;
         }
-        row_stages(v, 12, 8);
-        th.put_pieces(buf, v, false);
+        float ss[2] = {0.f, 0.f};
+        if (NH == 2) {                                        // the second piece goes on with the sums of the first
+            if (part == 1) asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (part == 1) ss[0] = carry[0][th.t], ss[1] = carry[1][th.t];
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) ss[k & 1] += v[2 * k] * v[2 * k] + v[2 * k + 1] * v[2 * k + 1];
+        if (NH == 2 && part == 0) {
+            carry[0][th.t] = ss[0], carry[1][th.t] = ss[1];
+            asm volatile("bar.arrive 1, 256;" ::: "memory");
+        }
+        if (part == NH - 1) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ss[i] += __shfl_xor_sync(0xFFFFFFFFu, ss[i], o);
+                if (th.lane == 0) red[4 * i + th.warp] = ss[i];
+            }
+        }
+        __syncthreads();
+        float tot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tot += red[i];
+        const float inv = rsqrtf(tot / n + p.eps);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float2 w = __half22float2(u32_as_half2(ws[k]));
+            const float2 f = __half22float2(__floats2half2_rn(v[2 * k] * inv * w.x, v[2 * k + 1] * inv * w.y));
+            v[2 * k] = f.x, v[2 * k + 1] = f.y;
+        }
+        th.put_pairs(buf, v);
+        __syncthreads();
+        th.get_pieces(buf, v);
+        piece_stages(v);
+        th.put_pieces(buf, v);
         __syncthreads();
         th.get_columns(buf, v);
         column_stages(v, 12);
         th.put_columns(buf, v);
         __syncthreads();
-        th.get_pieces(buf, v, true);
-        stage<8>(v);
-        stage<16>(v);
-        __half *orow = p.out + row * p.ld_out + 4096 * part;
+        th.get_pairs(buf, v);
+        far_stages(v, 12);
+        __half *orow = p.out + row * p.ld_out + col0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[8 * j + i] *= hn;
-            *reinterpret_cast<uint4 *>(orow + th.piece(j, true)) = pack8_from(v + 8 * j);
-        }
+        for (int k = 0; k < 16; ++k)
+            *reinterpret_cast<uint32_t *>(orow + th.pair(k)) = half2_as_u32(__floats2half2_rn(v[2 * k] * hn, v[2 * k + 1] * hn));
         __syncthreads();                                      // the buffer is free for the next row
     }
 }
@@ -334,15 +351,15 @@ __global__ void __launch_bounds__(256, 2) qkv_rows_kernel(const QkvRowsParams p)
         float v[32];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j, true);
+            const int c = th.piece(j);
             unpack8_at(col0 + c < n ? __ldcg(reinterpret_cast<const uint4 *>(src + c)) : make_uint4(0u, 0u, 0u, 0u), v + 8 * j);
         }
         float2 cs[8];
         const float2 *ang = p.angles + pos * 64 + (th.lane & 7);
 #pragma unroll
         for (int k = 0; k < 8; ++k) cs[k] = __ldg(ang + 8 * k);
-        row_stages(v, 7, 8);
-        th.put_pieces(buf, v, true);
+        piece_stages(v);
+        th.put_pieces(buf, v);
         __syncwarp();
         th.get_columns(buf, v);
         column_stages(v, 7);
@@ -363,10 +380,10 @@ __global__ void __launch_bounds__(256, 2) qkv_rows_kernel(const QkvRowsParams p)
         }
         th.put_columns(buf, v);
         __syncwarp();
-        th.get_pieces(buf, v, true);
+        th.get_pieces(buf, v);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j, true), head = (col0 + c) >> 7, i = c & 127;
+            const int c = th.piece(j), head = (col0 + c) >> 7, i = c & 127;
             if (col0 + c >= n) continue;
             __half *dst = head < p.hq ? src + c
                           : head < p.hq + p.hkv ? p.kcache + ((seq * p.max_pos + pos) * p.hkv + head - p.hq) * 128 + i
@@ -375,109 +392,6 @@ __global__ void __launch_bounds__(256, 2) qkv_rows_kernel(const QkvRowsParams p)
         }
         __syncwarp();
     }
-}
-
-// ---- gated MLP middle ---------------------------------------------------------------------------------------------------
-struct SwigluRowsParams {
-    const __half *in;                // [rows][ld_in >= 2n]: gate | up, before the output transform
-    int64_t ld_in;
-    __half *out;
-    int64_t ld_out;
-    const __half *signs_out, *signs_in;
-    int64_t rows, n;
-    int32_t block_bits;
-    float scale_out, scale_in;       // include the 1 / sqrt(block) of their transform
-};
-
-// A warp takes 1024 columns of a row (blocks up to 256).  Gate and up end their transforms in the column layout, the product
-// starts its own there, so that three transforms cost six passes through the exchange buffer instead of twelve.
-__global__ void __launch_bounds__(256, 2) swiglu_rows_kernel(const SwigluRowsParams p) {
-    __shared__ __align__(16) float smem[8 * kWarpSegFloats];
-    const SegThread<false> th;
-    const int unit = threadIdx.x >> 5;
-    float *buf = smem + unit * kWarpSegFloats;
-    const int segs = (int)((p.n + 1023) / 1024);
-    const int64_t worker = (int64_t)blockIdx.x * 8 + unit, workers = (int64_t)gridDim.x * 8 / segs * segs;
-    pdl_allow_next_grid();
-    if (worker >= workers) return;
-    const int64_t col0 = (worker % segs) * 1024;
-    uint32_t sgn_g = 0, sgn_u = 0, sgn_i = 0;                 // bit k: sign of this thread's column element k
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-        const int64_t c = col0 + th.column() + 8 * k;
-        if (c >= p.n) continue;
-        const unsigned short *so = reinterpret_cast<const unsigned short *>(p.signs_out), *si = reinterpret_cast<const unsigned short *>(p.signs_in);
-        if (so) sgn_g |= (uint32_t)(__ldg(so + c) >> 15) << k, sgn_u |= (uint32_t)(__ldg(so + p.n + c) >> 15) << k;
-        if (si) sgn_i |= (uint32_t)(__ldg(si + c) >> 15) << k;
-    }
-    pdl_wait_prior_grids();
-    for (int64_t row = worker / segs; row < p.rows; row += workers / segs) {
-        const __half *src = p.in + row * p.ld_in + col0;
-        uint4 ru[4];
-        float g[32], u[32];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j, true);
-            const bool in = col0 + c < p.n;
-            const uint4 rg = in ? __ldcg(reinterpret_cast<const uint4 *>(src + c)) : make_uint4(0u, 0u, 0u, 0u);
-            ru[j] = in ? __ldcg(reinterpret_cast<const uint4 *>(src + p.n + c)) : make_uint4(0u, 0u, 0u, 0u);
-            unpack8_at(rg, g + 8 * j);
-        }
-        row_stages(g, p.block_bits, 8);
-        th.put_pieces(buf, g, true);
-        __syncwarp();
-        th.get_columns(buf, g);
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) unpack8_at(ru[j], u + 8 * j);
-        row_stages(u, p.block_bits, 8);
-        th.put_pieces(buf, u, true);
-        __syncwarp();
-        th.get_columns(buf, u);
-        column_stages(g, p.block_bits);
-        column_stages(u, p.block_bits);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            // the layer's own output is fp16, and so is the gated product
-            const float gg = __half2float(__float2half_rn(g[k] * (((sgn_g >> k) & 1u) ? -p.scale_out : p.scale_out)));
-            const float uu = __half2float(__float2half_rn(u[k] * (((sgn_u >> k) & 1u) ? -p.scale_out : p.scale_out)));
-            const float m = __half2float(__float2half_rn(__fdividef(gg, 1.f + __expf(-gg)) * uu));
-            g[k] = ((sgn_i >> k) & 1u) ? -m : m;
-        }
-        column_stages(g, p.block_bits);
-        __syncwarp();
-        th.put_columns(buf, g);
-        __syncwarp();
-        th.get_pieces(buf, g, true);
-        row_stages(g, p.block_bits, 8);
-        __half *dst = p.out + row * p.ld_out + col0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j, true);
-            if (col0 + c >= p.n) continue;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) g[8 * j + i] *= p.scale_in;
-            *reinterpret_cast<uint4 *>(dst + c) = pack8_from(g + 8 * j);
-        }
-        __syncwarp();
-    }
-}
-
-int swiglu_rows(const void *gate_up, int64_t ld_in, void *out, int64_t ld_out, const void *signs_out, const void *signs_in, int64_t rows, int64_t n,
-                int block, float scale_out, float scale_in, cudaStream_t stream) {
-    SwigluRowsParams p;
-    p.in = static_cast<const __half *>(gate_up);
-    p.ld_in = ld_in;
-    p.out = static_cast<__half *>(out);
-    p.ld_out = ld_out;
-    p.signs_out = static_cast<const __half *>(signs_out);
-    p.signs_in = static_cast<const __half *>(signs_in);
-    p.rows = rows;
-    p.n = n;
-    p.block_bits = log2_of(block);
-    p.scale_out = scale_out * norm_of(block);
-    p.scale_in = scale_in * norm_of(block);
-    return launch(swiglu_rows_kernel, dim3(rows_grid(rows, (n + 1023) / 1024, 8, 2)), dim3(256), 0, stream, p);
 }
 
 }  // namespace rptc

@@ -110,8 +110,9 @@ class RPTCLinear(nn.Module):
 
     def product_t(self, xt: torch.Tensor) -> torch.Tensor:
         """W_hat xt for already-transformed activations xt fp16 [rows > 8, in]: the tensor-core GEMM, unscaled and
-        before the output transform."""
-        return ops.gemm(self.codes, self.lut, xt, self.out_features, self.in_features, self.fmt, carry_in=self.carry_in)
+        before the output transform.  A row's result does not depend on the number of rows: a prompt gives the same
+        caches and logits however many tokens go through the network with it."""
+        return ops.gemm(self.codes, self.lut, xt, self.out_features, self.in_features, self.fmt, carry_in=self.carry_in, invariant=True)
 
     def finish_t(self, y: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         """Output side of `product_t`: s_out * H(y) * scale (+ residual), fp16."""

@@ -170,8 +170,8 @@ class RPTCLlama:
                 and self.cfg.head_dim == 128 and self.blocks[0].qkv.block_out >= 128 and self.fused_tp)
 
     def _extra_launches(self) -> int:
-        """Launches beyond one per matvec: the output head takes up to eight activation rows per launch."""
-        return (self.rows - 1) // 8
+        """Launches beyond one per matvec: the output head takes up to sixteen activation rows per launch."""
+        return (self.rows - 1) // 16
 
     def step_eager(self) -> None:
         if self._glueable():

@@ -169,16 +169,17 @@ def gemv(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, m: int, n: int
 
 
 def gemm(codes: torch.Tensor, lut: torch.Tensor, x: torch.Tensor, m: int, n: int, fmt: Format,
-         out: torch.Tensor | None = None, carry_in: torch.Tensor | None = None) -> torch.Tensor:
-    """y[t] = W x[t] for a block of tokens on the tensor cores (rptc_gemm).  x: fp16 [tokens, n]."""
+         out: torch.Tensor | None = None, carry_in: torch.Tensor | None = None, invariant: bool = False) -> torch.Tensor:
+    """y[t] = W x[t] for a block of tokens on the tensor cores (rptc_gemm).  x: fp16 [tokens, n].  `invariant`: a token's
+    result does not depend on the number of tokens (rptc_gemm_invariant)."""
     _cuda_contig(codes, "codes", torch.int32)
     _cuda_contig(lut, "lut", torch.float16)
     if not x.is_cuda or x.dtype != torch.float16 or x.dim() != 2 or x.stride(1) != 1 or x.shape[1] != n:
         raise RuntimeError("x must be a CUDA fp16 [tokens, n] tensor with unit column stride")
     if out is None:
         out = torch.empty((x.shape[0], m), dtype=torch.float16, device=x.device)
-    call("rptc_gemm", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0), ptr(out), out.stride(0), m, n, x.shape[0],
-         ctypes.byref(fmt))
+    call("rptc_gemm_invariant" if invariant else "rptc_gemm", codes.device, ptr(codes), ptr(lut), ptr(carry_in), ptr(x), x.stride(0), ptr(out),
+         out.stride(0), m, n, x.shape[0], ctypes.byref(fmt))
     return out
 
 
@@ -311,8 +312,8 @@ def dense_gemv(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None
     if out is None:
         out = torch.empty((x.shape[0], m), dtype=torch.float16, device=x.device)
     o2 = out.unsqueeze(0) if out.dim() == 1 else out
-    for b0 in range(0, x.shape[0], 8):                  # the kernel takes up to eight activation rows per launch
-        xb, ob = x[b0:b0 + 8], o2[b0:b0 + 8]
+    for b0 in range(0, x.shape[0], 16):                 # the kernel takes up to sixteen activation rows per launch
+        xb, ob = x[b0:b0 + 16], o2[b0:b0 + 16]
         call("rptc_dense_gemv", W.device, ptr(W), W.stride(0), ptr(xb), _ld(xb, n), ptr(ob), _ld(ob, m), m, n, xb.shape[0])
     return out[0] if squeeze and out.dim() == 2 else out
 

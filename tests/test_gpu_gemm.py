@@ -139,3 +139,15 @@ def test_two_sm_kernel_passes_the_identity_cases():
 def test_gemm_tiles_and_splits(code, K, L, S, m, n, tokens):
     """One and two token halves, tiles past the last row, and a reduction shared by one, two and four CTAs (uneven parts)."""
     _run(code, K, L, S, m, n, tokens, seed=m + n + tokens)
+
+
+def test_gemm_invariant_gives_a_token_the_same_bits_in_any_company():
+    from rptc_b200 import Format, ops
+    fmt, (m, n) = Format(), (512, 4096)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, 2, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(512, dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn((5000, n), generator=g, device="cuda").half()
+    full = ops.gemm(codes, lut, x, m, n, fmt, invariant=True)
+    for tokens in (9, 128, 200, 1000):
+        assert torch.equal(ops.gemm(codes, lut, x[:tokens], m, n, fmt, invariant=True), full[:tokens]), tokens

@@ -150,3 +150,14 @@ def test_gemv_few_rows_at_tile_and_range_edges(code, K, L, S, m, n, batch):
     torch.cuda.synchronize()
     ops.device_status()
     check_product(y.float().cpu().numpy(), exact.cpu().numpy(), dense.norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(), GEMV_FP32_TOL)
+
+
+@pytest.mark.parametrize("m,n,batch", [(16, 8, 3), (17, 40, 5), (1000, 4096, 16), (40000, 520, 9), (37, 8200, 8), (2500, 8232, 13)])
+def test_dense_gemv_of_many_rows(m, n, batch):
+    """Rows and columns that are not whole tiles, x in one and in several chunks of columns, one and several rounds of tiles."""
+    from rptc_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    W, x = torch.randn((m, n), generator=g, device="cuda").half(), torch.randn((batch, n), generator=g, device="cuda").half()
+    exact = x.double() @ W.double().t()
+    y = ops.dense_gemv(W, x)
+    check_product(y.float().cpu().numpy(), exact.cpu().numpy(), W.double().norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(), GEMV_FP32_TOL)

@@ -175,31 +175,21 @@ def test_gemv_computing_its_own_input_from_8192_wide_rows(batch, with_acc):
 @pytest.mark.parametrize("n,block", [(256, 8), (256, 256), (768, 64), (11008, 256), (12288, 128), (512, 512), (3072, 1024), (6144, 2048), (4096, 4096), (12288, 4096)])
 @pytest.mark.parametrize("transpose,f32,residual", [(False, False, False), (True, False, True), (True, True, False), (True, True, True)])
 def test_hadamard_of_many_rows_matches_single_rows(n, block, transpose, f32, residual):
-    """The kernels that walk down the rows against the one-row kernels, over every block size class, partial segments included."""
+    """The kernels that walk down the rows give the bits of the one-row kernels, over every block size class, partial segments
+    included."""
     from rptc_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(n + block)
-    rows = 37
+    rows = 37 if block > 256 else (8 << 20) // n + 3
     x = torch.randn((rows, n), generator=g, device="cuda", dtype=torch.float32 if f32 else torch.float16)
     signs = (torch.randint(0, 2, (n,), generator=g, device="cuda") * 2 - 1).half()
     res = torch.randn((rows, n), generator=g, device="cuda").half() if residual else None
-    want = torch.cat([ops.hadamard(x[r:r + 1], signs, block, transpose, 0.7, residual=None if res is None else res[r:r + 1]) for r in range(rows)])
+    few = lambda r: ops.hadamard(x[r:r + 31], signs, block, transpose, 0.7, residual=None if res is None else res[r:r + 31])
+    want = torch.cat([few(r) for r in range(0, rows, 31)])
     got = ops.hadamard(x, signs, block, transpose, 0.7, residual=res, clear_in=f32)
-    assert (got.float() - want.float()).abs().max() <= 2e-3 * want.float().abs().max()
+    assert torch.equal(got, want)
     assert not f32 or not x.any()                        # the accumulator is left zeroed
     if not f32:                                          # in place
         assert torch.equal(ops.hadamard(x, signs, block, transpose, 0.7, residual=res, out=x), got)
-
-
-@pytest.mark.parametrize("n,block", [(256, 256), (512, 64), (2816, 256), (11008, 256)])
-def test_swiglu_of_many_rows_matches_single_rows(n, block):
-    from rptc_b200 import ops
-    g = torch.Generator(device="cuda").manual_seed(n)
-    rows = 45
-    gu = torch.randn((rows, 2 * n), generator=g, device="cuda").half()
-    so, si = [(torch.randint(0, 2, (k,), generator=g, device="cuda") * 2 - 1).half() for k in (2 * n, n)]
-    one = lambda a: ops.swiglu_hadamard_f16(a, torch.empty((a.shape[0], n), dtype=torch.float16, device="cuda"), so, si, n, block, 0.8, 1.1)
-    want, got = torch.cat([one(gu[r:r + 1]) for r in range(rows)]), one(gu)
-    assert (got.float() - want.float()).abs().max() <= 2e-3 * want.float().abs().max()
 
 
 @pytest.mark.parametrize("n", [4096, 8192])
@@ -211,11 +201,11 @@ def test_prompt_norm_matches_its_parts(n, with_y):
     f16 = lambda *s: torch.randn(*s, generator=g, device="cuda").half()
     h, y, w = f16(rows, n), f16(rows, n), (1 + 0.1 * f16(n))
     so, si = [(torch.randint(0, 2, (n,), generator=g, device="cuda") * 2 - 1).half() for _ in range(2)]
-    h_want = ops.hadamard(y, so, 4096, transpose=True, scale=0.3, residual=h) if with_y else h.clone()
-    want = ops.hadamard(ops.rmsnorm(h_want, w, torch.empty_like(h), eps), si, 4096)
+    few = lambda x, *a, **k: torch.cat([ops.hadamard(x[r:r + 25], *a, **{**k, "residual": h[r:r + 25] if k else None}) for r in range(0, rows, 25)])
+    h_want = few(y, so, 4096, transpose=True, scale=0.3) if with_y else h.clone()
+    want = few(ops.rmsnorm(h_want, w, torch.empty_like(h), eps), si, 4096)
     got = ops.prompt_norm(y if with_y else None, so, 0.3, h, w, eps, si, torch.empty_like(h))
-    assert (h.float() - h_want.float()).abs().max() <= 2e-3 * h_want.float().abs().max()
-    assert (got.float() - want.float()).norm() <= 2e-3 * want.float().norm()
+    assert torch.equal(h, h_want) and torch.equal(got, want)
 
 
 @pytest.mark.parametrize("rows,tokens,hq,hkv", [(1, 40, 4, 1), (2, 33, 32, 8), (1, 2048, 4, 4)])
@@ -230,4 +220,4 @@ def test_prompt_qkv_matches_its_parts(rows, tokens, hq, hkv):
     ops.rope_cache_prompt(want, rows, tokens, *caches[0], hq, hkv, 128, 10000.0)
     ops.prompt_qkv(qkv, signs, 0.5, rows, tokens, *caches[1], hq, hkv, ops.rope_angles(tokens, 10000.0, "cuda:0"))
     for a, b in ((qkv[:, : hq * 128], want[:, : hq * 128]), (caches[1][0], caches[0][0]), (caches[1][1], caches[0][1])):
-        assert (a.float() - b.float()).abs().max() <= 2e-3 * b.float().abs().max()
+        assert torch.equal(a, b)

@@ -388,3 +388,27 @@ def test_fused_matvec_sixteen_rows_matches_two_calls_of_eight():
     assert torch.equal(y, dense.t()[100:116])
     y13 = ops.gemv(codes, lut, x[:13], m, n, fmt)                           # 8 + 4 + 1
     assert torch.equal(y13, dense.t()[100:113])
+
+
+@pytest.mark.parametrize("rows,heads,kv_heads", [(5, 32, 32), (9, 32, 8), (16, 32, 32), (3, 8, 2)])
+def test_attention_of_many_rows_matches_single_rows(rows, heads, kv_heads):
+    """CTAs of 16, 8 and 4 warps (by the number of rows x heads) against one row at a time, contexts from the first position
+    to several chunks."""
+    from rptc_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    max_pos, n = 700, (heads + 2 * kv_heads) * 128
+    pos = torch.tensor([0, 1, 63, 64, 130, 255, 256, 600, 699, 7, 31, 400, 511, 512, 99, 128][:rows], dtype=torch.int32, device="cuda")
+    acc = torch.randn((rows, n), generator=g, device="cuda")
+    caches = [torch.randn((rows, max_pos, kv_heads, 128), generator=g, device="cuda").half() for _ in range(2)]
+    so, si = [(torch.randint(0, 2, (k,), generator=g, device="cuda") * 2 - 1).half() for k in (n, heads * 128)]
+
+    def attend(r):
+        k, v = caches[0][r].clone(), caches[1][r].clone()
+        out = torch.empty((k.shape[0], heads * 128), dtype=torch.float16, device="cuda")
+        ops.qkv_attn_decode(acc[r].clone(), so, 0.05, pos[r].clone(), k, v, out, heads, kv_heads, 10000.0, si)
+        return out, k, v
+
+    want = [torch.cat(parts) for parts in zip(*[attend(slice(r, r + 1)) for r in range(rows)])]
+    for a, b in zip(attend(slice(0, rows)), want):
+        assert (a.float() - b.float()).abs().max() <= 2e-3 * b.float().abs().max()
+    ops.device_status()
