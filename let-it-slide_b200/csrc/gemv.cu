@@ -54,8 +54,7 @@ struct GemvParams {
     SwigluParams sw;
     float *clear;
     int64_t clear_count;
-    // gemv_rows_kernel, MODE 0: CTAs per bank of rows, fp16 elements from one bank's table to the next
-    int32_t ctas;
+    // gemv_rows_kernel, MODE 0: fp16 elements from one bank's table to the next
     int64_t lut_stride;
 };
 
@@ -237,9 +236,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
         if (threadIdx.x == 0) atomicExch(p.status, kStatusSmemPlan);
         return;
     }
-    // the bank this CTA works on, and its number among the bank's CTAs
-    const uint32_t bank = MODE == 0 ? blockIdx.x / (uint32_t)p.ctas : 0u, n_ctas = MODE == 0 ? (uint32_t)p.ctas : gridDim.x;
-    const uint32_t cta = blockIdx.x - bank * n_ctas;
+    // the bank this CTA works on (MODE 0: one grid row per bank), and its number among the bank's CTAs
+    const uint32_t bank = MODE == 0 ? blockIdx.y : 0u, n_ctas = gridDim.x, cta = blockIdx.x;
     const __half *table = p.lut + (MODE == 0 ? (int64_t)bank * p.lut_stride : 0);
     const uint4 *codes = p.codes + (MODE == 0 ? (int64_t)bank * p.m * p.n_units : 0);
     float *acc = p.acc + (MODE == 0 ? (int64_t)bank * p.m : 0);
@@ -583,15 +581,15 @@ static int launch_gemv(const GemvParams &p, size_t smem, cudaStream_t stream) {
 }
 
 template <int CODE, int K, int BATCH, int MODE>
-static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t stream, int grid = num_sms()) {
+static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t stream, dim3 grid = dim3(num_sms())) {
     static SmemOptIn opted;
     auto kern = gemv_rows_kernel<CODE, K, BATCH, MODE>;
     if (int e = allow_max_smem(kern, opted)) return e;
-    return launch(kern, dim3(grid), dim3(kGemvThreads), smem, stream, p);
+    return launch(kern, grid, dim3(kGemvThreads), smem, stream, p);
 }
 
 template <int CODE, int K>
-static int dispatch(const GemvParams &p, int batch, bool tiled, size_t smem, int grid, cudaStream_t stream) {
+static int dispatch(const GemvParams &p, int batch, bool tiled, size_t smem, dim3 grid, cudaStream_t stream) {
     if (!tiled) return batch == 1 && !p.in.h_in ? launch_gemv<CODE, K>(p, smem, stream) : RPTC_ERR_UNSUPPORTED;
     if (p.in.h_in) {
         if (batch > 2) return RPTC_ERR_UNSUPPORTED;
@@ -631,9 +629,9 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
     const bool tma = f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE;
     p.in = in ? *in : rptc_gemv_input{};
     // one bank's table per CTA: the SMs are dealt out to the banks
-    p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
+    const int ctas = num_sms() / banks.banks;
+    const dim3 grid((unsigned)(ctas > 0 ? ctas : 1), (unsigned)banks.banks);
     p.lut_stride = banks.lut_stride;
-    const int grid = banks.banks * p.ctas;
 
     // shared-memory plan (must mirror the kernel's)
     const size_t kMaxSmem = 227 * 1024 - 1024;     // leave room for the 1 KiB the system may reserve

@@ -1,0 +1,269 @@
+// The layers' forward passes as the interpreter calls them.  The library itself (librptc_b200.so) knows no tensors; what lies
+// between a module's `forward` and its entry points -- reading the module's attributes, checks, the result and the
+// workspace, device and stream -- cost 12 us of Python and ctypes per call, as much as the kernels of a one-token pass.
+// Functions return the result, or the rptc_status of the entry point as an int (the caller raises).
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <exception>
+
+#include "../../include/rptc_b200.h"
+
+namespace {
+
+// Entry points of the library that the Python side has loaded.
+struct {
+    decltype(&rptc_linear_workspace_bytes) linear_workspace_bytes;
+    decltype(&rptc_linear_forward) linear_forward;
+    decltype(&rptc_packed_workspace_bytes) packed_workspace_bytes;
+    decltype(&rptc_packed_forward) packed_forward;
+    decltype(&rptc_gemv_timed) gemv_timed;
+} g_lib;
+
+#define RPTC_NAMES(X) X(in_features) X(out_features) X(block_in) X(block_out) X(scale) X(fmt) X(_buffers) X(codes) X(lut) X(carry_in) \
+    X(signs_in) X(signs_out) X(num_banks) X(bank_blocks) X(L) X(alphabets) X(biases_out) X(biases_in) X(scales_out) X(scales_in) X(bias)
+struct Names {
+#define RPTC_FIELD(n) PyObject *n;
+    RPTC_NAMES(RPTC_FIELD)
+} g_names;
+
+struct PyError : std::exception {};      // the interpreter's error is set
+[[noreturn]] void fail(const char *what) {
+    PyErr_SetString(PyExc_RuntimeError, what);
+    throw PyError();
+}
+
+// A module's instance attributes and buffers, without the module's __getattr__.
+class Attributes {
+public:
+    explicit Attributes(PyObject *module) : dict_(PyObject_GenericGetDict(module, nullptr)) {
+        if (!dict_) throw PyError();
+        buffers_ = get(dict_, g_names._buffers);
+    }
+    Attributes(const Attributes &) = delete;
+    ~Attributes() { Py_XDECREF(dict_); }
+    PyObject *object(PyObject *name) const { return get(dict_, name); }
+    int64_t integer(PyObject *name) const {
+        const long long v = PyLong_AsLongLong(get(dict_, name));
+        if (v == -1 && PyErr_Occurred()) throw PyError();
+        return v;
+    }
+    double number(PyObject *name) const {
+        const double v = PyFloat_AsDouble(get(dict_, name));
+        if (v == -1.0 && PyErr_Occurred()) throw PyError();
+        return v;
+    }
+    // a buffer's tensor, or null for None
+    const at::Tensor *buffer(PyObject *name) const {
+        PyObject *o = get(buffers_, name);
+        if (o == Py_None) return nullptr;
+        if (!THPVariable_Check(o)) fail("a buffer of the layer is not a tensor");
+        return &THPVariable_Unpack(o);
+    }
+    const void *pointer(PyObject *name) const {
+        const at::Tensor *t = buffer(name);
+        return t ? t->data_ptr() : nullptr;
+    }
+
+private:
+    static PyObject *get(PyObject *dict, PyObject *name) {
+        PyObject *o = PyDict_GetItemWithError(dict, name);
+        if (!o) {
+            if (!PyErr_Occurred()) PyErr_SetObject(PyExc_AttributeError, name);
+            throw PyError();
+        }
+        return o;
+    }
+    PyObject *dict_, *buffers_ = nullptr;
+};
+
+const at::Tensor &unpack(PyObject *o, const char *what) {
+    if (!THPVariable_Check(o)) fail(what);
+    return THPVariable_Unpack(o);
+}
+
+rptc_format format_of(PyObject *structure) {      // the ctypes mirror of rptc_format
+    rptc_format f;
+    Py_buffer view;
+    if (PyObject_GetBuffer(structure, &view, PyBUF_SIMPLE)) throw PyError();
+    const bool fits = view.len == (Py_ssize_t)sizeof(f);
+    if (fits) memcpy(&f, view.buf, sizeof(f));
+    PyBuffer_Release(&view);
+    if (!fits) fail("fmt is not a Format");
+    return f;
+}
+
+// The activations as the kernels read them: contiguous, 16-byte aligned.
+at::Tensor ready(const at::Tensor &x) {
+    at::Tensor t = x.contiguous();
+    if (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) t = t.clone(at::MemoryFormat::Contiguous);
+    return t;
+}
+
+at::Tensor result_like(const at::Tensor &x, int64_t columns) {
+    at::DimVector shape(x.sizes());
+    shape.back() = columns;
+    return at::empty(shape, x.options().requires_grad(false));
+}
+
+template <typename F>
+PyObject *guarded(F &&f) {
+    try {
+        return f();
+    } catch (const PyError &) {
+    } catch (const c10::Error &e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const std::exception &e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return nullptr;
+}
+
+cudaStream_t current_stream(const at::Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// linear_forward(module, x)
+PyObject *linear_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 2) fail("linear_forward(module, x)");
+        const Attributes a(args[0]);
+        const at::Tensor &x_in = unpack(args[1], "x must be a tensor");
+        rptc_linear l;
+        l.m = a.integer(g_names.out_features);
+        l.n = a.integer(g_names.in_features);
+        if (!x_in.is_cuda()) fail("x must be a CUDA tensor");
+        if (x_in.dim() < 1 || x_in.size(-1) != l.n || x_in.numel() == 0) fail("x must have in_features columns and at least one row");
+        const at::Tensor *codes = a.buffer(g_names.codes);
+        if (!codes) fail("the layer has no codes");
+        l.codes = codes->data_ptr();
+        l.lut = a.pointer(g_names.lut);
+        l.carry_in = static_cast<const uint32_t *>(a.pointer(g_names.carry_in));
+        l.signs_in = a.pointer(g_names.signs_in);
+        l.signs_out = a.pointer(g_names.signs_out);
+        l.block_in = (int32_t)a.integer(g_names.block_in);
+        l.block_out = (int32_t)a.integer(g_names.block_out);
+        l.scale = (float)a.number(g_names.scale);
+        l.fmt = format_of(a.object(g_names.fmt));
+        const c10::cuda::OptionalCUDAGuard guard(codes->device());
+        const at::Tensor x = ready(x_in.scalar_type() == at::kHalf ? x_in : x_in.to(at::kHalf));
+        const int64_t rows = x.numel() / l.n;
+        at::Tensor y = result_like(x, l.m);
+        const int64_t need = g_lib.linear_workspace_bytes(&l, rows);
+        at::Tensor ws = at::empty({need > 0 ? need : 1}, x.options().dtype(at::kByte));
+        const int status = g_lib.linear_forward(&l, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need, current_stream(*codes));
+        if (status != RPTC_OK) return PyLong_FromLong(status);
+        // beyond 64 rows the product of a layer without transforms leaves the scale to be applied
+        if (!l.signs_in && rows > 64 && l.scale != 1.f) y = y * a.number(g_names.scale);
+        return THPVariable_Wrap(std::move(y));
+    });
+}
+
+// packed_forward(module, x)
+PyObject *packed_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 2) fail("packed_forward(module, x)");
+        const Attributes a(args[0]);
+        const at::Tensor &x_in = unpack(args[1], "x must be a tensor");
+        rptc_packed l;
+        l.m = a.integer(g_names.out_features);
+        l.n = a.integer(g_names.in_features);
+        if (!x_in.is_cuda()) fail("x must be a CUDA tensor");
+        if (x_in.dim() < 1 || x_in.size(-1) != l.n) fail("x must have in_features columns");
+        const at::ScalarType type = x_in.scalar_type();
+        const int dtype = type == at::kHalf ? 0 : type == at::kBFloat16 ? 1 : 2;
+        const c10::cuda::OptionalCUDAGuard guard(x_in.device());
+        const at::Tensor x = ready(dtype == 2 && type != at::kFloat ? x_in.to(at::kFloat) : x_in);
+        at::Tensor y = result_like(x, l.m);
+        const int64_t tokens = x.numel() / l.n;
+        if (tokens > 0) {
+            l.codes = a.pointer(g_names.codes);
+            l.alphabets = a.pointer(g_names.alphabets);
+            l.biases_out = static_cast<const float *>(a.pointer(g_names.biases_out));
+            l.biases_in = static_cast<const float *>(a.pointer(g_names.biases_in));
+            l.scales_out = static_cast<const float *>(a.pointer(g_names.scales_out));
+            l.scales_in = static_cast<const float *>(a.pointer(g_names.scales_in));
+            l.bias = static_cast<const float *>(a.pointer(g_names.bias));
+            l.banks = (int32_t)a.integer(g_names.num_banks);
+            l.bank_blocks = (int32_t)a.integer(g_names.bank_blocks);
+            l.L = (int32_t)a.integer(g_names.L);
+            const int64_t most = tokens < 65535 ? tokens : 65535;      // tokens per native call
+            const int64_t need = g_lib.packed_workspace_bytes(&l, most);
+            if (need < 0) return PyLong_FromLong(RPTC_ERR_SHAPE);
+            at::Tensor ws = at::empty({need}, x.options().dtype(at::kByte));
+            const char *xp = static_cast<const char *>(x.data_ptr());
+            char *yp = static_cast<char *>(y.data_ptr());
+            const int64_t width = x.element_size();
+            for (int64_t t = 0; t < tokens; t += most) {
+                const int status = g_lib.packed_forward(&l, xp + t * l.n * width, dtype, yp + t * l.m * width, most < tokens - t ? most : tokens - t,
+                                                        ws.data_ptr(), need, current_stream(x));
+                if (status != RPTC_OK) return PyLong_FromLong(status);
+            }
+        }
+        if (y.scalar_type() != type) y = y.to(type);
+        return THPVariable_Wrap(std::move(y));
+    });
+}
+
+// gemv_timed(codes, lut, x, acc, y, m, n, x_order, accumulate, fmt): milliseconds, or the status
+PyObject *gemv_timed(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 10) fail("gemv_timed(codes, lut, x, acc, y, m, n, x_order, accumulate, fmt)");
+        const at::Tensor *t[5];
+        for (int i = 0; i < 5; ++i) t[i] = &unpack(args[i], "expected a tensor");
+        long long v[4];
+        for (int i = 0; i < 4; ++i) {
+            v[i] = PyLong_AsLongLong(args[5 + i]);
+            if (v[i] == -1 && PyErr_Occurred()) throw PyError();
+        }
+        const rptc_format fmt = format_of(args[9]);
+        const c10::cuda::OptionalCUDAGuard guard(t[4]->device());
+        const cudaStream_t s = current_stream(*t[4]);
+        float ms = 0.f;
+        int status;
+        Py_BEGIN_ALLOW_THREADS                                        // waits for the result
+        status = g_lib.gemv_timed(t[0]->data_ptr(), t[1]->data_ptr(), t[2]->data_ptr(), static_cast<float *>(t[3]->data_ptr()), t[4]->data_ptr(),
+                                  v[0], v[1], (int)v[2], (int)v[3], &fmt, &ms, s);
+        Py_END_ALLOW_THREADS
+        return status == RPTC_OK ? PyFloat_FromDouble(ms) : PyLong_FromLong(status);
+    });
+}
+
+// bind(linear_workspace_bytes, linear_forward, packed_workspace_bytes, packed_forward, gemv_timed): addresses
+PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 5) fail("bind(five addresses)");
+        void *p[5];
+        for (int i = 0; i < 5; ++i) {
+            p[i] = PyLong_AsVoidPtr(args[i]);
+            if (!p[i]) {
+                if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "null address");
+                throw PyError();
+            }
+        }
+        g_lib.linear_workspace_bytes = reinterpret_cast<decltype(g_lib.linear_workspace_bytes)>(p[0]);
+        g_lib.linear_forward = reinterpret_cast<decltype(g_lib.linear_forward)>(p[1]);
+        g_lib.packed_workspace_bytes = reinterpret_cast<decltype(g_lib.packed_workspace_bytes)>(p[2]);
+        g_lib.packed_forward = reinterpret_cast<decltype(g_lib.packed_forward)>(p[3]);
+        g_lib.gemv_timed = reinterpret_cast<decltype(g_lib.gemv_timed)>(p[4]);
+        Py_RETURN_NONE;
+    });
+}
+
+#define RPTC_METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
+PyMethodDef g_methods[] = {RPTC_METHOD(bind), RPTC_METHOD(linear_forward), RPTC_METHOD(packed_forward), RPTC_METHOD(gemv_timed),
+                           {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native() {
+#define RPTC_INTERN(n) \
+    g_names.n = PyUnicode_InternFromString(#n); \
+    if (!g_names.n) return nullptr;
+    RPTC_NAMES(RPTC_INTERN)
+    return PyModule_Create(&g_module);
+}

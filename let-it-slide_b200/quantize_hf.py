@@ -32,13 +32,10 @@ from torch import nn
 
 from rptc import pack_symbols, quantize_rows
 from rptc_b200 import CODE_LUT, LAYOUT_ROWMAJOR, LAYOUT_TILED, Format, ops
-from rptc_b200._lib import Packed, call, lib
+from rptc_b200._lib import RPTCError, native
 
 # Hugging Face projection name -> name of the fused layer its statistics are filed under (quantize_hf.py:14-22)
 hf_to_fused = {"q": "qkv", "k": "qkv", "v": "qkv", "o": "o", "up": "up", "gate": "up", "down": "down"}
-
-# activation types that rptc_packed_forward reads and writes as they are
-_NATIVE_DTYPES = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
 
 _PROJ = re.compile(r"model\.layers\.(\d+)\.(self_attn\.(\w+)_proj|mlp\.(\w+)_proj)")      # quantize_hf.py:189
 
@@ -197,30 +194,10 @@ class FactorizedRPTCLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """One native call (rptc_packed_forward): scaled fp16 activations and the two sums over x, the product of all banks
         in one launch, then scales and biases."""
-        m, n, dt = self.out_features, self.in_features, x.dtype
-        dtype = _NATIVE_DTYPES.get(dt)
-        if dtype is None:
-            x, dtype = x.float(), 2
-        if x.shape[-1] != n:
-            raise RuntimeError(f"x must have {n} columns, got {tuple(x.shape)}")
-        if not x.is_contiguous() or x.data_ptr() & 15:
-            x = x.clone(memory_format=torch.contiguous_format)
-        tokens = x.numel() // n
-        y = torch.empty((*x.shape[:-1], m), dtype=x.dtype, device=x.device)
-        if tokens == 0:
-            return y.to(dt)
-        buffers = self._buffers                       # not through Module.__getattr__: seven lookups per call
-        d = Packed(*[buffers[name].data_ptr() for name in ("codes", "alphabets", "biases_out", "biases_in", "scales_out", "scales_in")],
-                   None if buffers["bias"] is None else buffers["bias"].data_ptr(), m, n, self.num_banks, self.bank_blocks, self.L)
-        most = min(tokens, 65535)                     # tokens per native call
-        need = lib().rptc_packed_workspace_bytes(d, most)
-        if need < 0:
-            raise RuntimeError("rptc_packed_workspace_bytes: shape not supported")
-        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
-        for t in range(0, tokens, most):
-            call("rptc_packed_forward", x.device, d, x.data_ptr() + t * n * x.element_size(), dtype, y.data_ptr() + t * m * y.element_size(),
-                 min(most, tokens - t), ws.data_ptr(), need)
-        return y if y.dtype == dt else y.to(dt)
+        y = native().packed_forward(self, x)
+        if type(y) is int:
+            raise RPTCError(y, "rptc_packed_forward")
+        return y
 
     def extra_repr(self) -> str:
         return f"{self.in_features} -> {self.out_features}, L={self.L}, banks={self.num_banks}"

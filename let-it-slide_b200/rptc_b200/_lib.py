@@ -207,6 +207,22 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The extension module with the layers' forward passes (csrc/torch_ext.cpp), bound to the library loaded here.  Fails
+    loudly when it has not been built."""
+    global _native
+    if _native is None:
+        from . import _native as ext
+        L = lib()
+        ext.bind(*[ctypes.cast(getattr(L, "rptc_" + name), ctypes.c_void_p).value for name in (
+            "linear_workspace_bytes", "linear_forward", "packed_workspace_bytes", "packed_forward", "gemv_timed")])
+        _native = ext
+    return _native
+
+
 def exported_symbols() -> list[str]:
     return list(_SIGS)
 

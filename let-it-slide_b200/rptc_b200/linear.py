@@ -14,7 +14,7 @@ import torch
 from torch import nn
 
 from . import ops
-from ._lib import CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_TILED, Format, Linear, call, lib, ptr
+from ._lib import CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_TILED, Format, RPTCError, native
 
 
 def hadamard_block(n: int) -> int:
@@ -123,26 +123,19 @@ class RPTCLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """One native call (rptc_linear_forward): input transform, fused product, output transform."""
-        m, n = self.out_features, self.in_features
-        if x.dtype != torch.float16:
-            x = x.to(torch.float16)
-        if not x.is_contiguous() or x.data_ptr() & 15:
-            x = x.clone(memory_format=torch.contiguous_format)
-        rows = x.numel() // n
-        y = torch.empty((*x.shape[:-1], m), dtype=torch.float16, device=x.device)
-        if x.shape[-1] != n or rows == 0:
-            raise RuntimeError(f"x must have {n} columns and at least one row, got {tuple(x.shape)}")
-        buffers = self._buffers                       # not through Module.__getattr__: five lookups per call
-        codes = buffers["codes"]
-        d = Linear(codes.data_ptr(), buffers["lut"].data_ptr(), ptr(buffers["carry_in"]), ptr(buffers["signs_in"]), ptr(buffers["signs_out"]),
-                   m, n, self.block_in, self.block_out, self.scale, self.fmt)
-        fused_scale = self.incoherent or rows <= 64
-        need = lib().rptc_linear_workspace_bytes(d, rows)
-        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
-        call("rptc_linear_forward", codes.device, d, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need)
-        if not fused_scale and self.scale != 1.0:
-            y = y * self.scale
+        if self.fmt.layout != LAYOUT_TILED or self.fmt.quirk:
+            return self._forward_by_parts(x)
+        y = native().linear_forward(self, x)
+        if type(y) is int:
+            raise RPTCError(y, "rptc_linear_forward")
         return y
+
+    def _forward_by_parts(self, x: torch.Tensor) -> torch.Tensor:
+        """The reference's layouts: one row at a time goes through the general matvec kernel."""
+        x2 = x.reshape(-1, self.in_features).to(torch.float16).contiguous()
+        xt, acc = self.transform_in(x2), self.acc_buffer(x2.shape[0])
+        self.matvec_acc(xt, acc)
+        return self.finish(acc).reshape(*x.shape[:-1], self.out_features)
 
     # -- reference helpers ----------------------------------------------------------------------------
     def decoded(self) -> torch.Tensor:

@@ -25,7 +25,7 @@ import torch
 
 from rptc_b200 import (CODE_HASH, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_UNITMAJOR, QUIRK_K1_LANE0_SEED,
                        QUIRK_K2_LANE0_CARRY, QUIRK_NONE, XORDER_K2_LEGACY, XORDER_NATURAL, Format, ops)
-from rptc_b200._lib import call
+from rptc_b200._lib import RPTCError, call, native
 
 _quirks = False
 _scratch: dict[tuple[int, int, int], torch.Tensor] = {}
@@ -70,15 +70,11 @@ def _timed(device: torch.device, fn) -> float:
 
 def _timed_matvec(compressed, codebook, x, out, m: int, n: int, fmt: Format, x_order: int, accumulate: bool) -> float:
     """out = (or +=) W x and the device time it took, in one native call."""
-    device, ms = out.device, ctypes.c_float()
-    acc = _acc(device, m)
-    try:
-        call("rptc_gemv_timed", device, compressed.data_ptr(), codebook.data_ptr(), x.data_ptr(), acc.data_ptr(), out.data_ptr(), m, n, x_order,
-             int(accumulate), fmt, ms)
-    except Exception:
+    ms = native().gemv_timed(compressed, codebook, x, _acc(out.device, m), out, m, n, x_order, int(accumulate), fmt)
+    if type(ms) is int:
         _scratch.clear()      # an accumulator that was not finished is not zero
-        raise
-    return ms.value
+        raise RPTCError(ms, "rptc_gemv_timed")
+    return ms
 
 
 def matvec(decompressed: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> float:
