@@ -153,7 +153,8 @@ __device__ __forceinline__ float block_sum(float v, float *red) {      // red: >
 // (1) optional: h = residual + s_out * H(acc) * scale   (the output side of a row's previous layer; acc cleared)
 // (2) xn = rmsnorm(h) * w_norm
 // (3) out = H(s_in * xn) * norm   (the input side of the next layer), or out = xn when no transform is wanted.
-// One CTA per row: n / 8 threads; the row is one Hadamard block (n <= 4096) or two of 4096 (n = 8192).
+// One CTA per row: n / 8 threads, the row is one Hadamard block (finish_norm_row, n <= 2048); or 256 threads per 4096 elements
+// (finish_norm_unit, n = 4096 or 8192).
 struct FinishNormParams {
     float *acc;                  // fp32 [rows][ld_acc] or NULL (then h is read as it is)
     int64_t ld_acc;
@@ -172,43 +173,30 @@ struct FinishNormParams {
     int32_t block;               // Hadamard block of both transforms (n, or 4096 when n = 8192)
 };
 
-// One row; called by all n/8 threads of a CTA.  `owner`: this CTA is the one that clears the accumulator behind
-// its read and stores the updated residual.  When several CTAs compute the same row (each for its own use),
-// exactly one of them is the owner of the residual and nobody clears; the residual then needs h_out != h.
-// `ex_idle`: no thread can still be reading the exchange buffer when this call starts (first use in the kernel).
-// `after_loads`: called once the row's global loads have been issued and before their values are used -- a place for
-// work that should overlap the loads' trip through L2 (e.g. writing a lookup table to shared memory).
-template <typename Hook = NoHook>
-__device__ __forceinline__ void finish_norm_row(const FinishNormParams &p, int64_t row, float *ex, float *red, bool clear_acc,
-                                                bool write_h, bool ex_idle = false, Hook after_loads = Hook()) {
+// One row by all n / 8 threads of a CTA (n <= 2048): the accumulator is cleared behind its read, the residual updated in place.
+__device__ __forceinline__ void finish_norm_row(const FinishNormParams &p, int64_t row, float *ex, float *red) {
     const int t = threadIdx.x;
     const int col = 8 * t;
     const float hn = hadamard_norm_dev(p.block);
     // every global load is issued before the first dependent use: one memory round trip for the kernel
     const uint4 raw_so = raw8_or_ones(p.signs_out ? p.signs_out + col : nullptr);
-    const uint4 raw_h = clear_acc ? *reinterpret_cast<const uint4 *>(p.h + row * p.ld_h + col)
-                                  : __ldcg(reinterpret_cast<const uint4 *>(p.h + row * p.ld_h + col));
+    const uint4 raw_h = *reinterpret_cast<const uint4 *>(p.h + row * p.ld_h + col);
     const uint4 raw_w = *reinterpret_cast<const uint4 *>(p.w_norm + col);
     const uint4 raw_si = raw8_or_ones(p.signs_in ? p.signs_in + col : nullptr);
     float v[8], sg[8];
     if (p.acc) {
-        if (clear_acc) load8_f32(p.acc + row * p.ld_acc + col, v, true);
-        else load8_f32_cg(p.acc + row * p.ld_acc + col, v);
-    }
-    after_loads();
-    if (p.acc) {
-        fwht8(v, p.block, ex, !ex_idle);
+        load8_f32(p.acc + row * p.ld_acc + col, v, true);
+        fwht8(v, p.block, ex, false);
         unpack8(raw_so, sg);
         float r[8];
         unpack8(raw_h, r);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = r[i] + v[i] * (p.scale_out * hn) * sg[i];
-        if (write_h) store8_f16((p.h_out ? p.h_out : p.h) + row * p.ld_h + col, v);
+        store8_f16(p.h + row * p.ld_h + col, v);
         // continue from the rounded residual stream, as an unfused reader of h would
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __half2float(__float2half_rn(v[i]));
     } else {
-        if (write_h && p.h_out) *reinterpret_cast<uint4 *>(p.h_out + row * p.ld_h + col) = raw_h;
         unpack8(raw_h, v);
     }
     float ss = 0.f;
@@ -230,57 +218,173 @@ __device__ __forceinline__ void finish_norm_row(const FinishNormParams &p, int64
     store8_f16(p.out + row * p.ld_out + col, v);
 }
 
-// The same for a row of NH x 4096 elements handled by 512 threads (thread t holds elements 8t..8t+7 of every 4096-wide
-// piece; each piece is one Hadamard block): the form used inside a 512-thread matvec CTA for 8192-wide models.  Never
-// clears the accumulator (several CTAs read it); p.block must be 4096.
-template <int NH>
-__device__ __forceinline__ void finish_norm_row_wide(const FinishNormParams &p, int64_t row, float *ex, float *red, bool write_h,
-                                                     bool ex_idle) {
-    const int t = threadIdx.x;
-    const float hn = hadamard_norm_dev(4096);
-    float v[NH][8];
+// ---- the same for blocks of 4096, 256 threads ("a unit") per block -----------------------------------------------------------
+// Sixteen values a thread: 4096 = 16 x 16 x 16, so that a transform is three times four stages in registers with two exchanges
+// through shared memory between them, one of which stays inside the warp.  Against eight values a thread with shuffles (72
+// wavefronts of the shared-memory pipe per 256 elements, three barriers) it takes 48 and one barrier.
+//   far      element t + 256 k        (k = 0..15: bits 8-11)
+//   middle   element (t & 15) + 16 k + 256 (t >> 4)
+//   near     element 16 t + k: loads and stores of fp16 are 32 contiguous bytes
+// Element e sits at e + 4 (e >> 5) + 16 (e >> 8) of the exchange buffer: no bank conflicts in any of the three.
+constexpr int kUnitThreads = 256, kUnitFloats = 4096 + 4 * 128 + 16 * 16;
+__device__ __forceinline__ int unit_at(int e) { return e + 4 * (e >> 5) + 16 * (e >> 8); }
+__device__ __forceinline__ void unit_barrier(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kUnitThreads) : "memory"); }
+
+__device__ __forceinline__ void stages16(float (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const float a = v[i], b = v[i + 1];
+        v[i] = a + b;
+        v[i + 1] = a - b;
+    }
+#pragma unroll
+    for (int h = 2; h < 16; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 16; i += 2)
+            if ((i & h) == 0) {                // two neighbours at a time
+                const f32x2 a = pack2(v[i], v[i + 1]), b = pack2(v[i + h], v[i + h + 1]);
+                unpack2(add2(a, b), v[i], v[i + 1]);
+                unpack2(sub2(a, b), v[i + h], v[i + h + 1]);
+            }
+}
+// far -> near with all twelve stages; `bar`: a named barrier of the unit
+__device__ __forceinline__ void unit_transform_to_near(float (&v)[16], float *ex, int t, int bar) {
+    stages16(v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ex[unit_at(t + 256 * k)] = v[k];
+    unit_barrier(bar);
+    const int m = (t & 15) + 256 * (t >> 4);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = ex[unit_at(m + 16 * k)];
+    stages16(v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ex[unit_at(m + 16 * k)] = v[k];
+    __syncwarp();
+    const float4 *q = reinterpret_cast<const float4 *>(ex + unit_at(16 * t));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 f = q[j];
+        v[4 * j] = f.x, v[4 * j + 1] = f.y, v[4 * j + 2] = f.z, v[4 * j + 3] = f.w;
+    }
+    stages16(v);
+}
+// near -> far with all twelve stages.  The thread's own elements may still hold what it read above.
+__device__ __forceinline__ void unit_transform_to_far(float (&v)[16], float *ex, int t, int bar) {
+    stages16(v);
+    float4 *q = reinterpret_cast<float4 *>(ex + unit_at(16 * t));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+    const int m = (t & 15) + 256 * (t >> 4);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = ex[unit_at(m + 16 * k)];
+    stages16(v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ex[unit_at(m + 16 * k)] = v[k];
+    unit_barrier(bar);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = ex[unit_at(t + 256 * k)];
+    stages16(v);
+}
+
+__device__ __forceinline__ void unpack16(const uint4 (&r)[2], float (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint4 &q = r[i >> 2];
+        const float2 f = __half22float2(u32_as_half2((i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w));
+        v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void pack16(const float (&v)[16], uint4 (&r)[2]) {
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = half2_as_u32(__floats2half2_rn(v[2 * i], v[2 * i + 1]));
+    r[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    r[1] = make_uint4(o[4], o[5], o[6], o[7]);
+}
+
+// finish_norm_row for elements [4096 part, 4096 part + 4096) of a row of 4096 or 8192 by one unit of 256 threads; the two units
+// of a row of 8192 call it together.  ex: kUnitFloats of the unit's own; red: 16 floats of the row's; bar: named barrier of the
+// unit; pair_bar: named barrier of the 512 threads of both units.
+template <typename Hook = NoHook>
+__device__ __forceinline__ void finish_norm_unit(const FinishNormParams &p, int64_t row, int part, float *ex, float *red, int bar, int pair_bar,
+                                                 bool clear_acc, bool write_h, Hook after_loads = Hook()) {
+    const int t = threadIdx.x & (kUnitThreads - 1), lane = t & 31, warp = t >> 5;
+    const int col0 = 4096 * part, col = col0 + 16 * t;
+    const float hn = 0.015625f;                              // 1 / sqrt(4096)
+    const uint4 ones = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+    // every global load is issued before the first dependent use: one memory round trip
+    float v[16];
+    uint4 rh[2], rso[2], rw[2], rsi[2];
+    if (p.acc) {
+        float *acc = p.acc + row * p.ld_acc + col0 + t;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = __ldcg(acc + 256 * k);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        rh[i] = __ldcg(reinterpret_cast<const uint4 *>(p.h + row * p.ld_h + col) + i);
+        rso[i] = p.signs_out ? *(reinterpret_cast<const uint4 *>(p.signs_out + col) + i) : ones;
+        rw[i] = *(reinterpret_cast<const uint4 *>(p.w_norm + col) + i);
+        rsi[i] = p.signs_in ? *(reinterpret_cast<const uint4 *>(p.signs_in + col) + i) : ones;
+    }
+    after_loads();
+    if (p.acc) {
+        if (clear_acc) {
+            float *acc = p.acc + row * p.ld_acc + col0 + t;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) acc[256 * k] = 0.f;
+        }
+        unit_transform_to_near(v, ex, t, bar);
+        float so[16], r[16];
+        unpack16(rso, so);
+        unpack16(rh, r);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = r[i] + v[i] * (p.scale_out * hn) * so[i];
+        pack16(v, rh);
+    }
+    if (write_h && (p.acc || p.h_out)) {
+        uint4 *dst = reinterpret_cast<uint4 *>((p.h_out ? p.h_out : p.h) + row * p.ld_h + col);
+        dst[0] = rh[0];
+        dst[1] = rh[1];
+    }
+    unpack16(rh, v);                                         // continue from the rounded residual stream, as an unfused reader of h would
     float ss = 0.f;
 #pragma unroll
-    for (int hf = 0; hf < NH; ++hf) {
-        const int col = hf * 4096 + 8 * t;
-        const uint4 raw_h = __ldcg(reinterpret_cast<const uint4 *>(p.h + row * p.ld_h + col));
-        if (p.acc) {
-            const uint4 raw_so = raw8_or_ones(p.signs_out ? p.signs_out + col : nullptr);
-            load8_f32_cg(p.acc + row * p.ld_acc + col, v[hf]);
-            fwht8(v[hf], 4096, ex, !(ex_idle && hf == 0));
-            float sg[8], r[8];
-            unpack8(raw_so, sg);
-            unpack8(raw_h, r);
+    for (int i = 0; i < 16; ++i) ss += v[i] * v[i];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[hf][i] = r[i] + v[hf][i] * (p.scale_out * hn) * sg[i];
-            if (write_h) store8_f16((p.h_out ? p.h_out : p.h) + row * p.ld_h + col, v[hf]);
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+    const bool pair = p.n > 4096;
+    if (lane == 0) red[8 * part + warp] = ss;
+    if (pair) asm volatile("bar.sync %0, %1;" ::"r"(pair_bar), "n"(2 * kUnitThreads) : "memory");
+    else unit_barrier(bar);
+    float tot = 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[hf][i] = __half2float(__float2half_rn(v[hf][i]));
-        } else {
-            if (write_h && p.h_out) *reinterpret_cast<uint4 *>(p.h_out + row * p.ld_h + col) = raw_h;
-            unpack8(raw_h, v[hf]);
-        }
+    for (int i = 0; i < 8; ++i) tot += red[i];
+    if (pair) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss += v[hf][i] * v[hf][i];
+        for (int i = 8; i < 16; ++i) tot += red[i];
     }
-    const float inv = rsqrtf(block_sum(ss, red) / p.n + p.eps);
+    const float inv = rsqrtf(tot / p.n + p.eps);
+    float w[16];
+    unpack16(rw, w);
 #pragma unroll
-    for (int hf = 0; hf < NH; ++hf) {
-        const int col = hf * 4096 + 8 * t;
-        float w[8], sg[8];
-        unpack8(*reinterpret_cast<const uint4 *>(p.w_norm + col), w);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[hf][i] = __half2float(__float2half_rn(v[hf][i] * inv * w[i]));
-        if (p.transform_in) {
-            unpack8(raw8_or_ones(p.signs_in ? p.signs_in + col : nullptr), sg);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[hf][i] *= sg[i];
-            fwht8(v[hf], 4096, ex, hf != 0);      // before piece 0: block_sum's barriers; later pieces: the transform before
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[hf][i] *= hn;
-        }
-        store8_f16(p.out + row * p.ld_out + col, v[hf]);
+    for (int i = 0; i < 16; ++i) v[i] = v[i] * inv * w[i];
+    pack16(v, rh);
+    __half *out = p.out + row * p.ld_out;
+    if (!p.transform_in) {
+        reinterpret_cast<uint4 *>(out + col)[0] = rh[0];
+        reinterpret_cast<uint4 *>(out + col)[1] = rh[1];
+        return;
     }
+    unpack16(rh, v);
+    float si[16];
+    unpack16(rsi, si);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] *= si[i];
+    unit_transform_to_far(v, ex, t, bar);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) out[col0 + t + 256 * k] = __float2half_rn(v[k] * hn);
 }
 
 // Fused MLP middle: gate/up pre-activations arrive as the fp32 accumulator of the fused gate-up

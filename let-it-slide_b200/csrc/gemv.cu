@@ -31,7 +31,8 @@ constexpr int kStages = RPTC_GEMV_STAGES;        // ring depth per warp
 constexpr int kStageUnits = 2;                   // units per stage: one of each row block of a granule
 constexpr uint32_t kUnitBytes = 512;             // 32 rows x 128 bits
 constexpr uint32_t kStageBytes = kStageUnits * kUnitBytes;
-constexpr uint32_t kBarBytes = 1024;             // the barrier of the table's bulk copy; the ring starts behind it
+constexpr uint32_t kBarBytes = 1024;             // the barrier of the table's bulk copy, the glue's sums; the ring starts behind it
+constexpr uint32_t kGlueSums = 512;
 constexpr uint32_t kRingBytes = kGemvWarps * kStages * kStageBytes;
 static_assert(kBarBytes + kRingBytes + 1024 <= kHashLutWindow, "ring must fit below the HASH table window");
 
@@ -56,6 +57,8 @@ struct GemvParams {
     int64_t clear_count;
     // gemv_rows_kernel, MODE 0: fp16 elements from one bank's table to the next
     int64_t lut_stride;
+    // MODE 1: where the glue exchanges values
+    int32_t ex_on_ring;
 };
 
 // Source pair of stream pair s under the fused reference kernel's x staging (inference.cu:216-221,249).
@@ -420,8 +423,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
                      i += (int64_t)gridDim.x * kGemvThreads)
                     z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            if (p.n != 4096) late_prologue();      // the wide form has no hook
-            float *ex = reinterpret_cast<float *>(smem_raw + (xs - s0) + BATCH * x_batch_stride);
+            // Exchange buffers of the glue, one per unit of 256 threads: behind x, or, beside a table that leaves no room there, in
+            // the ring, which is then filled behind the glue.
+            const bool on_ring = p.ex_on_ring;
+            float *ex = reinterpret_cast<float *>(smem_raw + (on_ring ? kBarBytes : (xs - s0) + BATCH * x_batch_stride));
             FinishNormParams q;
             q.acc = const_cast<float *>(p.in.acc);
             q.ld_acc = p.in.ld_acc;
@@ -438,12 +443,23 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
             q.ld_out = x_batch_stride >> 1;
             q.n = (int32_t)p.n;
             q.block = 4096;
+            const int unit = warp >> 3;
+            float *unit_ex = ex + unit * kUnitFloats;
+            float *red = reinterpret_cast<float *>(smem_raw + kGlueSums);      // 16 floats per row
+            auto hook = [&]() {
+                if (!on_ring) late_prologue();
+            };
+            if (p.n == 4096) {                       // a unit per row
+                if (unit < BATCH)
+                    finish_norm_unit(q, unit, 0, unit_ex, red + 16 * unit, 1 + unit, 3, false, blockIdx.x == 0, hook);
+            } else {                                 // both units on one row after the other
 #pragma unroll 1
-            for (int b = 0; b < BATCH; ++b) {
-                if (p.n == 4096)
-                    finish_norm_row(q, b, ex, ex + 4096, false, blockIdx.x == 0, b == 0, late_prologue);
-                else finish_norm_row_wide<2>(q, b, ex, ex + 4096, blockIdx.x == 0, b == 0);
+                for (int b = 0; b < BATCH; ++b) {
+                    finish_norm_unit(q, b, unit, unit_ex, red + 16 * b, 1 + unit, 3, false, blockIdx.x == 0, hook);
+                    if (b + 1 < BATCH) __syncthreads();      // the buffers are read to the end before the next row
+                }
             }
+            if (on_ring) __syncthreads();
         } else {
             const int64_t col0 = (int64_t)useg0 * WPU;
             const int pairs = nu * PAIRS;
@@ -650,7 +666,10 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
     size_t smem = fixed + size_t(seg) * unit_x_bytes;
     if (in) {
         if (seg != p.n_units) return RPTC_ERR_TOO_LARGE;                        // computed activations live in one segment
-        smem += 4096 * sizeof(float) + 128;                                     // exchange buffer of the 4096-point transform
+        const size_t ex = (n > 4096 || batch > 1 ? 2 : 1) * kUnitFloats * sizeof(float);      // exchange buffers of the 4096-point transforms
+        static_assert(2 * kUnitFloats * sizeof(float) <= kRingBytes, "they must fit into the ring");
+        p.ex_on_ring = smem + ex > kMaxSmem;
+        if (!p.ex_on_ring) smem += ex;
         if (smem > kMaxSmem) return RPTC_ERR_TOO_LARGE;
     }
 

@@ -77,13 +77,22 @@ __global__ void __launch_bounds__(512) swiglu_hadamard_kernel(const SwigluParams
 // They exist to shorten the chain of small dependent launches between two fused dequant-GEMVs.
 
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) finish_norm_hadamard_kernel(const FinishNormParams p) {
-    __shared__ __align__(16) float ex[8 * THREADS];
+__global__ void __launch_bounds__(256) finish_norm_hadamard_kernel(const FinishNormParams p) {
+    __shared__ __align__(16) float ex[2048];
     __shared__ float red[36];
     pdl_allow_next_grid();
     pdl_wait_prior_grids();
-    finish_norm_row(p, blockIdx.x, ex, red, true, true, true);
+    finish_norm_row(p, blockIdx.x, ex, red);
+}
+
+// Rows of 4096 or 8192: 256 threads per 4096 elements.
+__global__ void __launch_bounds__(2 * kUnitThreads) finish_norm_unit_kernel(const FinishNormParams p) {
+    __shared__ __align__(16) float ex[2][kUnitFloats];
+    __shared__ float red[16];
+    pdl_allow_next_grid();
+    pdl_wait_prior_grids();
+    const int unit = threadIdx.x / kUnitThreads;
+    finish_norm_unit(p, blockIdx.x, unit, ex[unit], red, 1 + unit, 3, true, true);
 }
 
 // Output side of the fused qkv layer, rotary embedding and KV-cache append in one pass:
@@ -295,9 +304,9 @@ extern "C" int rptc_finish_norm_hadamard(float *acc, int64_t ld_acc, const void 
     p.ld_out = ld_out;
     p.n = (int32_t)n;
     p.block = (int32_t)(n > 4096 ? 4096 : n);
-    if (n > 4096)
-        return launch(finish_norm_hadamard_kernel<1024>, dim3((unsigned)rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), p);
-    return launch(finish_norm_hadamard_kernel<512>, dim3((unsigned)rows), dim3((unsigned)(n / 8)), 0, static_cast<cudaStream_t>(stream), p);
+    if (n >= 4096)
+        return launch(finish_norm_unit_kernel, dim3((unsigned)rows), dim3((unsigned)(n / 16)), 0, static_cast<cudaStream_t>(stream), p);
+    return launch(finish_norm_hadamard_kernel, dim3((unsigned)rows), dim3((unsigned)(n / 8)), 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int rptc_qkv_finish(float *acc, int64_t ld_acc, const void *signs_out, float scale, void *q_out, int64_t ld_q,
