@@ -72,7 +72,8 @@ __device__ __forceinline__ int64_t k2_legacy_pair(int64_t s, int64_t n) {
 }
 
 // The general kernel: any layout (strided 128-bit loads straight from memory, one unit of one row block per
-// step), the reference kernels' lane-0 deviations, batch 1.  The native TILED layout takes the two kernels below.
+// step), the reference kernels' lane-0 deviations, batch 1.  It is left with the layouts whose 32 rows of a unit lie
+// together (UNITMAJOR, TILED with a deviation); the others have kernels of their own below.
 template <int CODE, int K>
 __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams p) {
     constexpr int WPU = 128 / K;          // weights per unit
@@ -191,6 +192,125 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
         }
     }
     if (!waited_prior) pdl_wait_prior_grids();
+}
+
+// ---- layouts whose units of a row lie together (ROWMAJOR, CHUNKED), batch 1 ------------------------------------------------
+// lane = unit: a warp takes one row of a chunk of 32 units (2048 columns at two bits) per step, a single 512-byte request where
+// lane = row would touch 32 places 512 bytes or more apart (16384 x 16384, CHUNKED: 70 us).  The activations of a lane's
+// unit stay in registers while the warp walks down the rows of the chunk; the 16 bits in front of a unit come from the lane
+// to the left, in front of the chunk from memory.  Codes arrive through a private ring of asynchronous copies, four rows
+// ahead.  fp16 pair products per unit, fp32 sums across the lanes.
+constexpr int kUnitsAhead = 4;
+constexpr uint32_t kUnitsRing = kGemvWarps * kUnitsAhead * 512, kUnitsHist = kGemvWarps * kUnitsAhead * 4;
+static_assert(kBarBytes + kUnitsRing + kUnitsHist + 1024 <= kHashLutWindow, "ring must fit below the HASH table window");
+template <int CODE, int K>
+__global__ void __launch_bounds__(kGemvThreads, 1) gemv_units_kernel(const GemvParams p) {
+    constexpr int PAIRS = 64 / K, PPU = PAIRS / 4;            // activation pairs, 16-byte pieces of them, per unit
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t s0 = smem_addr(smem_raw);
+    const uint32_t ring = s0 + kBarBytes + (uint32_t)warp * (kUnitsAhead * 512) + 16u * lane;
+    const uint32_t hist = s0 + kBarBytes + kUnitsRing + (uint32_t)warp * (kUnitsAhead * 4);
+    const uint32_t lut_tab = CODE == RPTC_CODE_HASH ? kHashLutWindow : s0 + kBarBytes + kUnitsRing + kUnitsHist;
+    const uint32_t xs = lut_tab + lut_bytes<CODE>(p.L, p.S);
+    if (CODE == RPTC_CODE_LUT) {
+        if (threadIdx.x == 0) {
+            mbar_init(s0, 1);
+            mbar_fence_init();
+            mbar_expect_tx(s0, 2u << p.L);
+            bulk_g2s(lut_tab, p.lut, 2u << p.L, s0);
+        }
+    } else {
+        lut_fill<CODE>(lut_tab, p.lut, p.L, p.S);
+    }
+    const Lut<CODE> lut = lut_view<CODE>(lut_tab, p.L, p.S);
+    pdl_allow_next_grid();
+    // (chunk, row) pairs, chunk by chunk, in equal ranges per CTA; a warp takes every sixteenth row of the range
+    const uint32_t m = (uint32_t)p.m, chunks = (uint32_t)(p.n_units + 31) >> 5, T = chunks * m;
+    const uint32_t per = T / gridDim.x, extra = T - per * gridDim.x;
+    const uint32_t c0 = blockIdx.x * per + min(blockIdx.x, extra), c1 = c0 + per + (blockIdx.x < extra ? 1u : 0u);
+    bool first = true;
+    for (uint32_t pos = c0; pos < c1;) {
+        const uint32_t chunk = pos / m, r0 = pos - chunk * m, r1 = min(m, r0 + (c1 - pos));
+        pos += r1 - r0;
+        const int32_t u = (int32_t)(chunk * 32) + lane;
+        const bool active = u < p.n_units;
+        const uint4 *base = p.codes + (int64_t)chunk * p.st.hi + lane;
+        uint32_t f_row = r0 + warp, f_slot = 0;               // fetch cursor
+        auto fetch = [&]() {
+            if (f_row < r1) {
+                const uint4 *src = base + (int64_t)f_row * p.st.row;
+                if (active) cp_async16(ring + f_slot * 512u, src);
+                if (lane == 0) {
+                    if (chunk == 0) {
+                        const uint32_t v = p.carry_in ? __ldg(p.carry_in + f_row) : 0u;
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(hist + 4u * f_slot), "r"(v) : "memory");
+                    } else {      // the last word of the row's unit in front of the chunk
+                        const uint32_t *last = reinterpret_cast<const uint32_t *>(p.codes + (int64_t)(chunk - 1) * p.st.hi + 31 + (int64_t)f_row * p.st.row) + 3;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(hist + 4u * f_slot), "l"(last) : "memory");
+                    }
+                }
+            }
+            cp_async_commit();                                // an empty group when nothing is left keeps the count constant
+            f_row += kGemvWarps;
+            f_slot = (f_slot + 1) % kUnitsAhead;
+        };
+#pragma unroll 1
+        for (int i = 0; i < kUnitsAhead; ++i) fetch();
+        if (first) pdl_wait_prior_grids();
+        else __syncthreads();                                 // everyone is done with the chunk before
+        // activations of the chunk; piece j of unit q sits at piece j ^ swz(q), so that 32 lanes read theirs without conflicts
+        auto swz = [](int q) { return (uint32_t)(PPU == 8 ? q & 7 : (q >> 1) & 3); };
+        for (int i = threadIdx.x; i < 32 * PAIRS; i += kGemvThreads) {
+            const int q = i / PAIRS, w = i % PAIRS;
+            const int64_t s = (int64_t)chunk * (32 * PAIRS) + i;
+            uint32_t v = 0;
+            if (2 * s < p.n) v = ld_ordered_u32(reinterpret_cast<const uint32_t *>(p.x) + (p.x_order == RPTC_XORDER_K2_LEGACY ? k2_legacy_pair(s, p.n) : s));
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(xs + (((uint32_t)(q * PPU) + ((uint32_t)(w >> 2) ^ swz(q))) << 4) + 4u * (w & 3)), "r"(v) : "memory");
+        }
+        __syncthreads();
+        if (CODE == RPTC_CODE_LUT && first && !mbar_wait(s0, 0, p.status)) {
+            cp_async_wait<0>();
+            return;
+        }
+        first = false;
+        uint32_t xr[PAIRS];
+#pragma unroll
+        for (int j = 0; j < PPU; ++j) {
+            const uint4 v = lds128(xs + (((uint32_t)(lane * PPU) + ((uint32_t)j ^ swz(lane))) << 4));
+            xr[4 * j] = v.x, xr[4 * j + 1] = v.y, xr[4 * j + 2] = v.z, xr[4 * j + 3] = v.w;
+        }
+        uint32_t slot = 0;
+#pragma unroll 1
+        for (uint32_t row = r0 + warp; row < r1; row += kGemvWarps) {
+            cp_async_wait<kUnitsAhead - 1>();
+            const uint4 v = lds128(ring + slot * 512u);
+            uint32_t halo = __shfl_up_sync(0xFFFFFFFFu, v.w, 1);
+            if (lane == 0) {
+                halo = lds32(hist + 4u * slot);
+                if (p.quirk == RPTC_QUIRK_K2_LANE0_CARRY) halo = v.w;      // the reference kernels' lane-0 deviations
+                else if (p.quirk == RPTC_QUIRK_K1_LANE0_SEED && u > 0) halo >>= 16;
+            }
+            fetch();                                          // the words are in registers
+            slot = (slot + 1) % kUnitsAhead;
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            __half2 hacc[4];
+            decode_group<CODE, K>(w, halo, lut, [&](int pi, __half2 wp) {
+                const __half2 x2 = u32_as_half2(xr[pi]);
+                hacc[pi & 3] = pi < 4 ? __hmul2(wp, x2) : __hfma2(wp, x2, hacc[pi & 3]);
+            });
+            const float2 f2 = __half22float2(__hadd2(__hadd2(hacc[0], hacc[1]), __hadd2(hacc[2], hacc[3])));
+            float sum = active ? f2.x + f2.y : 0.f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+            if (lane == 0) atomicAdd(p.acc + row, sum);
+        }
+        cp_async_wait<0>();
+    }
+    if (first) {                                              // a CTA without work
+        pdl_wait_prior_grids();
+        if (CODE == RPTC_CODE_LUT && threadIdx.x == 0) mbar_wait(s0, 0, p.status);      // its table must not land in memory given back
+    }
 }
 
 // ---- batch 1-2: lane = row, products on the tensor cores -----------------------------------------------------------
@@ -596,6 +716,17 @@ static int launch_gemv(const GemvParams &p, size_t smem, cudaStream_t stream) {
     return launch(kern, dim3(num_sms()), dim3(kGemvThreads), smem, stream, p);
 }
 
+template <int CODE, int K>
+static int launch_gemv_units(const GemvParams &p, cudaStream_t stream) {
+    static SmemOptIn opted;
+    auto kern = gemv_units_kernel<CODE, K>;
+    if (int e = allow_max_smem(kern, opted)) return e;
+    const size_t x = 32 * (128 / K) * 2;                              // one chunk of activations
+    const size_t smem = CODE == RPTC_CODE_HASH ? kHashLutWindow + kHashLutBytes + x
+                                               : kBarBytes + kUnitsRing + kUnitsHist + (CODE == RPTC_CODE_LUT ? size_t(2) << p.L : size_t(128) << p.S) + x + 128;
+    return launch(kern, dim3(num_sms()), dim3(kGemvThreads), smem, stream, p);
+}
+
 template <int CODE, int K, int BATCH, int MODE>
 static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t stream, dim3 grid = dim3(num_sms())) {
     static SmemOptIn opted;
@@ -606,7 +737,10 @@ static int launch_gemv_rows(const GemvParams &p, size_t smem, cudaStream_t strea
 
 template <int CODE, int K>
 static int dispatch(const GemvParams &p, int batch, bool tiled, size_t smem, dim3 grid, cudaStream_t stream) {
-    if (!tiled) return batch == 1 && !p.in.h_in ? launch_gemv<CODE, K>(p, smem, stream) : RPTC_ERR_UNSUPPORTED;
+    if (!tiled) {
+        if (batch != 1 || p.in.h_in) return RPTC_ERR_UNSUPPORTED;
+        return p.st.lo == 1 ? launch_gemv_units<CODE, K>(p, stream) : launch_gemv<CODE, K>(p, smem, stream);
+    }
     if (p.in.h_in) {
         if (batch > 2) return RPTC_ERR_UNSUPPORTED;
         return batch == 1 ? launch_gemv_rows<CODE, K, 1, 1>(p, smem, stream) : launch_gemv_rows<CODE, K, 2, 1>(p, smem, stream);

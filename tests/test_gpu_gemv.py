@@ -161,3 +161,24 @@ def test_dense_gemv_of_many_rows(m, n, batch):
     exact = x.double() @ W.double().t()
     y = ops.dense_gemv(W, x)
     check_product(y.float().cpu().numpy(), exact.cpu().numpy(), W.double().norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(), GEMV_FP32_TOL)
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("layout", [o.LAYOUT_ROWMAJOR, o.LAYOUT_CHUNKED])
+@pytest.mark.parametrize("m,n", [(32, 2048), (64, 64), (96, 6208), (1056, 4096), (4096, 10240)])
+def test_gemv_of_layouts_with_a_row_together(code, K, L, S, layout, m, n):
+    """Fewer rows than CTAs, chunks of fewer than 32 units, ranges that start inside a chunk."""
+    from rptc_b200 import Format, ops
+    if layout == o.LAYOUT_CHUNKED and (n * K // 128) % 32:
+        pytest.skip("whole chunks only")
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    fmt = Format(code, K, L, S, layout)
+    codes = torch.randint(-2**31, 2**31 - 1, (m * n * K // 32,), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn((1, n), dtype=torch.float16, device="cuda", generator=g)
+    dense = ops.decompress(codes, lut, m, n, fmt).double()
+    y = ops.gemv(codes, lut, x, m, n, fmt)
+    torch.cuda.synchronize()
+    ops.device_status()
+    check_product(y.float().cpu().numpy(), (x.double() @ dense.t()).cpu().numpy(), dense.norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(),
+                  GEMV_HFMA2_TOL)
