@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
 // lane = row would touch 32 places 512 bytes or more apart (16384 x 16384, CHUNKED: 70 us).  The activations of a lane's
 // unit stay in registers while the warp walks down the rows of the chunk; the 16 bits in front of a unit come from the lane
 // to the left, in front of the chunk from memory.  Codes arrive through a private ring of asynchronous copies, four rows
-// ahead.  fp16 pair products per unit, fp32 sums across the lanes.
+// ahead.  fp16 pair products per unit, fp32 sums across the lanes.  Bound by the table look-ups; against lane = row, 16384 x
+// 16384: HASH 65 -> 54 us, LUT 145 -> 134 us, LITE 73 -> 66 us; 4096 x 4096 HASH in a drop-in call 32.4 -> 31 us.
 constexpr int kUnitsAhead = 4;
 constexpr uint32_t kUnitsRing = kGemvWarps * kUnitsAhead * 512, kUnitsHist = kGemvWarps * kUnitsAhead * 4;
 static_assert(kBarBytes + kUnitsRing + kUnitsHist + 1024 <= kHashLutWindow, "ring must fit below the HASH table window");

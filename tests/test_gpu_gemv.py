@@ -167,7 +167,8 @@ def test_dense_gemv_of_many_rows(m, n, batch):
 @pytest.mark.parametrize("layout", [o.LAYOUT_ROWMAJOR, o.LAYOUT_CHUNKED])
 @pytest.mark.parametrize("m,n", [(32, 2048), (64, 64), (96, 6208), (1056, 4096), (4096, 10240)])
 def test_gemv_of_layouts_with_a_row_together(code, K, L, S, layout, m, n):
-    """Fewer rows than CTAs, chunks of fewer than 32 units, ranges that start inside a chunk."""
+    """Fewer rows than CTAs, chunks of fewer than 32 units, ranges that start inside a chunk.  The fp16 roundings of the n / 64 units add
+    in quadrature, so the bound, measured at n = 4096, grows as n falls."""
     from rptc_b200 import Format, ops
     if layout == o.LAYOUT_CHUNKED and (n * K // 128) % 32:
         pytest.skip("whole chunks only")
@@ -181,4 +182,4 @@ def test_gemv_of_layouts_with_a_row_together(code, K, L, S, layout, m, n):
     torch.cuda.synchronize()
     ops.device_status()
     check_product(y.float().cpu().numpy(), (x.double() @ dense.t()).cpu().numpy(), dense.norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(),
-                  GEMV_HFMA2_TOL)
+                  GEMV_HFMA2_TOL * (4096 / min(n, 4096)) ** 0.5)
