@@ -5,7 +5,7 @@
 // its left they are the windows of its eight states.  A warp walks along contiguous pieces of 256 symbols, so that the
 // bits in front of a piece come from the piece before.  The alphabet sits in shared memory as fp16 (128 KiB at L = 16).
 // Bound: HBM, 8 bytes per weight.  4096 x 4096, L = 16: 381 us with the symbols packed by tensor operations in 64-bit
-// integers and decoded by the decompress kernel, 27 us as it is (floor 20.6 us).
+// integers and decoded by the decompress kernel, 33 us a call as it is, 26 of them in the kernel (floor 20.6 us).
 #include "common.cuh"
 
 namespace rptc {
