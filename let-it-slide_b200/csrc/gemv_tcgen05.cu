@@ -83,6 +83,10 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
     const uint32_t per = total / p.ctas, extra = total - per * p.ctas;
     const uint32_t c0 = cta * per + min(cta, extra), c1 = c0 + per + (cta < extra ? 1u : 0u);
 
+    // entries of the table that this thread spreads over the banks: asked for first, stored when its copies are under way
+    LutPending entries;
+    if (CODE != RPTC_CODE_LUT) entries = lut_fill_begin<CODE>(p.lut_addr, p.lut + (int64_t)bank * p.lut_stride, p.L, p.S);
+    if (warp == kFewTmaWarp && lane == 0) tma_prefetch_map(&x_map);
     if (tid == 0) {
         for (int i = 0; i < kFewMaxXStages; ++i) mbar_init(full_x + 8 * i, 1), mbar_init(empty_x + 8 * i, RB);
         for (int g = 0; g < 4; ++g) mbar_init(full_a + 8 * g, 4), mbar_init(empty_a + 8 * g, 1);
@@ -152,7 +156,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
 #pragma unroll 1
         for (int i = 0; i < kFewAhead; ++i) fetch();
     }
-    if (CODE != RPTC_CODE_LUT) lut_fill<CODE>(p.lut_addr, p.lut + (int64_t)bank * p.lut_stride, p.L, p.S);
+    // ---- table filled
+    if (CODE != RPTC_CODE_LUT) lut_fill_end<CODE>(p.lut_addr, entries, p.S);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -217,16 +222,23 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParam
 #pragma unroll 1
                     for (int a = 0; a < PARTS; ++a) {
                         if (g.part_begin<PARTS>(a) == g.part_begin<PARTS>(a + 1)) continue;      // no step of this segment
-                        for (int c = 0; c < p.n_sums; ++c) {
-                            uint32_t v[8];
-                            tmem_load8(tmem + lanes + (uint32_t)(((a * RB + block) * p.n_sums + c) * p.n_cols + t0), v);
+                        uint32_t v[8], w[8] = {};
+                        const uint32_t src = tmem + lanes + (uint32_t)((a * RB + block) * p.n_sums * p.n_cols + t0);
+                        tmem_load8_begin(src, v);
+                        if (p.n_sums == 2) tmem_load8_begin(src + (uint32_t)p.n_cols, w);
+                        tmem_load_wait(v, w);
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) sum[e] += __uint_as_float(v[e]);
-                        }
+                        for (int e = 0; e < 8; ++e) sum[e] += __uint_as_float(v[e]) + __uint_as_float(w[e]);
                     }
+                    float *to = dst + (int64_t)t0 * p.ld_acc;
+                    if (t0 + 8 <= p.tokens) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (t0 + e < p.tokens) atomicAdd(dst + (int64_t)(t0 + e) * p.ld_acc, sum[e]);
+                        for (int e = 0; e < 8; ++e) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 7; ++e)
+                            if (t0 + e < p.tokens) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
+                    }
                 }
             }
             tc_fence_before();

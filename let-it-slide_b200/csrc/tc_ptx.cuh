@@ -71,6 +71,23 @@ __device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&v)[8]) {
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// The same without the wait: `v` holds the values after tmem_load_wait, which names the registers so that no use of them
+// moves in front of it.
+__device__ __forceinline__ void tmem_load8_begin(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[8], uint32_t (&w)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(w[0]), "+r"(w[1]),
+                   "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_map(const void *map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
 
 // True in one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
