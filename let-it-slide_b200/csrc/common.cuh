@@ -50,6 +50,19 @@ inline int allow_max_smem(Kernel kern, SmemOptIn &seen, int bytes = 227 * 1024) 
     return RPTC_OK;
 }
 
+// For kernels whose CTAs are to share an SM with those of the kernel in front or behind: an SM that is busy cannot change its
+// split between L1 and shared memory, so they all ask for the largest shared memory.
+template <typename Kernel>
+inline int prefer_shared_memory(Kernel kern, SmemOptIn &seen) {
+    const int dev = current_device();
+    if (dev < 0) return cuda_fail(cudaErrorInvalidDevice);
+    if (!seen.done[dev]) {
+        RPTC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        seen.done[dev] = true;
+    }
+    return RPTC_OK;
+}
+
 // Launches `kernel` with or without the programmatic-dependent-launch attribute.
 template <typename... KArgs, typename... Args>
 inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

@@ -32,6 +32,12 @@ constexpr int kFewMaxXStages = 8;
 constexpr int kFewACols = 32 * 4;                    // tensor-memory columns of the decoded weights: 64 fp16 per group and lane
 constexpr int kFewTmemCols = 512;
 
+// 64 registers per thread and no more shared memory than the plan needs: the CTAs of the small kernels in front of and behind
+// this one in a decode step (norms, SwiGLU, attention) then fit on an SM beside one of its own, so that they are in place when the
+// last sum is in, one to an SM, and this kernel fetches codes and table under them.  Without it they were packed onto the first SMs
+// that came free, and those SMs started the next product 2 us late.
+constexpr int kFewRegisterThreads = 1024;
+
 struct FewParams {
     const uint4 *codes;
     const __half *lut;
@@ -64,7 +70,7 @@ struct FewSegment {
 };
 
 template <int CODE, int K, int RB>
-__global__ void __launch_bounds__(kFewThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
+__global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int UPS = K / 2;                       // 128-bit units per step
     constexpr int PARTS = 4 / RB;
     constexpr int NW = 4 * UPS;
@@ -331,8 +337,10 @@ template <int CODE, int K, int RB>
 static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t stream) {
     static SmemOptIn opted;
     auto kern = gemv_few_kernel<CODE, K, RB>;
+    static SmemOptIn preferred;
     if (int e = allow_max_smem(kern, opted)) return e;
-    return launch(kern, dim3(grid), dim3(kFewThreads), kFewTop, stream, p, map);
+    if (int e = prefer_shared_memory(kern, preferred)) return e;
+    return launch(kern, dim3(grid), dim3(kFewThreads), p.x_addr + (uint32_t)p.n_xstages * 128u * (uint32_t)p.n_cols, stream, p, map);
 }
 
 template <int CODE, int K>

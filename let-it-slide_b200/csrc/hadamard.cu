@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(256) finish_norm_hadamard_kernel(const FinishN
     finish_norm_row(p, blockIdx.x, ex, red);
 }
 
-// Rows of 4096 or 8192: 256 threads per 4096 elements.
-__global__ void __launch_bounds__(2 * kUnitThreads) finish_norm_unit_kernel(const FinishNormParams p) {
-    __shared__ __align__(16) float ex[2][kUnitFloats];
+// Rows of 4096 or 8192: 256 threads per 4096 elements (64 registers: see kFewRegisterThreads).
+template <int UNITS>
+__global__ void __launch_bounds__(UNITS * kUnitThreads, UNITS == 1 ? 4 : 1) finish_norm_unit_kernel(const FinishNormParams p) {
+    __shared__ __align__(16) float ex[UNITS][kUnitFloats];
     __shared__ float red[16];
     pdl_allow_next_grid();
     pdl_wait_prior_grids();
@@ -257,6 +258,8 @@ static int swiglu_launch(float *acc, const void *in16, int64_t ld_in, void *out,
     p.scale_in = scale_in * hadamard_norm(block);
     if (block <= 256 && n > 256) {      // a warp per 256 columns, eight warps per CTA
         p.chunk = 2048;
+        static SmemOptIn preferred;
+        if (int e = prefer_shared_memory(swiglu_hadamard_kernel, preferred)) return e;
         return launch(swiglu_hadamard_kernel, dim3((unsigned)((n + 2047) / 2048), (unsigned)rows), dim3(256), 0,
                       static_cast<cudaStream_t>(stream), p);
     }
@@ -304,8 +307,15 @@ extern "C" int rptc_finish_norm_hadamard(float *acc, int64_t ld_acc, const void 
     p.ld_out = ld_out;
     p.n = (int32_t)n;
     p.block = (int32_t)(n > 4096 ? 4096 : n);
-    if (n >= 4096)
-        return launch(finish_norm_unit_kernel, dim3((unsigned)rows), dim3((unsigned)(n / 16)), 0, static_cast<cudaStream_t>(stream), p);
+    static SmemOptIn one, two;
+    if (n == 4096) {
+        if (int e = prefer_shared_memory(finish_norm_unit_kernel<1>, one)) return e;
+        return launch(finish_norm_unit_kernel<1>, dim3((unsigned)rows), dim3(kUnitThreads), 0, static_cast<cudaStream_t>(stream), p);
+    }
+    if (n == 8192) {
+        if (int e = prefer_shared_memory(finish_norm_unit_kernel<2>, two)) return e;
+        return launch(finish_norm_unit_kernel<2>, dim3((unsigned)rows), dim3(2 * kUnitThreads), 0, static_cast<cudaStream_t>(stream), p);
+    }
     return launch(finish_norm_hadamard_kernel, dim3((unsigned)rows), dim3((unsigned)(n / 8)), 0, static_cast<cudaStream_t>(stream), p);
 }
 

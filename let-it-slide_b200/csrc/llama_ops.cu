@@ -364,6 +364,8 @@ template <typename... Args>
 static int launch_attn(int heads, int64_t rows, cudaStream_t stream, Args... args) {
     const dim3 grid((unsigned)heads, (unsigned)rows);
     const int64_t ctas = heads * rows, sms = num_sms();
+    static SmemOptIn preferred;
+    if (int e = prefer_shared_memory(attn_decode_kernel<4>, preferred)) return e;      // its CTAs fit beside those of gemv_few_kernel
     if (ctas <= sms) return launch(attn_decode_kernel<16>, grid, dim3(512), 0, stream, args...);
     if (ctas <= 2 * sms) return launch(attn_decode_kernel<8>, grid, dim3(256), 0, stream, args...);
     return launch(attn_decode_kernel<4>, grid, dim3(128), 0, stream, args...);
