@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
 #pragma unroll 1
             for (int32_t i = 0; i < len && ok; ++i) {
                 cp_async_wait<kFewAhead - 1>();      // this step's words have landed
-                uint32_t R[2 * NW], out[32];
+                uint32_t R[2 * NW], out[16];
                 if (i == 0) prevw = lds32(hist + 2048u * slot);
 #pragma unroll
                 for (int q = 0; q < UPS; ++q) {
@@ -206,12 +206,15 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                 for (int pi = 0; pi < 32; pi += 4) {
                     uint32_t four[4];
                     decode_quad_bits<CODE, K>(R, lut, pi, four);
-                    out[pi] = four[0], out[pi + 1] = four[1], out[pi + 2] = four[2], out[pi + 3] = four[3];
+                    out[pi & 15] = four[0], out[(pi & 15) + 1] = four[1], out[(pi & 15) + 2] = four[2], out[(pi & 15) + 3] = four[3];
+                    if (pi == 12) {                  // the MMAs have read the group's last step
+                        ok = mbar_wait(empty_a + 8 * group, a_phase, p.status);
+                        a_phase ^= 1u;
+                        tc_fence_after();
+                    }
+                    if ((pi & 15) == 12) tmem_store16_begin(a_cols + 32u * (uint32_t)group + (uint32_t)(pi & 16) + lanes, out);
                 }
-                ok = mbar_wait(empty_a + 8 * group, a_phase, p.status);      // the MMAs have read the group's last step
-                a_phase ^= 1u;
-                tc_fence_after();
-                tmem_store32(a_cols + 32u * (uint32_t)group + lanes, out);
+                tmem_store_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_a + 8 * group);
