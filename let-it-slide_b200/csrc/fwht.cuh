@@ -303,6 +303,18 @@ __device__ __forceinline__ void pack16(const float (&v)[16], uint4 (&r)[2]) {
     r[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
+// Before the wait for the kernel in front: the layer's constants (output signs, norm weights, input signs; last used a step ago and
+// since pushed out of L2 by the other layers) set out for L2.  Thread `i` of `threads` takes every `threads`-th 128-byte line.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_norm_constants(const __half *signs_out, const __half *w_norm, const __half *signs_in, int n, int i, int threads) {
+    const int lines = n / 64;
+    for (int l = i; l < 3 * lines; l += threads) {
+        const int a = l / lines;
+        const __half *v = a == 0 ? signs_out : a == 1 ? w_norm : signs_in;
+        if (v) prefetch_l2(v + 64 * (l - a * lines));
+    }
+}
+
 // finish_norm_row for elements [4096 part, 4096 part + 4096) of a row of 4096 or 8192 by one unit of 256 threads; the two units
 // of a row of 8192 call it together.  ex: kUnitFloats of the unit's own; red: 16 floats of the row's; bar: named barrier of the
 // unit; pair_bar: named barrier of the 512 threads of both units.
@@ -404,6 +416,12 @@ struct SwigluParams {
     float scale_out, scale_in;  // both include the 1/sqrt(block) of their transform
 };
 
+// Before the wait, like prefetch_norm_constants: the constants of columns col .. col + 7, by one thread in eight.
+__device__ __forceinline__ void prefetch_swiglu_constants(const SwigluParams &p, int64_t col) {
+    if (col >= p.n || (col & 63)) return;
+    if (p.signs_out) prefetch_l2(p.signs_out + col), prefetch_l2(p.signs_out + p.n + col);
+    if (p.signs_in) prefetch_l2(p.signs_in + col);
+}
 // Columns col .. col+7 of one row (thread t of the chunk holds 8t..8t+7); result to dst[0..7].
 template <typename Hook = NoHook>
 __device__ __forceinline__ void swiglu_chunk(const SwigluParams &p, int64_t row, int64_t col, float *ex, bool clear, __half *dst,

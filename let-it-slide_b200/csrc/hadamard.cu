@@ -66,9 +66,10 @@ __global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
 __global__ void __launch_bounds__(512) swiglu_hadamard_kernel(const SwigluParams p) {
     __shared__ __align__(16) float ex[4096];
     pdl_allow_next_grid();
-    pdl_wait_prior_grids();
     const int64_t row = blockIdx.y;
     const int64_t col = (int64_t)blockIdx.x * p.chunk + 8 * threadIdx.x;
+    prefetch_swiglu_constants(p, col);
+    pdl_wait_prior_grids();
     if (col >= p.n) return;     // only with blocks <= 256 (whole warps leave; such blocks need no CTA barrier)
     swiglu_chunk(p, row, col, ex, p.clear != 0, p.out + row * p.ld_out + col);
 }
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(UNITS * kUnitThreads, UNITS == 1 ? 4 : 1) fini
     __shared__ __align__(16) float ex[UNITS][kUnitFloats];
     __shared__ float red[16];
     pdl_allow_next_grid();
+    prefetch_norm_constants(p.signs_out, p.w_norm, p.signs_in, p.n, threadIdx.x, blockDim.x);
     pdl_wait_prior_grids();
     const int unit = threadIdx.x / kUnitThreads;
     finish_norm_unit(p, blockIdx.x, unit, ex[unit], red, 1 + unit, 3, true, true);
