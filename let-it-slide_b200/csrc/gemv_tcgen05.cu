@@ -17,6 +17,9 @@
 // an MMA warp and an accumulator of its own: issuing a step (two waits, four MMAs, two commits) takes one thread about
 // 600 clocks, as long as a group takes to decode it, so that one issuer for all four groups held the kernel to a
 // quarter of the speed.  A segment's sums are added to the caller's fp32 accumulator with atomics.
+// More activation rows (SHARED): a tile is RB x 128 weight rows (RB = 1, 2) x up to 256 (RB = 2: 192) tokens, and the groups that take parts
+// of the same rows' steps share one accumulator, filled by one MMA warp.  A step of 256 x 192 takes the tensor core 768
+// clocks and its decode about 430 issue slots per scheduler, so that decoding again for the next 192 tokens is free.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and returns.
 #include "common.cuh"
 #include "matmul.cuh"
@@ -24,7 +27,8 @@
 
 namespace rptc {
 
-static_assert(4 * kFewMaxTokens <= 512 - 128 && 4 * 2 * 48 <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
+constexpr int kFewOwnTokens = 96;                    // up to here a group has accumulators of its own
+static_assert(4 * kFewOwnTokens <= 512 - 128 && 4 * 2 * 48 <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
 constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * (kFewMmaWarp + 4);
 constexpr int kFewAhead = 4;                         // steps of a thread's code bits in flight
 constexpr uint32_t kFewBars = 0x400, kFewHistory = 0x800, kFewCodes = 0x2800, kFewTop = 0x38800;
@@ -48,28 +52,37 @@ struct FewParams {
     int32_t n_steps, n_units;                        // 64-column steps, 128-bit units per row
     int32_t tokens, n_cols;                          // activation rows, rounded up to 16
     int32_t tiles, ctas;                             // per bank
+    int32_t token_tiles;                             // tiles of the same weight rows, n_cols tokens each
     int32_t L, S;
     uint32_t lut_addr, x_addr;
     int32_t n_xstages;
+    bool shared;                                     // more than kFewOwnTokens activation rows (host side: SHARED)
     int32_t n_sums, max_steps;                       // accumulators per group (1 or 2), longest segment
     unsigned int *status;
 };
 
 // A segment: the steps [s0, s1) of one tile, and the part of them that one group takes.
 struct FewSegment {
-    int32_t tile, s0, s1;
+    int32_t tile, s0, s1;                            // tile: of weight rows
+    int32_t t0;                                      // first token
     uint32_t end;                                    // where the next segment starts in the CTA's range
     __device__ __forceinline__ FewSegment(uint32_t pos, uint32_t range_end, const FewParams &p) {
         tile = (int32_t)(pos / (uint32_t)p.n_steps);
         s0 = (int32_t)(pos - (uint32_t)tile * (uint32_t)p.n_steps);
         s1 = min(p.n_steps, s0 + min((int32_t)(range_end - pos), p.max_steps));
         end = pos + (uint32_t)(s1 - s0);
+        t0 = 0;
+        if (p.token_tiles > 1) {
+            const int32_t rows = tile / p.token_tiles;
+            t0 = (tile - rows * p.token_tiles) * p.n_cols;
+            tile = rows;
+        }
     }
     template <int PARTS>
     __device__ __forceinline__ int32_t part_begin(int part) const { return s0 + (s1 - s0) * part / PARTS; }
 };
 
-template <int CODE, int K, int RB>
+template <int CODE, int K, int RB, bool SHARED>
 __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int UPS = K / 2;                       // 128-bit units per step
     constexpr int PARTS = 4 / RB;
@@ -85,7 +98,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     const int bank = blockIdx.x / p.ctas;
     const uint32_t cta = blockIdx.x - bank * p.ctas;
     // this CTA's range of the bank's steps
-    const uint32_t total = (uint32_t)p.tiles * (uint32_t)p.n_steps;
+    const uint32_t total = (uint32_t)(p.tiles * p.token_tiles) * (uint32_t)p.n_steps;
     const uint32_t per = total / p.ctas, extra = total - per * p.ctas;
     const uint32_t c0 = cta * per + min(cta, extra), c1 = c0 + per + (cta < extra ? 1u : 0u);
 
@@ -96,7 +109,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     if (tid == 0) {
         for (int i = 0; i < kFewMaxXStages; ++i) mbar_init(full_x + 8 * i, 1), mbar_init(empty_x + 8 * i, RB);
         for (int g = 0; g < 4; ++g) mbar_init(full_a + 8 * g, 4), mbar_init(empty_a + 8 * g, 1);
-        mbar_init(sums, 4);
+        mbar_init(sums, SHARED ? RB : 4);
         mbar_init(drained, kFewWarps);
         mbar_init(table_bar, 1);
         mbar_fence_init();
@@ -226,11 +239,12 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
             if (ok && row < p.m) {                   // of a whole warp: m is a multiple of 32
                 float *dst = p.acc + (int64_t)bank * p.m + row;
 #pragma unroll 1
-                for (int t0 = 8 * part; t0 < p.tokens; t0 += 8 * PARTS) {
+                const int tokens = min(p.tokens - g.t0, p.n_cols);
+                for (int t0 = 8 * part; t0 < tokens; t0 += 8 * PARTS) {
                     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-                    for (int a = 0; a < PARTS; ++a) {
-                        if (g.part_begin<PARTS>(a) == g.part_begin<PARTS>(a + 1)) continue;      // no step of this segment
+                    for (int a = 0; a < (SHARED ? 1 : PARTS); ++a) {
+                        if (!SHARED && g.part_begin<PARTS>(a) == g.part_begin<PARTS>(a + 1)) continue;      // no step of this segment
                         uint32_t v[8], w[8] = {};
                         const uint32_t src = tmem + lanes + (uint32_t)((a * RB + block) * p.n_sums * p.n_cols + t0);
                         tmem_load8_begin(src, v);
@@ -239,14 +253,14 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
 #pragma unroll
                         for (int e = 0; e < 8; ++e) sum[e] += __uint_as_float(v[e]) + __uint_as_float(w[e]);
                     }
-                    float *to = dst + (int64_t)t0 * p.ld_acc;
-                    if (t0 + 8 <= p.tokens) {
+                    float *to = dst + (int64_t)(g.t0 + t0) * p.ld_acc;
+                    if (t0 + 8 <= tokens) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
                     } else {
 #pragma unroll
                         for (int e = 0; e < 7; ++e)
-                            if (t0 + e < p.tokens) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
+                            if (t0 + e < tokens) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
                     }
                 }
             }
@@ -272,19 +286,19 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                     ok = mbar_wait(empty_x + 8 * px.s, px.phase, p.status);
                     if (ok && elect_one()) {
                         mbar_expect_tx(full_x + 8 * px.s, bytes);
-                        tma_load_2d(p.x_addr + (uint32_t)px.s * bytes, &x_map, s * 64, 0, full_x + 8 * px.s);
+                        tma_load_2d(p.x_addr + (uint32_t)px.s * bytes, &x_map, s * 64, g.t0, full_x + 8 * px.s);
                     }
                     __syncwarp();
                     px.advance(p.n_xstages);
                 }
         }
-    } else {
-        // ================= MMA issue for one group: the whole warp waits, one lane issues =================
+    } else if (!SHARED || warp < kFewMmaWarp + RB) {
+        // ================= MMA issue for one accumulator (a group's, or SHARED a row block's): the whole warp waits, one lane issues =================
         const int grp = __shfl_sync(0xFFFFFFFFu, warp, 0) - kFewMmaWarp, mine = grp / RB;
         RingPos px = {0, 0u};
-        uint32_t a_phase = 0u, seg = 0;
+        uint32_t a_phase = 0u, seg = 0;              // a_phase: bit q for the group that takes part q
         const uint32_t bytes = 128u * (uint32_t)p.n_cols, idesc = instr_desc(p.n_cols);
-        const uint32_t d_tmem = tmem + (uint32_t)(grp * p.n_sums * p.n_cols), a_tmem = a_cols + 32u * (uint32_t)grp;
+        const uint32_t d_tmem = tmem + (uint32_t)(grp * p.n_sums * p.n_cols), a_first = a_cols + 32u * (uint32_t)grp;
         // the four MMAs of a step go round the accumulators
         const uint32_t d1 = p.n_sums == 2 ? (uint32_t)p.n_cols : 0u;
         for (uint32_t pos = c0; pos < c1 && ok; ++seg) {
@@ -298,11 +312,13 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
 #pragma unroll
                 for (int q = 0; q < PARTS; ++q) {
                     if (g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
-                    if (q == mine && ok) {
-                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * grp, a_phase, p.status);
-                        a_phase ^= 1u;
+                    if ((SHARED || q == mine) && ok) {
+                        const int from = SHARED ? q * RB : 0;                // + grp: the group whose step it is
+                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), (a_phase >> q) & 1u, p.status);
+                        a_phase ^= 1u << q;
                         if (ok) {
                             tc_fence_after();
+                            const uint32_t a_tmem = a_first + 32u * (uint32_t)from;
                             const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)px.s * bytes);
                             if (elect_one()) {
                                 // + 32 bytes of shared memory, + 8 columns of tensor memory per K = 16
@@ -310,7 +326,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                                 tc_mma_f16_ta(d_tmem + d1, a_tmem + 8u, xb + 2u, idesc, accumulate | (uint32_t)(p.n_sums == 1));
                                 tc_mma_f16_ta(d_tmem, a_tmem + 16u, xb + 4u, idesc, 1u);
                                 tc_mma_f16_ta(d_tmem + d1, a_tmem + 24u, xb + 6u, idesc, 1u);
-                                tc_commit(empty_a + 8 * grp);
+                                tc_commit(empty_a + 8 * (grp + from));
                                 tc_commit(empty_x + 8 * px.s);
                             }
                             __syncwarp();
@@ -336,10 +352,10 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     }
 }
 
-template <int CODE, int K, int RB>
+template <int CODE, int K, int RB, bool SHARED>
 static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t stream) {
     static SmemOptIn opted;
-    auto kern = gemv_few_kernel<CODE, K, RB>;
+    auto kern = gemv_few_kernel<CODE, K, RB, SHARED>;
     static SmemOptIn preferred;
     if (int e = allow_max_smem(kern, opted)) return e;
     if (int e = prefer_shared_memory(kern, preferred)) return e;
@@ -348,18 +364,20 @@ static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid,
 
 template <int CODE, int K>
 static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t s) {
+    if (p.shared) return rb == 1 ? launch_few<CODE, K, 1, true>(p, map, grid, s) : launch_few<CODE, K, 2, true>(p, map, grid, s);
     switch (rb) {
-        case 1: return launch_few<CODE, K, 1>(p, map, grid, s);
-        case 2: return launch_few<CODE, K, 2>(p, map, grid, s);
+        case 1: return launch_few<CODE, K, 1, false>(p, map, grid, s);
+        case 2: return launch_few<CODE, K, 2, false>(p, map, grid, s);
     }
-    return launch_few<CODE, K, 4>(p, map, grid, s);
+    return launch_few<CODE, K, 4, false>(p, map, grid, s);
 }
 
 // Row blocks per tile.  With four of them a step of activations is loaded, waited for and handed back once per 512 rows;
 // the relative times of a 128-row block are measured (28672 x 8192, 8 tokens: 31.0 us with four, 33.9 with two, 47.0
 // with one).  A bank that is not a whole number of tiles leaves groups without rows: count the blocks that are walked.
-static int few_row_blocks(int64_t m) {
+static int few_row_blocks(int64_t m, int64_t tokens) {
     const int64_t blocks = (m + 127) / 128;
+    if (tokens > kFewOwnTokens) return blocks == 1 ? 1 : 2;
     int best = 4;
     double best_cost = 0;
     for (int rb = 4; rb >= 1; rb >>= 1) {
@@ -370,7 +388,7 @@ static int few_row_blocks(int64_t m) {
 }
 
 // Where the table and the activation ring go; false when two stages do not fit.
-static bool few_plan(FewParams &p, const rptc_format &f) {
+static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb) {
     const uint32_t codes_end = kFewCodes + kFewWarps * kFewAhead * (f.K / 2) * 512;
     uint32_t free;
     if (f.code == RPTC_CODE_HASH) {
@@ -382,6 +400,14 @@ static bool few_plan(FewParams &p, const rptc_format &f) {
     }
     if (free >= kFewTop) return false;
     p.x_addr = free;
+    p.shared = tokens > kFewOwnTokens;
+    p.token_tiles = 1;
+    if (p.shared) {      // three stages of activations and the accumulators (RB x n_cols columns beside the decoded weights) bound the tile
+        const int64_t fit = (kFewTop - free) / (3 * 128) / 16 * 16, most = rb == 1 ? 256 : 192, cols = fit < most ? fit : most;
+        if (cols < 16) return false;
+        p.token_tiles = (int32_t)((tokens + cols - 1) / cols);
+    }
+    p.n_cols = (int32_t)(((tokens + p.token_tiles - 1) / p.token_tiles + 15) / 16 * 16);
     p.n_xstages = (int32_t)((kFewTop - free) / (128u * (uint32_t)p.n_cols));
     if (p.n_xstages > kFewMaxXStages) p.n_xstages = kFewMaxXStages;
     return p.n_xstages >= 2;
@@ -389,18 +415,16 @@ static bool few_plan(FewParams &p, const rptc_format &f) {
 
 bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x) {
     FewParams p;
-    p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
     return f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE && (f.K == 2 || f.K == 4) && n % 64 == 0 && tokens <= kFewMaxTokens &&
            (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % 8 == 0 &&
-           few_plan(p, f);
+           few_plan(p, f, tokens, 2);
 }
 
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s) {
     FewParams p;
-    p.n_cols = (int32_t)((tokens + 15) / 16 * 16);
-    if (!few_plan(p, f)) return RPTC_ERR_UNSUPPORTED;
-    const int rb = few_row_blocks(m);
+    const int rb = few_row_blocks(m, tokens);
+    if (!few_plan(p, f, tokens, rb)) return RPTC_ERR_UNSUPPORTED;
     CUtensorMap map;
     if (int e = encode_map(map, x, n, tokens, ld_x, p.n_cols)) return e;
     p.codes = static_cast<const uint4 *>(codes);
@@ -414,16 +438,18 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
     p.n_units = (int32_t)(n * f.K / 128);
     p.tokens = (int32_t)tokens;
     p.tiles = (int32_t)((m + rb * 128 - 1) / (rb * 128));
-    if ((int64_t)p.tiles * p.n_steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
+    const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
+    if (steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
     // one bank's table per CTA: the SMs are dealt out to the banks
     p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
-    if ((int64_t)p.ctas > (int64_t)p.tiles * p.n_steps) p.ctas = p.tiles * p.n_steps;
+    if (p.ctas > steps) p.ctas = (int32_t)steps;
     // The tensor core rounds its running sums towards zero, so the error of a sum grows with the number of MMAs behind it.
     // Two accumulators per group keep it where the mma.sync kernel had it (22016 x 4096, 16 rows: relative error 0.7e-6
     // against 1.3e-6 with one); where there is room for one only, a CTA's range goes into the result in two halves.
-    p.n_sums = p.n_cols <= 48 ? 2 : 1;
-    const int64_t range = ((int64_t)p.tiles * p.n_steps + p.ctas - 1) / p.ctas;
-    p.max_steps = (int32_t)(p.n_sums == 2 ? range : (range + 1) / 2);
+    // SHARED: no chain is longer than those of the fused GEMM, whose place it takes.
+    p.n_sums = !p.shared && p.n_cols <= 48 ? 2 : 1;
+    const int64_t range = (steps + p.ctas - 1) / p.ctas;
+    p.max_steps = (int32_t)(p.n_sums == 2 || p.shared ? range : (range + 1) / 2);
     p.L = f.L;
     p.S = f.S;
     p.status = device_status_word();
