@@ -586,7 +586,7 @@ static int64_t cluster_places(int split) {
 // tile feeds the tensor pipe about 1.35 times faster per weight row, but there are half as many of it; sharing a tile's
 // reduction over two or four CTAs fills SMs that would be idle (4096 rows x 512 tokens are 32 wide tiles for 148 SMs)
 // at the price of the exchange.  A CTA keeps at least eight steps.
-static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
+static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, double *estimate = nullptr) {
     GemmShape best = {0, 0, 0};
     double best_us = 0;
     const int64_t steps = n / kStepCols;
@@ -603,7 +603,14 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks 
             }
         }
     }
+    if (estimate) *estimate = best_us;
     return best;
+}
+
+double gemm_us(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
+    double us;
+    choose_shape(m, n, tokens, banks, f, &us);
+    return us;
 }
 
 int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {

@@ -828,7 +828,7 @@ int check_format(const rptc_format *f);   // api.cu
 
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
                 const Banks &banks, const rptc_format &f, cudaStream_t stream) {
-    if (tokens > 2 && gemv_few_takes(n, tokens, f, x, ld_x))
+    if (tokens > 2 && gemv_few_takes(m, n, tokens, banks, f, x, ld_x))
         return gemv_few(codes, lut, nullptr, x, ld_x, acc, ld_acc, m, n, tokens, banks, f, stream);
     for (int64_t t = 0; t < tokens; t += 2) {
         const int e = gemv_one(codes, lut, nullptr, static_cast<const __half *>(x) + t * ld_x, ld_x, acc + t * ld_acc, ld_acc, m, n,
@@ -870,7 +870,7 @@ extern "C" int rptc_gemv(const void *codes, const void *lut, const uint32_t *car
     if (int e = validate_gemv_args(codes, lut, x, ld_x, acc, ld_acc, m, n, batch, x_order, fmt)) return e;
     if (int e = rptc_check_device()) return e;
     // Up to two rows the lane-per-row kernel is the faster one (28672 x 8192: 28.0 against 30.6 us).
-    if (batch > 2 && x_order == RPTC_XORDER_NATURAL && gemv_few_takes(n, batch, *fmt, x, ld_x))
+    if (batch > 2 && x_order == RPTC_XORDER_NATURAL && gemv_few_takes(m, n, batch, Banks(), *fmt, x, ld_x))
         return gemv_few(codes, lut, carry_in, x, ld_x, acc, ld_acc, m, n, batch, Banks(), *fmt, static_cast<cudaStream_t>(stream));
     // what the kernel for a few rows does not take (rows of x that are not 16-byte aligned, the legacy order): pairs of rows
     int done = 0;

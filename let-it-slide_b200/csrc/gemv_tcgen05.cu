@@ -27,7 +27,6 @@
 
 namespace rptc {
 
-constexpr int kFewOwnTokens = 96;                    // up to here a group has accumulators of its own
 static_assert(4 * kFewOwnTokens <= 512 - 128 && 4 * 2 * 48 <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
 constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * (kFewMmaWarp + 4);
 constexpr int kFewAhead = 4;                         // steps of a thread's code bits in flight
@@ -372,12 +371,11 @@ static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, uns
     return launch_few<CODE, K, 4, false>(p, map, grid, s);
 }
 
-// Row blocks per tile.  With four of them a step of activations is loaded, waited for and handed back once per 512 rows;
+// Row blocks per tile up to kFewOwnTokens activation rows.  With four of them a step of activations is loaded, waited for and handed back once per 512 rows;
 // the relative times of a 128-row block are measured (28672 x 8192, 8 tokens: 31.0 us with four, 33.9 with two, 47.0
 // with one).  A bank that is not a whole number of tiles leaves groups without rows: count the blocks that are walked.
-static int few_row_blocks(int64_t m, int64_t tokens) {
+static int few_row_blocks(int64_t m) {
     const int64_t blocks = (m + 127) / 128;
-    if (tokens > kFewOwnTokens) return blocks == 1 ? 1 : 2;
     int best = 4;
     double best_cost = 0;
     for (int rb = 4; rb >= 1; rb >>= 1) {
@@ -386,8 +384,14 @@ static int few_row_blocks(int64_t m, int64_t tokens) {
     }
     return best;
 }
+// SHARED: microseconds of a 64-column step of a tile.  The decode (a 65,536-entry table: bank conflicts), the tensor core (four
+// clocks per token and pair of row blocks), or one thread's issue of the step.
+static double shared_step_us(int rb, int n_cols, int code) {
+    const double decode = rb * (code == RPTC_CODE_LUT ? 0.60 : 0.14), mma = rb * n_cols * 2 / 1900.0, issue = 0.34;
+    return decode > mma ? (decode > issue ? decode : issue) : (mma > issue ? mma : issue);
+}
 
-// Where the table and the activation ring go; false when two stages do not fit.
+// Tile of `rb` row blocks, where the table and the activation ring go; false when they do not fit.
 static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb) {
     const uint32_t codes_end = kFewCodes + kFewWarps * kFewAhead * (f.K / 2) * 512;
     uint32_t free;
@@ -402,7 +406,7 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
     p.x_addr = free;
     p.shared = tokens > kFewOwnTokens;
     p.token_tiles = 1;
-    if (p.shared) {      // three stages of activations and the accumulators (RB x n_cols columns beside the decoded weights) bound the tile
+    if (p.shared) {      // three stages of activations, and the accumulators beside the decoded weights, bound the tile
         const int64_t fit = (kFewTop - free) / (3 * 128) / 16 * 16, most = rb == 1 ? 256 : 192, cols = fit < most ? fit : most;
         if (cols < 16) return false;
         p.token_tiles = (int32_t)((tokens + cols - 1) / cols);
@@ -412,19 +416,67 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
     if (p.n_xstages > kFewMaxXStages) p.n_xstages = kFewMaxXStages;
     return p.n_xstages >= 2;
 }
+static int64_t few_tiles(int64_t m, int rb) { return (m + rb * 128 - 1) / (rb * 128); }
+// The plan for `tokens` activation rows: row blocks per tile, or 0 where there is none.
+static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tokens) {
+    int rb = few_row_blocks(m);
+    if (tokens > kFewOwnTokens) {
+        FewParams one, two;
+        const bool has_one = few_plan(one, f, tokens, 1), has_two = few_plan(two, f, tokens, 2);
+        if (!has_one && !has_two) return 0;
+        rb = !has_two || (has_one && few_tiles(m, 1) * one.token_tiles * shared_step_us(1, one.n_cols, f.code) <
+                                         few_tiles(m, 2) * two.token_tiles * shared_step_us(2, two.n_cols, f.code))
+                 ? 1
+                 : 2;
+    }
+    return few_plan(p, f, tokens, rb) ? rb : 0;
+}
 
-bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x) {
+// Up to kFewOwnTokens activation rows always (a step costs its decode), beyond that where it is estimated to finish before
+// the fused GEMM: a GEMM tile of 256 x 256 feeds the tensor core better and its result is fp16, but its decode goes through
+// shared memory and half of its SMs are idle for a few hundred tokens.  Here a CTA has its equal share of the steps, adds
+// its tiles' sums to memory (0.021 us per token and pair of row blocks), and the fp32 accumulator is zeroed in front and
+// read behind.  The time around the steps is fitted to whole layers of both codes.  Measured, whole layers, GEMM -> this: 4096 x 11008
+// HASH, 128 tokens 44.5 -> 29.2 us, 512 61.5 -> 56.1; 1024 x 14336, 256 tokens 53.8 -> 29.9; 4096 x 4096 in 32 banks, 112 tokens 36.9 ->
+// 20.6; on the other side of the line 14336 x 1024, 512 tokens 38.7 -> 51.7, 22016 x 4096, 2048 tokens 350 -> 406.
+static bool few_is_faster(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     FewParams p;
-    return f.layout == RPTC_LAYOUT_TILED && f.quirk == RPTC_QUIRK_NONE && (f.K == 2 || f.K == 4) && n % 64 == 0 && tokens <= kFewMaxTokens &&
-           (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ld_x % 8 == 0 &&
-           few_plan(p, f, tokens, 2);
+    const int rb = few_choose(p, f, m, tokens);
+    if (!rb || !p.shared) return rb != 0;
+    const int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1, waves = (banks.banks * ctas + num_sms() - 1) / num_sms();
+    const int64_t n_steps = n / 64, steps = (few_tiles(m, rb) * p.token_tiles * n_steps + ctas - 1) / ctas;
+    const double drains = 1 + steps / n_steps;
+    const double us = waves * ((f.code == RPTC_CODE_LUT ? 8.0 : 12.0) + steps * shared_step_us(rb, p.n_cols, f.code) + drains * 0.0105 * rb * p.n_cols) +
+                      (double)banks.banks * m * tokens * 8 / 4.5e6;
+    const double gemm = gemm_us(m, n, tokens, banks, f);
+    return gemm == 0 || us < gemm;
+}
+
+bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, const void *x, int64_t ld_x) {
+    if (f.layout != RPTC_LAYOUT_TILED || f.quirk != RPTC_QUIRK_NONE || (f.K != 2 && f.K != 4) || n % 64 || (reinterpret_cast<uintptr_t>(x) & 15) || ld_x % 8)
+        return false;
+    // a layer asks several times per call, and mostly the question of the call before
+    struct Question {
+        int64_t m, n, tokens;
+        int32_t banks, code, K, L, S;
+        bool operator==(const Question &o) const {
+            return m == o.m && n == o.n && tokens == o.tokens && banks == o.banks && code == o.code && K == o.K && L == o.L && S == o.S;
+        }
+    };
+    static thread_local Question last = {};
+    static thread_local bool last_answer = false;
+    const Question q = {m, n, tokens, banks.banks, f.code, f.K, f.L, f.S};
+    if (q == last) return last_answer;
+    last_answer = few_is_faster(m, n, tokens, banks, f);
+    last = q;
+    return last_answer;
 }
 
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s) {
     FewParams p;
-    const int rb = few_row_blocks(m, tokens);
-    if (!few_plan(p, f, tokens, rb)) return RPTC_ERR_UNSUPPORTED;
+    const int rb = few_choose(p, f, m, tokens);
+    if (!rb) return RPTC_ERR_UNSUPPORTED;
     CUtensorMap map;
     if (int e = encode_map(map, x, n, tokens, ld_x, p.n_cols)) return e;
     p.codes = static_cast<const uint4 *>(codes);
@@ -437,7 +489,7 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
     p.n_steps = (int32_t)(n / 64);
     p.n_units = (int32_t)(n * f.K / 128);
     p.tokens = (int32_t)tokens;
-    p.tiles = (int32_t)((m + rb * 128 - 1) / (rb * 128));
+    p.tiles = (int32_t)few_tiles(m, rb);
     const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
     if (steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
     // one bank's table per CTA: the SMs are dealt out to the banks

@@ -124,9 +124,10 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
 // Which product a packed layer takes, and how many columns it gives per bank.
 static bool packed_plan(const rptc_packed &l, int64_t tokens, int64_t &cols) {
     const rptc_format f = {RPTC_CODE_LUT, 2, l.L, 0, RPTC_LAYOUT_TILED, RPTC_QUIRK_NONE};
-    const bool few = tokens <= kFewMaxTokens;
     Banks banks;
     banks.banks = l.banks;
+    banks.lut_stride = int64_t(1) << l.L;
+    const bool few = tokens <= kFewOwnTokens || gemv_few_takes((int64_t)l.bank_blocks * 32, l.n, tokens, banks, f, nullptr, l.n);
     cols = few ? (int64_t)l.bank_blocks * 32 : gemm_bank_columns((int64_t)l.bank_blocks * 32, l.n, tokens, banks, f);
     return few;
 }
@@ -180,7 +181,7 @@ extern "C" int rptc_packed_forward(const rptc_packed *l, const void *x, int dtyp
 // Whether the product goes through the fp32 accumulator: one or two rows, whatever the kernel for a few rows takes, and
 // up to 64 rows of a shape that the tiled product does not cover.
 static bool linear_few(const rptc_linear &l, int64_t rows) {
-    return rows <= 2 || gemv_few_takes(l.n, rows, l.fmt, nullptr, l.n) || (rows <= 64 && (l.m % 128 || l.n % 64));
+    return rows <= 2 || gemv_few_takes(l.m, l.n, rows, Banks(), l.fmt, nullptr, l.n) || (rows <= 64 && (l.m % 128 || l.n % 64));
 }
 
 extern "C" int64_t rptc_linear_workspace_bytes(const rptc_linear *l, int64_t rows) {

@@ -19,9 +19,12 @@ int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, const Banks &ban
 // result.  Shapes and alignments as rptc_gemm's, with m % 32 == 0 where banks > 1.
 int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
                 int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
-// acc[b][bank * m + row] += sum_c W[bank][row][c] x[b][c], up to kFewMaxTokens activation rows, where gemv_few_takes says so.
-constexpr int64_t kFewMaxTokens = 96;
-bool gemv_few_takes(int64_t n, int64_t tokens, const rptc_format &f, const void *x, int64_t ld_x);
+// The estimate that gemm_banked's choice of tiles rests on, microseconds; 0 where it takes no such product.
+double gemm_us(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f);
+// acc[b][bank * m + row] += sum_c W[bank][row][c] x[b][c] for any number of activation rows that gemv_few_takes says yes to (up to
+// kFewOwnTokens whatever the shape).
+constexpr int64_t kFewOwnTokens = 96;
+bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, const void *x, int64_t ld_x);
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
 // The same for any number of activation rows (TILED codes, no quirk, no carry): gemv_few where it takes them, else the

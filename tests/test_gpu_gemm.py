@@ -151,3 +151,24 @@ def test_gemm_invariant_gives_a_token_the_same_bits_in_any_company():
     full = ops.gemm(codes, lut, x, m, n, fmt, invariant=True)
     for tokens in (9, 128, 200, 1000):
         assert torch.equal(ops.gemm(codes, lut, x[:tokens], m, n, fmt, invariant=True), full[:tokens]), tokens
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 16, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("m,n,tokens", [(32, 8192, 97), (160, 11008, 112), (1056, 8256, 193), (288, 4160, 385), (4096, 4096, 160)])
+def test_layer_of_some_hundred_tokens(code, K, L, S, m, n, tokens):
+    """Products that share an accumulator between the groups of a row block: rows past a tile's end, a last tile of few tokens, ranges
+    that start inside a tile."""
+    from rptc_b200 import Format, ops
+    from rptc_b200.linear import RPTCLinear
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    fmt = Format(code, K, L, S, o.LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, K, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn((tokens, n), dtype=torch.float16, device="cuda", generator=g)
+    y = RPTCLinear(n, m, fmt, codes, lut, 1.0)(x)
+    torch.cuda.synchronize()
+    ops.device_status()
+    dense = ops.decompress(codes, lut, m, n, fmt).double()
+    err = (y.double() - x.double() @ dense.t()).abs()
+    bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
+    assert float((err / bound).max()) <= 1.0
