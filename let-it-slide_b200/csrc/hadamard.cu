@@ -173,6 +173,7 @@ int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int
 // against 19.3; up to 128 rows both take 3.3).  Smaller blocks need no barrier in the kernels with eight values per thread,
 // which have more warps in flight: those stay ahead until the memory traffic is what counts (512 x 11008: 8.8 us against
 // 9.6; 2048 x 12288: 31.5 against 27.1).
+int swiglu_rows(const SwigluParams &p, int64_t rows, cudaStream_t stream);
 static bool many_rows(int64_t rows, int64_t n, int block) { return block > 256 ? rows >= 32 : rows * n >= (int64_t(8) << 20); }
 
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
@@ -258,6 +259,10 @@ static int swiglu_launch(float *acc, const void *in16, int64_t ld_in, void *out,
     p.clear = acc ? clear : 0;
     p.scale_out = scale_out * hadamard_norm(block);
     p.scale_in = scale_in * hadamard_norm(block);
+    // Prompts: from a full set of warps on (16 per SM, 512 columns of a row each), with rows on 32-byte boundaries.
+    if (in16 && block == 256 && rows * n >= (int64_t)num_sms() * 16 * 512 && ld_in % 16 == 0 && ld_out % 16 == 0 &&
+        ((reinterpret_cast<uintptr_t>(in16) | reinterpret_cast<uintptr_t>(out)) & 31) == 0)
+        return swiglu_rows(p, rows, static_cast<cudaStream_t>(stream));
     if (block <= 256 && n > 256) {      // a warp per 256 columns, eight warps per CTA
         p.chunk = 2048;
         static SmemOptIn preferred;

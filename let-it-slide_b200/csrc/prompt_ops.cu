@@ -177,6 +177,147 @@ int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int
                      : launch(hadamard_rows_kernel<true, false>, grid, dim3(128), 0, stream, p);
 }
 
+// ---- SwiGLU between its transforms, blocks of 256 ---------------------------------------------------------------------
+// out = H(s_in * fp16(silu(g) * u)) * scale_in with (g | u) = fp16(s_out * H(in) * scale_out): the arithmetic and the order of
+// stages of swiglu_hadamard_kernel, so the results are the same bits.  A warp takes 512 columns (a half-warp per block) and walks down
+// the rows, the next row's values under way.  A thread holds sixteen values of a block,
+//   near   elements 16 t .. 16 t + 15: the stages of bits 0-3, loads and stores of 32 bytes
+//   far    elements t + 16 k: the stages of bits 4-7, signs, the SwiGLU
+// and an exchange through shared memory costs a fifth of the five shuffle stages per value that bound the kernel with
+// eight values per thread (2048 x 11008: 88 us there).
+// The four 16-byte pieces of sixteen values sit at piece ^ (t >> 1): no bank conflicts in either layout.
+constexpr int kSwHalfFloats = 256 + 16, kSwWarpFloats = 2 * kSwHalfFloats;
+struct Near16 {
+    float *row;
+    int x;
+    __device__ __forceinline__ Near16(float *half, int t) : row(half + 16 * t), x((t >> 1) & 3) {}
+    __device__ __forceinline__ void put(const float (&v)[16]) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) *reinterpret_cast<float4 *>(row + 4 * (c ^ x)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    }
+    __device__ __forceinline__ void get(float (&v)[16]) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 f = *reinterpret_cast<const float4 *>(row + 4 * (c ^ x));
+            v[4 * c] = f.x, v[4 * c + 1] = f.y, v[4 * c + 2] = f.z, v[4 * c + 3] = f.w;
+        }
+    }
+};
+struct Far16 {
+    float *at[4];
+    __device__ __forceinline__ Far16(float *half, int t) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) at[q] = half + 4 * ((t >> 2) ^ q) + (t & 3);
+    }
+    __device__ __forceinline__ void put(const float (&v)[16]) const {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) at[(k >> 1) & 3][16 * k] = v[k];
+    }
+    __device__ __forceinline__ void get(float (&v)[16]) const {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = at[(k >> 1) & 3][16 * k];
+    }
+};
+__device__ __forceinline__ void ld_32_bytes(const __half *p, uint32_t (&r)[8]) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st_32_bytes(__half *p, const uint32_t (&r)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
+                 "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void unpack_pairs(const uint32_t (&r)[8], float (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float2 f = __half22float2(u32_as_half2(r[i]));
+        v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+}
+
+__global__ void __launch_bounds__(256, 2) swiglu_rows_kernel(const SwigluParams p, int64_t rows) {
+    __shared__ __align__(16) float smem[8 * kSwWarpFloats];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 15, half = lane >> 4;
+    float *buf = smem + warp * kSwWarpFloats + half * kSwHalfFloats;
+    const Near16 near(buf, t);
+    const Far16 far(buf, t);
+    const int segs = (int)((p.n + 511) / 512);
+    const int64_t worker = (int64_t)blockIdx.x * 8 + warp, workers = (int64_t)gridDim.x * 8 / segs * segs;
+    pdl_allow_next_grid();
+    // A last segment of one block: both halves of the warp take it, one stores.  (Zeros instead cost 1.6 times the kernel's time:
+    // a division of zero takes the slow path.)
+    const int64_t first = (worker % segs) * 512 + 256 * half;
+    const bool active = first < p.n;
+    const int64_t block0 = active ? first : p.n - 256;
+    uint32_t sg[8], su[8], si[8];                            // signs in the far layout, two to a register
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        auto pair = [&](const __half *s) {
+            return s ? half2_as_u32(__halves2half2(s[block0 + t + 32 * i], s[block0 + t + 32 * i + 16])) : 0x3C003C00u;
+        };
+        sg[i] = pair(p.signs_out), su[i] = pair(p.signs_out ? p.signs_out + p.n : nullptr), si[i] = pair(p.signs_in);
+    }
+    pdl_wait_prior_grids();
+    if (worker >= workers) return;
+    const int64_t step = workers / segs;
+    uint32_t rg[8], ru[8];
+    auto fetch = [&](int64_t row) {
+        const __half *src = p.in16 + row * p.ld_acc + block0 + 16 * t;
+        ld_32_bytes(src, rg);
+        ld_32_bytes(src + p.n, ru);
+    };
+    int64_t row = worker / segs;
+    if (row < rows) fetch(row);
+    for (; row < rows; row += step) {
+        float g[16], u[16], s[16];
+        unpack_pairs(rg, g);
+        unpack_pairs(ru, u);
+        if (row + step < rows) fetch(row + step);
+        stages16(g);
+        near.put(g);
+        stages16(u);
+        __syncwarp();
+        far.get(g);
+        __syncwarp();
+        near.put(u);
+        stages16(g);
+        __syncwarp();
+        far.get(u);
+        stages16(u);
+        unpack_pairs(sg, s);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) g[k] *= p.scale_out * s[k];
+        unpack_pairs(su, s);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) u[k] *= p.scale_out * s[k];
+        unpack_pairs(si, s);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {                       // fp16 where the unfused path stores fp16
+            const float gg = __half2float(__float2half_rn(g[k])), uu = __half2float(__float2half_rn(u[k]));
+            g[k] = __half2float(__float2half_rn(gg / (1.f + __expf(-gg)) * uu)) * s[k];
+        }
+        far.put(g);                                          // where this thread has read
+        __syncwarp();
+        near.get(g);
+        stages16(g);
+        near.put(g);
+        __syncwarp();
+        far.get(g);
+        stages16(g);
+        far.put(g);
+        __syncwarp();
+        near.get(g);
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = half2_as_u32(__floats2half2_rn(g[2 * i] * p.scale_in, g[2 * i + 1] * p.scale_in));
+        if (active) st_32_bytes(p.out + row * p.ld_out + block0 + 16 * t, o);
+    }
+}
+int swiglu_rows(const SwigluParams &p, int64_t rows, cudaStream_t stream) {
+    return launch(swiglu_rows_kernel, dim3(rows_grid(rows, (p.n + 511) / 512, 8, 2)), dim3(256), 0, stream, p, rows);
+}
+
 // ---- residual + RMSNorm + input transform -----------------------------------------------------------------------------
 struct NormRowsParams {
     const __half *y;                 // [rows][ld_y]: the product in front, before its output transform, or NULL
