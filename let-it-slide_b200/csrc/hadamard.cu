@@ -170,11 +170,15 @@ int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int
                   int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
                   cudaStream_t stream);
 // Which inputs go to the kernels that walk down the rows.  Blocks above 256 columns: from 32 rows on (2048 x 4096: 13.4 us
-// against 19.3; up to 128 rows both take 3.3).  Smaller blocks need no barrier in the kernels with eight values per thread,
-// which have more warps in flight: those stay ahead until the memory traffic is what counts (512 x 11008: 8.8 us against
-// 9.6; 2048 x 12288: 31.5 against 27.1).
+// against 19.3; up to 128 rows both take 3.3).  Smaller blocks, with rows on 32-byte boundaries: from 2.5 million values on (512 x 11008:
+// 7.6 us against 8.9, 512 x 4096: 4.5 against 4.2).
 int swiglu_rows(const SwigluParams &p, int64_t rows, cudaStream_t stream);
-static bool many_rows(int64_t rows, int64_t n, int block) { return block > 256 ? rows >= 32 : rows * n >= (int64_t(8) << 20); }
+static bool many_rows(int64_t rows, int64_t n, int block, const HadParams &p) {
+    if (block > 256) return rows >= 32;
+    auto on_32_bytes = [](const void *q, int64_t ld_bytes) { return ((reinterpret_cast<uintptr_t>(q) | (uintptr_t)ld_bytes) & 31) == 0; };
+    return block >= 16 && rows * n >= (int64_t(5) << 19) && on_32_bytes(p.in, p.ld_in * (p.in_is_f32 ? 4 : 2)) && on_32_bytes(p.out, p.ld_out * 2) &&
+           (!p.residual || on_32_bytes(p.residual, p.ld_res * 2));
+}
 
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
@@ -191,9 +195,6 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
         return RPTC_ERR_ALIGN;
     if (clear_in && !in_is_f32) return RPTC_ERR_ARG;
     if (int e = rptc_check_device()) return e;
-    if (many_rows(rows, n, block))
-        return hadamard_rows(in, in_is_f32, ld_in, static_cast<__half *>(out), ld_out, static_cast<const __half *>(signs),
-                             static_cast<const __half *>(residual), ld_res, rows, n, block, transpose, scale, clear_in, clear, clear_count, stream);
     HadParams p;
     p.in = in;
     p.ld_in = ld_in;
@@ -206,6 +207,9 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
     p.chunk = chunk;
     p.in_is_f32 = in_is_f32;
     p.transpose = transpose;
+    if (many_rows(rows, n, block, p))
+        return hadamard_rows(in, in_is_f32, ld_in, static_cast<__half *>(out), ld_out, static_cast<const __half *>(signs),
+                             static_cast<const __half *>(residual), ld_res, rows, n, block, transpose, scale, clear_in, clear, clear_count, stream);
     p.clear_in = clear_in;
     p.scale = scale * hadamard_norm(block);
     p.n = n;

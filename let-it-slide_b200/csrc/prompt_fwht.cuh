@@ -1,12 +1,11 @@
 // Walsh-Hadamard building blocks for many rows (prompts): 32 values per thread, exchanges through shared memory.
 //
-// A segment is 1024 columns for a warp (blocks of at most 256) or 4096 for a CTA of 128 threads (any block up to 4096); it
+// A segment is 4096 columns for a CTA of 128 threads (blocks of more than 256, up to 4096); it
 // may hold several blocks.  Element e of a segment is at e + 8 (e >> 8) in the exchange buffer, which keeps all accesses
 // below free of bank conflicts.  The layouts of a thread's 32 values, by the bits of e that vary inside the thread:
-//   pieces   bits 0-2 and two more (warp: 8, 9; CTA: 10, 11): four pieces of eight consecutive elements, loaded and stored
-//            as 16 bytes of fp16 each
+//   pieces   bits 0-2, 10 and 11: four pieces of eight consecutive elements, loaded and stored as 16 bytes of fp16 each
 //   columns  bits 3-7
-//   far      (CTA) bits 0 and 8-11: sixteen pairs, 256 elements apart
+//   far      bits 0 and 8-11: sixteen pairs, 256 elements apart
 // A transform does the stages of bits 0-2 in pieces, 3-7 in columns, 8-11 in far: in ascending order, the order of the
 // kernels with eight values per thread, so that the results of both are the same bits.  Stages at or above the block size
 // are skipped.  A thread that has read its values in one layout may write them in the same layout without a barrier.
@@ -18,7 +17,7 @@
 
 namespace rptc {
 
-constexpr int kWarpSegFloats = 1024 + 32, kCtaSegFloats = 4096 + 128;
+constexpr int kCtaSegFloats = 4096 + 128;
 
 // One butterfly stage over bit `H` of the index of v.
 template <int H>
@@ -55,20 +54,16 @@ __device__ __forceinline__ void far_stages(float (&v)[32], int block_bits) {
 }
 
 // Where a thread's values are; t of 128 threads in a CTA segment.
-template <bool CTA>
 struct SegThread {
     int lane, warp, t;
-    __device__ __forceinline__ SegThread() : lane(threadIdx.x & 31), warp(CTA ? (threadIdx.x >> 5) & 3 : 0), t(threadIdx.x & 127) {}
-    __device__ __forceinline__ int piece(int j) const { return CTA ? 8 * t + 1024 * j : 8 * lane + 256 * j; }
+    __device__ __forceinline__ SegThread() : lane(threadIdx.x & 31), warp((threadIdx.x >> 5) & 3), t(threadIdx.x & 127) {}
+    __device__ __forceinline__ int piece(int j) const { return 8 * t + 1024 * j; }
     __device__ __forceinline__ int pair(int k) const { return 2 * t + 256 * k; }
     __device__ __forceinline__ int column() const {      // element of k = 0: bits 0-2 from the lane, bits 8 up from the rest
         return (lane & 7) + 256 * ((lane >> 3) + 4 * warp);
     }
     static __device__ __forceinline__ int at(int e) { return e + 8 * (e >> 8); }
-    static __device__ __forceinline__ void sync() {
-        if (CTA) __syncthreads();
-        else __syncwarp();
-    }
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
     // The two halves of a piece as 16-byte accesses; lanes with bit 2 set take the upper half first, so that eight lanes
     // with a stride of 32 bytes meet all banks once.
     __device__ __forceinline__ void put_pieces(float *buf, const float (&v)[32]) const {

@@ -36,18 +36,15 @@ struct HadRowsParams {
 
 __device__ __forceinline__ uint32_t ldcg_u32(const void *p) { return __ldcg(static_cast<const uint32_t *>(p)); }
 
-// One segment of a row per warp (blocks up to 256, results in the layout of the pieces) or per CTA of 128 threads (results in
-// the layout of the pairs).
-template <bool CTA, bool IN_F32>
-__global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_kernel(const HadRowsParams p) {
-    constexpr int kSeg = CTA ? 4096 : 1024, kUnits = CTA ? 1 : 8;       // segments per CTA
+// Blocks above 256: one segment of a row per CTA of 128 threads, results in the layout of the pairs.
+template <bool IN_F32>
+__global__ void __launch_bounds__(128, 4) hadamard_rows_kernel(const HadRowsParams p) {
+    constexpr int kSeg = 4096;
     constexpr uint32_t kOnes = 0x3C003C00u;
-    __shared__ __align__(16) float smem[CTA ? kCtaSegFloats : 8 * kWarpSegFloats];
-    const SegThread<CTA> th;
-    const int unit = CTA ? 0 : threadIdx.x >> 5;
-    float *buf = smem + unit * kWarpSegFloats;
+    __shared__ __align__(16) float buf[kCtaSegFloats];
+    const SegThread th;
     const int segs = (int)((p.n + kSeg - 1) / kSeg);
-    const int64_t worker = (int64_t)blockIdx.x * kUnits + unit, workers = (int64_t)gridDim.x * kUnits / segs * segs;
+    const int64_t worker = blockIdx.x, workers = (int64_t)gridDim.x / segs * segs;
     pdl_allow_next_grid();
     pdl_wait_prior_grids();
     if (p.clear) {
@@ -59,7 +56,7 @@ __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_ke
     const int64_t col0 = (worker % segs) * kSeg;
     // the columns of pair of values i (v[2 i], v[2 i + 1]) as loaded and as stored
     auto col_in = [&](int i) { return col0 + th.piece(i >> 2) + 2 * (i & 3); };
-    auto col_out = [&](int i) { return CTA ? col0 + th.pair(i) : col_in(i); };
+    auto col_out = [&](int i) { return col0 + th.pair(i); };
     uint32_t sg[16];                                         // signs of the columns where they apply, two to a register
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -105,12 +102,8 @@ __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_ke
         column_stages(v, p.block_bits);
         th.put_columns(buf, v);
         th.sync();
-        if (CTA) {
-            th.get_pairs(buf, v);
-            far_stages(v, p.block_bits);
-        } else {
-            th.get_pieces(buf, v);
-        }
+        th.get_pairs(buf, v);
+        far_stages(v, p.block_bits);
         uint32_t o[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -127,66 +120,21 @@ __global__ void __launch_bounds__(CTA ? 128 : 256, CTA ? 4 : 2) hadamard_rows_ke
             o[i] = half2_as_u32(__floats2half2_rn(w.x, w.y));
         }
         __half *dst = p.out + row * p.ld_out;
-        if (CTA) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (col_out(i) < p.n) *reinterpret_cast<uint32_t *>(dst + col_out(i)) = o[i];
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (col0 + th.piece(j) < p.n) *reinterpret_cast<uint4 *>(dst + col0 + th.piece(j)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-        }
+        for (int i = 0; i < 16; ++i)
+            if (col_out(i) < p.n) *reinterpret_cast<uint32_t *>(dst + col_out(i)) = o[i];
         th.sync();                                           // the buffer is free for the next row
     }
 }
 
-// Grid of a kernel whose CTAs walk down the rows: as many as are resident at once, no more than there is work for.
-static unsigned rows_grid(int64_t rows, int64_t segs, int units, int resident) {
-    const int64_t want = (rows * segs + units - 1) / units, most = (int64_t)num_sms() * resident;
-    const int64_t least = (segs + units - 1) / units;        // every segment needs a worker
-    const int64_t g = want < most ? want : most;
-    return (unsigned)(g > least ? g : least);
-}
-
-int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int64_t ld_out, const __half *signs, const __half *residual,
-                  int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
-                  cudaStream_t stream) {
-    HadRowsParams p;
-    p.in = in;
-    p.ld_in = ld_in;
-    p.out = out;
-    p.ld_out = ld_out;
-    p.signs = signs;
-    p.residual = residual;
-    p.ld_res = ld_res;
-    p.rows = rows;
-    p.n = n;
-    p.block_bits = log2_of(block);
-    p.transpose = transpose;
-    p.clear_in = clear_in;
-    p.scale = scale * norm_of(block);
-    p.clear = clear_count > 0 ? clear : nullptr;
-    p.clear_count = clear_count;
-    if (block <= 256) {
-        const dim3 grid(rows_grid(rows, (n + 1023) / 1024, 8, 2));
-        return in_is_f32 ? launch(hadamard_rows_kernel<false, true>, grid, dim3(256), 0, stream, p)
-                         : launch(hadamard_rows_kernel<false, false>, grid, dim3(256), 0, stream, p);
-    }
-    const dim3 grid(rows_grid(rows, (n + 4095) / 4096, 1, 4));
-    return in_is_f32 ? launch(hadamard_rows_kernel<true, true>, grid, dim3(128), 0, stream, p)
-                     : launch(hadamard_rows_kernel<true, false>, grid, dim3(128), 0, stream, p);
-}
-
-// ---- SwiGLU between its transforms, blocks of 256 ---------------------------------------------------------------------
-// out = H(s_in * fp16(silu(g) * u)) * scale_in with (g | u) = fp16(s_out * H(in) * scale_out): the arithmetic and the order of
-// stages of swiglu_hadamard_kernel, so the results are the same bits.  A warp takes 512 columns (a half-warp per block) and walks down
-// the rows, the next row's values under way.  A thread holds sixteen values of a block,
+// ---- blocks of at most 256: sixteen values per thread ------------------------------------------------------------------
+// A warp takes 512 columns (a half-warp 256, thread t of 16) and walks down the rows, the next row's values under way:
 //   near   elements 16 t .. 16 t + 15: the stages of bits 0-3, loads and stores of 32 bytes
-//   far    elements t + 16 k: the stages of bits 4-7, signs, the SwiGLU
-// and an exchange through shared memory costs a fifth of the five shuffle stages per value that bound the kernel with
-// eight values per thread (2048 x 11008: 88 us there).
-// The four 16-byte pieces of sixteen values sit at piece ^ (t >> 1): no bank conflicts in either layout.
-constexpr int kSwHalfFloats = 256 + 16, kSwWarpFloats = 2 * kSwHalfFloats;
+//   far    elements t + 16 k: the stages of bits 4-7
+// with an exchange through shared memory in between, a fifth of the cost of a shuffle per value and stage.  The four 16-byte pieces
+// of sixteen values sit at piece ^ (t >> 1): no bank conflicts in either layout.  Bound: HBM.  2048 x 11008 with 32 values per thread and no
+// row ahead 26.8 us, with eight values and shuffles 31.5, as it is 20.1 (fp32 input 26.5); four CTAs per SM spill registers: 25.3.
+constexpr int kHalfFloats = 256 + 16, kPairFloats = 2 * kHalfFloats;
 struct Near16 {
     float *row;
     int x;
@@ -218,12 +166,12 @@ struct Far16 {
         for (int k = 0; k < 16; ++k) v[k] = at[(k >> 1) & 3][16 * k];
     }
 };
-__device__ __forceinline__ void ld_32_bytes(const __half *p, uint32_t (&r)[8]) {
+__device__ __forceinline__ void ld_32_bytes(const void *p, uint32_t (&r)[8]) {
     asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "l"(p));
 }
-__device__ __forceinline__ void st_32_bytes(__half *p, const uint32_t (&r)[8]) {
+__device__ __forceinline__ void st_32_bytes(void *p, const uint32_t (&r)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
                  "r"(r[6]), "r"(r[7])
                  : "memory");
@@ -236,10 +184,150 @@ __device__ __forceinline__ void unpack_pairs(const uint32_t (&r)[8], float (&v)[
     }
 }
 
-__global__ void __launch_bounds__(256, 2) swiglu_rows_kernel(const SwigluParams p, int64_t rows) {
-    __shared__ __align__(16) float smem[8 * kSwWarpFloats];
+// Bits 4-7 of blocks of 32 to 256: v[k] is element bits 4-7 = k.
+__device__ __forceinline__ void far_stages16(float (&v)[16], int block_bits) {
+    if (block_bits == 8) return stages16(v);
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+        if (block_bits > 4 + (h == 1 ? 0 : h == 2 ? 1 : 2)) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if ((i & h) == 0) {
+                    const float a = v[i], b = v[i + h];
+                    v[i] = a + b;
+                    v[i + h] = a - b;
+                }
+        }
+}
+template <bool IN_F32>
+__global__ void __launch_bounds__(256, IN_F32 ? 2 : 3) hadamard_half_rows_kernel(const HadRowsParams p) {
+    __shared__ __align__(16) float smem[8 * kPairFloats];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 15, half = lane >> 4;
-    float *buf = smem + warp * kSwWarpFloats + half * kSwHalfFloats;
+    float *buf = smem + warp * kPairFloats + half * kHalfFloats;
+    const Near16 near(buf, t);
+    const Far16 far(buf, t);
+    const int segs = (int)((p.n + 511) / 512);
+    const int64_t worker = (int64_t)blockIdx.x * 8 + warp, workers = (int64_t)gridDim.x * 8 / segs * segs;
+    pdl_allow_next_grid();
+    const int64_t col = (worker % segs) * 512 + 256 * half + 16 * t;
+    const bool active = col < p.n;                           // a last segment of 256 columns leaves half of the warp without
+    uint32_t sg[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sg[i] = p.signs && active ? __ldg(reinterpret_cast<const uint32_t *>(p.signs + col) + i) : 0x3C003C00u;
+    pdl_wait_prior_grids();
+    if (p.clear) {
+        float4 *z = reinterpret_cast<float4 *>(p.clear);
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < p.clear_count; i += (int64_t)gridDim.x * blockDim.x)
+            z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (worker >= workers) return;
+    const int64_t step = workers / segs;
+    uint32_t raw[IN_F32 ? 2 : 1][8] = {};
+    auto fetch = [&](int64_t row) {
+        if (!active) return;
+        if (IN_F32) {
+            float *src = const_cast<float *>(static_cast<const float *>(p.in)) + row * p.ld_in + col;
+            ld_32_bytes(src, raw[0]);
+            ld_32_bytes(src + 8, raw[IN_F32 ? 1 : 0]);
+            if (p.clear_in) {
+                const uint32_t zero[8] = {};
+                st_32_bytes(src, zero);
+                st_32_bytes(src + 8, zero);
+            }
+        } else {
+            ld_32_bytes(static_cast<const __half *>(p.in) + row * p.ld_in + col, raw[0]);
+        }
+    };
+    int64_t row = worker / segs;
+    if (row < p.rows) fetch(row);
+    for (; row < p.rows; row += step) {
+        float v[16], s[16];
+        if (IN_F32) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[IN_F32 ? i >> 3 : 0][i & 7]);
+        } else {
+            unpack_pairs(raw[0], v);
+        }
+        uint32_t res[8];
+        if (p.residual && active) ld_32_bytes(p.residual + row * p.ld_res + col, res);
+        if (row + step < p.rows) fetch(row + step);
+        unpack_pairs(sg, s);
+        if (!p.transpose) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] *= s[i];
+        }
+        stages16(v);
+        if (p.block_bits > 4) {
+            near.put(v);                                     // where this thread has read
+            __syncwarp();
+            far.get(v);
+            far_stages16(v, p.block_bits);
+            far.put(v);
+            __syncwarp();
+            near.get(v);
+        }
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float2 f = make_float2(p.scale, p.scale);
+            if (p.transpose) f.x *= s[2 * i], f.y *= s[2 * i + 1];
+            float2 w = make_float2(__fmul_rn(v[2 * i], f.x), __fmul_rn(v[2 * i + 1], f.y));
+            if (p.residual) {
+                const float2 r = __half22float2(u32_as_half2(res[i]));
+                w.x = __fadd_rn(w.x, r.x), w.y = __fadd_rn(w.y, r.y);
+            }
+            o[i] = half2_as_u32(__floats2half2_rn(w.x, w.y));
+        }
+        if (active) st_32_bytes(p.out + row * p.ld_out + col, o);
+    }
+}
+
+// Grid of a kernel whose CTAs walk down the rows: as many as are resident at once, no more than there is work for.
+static unsigned rows_grid(int64_t rows, int64_t segs, int units, int resident) {
+    const int64_t want = (rows * segs + units - 1) / units, most = (int64_t)num_sms() * resident;
+    const int64_t least = (segs + units - 1) / units;        // every segment needs a worker
+    const int64_t g = want < most ? want : most;
+    return (unsigned)(g > least ? g : least);
+}
+
+int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int64_t ld_out, const __half *signs, const __half *residual,
+                  int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
+                  cudaStream_t stream) {
+    HadRowsParams p;
+    p.in = in;
+    p.ld_in = ld_in;
+    p.out = out;
+    p.ld_out = ld_out;
+    p.signs = signs;
+    p.residual = residual;
+    p.ld_res = ld_res;
+    p.rows = rows;
+    p.n = n;
+    p.block_bits = log2_of(block);
+    p.transpose = transpose;
+    p.clear_in = clear_in;
+    p.scale = scale * norm_of(block);
+    p.clear = clear_count > 0 ? clear : nullptr;
+    p.clear_count = clear_count;
+    if (block <= 256) {
+        const dim3 grid(rows_grid(rows, (n + 511) / 512, 8, in_is_f32 ? 2 : 3));
+        return in_is_f32 ? launch(hadamard_half_rows_kernel<true>, grid, dim3(256), 0, stream, p)
+                         : launch(hadamard_half_rows_kernel<false>, grid, dim3(256), 0, stream, p);
+    }
+    const dim3 grid(rows_grid(rows, (n + 4095) / 4096, 1, 4));
+    return in_is_f32 ? launch(hadamard_rows_kernel<true>, grid, dim3(128), 0, stream, p)
+                     : launch(hadamard_rows_kernel<false>, grid, dim3(128), 0, stream, p);
+}
+
+// ---- SwiGLU between its transforms, blocks of 256 ---------------------------------------------------------------------
+// out = H(s_in * fp16(silu(g) * u)) * scale_in with (g | u) = fp16(s_out * H(in) * scale_out): the arithmetic and the order of
+// stages of swiglu_hadamard_kernel, so the results are the same bits.  A warp takes 512 columns (a half-warp per block) and walks down
+// the rows, the next row's values under way.  The kernel with eight values per thread is bound by its five shuffle stages per value.  2048 x
+// 11008: 84.8 -> 55.5 us (bound by instruction issue, the division most of all).
+__global__ void __launch_bounds__(256, 2) swiglu_rows_kernel(const SwigluParams p, int64_t rows) {
+    __shared__ __align__(16) float smem[8 * kPairFloats];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 15, half = lane >> 4;
+    float *buf = smem + warp * kPairFloats + half * kHalfFloats;
     const Near16 near(buf, t);
     const Far16 far(buf, t);
     const int segs = (int)((p.n + 511) / 512);
@@ -341,7 +429,7 @@ __global__ void __launch_bounds__(128 * NH, 4 / NH) norm_rows_kernel(const NormR
     constexpr int n = 4096 * NH;
     __shared__ __align__(16) float smem[NH * kCtaSegFloats];
     __shared__ float red[8], carry[2][128];
-    const SegThread<true> th;
+    const SegThread th;
     const int part = threadIdx.x >> 7;
     float *buf = smem + part * kCtaSegFloats;
     const int col0 = 4096 * part;
@@ -463,75 +551,87 @@ __global__ void __launch_bounds__(64) rope_angles_kernel(float2 *__restrict__ ou
     out[(int64_t)blockIdx.x * 64 + threadIdx.x] = make_float2(cs, sn);
 }
 
-// A warp takes eight heads of a token: after the column stages a thread holds both members of every rotated pair
-// (elements i and i + 64 differ in bit 6).
-__global__ void __launch_bounds__(256, 2) qkv_rows_kernel(const QkvRowsParams p) {
-    __shared__ __align__(16) float smem[8 * kWarpSegFloats];
-    const SegThread<false> th;
-    const int unit = threadIdx.x >> 5;
-    float *buf = smem + unit * kWarpSegFloats;
-    const int heads = p.hq + 2 * p.hkv, n = heads * 128, segs = (n + 1023) / 1024;
-    const int64_t worker = (int64_t)blockIdx.x * 8 + unit, workers = (int64_t)gridDim.x * 8 / segs * segs;
+// A half-warp takes two heads of a token: in the far layout a thread holds both members of every rotated pair (elements i and
+// i + 64 differ in bit 6).  WIDE: everything on 32-byte boundaries.  Bound: HBM, with the next token's values under way.
+template <bool WIDE>
+__device__ __forceinline__ void ld_half_row(const __half *p, uint32_t (&r)[8]) {
+    if (WIDE) return ld_32_bytes(p, r);
+    const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(p)), b = __ldcg(reinterpret_cast<const uint4 *>(p) + 1);
+    r[0] = a.x, r[1] = a.y, r[2] = a.z, r[3] = a.w, r[4] = b.x, r[5] = b.y, r[6] = b.z, r[7] = b.w;
+}
+template <bool WIDE>
+__global__ void __launch_bounds__(256, 3) qkv_rows_kernel(const QkvRowsParams p) {
+    __shared__ __align__(16) float smem[8 * kPairFloats];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 15, half = lane >> 4;
+    float *buf = smem + warp * kPairFloats + half * kHalfFloats;
+    const Near16 near(buf, t);
+    const Far16 far(buf, t);
+    const int heads = p.hq + 2 * p.hkv, n = heads * 128, segs = (n + 511) / 512;
+    const int64_t worker = (int64_t)blockIdx.x * 8 + warp, workers = (int64_t)gridDim.x * 8 / segs * segs;
     pdl_allow_next_grid();
     if (worker >= workers) return;
-    const int col0 = (int)(worker % segs) * 1024;
-    uint32_t signs = 0;                                       // bit k: the sign of this thread's column element k
+    const int col0 = (int)(worker % segs) * 512 + 256 * half, head0 = col0 >> 7, col = col0 + 16 * t, head = col >> 7;
+    const bool active = col < n;
+    uint32_t signs = 0;                                       // bit k: the sign of this thread's far element k
     if (p.signs_out) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            const int c = col0 + th.column() + 8 * k;
+        for (int k = 0; k < 16; ++k) {
+            const int c = col0 + t + 16 * k;
             if (c < n) signs |= (uint32_t)(__ldg(reinterpret_cast<const unsigned short *>(p.signs_out) + c) >> 15) << k;
         }
     }
-    const int head0 = (col0 >> 7) + 2 * (th.lane >> 3);       // of k < 16; k >= 16 belong to the next head
-    const bool rot0 = head0 < p.hq + p.hkv, rot1 = head0 + 1 < p.hq + p.hkv;
+    const int rotated = p.hq + p.hkv - head0;                 // how many of the two heads, if positive
+    const int64_t step = workers / segs, last = p.rows * p.tokens;
     pdl_wait_prior_grids();
-    for (int64_t row = worker / segs; row < p.rows * p.tokens; row += workers / segs) {
+    uint32_t raw[8] = {};
+    int64_t row = worker / segs;
+    if (row < last && active) ld_half_row<WIDE>(p.qkv + row * p.ld + col, raw);
+    for (; row < last; row += step) {
         const int64_t seq = row / p.tokens, pos = row - seq * p.tokens;
-        __half *src = p.qkv + row * p.ld + col0;
-        float v[32];
+        float v[16];
+        unpack_pairs(raw, v);
+        float2 cs[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j);
-            unpack8_at(col0 + c < n ? __ldcg(reinterpret_cast<const uint4 *>(src + c)) : make_uint4(0u, 0u, 0u, 0u), v + 8 * j);
-        }
-        float2 cs[8];
-        const float2 *ang = p.angles + pos * 64 + (th.lane & 7);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) cs[k] = __ldg(ang + 8 * k);
-        piece_stages(v);
-        th.put_pieces(buf, v);
+        for (int k = 0; k < 4; ++k) cs[k] = __ldg(p.angles + pos * 64 + t + 16 * k);
+        if (row + step < last && active) ld_half_row<WIDE>(p.qkv + (row + step) * p.ld + col, raw);
+        stages16(v);
+        near.put(v);                                          // where this thread has read
         __syncwarp();
-        th.get_columns(buf, v);
-        column_stages(v, 7);
+        far.get(v);
+        far_stages16(v, 7);
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {                        // the layer's fp16 output
+        for (int k = 0; k < 16; ++k) {                        // the layer's fp16 output
             const float sc = ((signs >> k) & 1u) ? -p.scale : p.scale;
             v[k] = __half2float(__float2half_rn(v[k] * sc));
         }
 #pragma unroll
         for (int hd = 0; hd < 2; ++hd) {
-            if (!(hd ? rot1 : rot0)) continue;
+            if (hd >= rotated) continue;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float a = v[16 * hd + k], b = v[16 * hd + 8 + k];
-                v[16 * hd + k] = a * cs[k].x - b * cs[k].y;
-                v[16 * hd + 8 + k] = b * cs[k].x + a * cs[k].y;
+            for (int k = 0; k < 4; ++k) {
+                const float a = v[8 * hd + k], b = v[8 * hd + 4 + k];
+                v[8 * hd + k] = a * cs[k].x - b * cs[k].y;
+                v[8 * hd + 4 + k] = b * cs[k].x + a * cs[k].y;
             }
         }
-        th.put_columns(buf, v);
+        far.put(v);
         __syncwarp();
-        th.get_pieces(buf, v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = th.piece(j), head = (col0 + c) >> 7, i = c & 127;
-            if (col0 + c >= n) continue;
-            __half *dst = head < p.hq ? src + c
+        near.get(v);
+        if (active) {
+            const int i = col & 127;
+            __half *dst = head < p.hq ? p.qkv + row * p.ld + col
                           : head < p.hq + p.hkv ? p.kcache + ((seq * p.max_pos + pos) * p.hkv + head - p.hq) * 128 + i
                                                 : p.vcache + ((seq * p.max_pos + pos) * p.hkv + head - p.hq - p.hkv) * 128 + i;
-            *reinterpret_cast<uint4 *>(dst) = pack8_from(v + 8 * j);
+            uint32_t o[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o[q] = half2_as_u32(__floats2half2_rn(v[2 * q], v[2 * q + 1]));
+            if (WIDE) {
+                st_32_bytes(dst, o);
+            } else {
+                reinterpret_cast<uint4 *>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                reinterpret_cast<uint4 *>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            }
         }
-        __syncwarp();
     }
 }
 
@@ -588,7 +688,9 @@ extern "C" int rptc_prompt_qkv(void *qkv, int64_t ld, const void *signs_out, flo
     p.hkv = hkv;
     p.max_pos = max_pos;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return launch(qkv_rows_kernel, dim3(rows_grid(rows * tokens, ((int64_t)(hq + 2 * hkv) * 128 + 1023) / 1024, 8, 2)), dim3(256), 0, s, p);
+    const dim3 grid(rows_grid(rows * tokens, ((int64_t)(hq + 2 * hkv) * 128 + 511) / 512, 8, 3));
+    const bool wide = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 31) == 0 && ld % 16 == 0;
+    return wide ? launch(qkv_rows_kernel<true>, grid, dim3(256), 0, s, p) : launch(qkv_rows_kernel<false>, grid, dim3(256), 0, s, p);
 }
 
 extern "C" int rptc_rope_angles(void *angles, int64_t tokens, float theta, rptc_stream_t stream) {

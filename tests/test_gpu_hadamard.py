@@ -221,3 +221,32 @@ def test_prompt_qkv_matches_its_parts(rows, tokens, hq, hkv):
     ops.prompt_qkv(qkv, signs, 0.5, rows, tokens, *caches[1], hq, hkv, ops.rope_angles(tokens, 10000.0, "cuda:0"))
     for a, b in ((qkv[:, : hq * 128], want[:, : hq * 128]), (caches[1][0], caches[0][0]), (caches[1][1], caches[0][1])):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,n", [(111, 11008), (2100, 768), (301, 4096), (4800, 256)])
+def test_swiglu_of_many_rows_matches_few_rows(rows, n):
+    """The kernel that walks down the rows gives the bits of the one with a warp per block: whole and half segments, one row per warp and
+    several, zeros in the input."""
+    from rptc_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((rows, 2 * n), generator=g, device="cuda").half()
+    x[::7, : n // 2] = 0
+    so, si = [(torch.randint(0, 2, (k,), generator=g, device="cuda") * 2 - 1).half() for k in (2 * n, n)]
+    part = lambda r: ops.swiglu_hadamard_f16(x[r:r + 50], torch.empty((min(50, rows - r), n), dtype=torch.float16, device="cuda"), so, si, n, 256, 1.3, 0.6)
+    got = ops.swiglu_hadamard_f16(x, torch.empty((rows, n), dtype=torch.float16, device="cuda"), so, si, n, 256, 1.3, 0.6)
+    assert torch.equal(got, torch.cat([part(r) for r in range(0, rows, 50)]))
+
+
+def test_prompt_qkv_off_32_byte_boundaries():
+    from rptc_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    hq, hkv, tokens = 3, 2, 70
+    n = (hq + 2 * hkv) * 128
+    signs = (torch.randint(0, 2, (n,), generator=g, device="cuda") * 2 - 1).half()
+    x = torch.randn((tokens, n), generator=g, device="cuda").half()
+    off = torch.zeros(tokens * n + 8, dtype=torch.float16, device="cuda")[8:].view(tokens, n).copy_(x)
+    caches = [[torch.zeros((1, tokens, hkv, 128), dtype=torch.float16, device="cuda") for _ in range(2)] for _ in range(2)]
+    for qkv, kv in ((x, caches[0]), (off, caches[1])):
+        ops.prompt_qkv(qkv, signs, 0.5, 1, tokens, *kv, hq, hkv, ops.rope_angles(tokens, 10000.0, "cuda:0"))
+    assert off.data_ptr() % 32 == 16 and torch.equal(x, off)
+    assert all(torch.equal(a, b) for a, b in zip(*caches))
