@@ -227,7 +227,8 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
         }
         if (l->signs_out)
             return hadamard_and_clear(acc, 1, m, y, m, l->signs_out, nullptr, 0, rows, m, l->block_out, 1, l->scale, 0, nullptr, 0, s);
-        return rptc_gemv_finish(acc, m, y, m, m, (int)rows, l->scale, 0, 0, stream);
+        // without transforms, beyond 64 rows, the scale is left to the caller whichever product was taken
+        return rptc_gemv_finish(acc, m, y, m, m, (int)rows, rows > 64 ? 1.f : l->scale, 0, 0, stream);
     }
     if (int e = rptc_gemm(l->codes, l->lut, l->carry_in, xt, n, y, m, m, n, rows, &l->fmt, stream)) return e;
     if (l->signs_out) return hadamard_and_clear(y, 0, m, y, m, l->signs_out, nullptr, 0, rows, m, l->block_out, 1, l->scale, 0, nullptr, 0, s);
