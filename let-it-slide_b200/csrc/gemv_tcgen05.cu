@@ -61,6 +61,7 @@ struct FewParams {
 };
 
 // A segment: the steps [s0, s1) of one tile, and the part of them that one group takes.
+template <bool SHARED>
 struct FewSegment {
     int32_t tile, s0, s1;                            // tile: of weight rows
     int32_t t0;                                      // first token
@@ -71,7 +72,7 @@ struct FewSegment {
         s1 = min(p.n_steps, s0 + min((int32_t)(range_end - pos), p.max_steps));
         end = pos + (uint32_t)(s1 - s0);
         t0 = 0;
-        if (p.token_tiles > 1) {
+        if (SHARED && p.token_tiles > 1) {
             const int32_t rows = tile / p.token_tiles;
             t0 = (tile - rows * p.token_tiles) * p.n_cols;
             tile = rows;
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     const int bank = blockIdx.x / p.ctas;
     const uint32_t cta = blockIdx.x - bank * p.ctas;
     // this CTA's range of the bank's steps
-    const uint32_t total = (uint32_t)(p.tiles * p.token_tiles) * (uint32_t)p.n_steps;
+    const uint32_t total = (uint32_t)(SHARED ? p.tiles * p.token_tiles : p.tiles) * (uint32_t)p.n_steps;
     const uint32_t per = total / p.ctas, extra = total - per * p.ctas;
     const uint32_t c0 = cta * per + min(cta, extra), c1 = c0 + per + (cta < extra ? 1u : 0u);
 
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         int32_t s = 0;
         int64_t row = 0;
         while (f_left == 0 && f_next < c1) {                              // the next segment in which this part has steps
-            const FewSegment g(f_next, c1, p);
+            const FewSegment<SHARED> g(f_next, c1, p);
             f_next = g.end;
             s = g.part_begin<PARTS>(part);
             f_left = g.part_begin<PARTS>(part + 1) - s;
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         uint32_t a_phase = 1u, seg_phase = 0u;
         for (uint32_t pos = c0; pos < c1 && ok;) {
-            const FewSegment g(pos, c1, p);
+            const FewSegment<SHARED> g(pos, c1, p);
             pos = g.end;
             const int64_t row = (int64_t)g.tile * (RB * 128) + lane_row;
             const int32_t len = g.part_begin<PARTS>(part + 1) - g.part_begin<PARTS>(part);
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
             if (ok && row < p.m) {                   // of a whole warp: m is a multiple of 32
                 float *dst = p.acc + (int64_t)bank * p.m + row;
 #pragma unroll 1
-                const int tokens = min(p.tokens - g.t0, p.n_cols);
+                const int tokens = SHARED ? min(p.tokens - g.t0, p.n_cols) : p.tokens;
                 for (int t0 = 8 * part; t0 < tokens; t0 += 8 * PARTS) {
                     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         RingPos px = {0, 1u};
         const uint32_t bytes = 128u * (uint32_t)p.n_cols;
         for (uint32_t pos = c0; pos < c1 && ok;) {
-            const FewSegment g(pos, c1, p);
+            const FewSegment<SHARED> g(pos, c1, p);
             pos = g.end;
             const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
             for (int32_t j = 0; j < rounds && ok; ++j)
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         // the four MMAs of a step go round the accumulators
         const uint32_t d1 = p.n_sums == 2 ? (uint32_t)p.n_cols : 0u;
         for (uint32_t pos = c0; pos < c1 && ok; ++seg) {
-            const FewSegment g(pos, c1, p);
+            const FewSegment<SHARED> g(pos, c1, p);
             pos = g.end;
             if (seg > 0) ok = mbar_wait(drained, (seg - 1) & 1u, p.status);      // the last segment's sums have been taken
             tc_fence_after();
@@ -313,8 +314,8 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                     if (g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
                     if ((SHARED || q == mine) && ok) {
                         const int from = SHARED ? q * RB : 0;                // + grp: the group whose step it is
-                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), (a_phase >> q) & 1u, p.status);
-                        a_phase ^= 1u << q;
+                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), SHARED ? (a_phase >> q) & 1u : a_phase, p.status);
+                        a_phase ^= SHARED ? 1u << q : 1u;
                         if (ok) {
                             tc_fence_after();
                             const uint32_t a_tmem = a_first + 32u * (uint32_t)from;
