@@ -13,8 +13,10 @@
 // form four groups of four (a warp reaches the 32 tensor-memory lanes of its number modulo four): a group owns one of the
 // RB row blocks and one of 4 / RB equal parts of a segment's steps, so that it walks along its rows and keeps the 16 bits
 // of history.  A thread owns a row: its code bits arrive through a private ring of asynchronous copies, four steps ahead.
-// Warp 16 loads the activations, taking the parts' steps in turn: position j of part 0, 1, ...  Each group has
-// an MMA warp and an accumulator of its own: issuing a step (two waits, four MMAs, two commits) takes one thread about
+// Warp 16 loads the activations, taking the parts' steps in turn: position j of part 0, 1, ...  A part has a ring of stages of its
+// own: a stage's full barrier tells only whether its phase is odd or even, so whoever waits on it has to have seen every phase
+// before (one ring for all parts let a warp that skips the others' positions take a stage that still held an older one).  Each
+// group has an MMA warp and an accumulator of its own: issuing a step (two waits, four MMAs, two commits) takes one thread about
 // 600 clocks, as long as a group takes to decode it, so that one issuer for all four groups held the kernel to a
 // quarter of the speed.  A segment's sums are added to the caller's fp32 accumulator with atomics.
 // More activation rows (SHARED): a tile is RB x 128 weight rows (RB = 1, 2) x up to 256 (RB = 2: 192) tokens, and the groups that take parts
@@ -54,7 +56,7 @@ struct FewParams {
     int32_t token_tiles;                             // tiles of the same weight rows, n_cols tokens each
     int32_t L, S;
     uint32_t lut_addr, x_addr;
-    int32_t n_xstages;
+    int32_t n_xstages;                               // per ring: one for each part, SHARED one
     bool shared;                                     // more than kFewOwnTokens activation rows (host side: SHARED)
     int32_t n_sums, max_steps;                       // accumulators per group (1 or 2), longest segment
     unsigned int *status;
@@ -85,7 +87,7 @@ struct FewSegment {
 template <int CODE, int K, int RB, bool SHARED>
 __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int UPS = K / 2;                       // 128-bit units per step
-    constexpr int PARTS = 4 / RB;
+    constexpr int PARTS = 4 / RB, RINGS = SHARED ? 1 : PARTS;
     constexpr int NW = 4 * UPS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -272,7 +274,9 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     } else if (warp == kFewTmaWarp) {
         // ================= activations =================
         pdl_wait_prior_grids();
-        RingPos px = {0, 1u};
+        RingPos px[RINGS];
+#pragma unroll
+        for (int q = 0; q < RINGS; ++q) px[q] = {0, 1u};
         const uint32_t bytes = 128u * (uint32_t)p.n_cols;
         for (uint32_t pos = c0; pos < c1 && ok;) {
             const FewSegment<SHARED> g(pos, c1, p);
@@ -283,18 +287,19 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                 for (int q = 0; q < PARTS; ++q) {
                     const int32_t s = g.part_begin<PARTS>(q) + j;
                     if (s >= g.part_begin<PARTS>(q + 1) || !ok) continue;
-                    ok = mbar_wait(empty_x + 8 * px.s, px.phase, p.status);
+                    const int ring = SHARED ? 0 : q, stage = ring * p.n_xstages + px[ring].s;
+                    ok = mbar_wait(empty_x + 8 * stage, px[ring].phase, p.status);
                     if (ok && elect_one()) {
-                        mbar_expect_tx(full_x + 8 * px.s, bytes);
-                        tma_load_2d(p.x_addr + (uint32_t)px.s * bytes, &x_map, s * 64, g.t0, full_x + 8 * px.s);
+                        mbar_expect_tx(full_x + 8 * stage, bytes);
+                        tma_load_2d(p.x_addr + (uint32_t)stage * bytes, &x_map, s * 64, g.t0, full_x + 8 * stage);
                     }
                     __syncwarp();
-                    px.advance(p.n_xstages);
+                    px[ring].advance(p.n_xstages);
                 }
         }
     } else if (!SHARED || warp < kFewMmaWarp + RB) {
         // ================= MMA issue for one accumulator (a group's, or SHARED a row block's): the whole warp waits, one lane issues =================
-        const int grp = __shfl_sync(0xFFFFFFFFu, warp, 0) - kFewMmaWarp, mine = grp / RB;
+        const int grp = __shfl_sync(0xFFFFFFFFu, warp, 0) - kFewMmaWarp, mine = grp / RB, ring = SHARED ? 0 : mine * p.n_xstages;
         RingPos px = {0, 0u};
         uint32_t a_phase = 0u, seg = 0;              // a_phase: bit q for the group that takes part q
         const uint32_t bytes = 128u * (uint32_t)p.n_cols, idesc = instr_desc(p.n_cols);
@@ -311,15 +316,16 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
             for (int32_t j = 0; j < rounds && ok; ++j)
 #pragma unroll
                 for (int q = 0; q < PARTS; ++q) {
-                    if (g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
-                    if ((SHARED || q == mine) && ok) {
+                    if (!(SHARED || q == mine) || g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
+                    if (ok) {
                         const int from = SHARED ? q * RB : 0;                // + grp: the group whose step it is
-                        ok = mbar_wait(full_x + 8 * px.s, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), SHARED ? (a_phase >> q) & 1u : a_phase, p.status);
+                        const int stage = ring + px.s;
+                        ok = mbar_wait(full_x + 8 * stage, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), SHARED ? (a_phase >> q) & 1u : a_phase, p.status);
                         a_phase ^= SHARED ? 1u << q : 1u;
                         if (ok) {
                             tc_fence_after();
                             const uint32_t a_tmem = a_first + 32u * (uint32_t)from;
-                            const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)px.s * bytes);
+                            const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)stage * bytes);
                             if (elect_one()) {
                                 // + 32 bytes of shared memory, + 8 columns of tensor memory per K = 16
                                 tc_mma_f16_ta(d_tmem, a_tmem, xb, idesc, accumulate);
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                                 tc_mma_f16_ta(d_tmem, a_tmem + 16u, xb + 4u, idesc, 1u);
                                 tc_mma_f16_ta(d_tmem + d1, a_tmem + 24u, xb + 6u, idesc, 1u);
                                 tc_commit(empty_a + 8 * (grp + from));
-                                tc_commit(empty_x + 8 * px.s);
+                                tc_commit(empty_x + 8 * stage);
                             }
                             __syncwarp();
                             accumulate = 1u;
@@ -359,7 +365,7 @@ static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid,
     static SmemOptIn preferred;
     if (int e = allow_max_smem(kern, opted)) return e;
     if (int e = prefer_shared_memory(kern, preferred)) return e;
-    return launch(kern, dim3(grid), dim3(kFewThreads), p.x_addr + (uint32_t)p.n_xstages * 128u * (uint32_t)p.n_cols, stream, p, map);
+    return launch(kern, dim3(grid), dim3(kFewThreads), p.x_addr + (uint32_t)(p.n_xstages * (SHARED ? 1 : 4 / RB)) * 128u * (uint32_t)p.n_cols, stream, p, map);
 }
 
 template <int CODE, int K>
@@ -413,9 +419,10 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
         p.token_tiles = (int32_t)((tokens + cols - 1) / cols);
     }
     p.n_cols = (int32_t)(((tokens + p.token_tiles - 1) / p.token_tiles + 15) / 16 * 16);
-    p.n_xstages = (int32_t)((kFewTop - free) / (128u * (uint32_t)p.n_cols));
-    if (p.n_xstages > kFewMaxXStages) p.n_xstages = kFewMaxXStages;
-    return p.n_xstages >= 2;
+    int32_t stages = (int32_t)((kFewTop - free) / (128u * (uint32_t)p.n_cols));
+    if (stages > kFewMaxXStages) stages = kFewMaxXStages;
+    p.n_xstages = p.shared ? stages : stages / (4 / rb);      // four, two or one part: a ring each
+    return stages >= 2 && p.n_xstages >= 1;
 }
 static int64_t few_tiles(int64_t m, int rb) { return (m + rb * 128 - 1) / (rb * 128); }
 // The plan for `tokens` activation rows: row blocks per tile, or 0 where there is none.
@@ -430,7 +437,12 @@ static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tok
                  ? 1
                  : 2;
     }
-    return few_plan(p, f, tokens, rb) ? rb : 0;
+    // a table and tokens that leave no stage for each of the parts take tiles of more row blocks, which have fewer of them
+    for (; rb <= 4; rb *= 2) {
+        if (few_plan(p, f, tokens, rb)) return rb;
+        if (p.shared) break;
+    }
+    return 0;
 }
 
 // Up to kFewOwnTokens activation rows always (a step costs its decode), beyond that where it is estimated to finish before

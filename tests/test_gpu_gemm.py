@@ -172,3 +172,27 @@ def test_layer_of_some_hundred_tokens(code, K, L, S, m, n, tokens):
     err = (y.double() - x.double() @ dense.t()).abs()
     bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
     assert float((err / bound).max()) <= 1.0
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_A, 4, 16, 0), (o.CODE_A, 2, 16, 0), (o.CODE_B, 2, 16, 8)])
+@pytest.mark.parametrize("m,n,tokens", [(1280, 4160, 49), (1792, 1088, 64), (2304, 2240, 57), (1280, 4160, 96), (128, 40960, 50), (128, 41024, 96), (96, 38400, 17)])
+def test_layer_whose_tiles_have_several_parts(code, K, L, S, m, n, tokens):
+    """Few row blocks, so that two or four groups of warps take parts of the same rows' steps, segments that are not a multiple of
+    the parts, and tables that leave few stages of activations.  The layer twice on inputs that differ in every step: a step's
+    sums taken from another step's activations cannot come out right in both."""
+    from rptc_b200 import Format, ops
+    from rptc_b200.linear import RPTCLinear
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    fmt = Format(code, K, L, S, o.LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, K, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    layer = RPTCLinear(n, m, fmt, codes, lut, 0.25)
+    dense = ops.decompress(codes, lut, m, n, fmt).double()
+    for _ in range(2):
+        x = torch.randn((tokens, n), dtype=torch.float16, device="cuda", generator=g)
+        y = layer(x) * 4
+        torch.cuda.synchronize()
+        ops.device_status()
+        err = (y.double() - x.double() @ dense.t()).abs()
+        bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
+        assert float((err / bound).max()) <= 1.0
