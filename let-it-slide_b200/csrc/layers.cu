@@ -179,9 +179,9 @@ extern "C" int rptc_packed_forward(const rptc_packed *l, const void *x, int dtyp
 
 // ---- the incoherent layer ----
 // Whether the product goes through the fp32 accumulator: one or two rows, whatever the kernel for a few rows takes, and
-// up to 64 rows of a shape that the tiled product does not cover.
+// up to 64 rows of a reduction that is not whole steps of 64 columns.  The others take the tiled product, whose last tile may be partial.
 static bool linear_few(const rptc_linear &l, int64_t rows) {
-    return rows <= 2 || gemv_few_takes(l.m, l.n, rows, Banks(), l.fmt, nullptr, l.n) || (rows <= 64 && (l.m % 128 || l.n % 64));
+    return rows <= 2 || gemv_few_takes(l.m, l.n, rows, Banks(), l.fmt, nullptr, l.n) || (rows <= 64 && l.n % 64);
 }
 
 extern "C" int64_t rptc_linear_workspace_bytes(const rptc_linear *l, int64_t rows) {
@@ -198,7 +198,7 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     if (!l->signs_in != !l->signs_out) return RPTC_ERR_ARG;
     if (l->m <= 0 || l->n <= 0 || rows <= 0 || (l->m % 32) || (l->n % (128 / l->fmt.K)) || (l->m % 4)) return RPTC_ERR_SHAPE;
     const bool few = linear_few(*l, rows);
-    if (!few && ((l->m % 128) || (l->n % 64))) return RPTC_ERR_SHAPE;
+    if (!few && (l->n % 64)) return RPTC_ERR_SHAPE;
     if (l->m > (int64_t(1) << 30) || l->n > (int64_t(1) << 30) || rows > 65535 || (l->m / 32) * (l->n / (128 / l->fmt.K)) >= (int64_t(1) << 31))
         return RPTC_ERR_TOO_LARGE;
     const int64_t need = rptc_linear_workspace_bytes(l, rows);
@@ -230,7 +230,7 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
         // without transforms, beyond 64 rows, the scale is left to the caller whichever product was taken
         return rptc_gemv_finish(acc, m, y, m, m, (int)rows, rows > 64 ? 1.f : l->scale, 0, 0, stream);
     }
-    if (int e = rptc_gemm(l->codes, l->lut, l->carry_in, xt, n, y, m, m, n, rows, &l->fmt, stream)) return e;
+    if (int e = gemm_banked(l->codes, l->lut, l->carry_in, xt, n, y, m, m, n, rows, Banks(), l->fmt, s)) return e;
     if (l->signs_out) return hadamard_and_clear(y, 0, m, y, m, l->signs_out, nullptr, 0, rows, m, l->block_out, 1, l->scale, 0, nullptr, 0, s);
     return RPTC_OK;
 }

@@ -16,7 +16,8 @@ struct Banks {
 // Columns of y per bank: a bank's rows rounded up to whole tiles.
 int64_t gemm_bank_columns(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f);
 // y[t][bank * gemm_bank_columns + row] = fp16(sum_c x[t][c] W[bank][row][c]); columns beyond a bank's m rows hold no
-// result.  Shapes and alignments as rptc_gemm's, with m % 32 == 0 where banks > 1.
+// result.  Shapes and alignments as rptc_gemm's, with any m % 32 == 0; banks == 1: ld_y >= m,
+// nothing is stored behind column m.
 int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, void *y, int64_t ld_y, int64_t m,
                 int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
 // The estimate that gemm_banked's choice of tiles rests on, microseconds; 0 where it takes no such product.

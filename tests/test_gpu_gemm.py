@@ -196,3 +196,23 @@ def test_layer_whose_tiles_have_several_parts(code, K, L, S, m, n, tokens):
         err = (y.double() - x.double() @ dense.t()).abs()
         bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
         assert float((err / bound).max()) <= 1.0
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("m,n,tokens", [(288, 64, 700), (14368, 1024, 512), (32, 128, 3000), (1056, 192, 65)])
+def test_layer_of_many_rows_with_a_partial_last_tile(code, K, L, S, m, n, tokens):
+    """Any multiple of 32 weight rows and any number of activation rows, whichever product is estimated to be the faster one."""
+    from rptc_b200 import Format, ops
+    from rptc_b200.linear import RPTCLinear
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    fmt = Format(code, K, L, S, o.LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, K, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn((tokens, n), dtype=torch.float16, device="cuda", generator=g)
+    y = RPTCLinear(n, m, fmt, codes, lut, 0.5)(x) * 2
+    torch.cuda.synchronize()
+    ops.device_status()
+    dense = ops.decompress(codes, lut, m, n, fmt).double()
+    err = (y.double() - x.double() @ dense.t()).abs()
+    bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
+    assert float((err / bound).max()) <= 1.0
