@@ -827,9 +827,9 @@ static int gemv_one(const void *codes, const void *lut, const uint32_t *carry_in
 int check_format(const rptc_format *f);   // api.cu
 
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
-                const Banks &banks, const rptc_format &f, cudaStream_t stream) {
+                const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered, float *partial) {
     if (tokens > 2 && gemv_few_takes(m, n, tokens, banks, f, x, ld_x))
-        return gemv_few(codes, lut, nullptr, x, ld_x, acc, ld_acc, m, n, tokens, banks, f, stream);
+        return gemv_few(codes, lut, nullptr, x, ld_x, acc, ld_acc, m, n, tokens, banks, f, stream, ordered, partial);
     for (int64_t t = 0; t < tokens; t += 2) {
         const int e = gemv_one(codes, lut, nullptr, static_cast<const __half *>(x) + t * ld_x, ld_x, acc + t * ld_acc, ld_acc, m, n,
                                tokens - t >= 2 ? 2 : 1, RPTC_XORDER_NATURAL, f, stream, nullptr, banks);

@@ -22,6 +22,7 @@
 // More activation rows (SHARED): a tile is RB x 128 weight rows (RB = 1, 2) x up to 256 (RB = 2: 192) tokens, and the groups that take parts
 // of the same rows' steps share one accumulator, filled by one MMA warp.  A step of 256 x 192 takes the tensor core 768
 // clocks and its decode about 430 issue slots per scheduler, so that decoding again for the next 192 tokens is free.
+// ORDERED: segments' sums are put down side by side instead, and a second kernel adds them up in their order.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and returns.
 #include "common.cuh"
 #include "matmul.cuh"
@@ -47,7 +48,7 @@ struct FewParams {
     const uint4 *codes;
     const __half *lut;
     const uint32_t *carry_in;
-    float *acc;
+    float *acc;                                      // ORDERED: the partial sums
     int64_t ld_acc;
     int64_t m, lut_stride;                           // rows of a bank, fp16 elements from one bank's table to the next
     int32_t n_steps, n_units;                        // 64-column steps, 128-bit units per row
@@ -61,6 +62,9 @@ struct FewParams {
     int32_t n_sums, max_steps;                       // accumulators per group (1 or 2), longest segment
     unsigned int *status;
 };
+// The tensor map behind the parameters starts on a 64-byte boundary: with one byte more it would move up, and a launch with more
+// than 256 bytes of parameters starts later (22016 x 4096, 8 rows: the layer takes 24.5 instead of 24.0 us).
+static_assert(sizeof(FewParams) <= 128, "parameters of gemv_few_kernel");
 
 // A segment: the steps [s0, s1) of one tile, and the part of them that one group takes.
 template <bool SHARED>
@@ -84,7 +88,7 @@ struct FewSegment {
     __device__ __forceinline__ int32_t part_begin(int part) const { return s0 + (s1 - s0) * part / PARTS; }
 };
 
-template <int CODE, int K, int RB, bool SHARED>
+template <int CODE, int K, int RB, bool SHARED, bool ORDERED>
 __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int UPS = K / 2;                       // 128-bit units per step
     constexpr int PARTS = 4 / RB, RINGS = SHARED ? 1 : PARTS;
@@ -240,6 +244,18 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
             tc_fence_after();
             if (ok && row < p.m) {                   // of a whole warp: m is a multiple of 32
                 float *dst = p.acc + (int64_t)bank * p.m + row;
+                bool again = false;                  // ORDERED: the CTA's second segment of this tile, added to its first
+                if (ORDERED) {
+                    const uint32_t from = g.end - (uint32_t)(g.s1 - g.s0), tile_from = from - (uint32_t)g.s0;
+                    const uint32_t first = tile_from < extra * (per + 1) ? tile_from / (per + 1) : extra + (tile_from - extra * (per + 1)) / per;
+                    dst += (int64_t)(cta - first) * p.tokens * p.ld_acc;
+                    again = from > max(tile_from, c0);
+                }
+                auto put = [&](float *to, float v) {
+                    if (!ORDERED) atomicAdd(to, v);
+                    else if (again) __stcg(to, __ldcg(to) + v);
+                    else __stcg(to, v);
+                };
 #pragma unroll 1
                 const int tokens = SHARED ? min(p.tokens - g.t0, p.n_cols) : p.tokens;
                 for (int t0 = 8 * part; t0 < tokens; t0 += 8 * PARTS) {
@@ -258,11 +274,11 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                     float *to = dst + (int64_t)(g.t0 + t0) * p.ld_acc;
                     if (t0 + 8 <= tokens) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
+                        for (int e = 0; e < 8; ++e) put(to + (int64_t)e * p.ld_acc, sum[e]);
                     } else {
 #pragma unroll
                         for (int e = 0; e < 7; ++e)
-                            if (t0 + e < tokens) atomicAdd(to + (int64_t)e * p.ld_acc, sum[e]);
+                            if (t0 + e < tokens) put(to + (int64_t)e * p.ld_acc, sum[e]);
                     }
                 }
             }
@@ -358,24 +374,60 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     }
 }
 
-template <int CODE, int K, int RB, bool SHARED>
+template <int CODE, int K, int RB, bool SHARED, bool ORDERED>
 static int launch_few(const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t stream) {
     static SmemOptIn opted;
-    auto kern = gemv_few_kernel<CODE, K, RB, SHARED>;
+    auto kern = gemv_few_kernel<CODE, K, RB, SHARED, ORDERED>;
     static SmemOptIn preferred;
     if (int e = allow_max_smem(kern, opted)) return e;
     if (int e = prefer_shared_memory(kern, preferred)) return e;
     return launch(kern, dim3(grid), dim3(kFewThreads), p.x_addr + (uint32_t)(p.n_xstages * (SHARED ? 1 : 4 / RB)) * 128u * (uint32_t)p.n_cols, stream, p, map);
 }
 
-template <int CODE, int K>
+template <int CODE, int K, bool ORDERED>
 static int launch_few_rb(int rb, const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t s) {
-    if (p.shared) return rb == 1 ? launch_few<CODE, K, 1, true>(p, map, grid, s) : launch_few<CODE, K, 2, true>(p, map, grid, s);
+    if (p.shared) return rb == 1 ? launch_few<CODE, K, 1, true, ORDERED>(p, map, grid, s) : launch_few<CODE, K, 2, true, ORDERED>(p, map, grid, s);
     switch (rb) {
-        case 1: return launch_few<CODE, K, 1, false>(p, map, grid, s);
-        case 2: return launch_few<CODE, K, 2, false>(p, map, grid, s);
+        case 1: return launch_few<CODE, K, 1, false, ORDERED>(p, map, grid, s);
+        case 2: return launch_few<CODE, K, 2, false, ORDERED>(p, map, grid, s);
     }
-    return launch_few<CODE, K, 4, false>(p, map, grid, s);
+    return launch_few<CODE, K, 4, false, ORDERED>(p, map, grid, s);
+}
+template <int CODE, int K>
+static int launch_few_sums(int rb, const FewParams &p, const CUtensorMap &map, unsigned grid, cudaStream_t s, bool ordered) {
+    return ordered ? launch_few_rb<CODE, K, true>(rb, p, map, grid, s) : launch_few_rb<CODE, K, false>(rb, p, map, grid, s);
+}
+
+// acc[token][column] = the partial sums of the column's tile, first segment first.  One thread per four columns of a token (of one tile and
+// bank: m is a multiple of 32); where they lie is worked out under the product.  Bound: one or two trips to L2.
+struct SumParams {
+    const float *partial;                            // [CTA within the tile][token][ld]
+    float *acc;
+    int64_t plane, ld;
+    uint32_t per, extra, n_steps;                    // the CTAs' ranges of steps: `per`, the first `extra` one more; steps of a tile
+    int32_t columns, m, tile_rows, token_tiles, n_cols;
+    __device__ __forceinline__ uint32_t cta_of(uint32_t pos) const {
+        return pos < extra * (per + 1) ? pos / (per + 1) : extra + (pos - extra * (per + 1)) / per;
+    }
+};
+__global__ void __launch_bounds__(128) ordered_sum_kernel(const SumParams p) {
+    constexpr int kAhead = 8;
+    pdl_allow_next_grid();
+    const int col = 4 * (blockIdx.x * 128 + threadIdx.x), token = blockIdx.y;
+    const uint32_t from = (uint32_t)(col % p.m / p.tile_rows * p.token_tiles + token / p.n_cols) * p.n_steps;
+    const int slots = (int)(p.cta_of(from + p.n_steps - 1) - p.cta_of(from)) + 1;
+    const float *src = p.partial + (int64_t)token * p.ld + col;
+    pdl_wait_prior_grids();
+    if (col >= p.columns) return;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < slots; s += kAhead, src += kAhead * p.plane) {
+        float4 v[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) v[i] = s + i < slots ? __ldcg(reinterpret_cast<const float4 *>(src + i * p.plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) sum.x += v[i].x, sum.y += v[i].y, sum.z += v[i].z, sum.w += v[i].w;
+    }
+    *reinterpret_cast<float4 *>(p.acc + (int64_t)token * p.ld + col) = sum;
 }
 
 // Row blocks per tile up to kFewOwnTokens activation rows.  With four of them a step of activations is loaded, waited for and handed back once per 512 rows;
@@ -390,6 +442,13 @@ static int few_row_blocks(int64_t m) {
         if (rb == 4 || cost < best_cost) best = rb, best_cost = cost;
     }
     return best;
+}
+// The same for ordered sums: every CTA that has a part of a tile puts down sums for all of its rows, so narrow tiles leave fewer of
+// them to write and read.  Layers of 4096 x 4096, HASH, one, two and four row blocks: 16 rows 17.0, 19.7, 18.8 us, 64 rows 25.8, 31.3, 36.9;
+// 22016 x 4096: 31.4, 29.2, 27.7 and 44.0, 43.3, 50.6.  The table code, bound by its look-ups, takes one: 11008 x 4096 in 32 banks, 16 rows
+// 35.1, 40.0, 40.9.
+static int ordered_row_blocks(int64_t m, int64_t tokens, int code) {
+    return code == RPTC_CODE_LUT || m <= 32 * 128 || tokens > 48 ? 1 : 2;
 }
 // SHARED: microseconds of a 64-column step of a tile.  The decode (a 65,536-entry table: bank conflicts), the tensor core (four
 // clocks per token and pair of row blocks), or one thread's issue of the step.
@@ -426,8 +485,8 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
 }
 static int64_t few_tiles(int64_t m, int rb) { return (m + rb * 128 - 1) / (rb * 128); }
 // The plan for `tokens` activation rows: row blocks per tile, or 0 where there is none.
-static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tokens) {
-    int rb = few_row_blocks(m);
+static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tokens, bool ordered) {
+    int rb = ordered ? ordered_row_blocks(m, tokens, f.code) : few_row_blocks(m);
     if (tokens > kFewOwnTokens) {
         FewParams one, two;
         const bool has_one = few_plan(one, f, tokens, 1), has_two = few_plan(two, f, tokens, 2);
@@ -445,22 +504,54 @@ static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tok
     return 0;
 }
 
+// How the chosen plan's steps are cut into CTAs and segments.
+static int few_ranges(FewParams &p, int rb, int64_t m, int64_t n, const Banks &banks) {
+    p.n_steps = (int32_t)(n / 64);
+    p.tiles = (int32_t)few_tiles(m, rb);
+    const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
+    if (steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
+    // one bank's table per CTA: the SMs are dealt out to the banks
+    p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
+    if (p.ctas > steps) p.ctas = (int32_t)steps;
+    // The tensor core rounds its running sums towards zero, so the error of a sum grows with the number of MMAs behind it.
+    // Two accumulators per group keep it where the mma.sync kernel had it (22016 x 4096, 16 rows: relative error 0.7e-6
+    // against 1.3e-6 with one); where there is room for one only, a CTA's range goes into the result in two halves.
+    // SHARED: no chain is longer than those of the fused GEMM, whose place it takes.
+    p.n_sums = !p.shared && p.n_cols <= 48 ? 2 : 1;
+    const int64_t range = (steps + p.ctas - 1) / p.ctas;
+    p.max_steps = (int32_t)(p.n_sums == 2 || p.shared ? range : (range + 1) / 2);
+    return RPTC_OK;
+}
+
+int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
+    FewParams p;
+    const int rb = few_choose(p, f, m, tokens, true);
+    if (!rb || few_ranges(p, rb, m, n, banks)) return 0;
+    // CTAs that meet in a tile: its first step may be a range's last, unless whole ranges make up a tile; those behind are full ones
+    const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps, per = steps / p.ctas;
+    const bool whole = steps % p.ctas == 0 && p.n_steps % per == 0;
+    const int64_t slots = whole ? p.n_steps / per : 1 + (p.n_steps - 1 + per - 1) / per;
+    const bool two_each = p.max_steps < (steps + p.ctas - 1) / p.ctas;
+    return slots * (two_each ? 2 : 1) <= 2 ? 0 : slots * tokens * banks.banks * m;
+}
+
 // Up to kFewOwnTokens activation rows always (a step costs its decode), beyond that where it is estimated to finish before
 // the fused GEMM: a GEMM tile of 256 x 256 feeds the tensor core better and its result is fp16, but its decode goes through
-// shared memory and half of its SMs are idle for a few hundred tokens.  Here a CTA has its equal share of the steps, adds
-// its tiles' sums to memory (0.021 us per token and pair of row blocks), and the fp32 accumulator is zeroed in front and
-// read behind.  The time around the steps is fitted to whole layers of both codes.  Measured, whole layers, GEMM -> this: 4096 x 11008
-// HASH, 128 tokens 44.5 -> 29.2 us, 512 61.5 -> 56.1; 1024 x 14336, 256 tokens 53.8 -> 29.9; 4096 x 4096 in 32 banks, 112 tokens 36.9 ->
-// 20.6; on the other side of the line 14336 x 1024, 512 tokens 38.7 -> 51.7, 22016 x 4096, 2048 tokens 350 -> 406.
+// shared memory and half of its SMs are idle for a few hundred tokens.  Here a CTA has its equal share of the steps, takes
+// its tiles' sums to memory (0.021 us per token and pair of row blocks), where more than two of them for a tile cost about 2.5 us
+// (they are added up in order by a second kernel), and the fp32 result is read behind.  The time around the steps is fitted to
+// whole layers of both codes.  Measured, whole layers, GEMM against this: 4096 x 11008 HASH, 128 tokens 44.5 and 31.6 us, 512 57.1 and
+// 58.6; 22016 x 4096, 192 tokens 67.4 and 57.6; 1024 x 14336, 256 tokens 53.8 and 34; 4096 x 4096 in 32 banks, 112 tokens 36.9 and
+// 23; on the other side of the line 14336 x 1024, 512 tokens 38.7 and 51.7, 22016 x 4096, 2048 tokens 350 and 406.
 static bool few_is_faster(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     FewParams p;
-    const int rb = few_choose(p, f, m, tokens);
+    const int rb = few_choose(p, f, m, tokens, true);
     if (!rb || !p.shared) return rb != 0;
     const int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1, waves = (banks.banks * ctas + num_sms() - 1) / num_sms();
     const int64_t n_steps = n / 64, steps = (few_tiles(m, rb) * p.token_tiles * n_steps + ctas - 1) / ctas;
     const double drains = 1 + steps / n_steps;
     const double us = waves * ((f.code == RPTC_CODE_LUT ? 8.0 : 12.0) + steps * shared_step_us(rb, p.n_cols, f.code) + drains * 0.0105 * rb * p.n_cols) +
-                      (double)banks.banks * m * tokens * 8 / 4.5e6;
+                      (double)banks.banks * m * tokens * 8 / 4.5e6 + (gemv_few_partials(m, n, tokens, banks, f) ? 2.5 : 0.0);
     const double gemm = gemm_us(m, n, tokens, banks, f);
     return gemm == 0 || us < gemm;
 }
@@ -486,10 +577,11 @@ bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, co
 }
 
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
-             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s) {
+             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s, bool ordered, float *partial) {
     FewParams p;
-    const int rb = few_choose(p, f, m, tokens);
+    const int rb = few_choose(p, f, m, tokens, ordered);
     if (!rb) return RPTC_ERR_UNSUPPORTED;
+    if (int e = few_ranges(p, rb, m, n, banks)) return e;
     CUtensorMap map;
     if (int e = encode_map(map, x, n, tokens, ld_x, p.n_cols)) return e;
     p.codes = static_cast<const uint4 *>(codes);
@@ -499,33 +591,41 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
     p.ld_acc = ld_acc;
     p.m = m;
     p.lut_stride = banks.lut_stride;
-    p.n_steps = (int32_t)(n / 64);
     p.n_units = (int32_t)(n * f.K / 128);
     p.tokens = (int32_t)tokens;
-    p.tiles = (int32_t)few_tiles(m, rb);
-    const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
-    if (steps >= (int64_t(1) << 31)) return RPTC_ERR_TOO_LARGE;
-    // one bank's table per CTA: the SMs are dealt out to the banks
-    p.ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
-    if (p.ctas > steps) p.ctas = (int32_t)steps;
-    // The tensor core rounds its running sums towards zero, so the error of a sum grows with the number of MMAs behind it.
-    // Two accumulators per group keep it where the mma.sync kernel had it (22016 x 4096, 16 rows: relative error 0.7e-6
-    // against 1.3e-6 with one); where there is room for one only, a CTA's range goes into the result in two halves.
-    // SHARED: no chain is longer than those of the fused GEMM, whose place it takes.
-    p.n_sums = !p.shared && p.n_cols <= 48 ? 2 : 1;
-    const int64_t range = (steps + p.ctas - 1) / p.ctas;
-    p.max_steps = (int32_t)(p.n_sums == 2 || p.shared ? range : (range + 1) / 2);
+    if (partial) p.acc = partial;
     p.L = f.L;
     p.S = f.S;
     p.status = device_status_word();
     if (!p.status) return RPTC_ERR_CUDA;
     const unsigned grid = (unsigned)(banks.banks * p.ctas);
+    const bool apart = partial != nullptr;
+    int e = RPTC_ERR_UNSUPPORTED;
     switch (f.code) {
-        case RPTC_CODE_LUT: return f.K == 2 ? launch_few_rb<RPTC_CODE_LUT, 2>(rb, p, map, grid, s) : launch_few_rb<RPTC_CODE_LUT, 4>(rb, p, map, grid, s);
-        case RPTC_CODE_HASH: return launch_few_rb<RPTC_CODE_HASH, 2>(rb, p, map, grid, s);
-        case RPTC_CODE_LITE: return f.K == 2 ? launch_few_rb<RPTC_CODE_LITE, 2>(rb, p, map, grid, s) : launch_few_rb<RPTC_CODE_LITE, 4>(rb, p, map, grid, s);
+        case RPTC_CODE_LUT:
+            e = f.K == 2 ? launch_few_sums<RPTC_CODE_LUT, 2>(rb, p, map, grid, s, apart) : launch_few_sums<RPTC_CODE_LUT, 4>(rb, p, map, grid, s, apart);
+            break;
+        case RPTC_CODE_HASH: e = launch_few_sums<RPTC_CODE_HASH, 2>(rb, p, map, grid, s, apart); break;
+        case RPTC_CODE_LITE:
+            e = f.K == 2 ? launch_few_sums<RPTC_CODE_LITE, 2>(rb, p, map, grid, s, apart) : launch_few_sums<RPTC_CODE_LITE, 4>(rb, p, map, grid, s, apart);
+            break;
     }
-    return RPTC_ERR_UNSUPPORTED;
+    if (e || !apart) return e;
+    const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
+    SumParams q;
+    q.partial = partial;
+    q.acc = acc;
+    q.plane = tokens * ld_acc;
+    q.ld = ld_acc;
+    q.per = (uint32_t)(steps / p.ctas);
+    q.extra = (uint32_t)(steps % p.ctas);
+    q.n_steps = (uint32_t)p.n_steps;
+    q.columns = (int32_t)(banks.banks * m);
+    q.m = (int32_t)m;
+    q.tile_rows = rb * 128;
+    q.token_tiles = p.token_tiles;
+    q.n_cols = p.n_cols;
+    return launch(ordered_sum_kernel, dim3((unsigned)((q.columns + 511) / 512), (unsigned)tokens), dim3(128), 0, s, q);
 }
 
 }  // namespace rptc

@@ -26,11 +26,15 @@ double gemm_us(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const r
 // kFewOwnTokens whatever the shape).
 constexpr int64_t kFewOwnTokens = 96;
 bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, const void *x, int64_t ld_x);
+// Ordered sums: every sum is taken in the same order on every run, so that equal calls give equal bits.  `partial` is room for
+// gemv_few_partials fp32 values (16-byte aligned; ld_acc a multiple of 4), and acc = instead of +=.  Where that is 0 the sums meet in acc as
+// they do without (+=, from zeros): there are two of them at most, and a + b is b + a.
+int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f);
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
-             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream);
+             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr);
 // The same for any number of activation rows (TILED codes, no quirk, no carry): gemv_few where it takes them, else the
 // lane-per-row kernel for one or two rows at a time.
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
-                const Banks &banks, const rptc_format &f, cudaStream_t stream);
+                const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr);
 
 }  // namespace rptc

@@ -216,3 +216,21 @@ def test_layer_of_many_rows_with_a_partial_last_tile(code, K, L, S, m, n, tokens
     err = (y.double() - x.double() @ dense.t()).abs()
     bound = y.double().abs() * 2.0**-11 + 2e-5 * dense.norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None] + 1e-4
     assert float((err / bound).max()) <= 1.0
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0)])
+@pytest.mark.parametrize("m,n,tokens", [(4096, 11008, 512), (4096, 4096, 9), (1280, 4160, 96), (160, 11008, 112), (1056, 8256, 193), (128, 41024, 50), (8192, 4096, 40),
+                                        (1024, 14336, 256)])
+def test_layers_of_nine_rows_and_more_repeat_themselves(code, K, L, S, m, n, tokens):
+    """Several segments to a tile: their sums are added up in one order, so equal calls give equal bits, transforms or none."""
+    from rptc_b200 import Format, ops
+    from rptc_b200.linear import RPTCLinear
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    layer = RPTCLinear.random(n, m, Format(code, K, L, S, o.LAYOUT_TILED), 0.02, 1, incoherent=m % 256 == 0 and n % 256 == 0)
+    x = torch.randn((tokens, n), dtype=torch.float16, device="cuda", generator=g)
+    first = layer(x)
+    for _ in range(20):
+        assert torch.equal(layer(x), first)
+    ref = x.float() @ layer.effective_weight().t()
+    assert (first.float() - ref).abs().max() <= 1e-2 * ref.abs().max()
+    ops.device_status()

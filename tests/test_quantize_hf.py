@@ -181,3 +181,20 @@ def test_packed_layer_forward_over_its_products(m, n, banks, L, tokens, dtype):
     got = layer(x)
     assert got.dtype == dtype
     assert (got.double() - want).norm() <= (4e-3 if dtype == torch.bfloat16 else 6e-4) * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,banks,L,tokens", [(4096, 1088, 8, 16, 40), (1376, 4096, 4, 14, 97), (11008, 1024, 32, 16, 12), (1024, 11008, 8, 16, 256)])
+def test_packed_layers_of_nine_tokens_and_more_repeat_themselves(m, n, banks, L, tokens):
+    import quantize_hf as q
+    g = torch.Generator(device="cuda").manual_seed(m + tokens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    symbols = torch.randint(0, 4, (m, n), generator=g, device="cuda", dtype=torch.int32)
+    layer = q.FactorizedRPTCLinear.from_parts(symbols, rnd(banks, 1 << L), 0.1 * rnd(m), 0.1 * rnd(n), 0.5 + rnd(m).abs(), 0.5 + rnd(n).abs())
+    x = rnd(tokens, n)
+    first = layer(x)
+    for _ in range(20):
+        assert torch.equal(layer(x), first)
+    want = ((x * layer.scales_in).half().double() @ layer.decoded().double().t()) * layer.scales_out.double() \
+        + x.double().sum(1, keepdim=True) * layer.biases_out.double() + (x.double() @ layer.biases_in.double())[:, None]
+    assert (first.double() - want).norm() <= 6e-4 * want.norm()
