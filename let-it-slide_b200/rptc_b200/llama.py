@@ -544,16 +544,23 @@ class RPTCLlama:
             finally:
                 lib().rptc_set_pdl(0)
         else:
+
+            def apply(lin, x):
+                # like the fused path a row's results do not depend on the number of rows that go with it
+                if R * T > 8 and lin.out_features % 128 == 0:
+                    return lin.finish_t(lin.product_t(lin.transform_in(x)))
+                return lin(x)
+
             xn = torch.empty_like(h)
             for i, b in enumerate(self.blocks):
                 ops.rmsnorm(h, b.norm1, xn, cfg.rms_eps)
-                qkv = b.qkv(xn)
+                qkv = apply(b.qkv, xn)
                 ops.rope_cache_prompt(qkv, R, T, self.kcache[i], self.vcache[i], self.heads_l, self.kv_heads_l, D, cfg.rope_theta)
-                h = h + reduce(b.o(self._prompt_attention(qkv, i, R, T)))
+                h = h + reduce(apply(b.o, self._prompt_attention(qkv, i, R, T)))
                 ops.rmsnorm(h, b.norm2, xn, cfg.rms_eps)
-                gu = b.gate_up(xn)
+                gu = apply(b.gate_up, xn)
                 mlp = torch.nn.functional.silu(gu[:, : self.ffn_l]).mul_(gu[:, self.ffn_l:])      # fp32 inside, fp16 in and out
-                h = h + reduce(b.down(mlp))
+                h = h + reduce(apply(b.down, mlp))
             last = h.reshape(R, T, cfg.hidden)[:, -1].contiguous()
         ops.rmsnorm(last, self.norm_f, self.xn, cfg.rms_eps)
         ops.dense_gemv(self.head, self.xn, out=self.logits)

@@ -412,3 +412,18 @@ def test_attention_of_many_rows_matches_single_rows(rows, heads, kv_heads):
     for a, b in zip(attend(slice(0, rows)), want):
         assert (a.float() - b.float()).abs().max() <= 2e-3 * b.float().abs().max()
     ops.device_status()
+
+
+def test_prefill_without_transforms_gives_a_position_the_same_bits_in_any_company():
+    """The path of tensor-parallel and transform-free models: what the first layer puts into the caches for a position does not depend on
+    how long the prompt is, and a prompt repeats itself."""
+    from rptc_b200.llama import LlamaConfig, RPTCLlama
+    cfg = LlamaConfig(hidden=1024, layers=2, heads=8, kv_heads=4, ffn=2816, vocab=256, max_pos=400)
+    model = RPTCLlama(cfg, rows=1, seed=3, incoherent=False)
+    tokens = torch.randint(0, 256, (1, 400), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    logits = model.prefill(tokens).clone()
+    k, v = model.kcache[0].clone(), model.vcache[0].clone()
+    assert torch.equal(model.prefill(tokens), logits)
+    for T in (9, 40, 130, 300):
+        model.prefill(tokens[:, :T])
+        assert torch.equal(model.kcache[0][:, :T], k[:, :T]) and torch.equal(model.vcache[0][:, :T], v[:, :T]), T
