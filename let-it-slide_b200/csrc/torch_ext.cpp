@@ -11,6 +11,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <exception>
+#include <optional>
+#include <string>
 
 #include "../../include/rptc_b200.h"
 
@@ -58,16 +60,26 @@ public:
         if (v == -1.0 && PyErr_Occurred()) throw PyError();
         return v;
     }
-    // a buffer's tensor, or null for None
-    const at::Tensor *buffer(PyObject *name) const {
+    // A buffer as a kernel reads it: `count` values of `type`, contiguous, and (device_with) on one GPU with the others; null for
+    // None where the layer may do without.  (`.half()` and the like change buffers of a module, `.to()` may have been missed.)
+    const void *pointer(PyObject *name, at::ScalarType type, int64_t count, bool optional = false) {
         PyObject *o = get(buffers_, name);
-        if (o == Py_None) return nullptr;
-        if (!THPVariable_Check(o)) fail("a buffer of the layer is not a tensor");
-        return &THPVariable_Unpack(o);
+        if (o == Py_None && optional) return nullptr;
+        if (!THPVariable_Check(o)) refuse(name, "must be a tensor");
+        const at::Tensor &t = THPVariable_Unpack(o);
+        if (t.scalar_type() != type) refuse(name, (std::string("must have dtype ") + c10::toString(type) + ", got " + c10::toString(t.scalar_type())).c_str());
+        if (t.numel() != count) refuse(name, ("must have " + std::to_string(count) + " elements, got " + std::to_string(t.numel())).c_str());
+        if (!t.is_contiguous()) refuse(name, "must be contiguous");
+        if (!device_) device_ = t.device();
+        if (!elsewhere_ && (!t.is_cuda() || *device_ != t.device())) elsewhere_ = name;
+        return t.data_ptr();
     }
-    const void *pointer(PyObject *name) const {
-        const at::Tensor *t = buffer(name);
-        return t ? t->data_ptr() : nullptr;
+    // The device of all buffers asked for; x has to be there too.
+    c10::Device device_with(const at::Tensor &x) const {
+        if (elsewhere_) refuse(elsewhere_, "must be a CUDA tensor on the GPU of the layer's other buffers");
+        if (!x.is_cuda()) fail("x must be a CUDA tensor");
+        if (x.device() != *device_) fail("x is on another GPU than the layer");
+        return *device_;
     }
 
 private:
@@ -79,7 +91,12 @@ private:
         }
         return o;
     }
-    PyObject *dict_, *buffers_ = nullptr;
+    [[noreturn]] static void refuse(PyObject *name, const char *what) {
+        const char *n = PyUnicode_AsUTF8(name);
+        fail((std::string(n ? n : "a buffer") + " " + what).c_str());
+    }
+    PyObject *dict_, *buffers_ = nullptr, *elsewhere_ = nullptr;
+    std::optional<c10::Device> device_;
 };
 
 const at::Tensor &unpack(PyObject *o, const char *what) {
@@ -130,31 +147,29 @@ cudaStream_t current_stream(const at::Tensor &t) { return c10::cuda::getCurrentC
 PyObject *linear_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
         if (nargs != 2) fail("linear_forward(module, x)");
-        const Attributes a(args[0]);
+        Attributes a(args[0]);
         const at::Tensor &x_in = unpack(args[1], "x must be a tensor");
         rptc_linear l;
         l.m = a.integer(g_names.out_features);
         l.n = a.integer(g_names.in_features);
-        if (!x_in.is_cuda()) fail("x must be a CUDA tensor");
+        l.fmt = format_of(a.object(g_names.fmt));
         if (x_in.dim() < 1 || x_in.size(-1) != l.n || x_in.numel() == 0) fail("x must have in_features columns and at least one row");
-        const at::Tensor *codes = a.buffer(g_names.codes);
-        if (!codes) fail("the layer has no codes");
-        l.codes = codes->data_ptr();
-        l.lut = a.pointer(g_names.lut);
-        l.carry_in = static_cast<const uint32_t *>(a.pointer(g_names.carry_in));
-        l.signs_in = a.pointer(g_names.signs_in);
-        l.signs_out = a.pointer(g_names.signs_out);
+        if (l.fmt.L < 1 || l.fmt.L > 16 || l.fmt.S < 0 || l.fmt.S > 16) fail("fmt has no such code");
+        l.codes = a.pointer(g_names.codes, at::kInt, l.m * l.n * l.fmt.K / 32);
+        l.lut = a.pointer(g_names.lut, at::kHalf, l.fmt.code == RPTC_CODE_LUT ? int64_t(1) << l.fmt.L : int64_t(2) << l.fmt.S);
+        l.carry_in = static_cast<const uint32_t *>(a.pointer(g_names.carry_in, at::kInt, l.m, true));
+        l.signs_in = a.pointer(g_names.signs_in, at::kHalf, l.n, true);
+        l.signs_out = a.pointer(g_names.signs_out, at::kHalf, l.m, true);
         l.block_in = (int32_t)a.integer(g_names.block_in);
         l.block_out = (int32_t)a.integer(g_names.block_out);
         l.scale = (float)a.number(g_names.scale);
-        l.fmt = format_of(a.object(g_names.fmt));
-        const c10::cuda::OptionalCUDAGuard guard(codes->device());
+        const c10::cuda::OptionalCUDAGuard guard(a.device_with(x_in));
         const at::Tensor x = ready(x_in.scalar_type() == at::kHalf ? x_in : x_in.to(at::kHalf));
         const int64_t rows = x.numel() / l.n;
         at::Tensor y = result_like(x, l.m);
         const int64_t need = g_lib.linear_workspace_bytes(&l, rows);
         at::Tensor ws = at::empty({need > 0 ? need : 1}, x.options().dtype(at::kByte));
-        const int status = g_lib.linear_forward(&l, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need, current_stream(*codes));
+        const int status = g_lib.linear_forward(&l, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need, current_stream(x));
         if (status != RPTC_OK) return PyLong_FromLong(status);
         // beyond 64 rows the product of a layer without transforms leaves the scale to be applied
         if (!l.signs_in && rows > 64 && l.scale != 1.f) y = y * a.number(g_names.scale);
@@ -166,30 +181,30 @@ PyObject *linear_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 PyObject *packed_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
         if (nargs != 2) fail("packed_forward(module, x)");
-        const Attributes a(args[0]);
+        Attributes a(args[0]);
         const at::Tensor &x_in = unpack(args[1], "x must be a tensor");
         rptc_packed l;
         l.m = a.integer(g_names.out_features);
         l.n = a.integer(g_names.in_features);
-        if (!x_in.is_cuda()) fail("x must be a CUDA tensor");
+        l.banks = (int32_t)a.integer(g_names.num_banks);
+        l.bank_blocks = (int32_t)a.integer(g_names.bank_blocks);
+        l.L = (int32_t)a.integer(g_names.L);
         if (x_in.dim() < 1 || x_in.size(-1) != l.n) fail("x must have in_features columns");
+        if (l.L < 1 || l.L > 16) fail("L must be 1 to 16");
+        l.codes = a.pointer(g_names.codes, at::kInt, (int64_t)l.banks * l.bank_blocks * 32 * l.n / 16);
+        l.alphabets = a.pointer(g_names.alphabets, at::kHalf, (int64_t)l.banks << l.L);
+        l.biases_out = static_cast<const float *>(a.pointer(g_names.biases_out, at::kFloat, l.m));
+        l.biases_in = static_cast<const float *>(a.pointer(g_names.biases_in, at::kFloat, l.n));
+        l.scales_out = static_cast<const float *>(a.pointer(g_names.scales_out, at::kFloat, l.m));
+        l.scales_in = static_cast<const float *>(a.pointer(g_names.scales_in, at::kFloat, l.n));
+        l.bias = static_cast<const float *>(a.pointer(g_names.bias, at::kFloat, l.m, true));
         const at::ScalarType type = x_in.scalar_type();
         const int dtype = type == at::kHalf ? 0 : type == at::kBFloat16 ? 1 : 2;
-        const c10::cuda::OptionalCUDAGuard guard(x_in.device());
+        const c10::cuda::OptionalCUDAGuard guard(a.device_with(x_in));
         const at::Tensor x = ready(dtype == 2 && type != at::kFloat ? x_in.to(at::kFloat) : x_in);
         at::Tensor y = result_like(x, l.m);
         const int64_t tokens = x.numel() / l.n;
         if (tokens > 0) {
-            l.codes = a.pointer(g_names.codes);
-            l.alphabets = a.pointer(g_names.alphabets);
-            l.biases_out = static_cast<const float *>(a.pointer(g_names.biases_out));
-            l.biases_in = static_cast<const float *>(a.pointer(g_names.biases_in));
-            l.scales_out = static_cast<const float *>(a.pointer(g_names.scales_out));
-            l.scales_in = static_cast<const float *>(a.pointer(g_names.scales_in));
-            l.bias = static_cast<const float *>(a.pointer(g_names.bias));
-            l.banks = (int32_t)a.integer(g_names.num_banks);
-            l.bank_blocks = (int32_t)a.integer(g_names.bank_blocks);
-            l.L = (int32_t)a.integer(g_names.L);
             const int64_t most = tokens < 65535 ? tokens : 65535;      // tokens per native call
             const int64_t need = g_lib.packed_workspace_bytes(&l, most);
             if (need < 0) return PyLong_FromLong(RPTC_ERR_SHAPE);

@@ -1,0 +1,75 @@
+"""What the layers' native calls refuse: buffers of another type, size or place than the kernels read.  The checks come before anything
+is launched, so that everything here but the tests of devices runs without a GPU."""
+import pytest
+import torch
+
+
+def _packed(device="cpu", bias=True):
+    import quantize_hf as q
+    return q.FactorizedRPTCLinear(64, 128, 8, 2, bias, device=device)
+
+
+def _linear(device="cpu"):
+    from rptc_b200 import Format
+    from rptc_b200.linear import RPTCLinear
+    return RPTCLinear.random(256, 256, Format(), 0.02, 1, device=device)
+
+
+PACKED = ["codes", "alphabets", "biases_out", "biases_in", "scales_out", "scales_in", "bias"]
+LINEAR = ["codes", "lut", "signs_in", "signs_out"]
+MAKE = {"packed": (_packed, 128, PACKED), "linear": (_linear, 256, LINEAR)}
+
+
+@pytest.mark.parametrize("kind,cast,name", [("packed", torch.float16, "biases_out"), ("packed", torch.bfloat16, "alphabets"), ("packed", torch.float64, "alphabets"),
+                                            ("linear", torch.float32, "lut"), ("linear", torch.bfloat16, "lut")])
+def test_a_layer_that_was_cast_is_refused(kind, cast, name):
+    make, n, _ = MAKE[kind]
+    layer = make().to(cast)
+    with pytest.raises(RuntimeError, match=f"{name} must have dtype"):
+        layer(torch.zeros(1, n, dtype=torch.float16))
+
+
+@pytest.mark.parametrize("kind,name", [(k, n) for k in MAKE for n in MAKE[k][2]])
+def test_a_buffer_of_another_type_size_or_stride_is_refused(kind, name):
+    make, n, _ = MAKE[kind]
+    x = torch.zeros(3, n, dtype=torch.float16)
+    good = make()
+    t = getattr(good, name)
+    for bad, what in ((t.to(torch.int16), "must have dtype"), (t.reshape(-1)[:-8].clone(), "elements, got"), (t.reshape(-1).repeat_interleave(2)[::2], "must be contiguous")):
+        layer = make()
+        layer._buffers[name] = bad
+        with pytest.raises(RuntimeError, match=f"{name} .*{what}"):
+            layer(x)
+
+
+@pytest.mark.parametrize("kind", list(MAKE))
+def test_a_layer_on_the_cpu_is_refused(kind):
+    make, n, _ = MAKE[kind]
+    with pytest.raises(RuntimeError, match="codes must be a CUDA tensor"):
+        make()(torch.zeros(1, n, dtype=torch.float16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,name", [(k, n) for k in MAKE for n in MAKE[k][2]])
+def test_a_buffer_that_does_not_fit_is_refused_on_the_gpu(kind, name):
+    make, n, _ = MAKE[kind]
+    x = torch.zeros(3, n, dtype=torch.float16, device="cuda")
+    layer = make("cuda")
+    t = getattr(layer, name)
+    for bad, what in ((t.to(torch.int16), "must have dtype"), (t.reshape(-1)[:-8].clone(), "elements, got"), (t.reshape(-1).repeat_interleave(2)[::2], "must be contiguous"),
+                      (t.cpu(), "must be a CUDA tensor")):
+        layer._buffers[name] = bad
+        with pytest.raises(RuntimeError, match=f"{name} .*{what}"):
+            layer(x)
+    layer._buffers[name] = t
+    assert torch.isfinite(layer(x)).all()
+    with pytest.raises(RuntimeError, match="x must be a CUDA tensor"):
+        layer(x.cpu())
+
+
+@pytest.mark.gpu
+def test_a_cast_packed_layer_is_refused_on_the_gpu():
+    x = torch.zeros(1, 128, dtype=torch.float16, device="cuda")
+    for cast in (torch.float16, torch.bfloat16):
+        with pytest.raises(RuntimeError, match="must have dtype"):
+            _packed("cuda").to(cast)(x)
