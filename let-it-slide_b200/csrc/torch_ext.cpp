@@ -8,6 +8,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <exception>
@@ -133,10 +134,8 @@ PyObject *guarded(F &&f) {
     try {
         return f();
     } catch (const PyError &) {
-    } catch (const c10::Error &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {      // torch's own classes: out of memory is torch.OutOfMemoryError here too
+        torch::translate_exception_to_python(std::current_exception());
     }
     return nullptr;
 }

@@ -73,3 +73,21 @@ def test_a_cast_packed_layer_is_refused_on_the_gpu():
     for cast in (torch.float16, torch.bfloat16):
         with pytest.raises(RuntimeError, match="must have dtype"):
             _packed("cuda").to(cast)(x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", list(MAKE))
+def test_out_of_memory_is_torchs_own_exception(kind):
+    import quantize_hf as q
+    from rptc_b200 import Format
+    from rptc_b200.linear import RPTCLinear
+    layer = q.FactorizedRPTCLinear(8192, 256, 8, 2, device="cuda") if kind == "packed" else RPTCLinear.random(256, 8192, Format(), 0.02, 1)
+    x = torch.zeros(60000, 256, dtype=torch.float16, device="cuda")               # a result of 1 GB
+    torch.cuda.empty_cache()
+    limit = (torch.cuda.memory_reserved() + (64 << 20)) / torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction(limit)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            layer(x)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
