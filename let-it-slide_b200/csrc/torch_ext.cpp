@@ -14,6 +14,7 @@
 #include <exception>
 #include <optional>
 #include <string>
+#include <vector>
 
 #include "../../include/rptc_b200.h"
 
@@ -41,22 +42,26 @@ struct PyError : std::exception {};      // the interpreter's error is set
     throw PyError();
 }
 
-// A module's instance attributes and buffers, without the module's __getattr__.
+// A module's instance attributes and buffers, where they usually lie without the module's __getattr__; what lies elsewhere (a buffer
+// that was replaced by a parameter, a property of a subclass) is asked of the module.
 class Attributes {
 public:
-    explicit Attributes(PyObject *module) : dict_(PyObject_GenericGetDict(module, nullptr)) {
+    explicit Attributes(PyObject *module) : module_(module), dict_(PyObject_GenericGetDict(module, nullptr)) {
         if (!dict_) throw PyError();
         buffers_ = get(dict_, g_names._buffers);
     }
     Attributes(const Attributes &) = delete;
-    ~Attributes() { Py_XDECREF(dict_); }
-    PyObject *object(PyObject *name) const { return get(dict_, name); }
-    int64_t integer(PyObject *name) const {
+    ~Attributes() {
+        for (PyObject *o : owned_) Py_DECREF(o);
+        Py_XDECREF(dict_);
+    }
+    PyObject *object(PyObject *name) { return get(dict_, name); }
+    int64_t integer(PyObject *name) {
         const long long v = PyLong_AsLongLong(get(dict_, name));
         if (v == -1 && PyErr_Occurred()) throw PyError();
         return v;
     }
-    double number(PyObject *name) const {
+    double number(PyObject *name) {
         const double v = PyFloat_AsDouble(get(dict_, name));
         if (v == -1.0 && PyErr_Occurred()) throw PyError();
         return v;
@@ -84,19 +89,20 @@ public:
     }
 
 private:
-    static PyObject *get(PyObject *dict, PyObject *name) {
+    PyObject *get(PyObject *dict, PyObject *name) {
         PyObject *o = PyDict_GetItemWithError(dict, name);
-        if (!o) {
-            if (!PyErr_Occurred()) PyErr_SetObject(PyExc_AttributeError, name);
-            throw PyError();
-        }
+        if (o) return o;
+        if (!PyErr_Occurred()) o = PyObject_GetAttr(module_, name);
+        if (!o) throw PyError();
+        owned_.push_back(o);
         return o;
     }
     [[noreturn]] static void refuse(PyObject *name, const char *what) {
         const char *n = PyUnicode_AsUTF8(name);
         fail((std::string(n ? n : "a buffer") + " " + what).c_str());
     }
-    PyObject *dict_, *buffers_ = nullptr, *elsewhere_ = nullptr;
+    PyObject *module_, *dict_, *buffers_ = nullptr, *elsewhere_ = nullptr;
+    std::vector<PyObject *> owned_;
     std::optional<c10::Device> device_;
 };
 

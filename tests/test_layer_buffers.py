@@ -67,6 +67,27 @@ def test_a_buffer_that_does_not_fit_is_refused_on_the_gpu(kind, name):
         layer(x.cpu())
 
 
+@pytest.mark.parametrize("kind", list(MAKE))
+def test_an_attribute_that_is_missing_is_an_attribute_error(kind):
+    make, n, names = MAKE[kind]
+    layer = make()
+    delattr(layer, names[1])
+    with pytest.raises(AttributeError, match=names[1]):
+        layer(torch.zeros(1, n, dtype=torch.float16))
+
+
+@pytest.mark.gpu
+def test_buffers_replaced_by_parameters_are_found():
+    """Assigning an nn.Parameter to the name of a buffer moves it among the module's parameters (a bias that is to be trained)."""
+    layer, x = _packed("cuda"), torch.ones(3, 128, device="cuda")
+    layer.bias.copy_(torch.arange(64.0))
+    want = layer(x)
+    layer.bias = torch.nn.Parameter(layer.bias.clone())
+    layer.scales_out = torch.nn.Parameter(layer.scales_out.clone())
+    assert "bias" not in layer._buffers
+    assert torch.equal(layer(x), want)
+
+
 @pytest.mark.gpu
 def test_a_cast_packed_layer_is_refused_on_the_gpu():
     x = torch.zeros(1, 128, dtype=torch.float16, device="cuda")
