@@ -76,6 +76,8 @@ public:
         if (t.scalar_type() != type) refuse(name, (std::string("must have dtype ") + c10::toString(type) + ", got " + c10::toString(t.scalar_type())).c_str());
         if (t.numel() != count) refuse(name, ("must have " + std::to_string(count) + " elements, got " + std::to_string(t.numel())).c_str());
         if (!t.is_contiguous()) refuse(name, "must be contiguous");
+        if (held_n_ == sizeof(held_) / sizeof(held_[0])) fail("too many buffers");
+        held_[held_n_++] = t;
         if (!device_) device_ = t.device();
         if (!elsewhere_ && (!t.is_cuda() || *device_ != t.device())) elsewhere_ = name;
         return t.data_ptr();
@@ -103,6 +105,8 @@ private:
     }
     PyObject *module_, *dict_, *buffers_ = nullptr, *elsewhere_ = nullptr;
     std::vector<PyObject *> owned_;
+    at::Tensor held_[7];      // a launch lets other threads run, and they may give the module new buffers
+    size_t held_n_ = 0;
     std::optional<c10::Device> device_;
 };
 
@@ -174,7 +178,11 @@ PyObject *linear_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         at::Tensor y = result_like(x, l.m);
         const int64_t need = g_lib.linear_workspace_bytes(&l, rows);
         at::Tensor ws = at::empty({need > 0 ? need : 1}, x.options().dtype(at::kByte));
-        const int status = g_lib.linear_forward(&l, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need, current_stream(x));
+        const cudaStream_t s = current_stream(x);
+        int status;
+        Py_BEGIN_ALLOW_THREADS                                        // a launch waits where the stream's queue is full
+        status = g_lib.linear_forward(&l, x.data_ptr(), y.data_ptr(), rows, ws.data_ptr(), need, s);
+        Py_END_ALLOW_THREADS
         if (status != RPTC_OK) return PyLong_FromLong(status);
         // beyond 64 rows the product of a layer without transforms leaves the scale to be applied
         if (!l.signs_in && rows > 64 && l.scale != 1.f) y = y * a.number(g_names.scale);
@@ -217,11 +225,13 @@ PyObject *packed_forward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
             const char *xp = static_cast<const char *>(x.data_ptr());
             char *yp = static_cast<char *>(y.data_ptr());
             const int64_t width = x.element_size();
-            for (int64_t t = 0; t < tokens; t += most) {
-                const int status = g_lib.packed_forward(&l, xp + t * l.n * width, dtype, yp + t * l.m * width, most < tokens - t ? most : tokens - t,
-                                                        ws.data_ptr(), need, current_stream(x));
-                if (status != RPTC_OK) return PyLong_FromLong(status);
-            }
+            const cudaStream_t s = current_stream(x);
+            int status = RPTC_OK;
+            Py_BEGIN_ALLOW_THREADS
+            for (int64_t t = 0; t < tokens && status == RPTC_OK; t += most)
+                status = g_lib.packed_forward(&l, xp + t * l.n * width, dtype, yp + t * l.m * width, most < tokens - t ? most : tokens - t, ws.data_ptr(), need, s);
+            Py_END_ALLOW_THREADS
+            if (status != RPTC_OK) return PyLong_FromLong(status);
         }
         if (y.scalar_type() != type) y = y.to(type);
         return THPVariable_Wrap(std::move(y));

@@ -112,3 +112,37 @@ def test_out_of_memory_is_torchs_own_exception(kind):
             layer(x)
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", list(MAKE))
+def test_other_threads_run_while_a_layer_waits_for_room_in_the_stream(kind):
+    """A stream holds about a thousand launches; a call that finds it full waits, and the interpreter does not wait with it."""
+    import threading
+    import time
+    make, n, _ = MAKE[kind]
+    layer, x = make("cuda"), torch.zeros(1, n, dtype=torch.float16, device="cuda")
+    layer(x)
+    torch.cuda.synchronize()
+    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    gaps, done = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps[0], last = max(gaps[0], now - last), now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    start.record()
+    torch.cuda._sleep(1_500_000_000)                # the better part of a second
+    for _ in range(1500):
+        layer(x)
+    stop.record()
+    torch.cuda.synchronize()
+    done.set()
+    thread.join()
+    busy = start.elapsed_time(stop) * 1e-3
+    assert busy > 0.4 and gaps[0] < 0.5 * busy, (busy, gaps[0])
