@@ -146,3 +146,34 @@ def test_other_threads_run_while_a_layer_waits_for_room_in_the_stream(kind):
     thread.join()
     busy = start.elapsed_time(stop) * 1e-3
     assert busy > 0.4 and gaps[0] < 0.5 * busy, (busy, gaps[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", list(MAKE))
+def test_buffers_written_right_in_front_of_a_call_are_the_ones_it_reads(kind):
+    """Stream order holds for a layer's buffers: a product that fetches codes and table ahead of its activations does not run
+    ahead of a copy into them."""
+    import quantize_hf as q
+    from rptc_b200 import CODE_LUT, LAYOUT_TILED, Format
+    from rptc_b200.linear import RPTCLinear
+    n, m = 1024, 4096
+    g = torch.Generator(device="cuda").manual_seed(7)
+
+    def make():
+        if kind == "linear":
+            return RPTCLinear.random(n, m, Format(CODE_LUT, 2, 16, 0, LAYOUT_TILED), 0.02, int(torch.randint(0, 1000, (1,))))
+        rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+        return q.FactorizedRPTCLinear.from_parts(torch.randint(0, 4, (m, n), generator=g, device="cuda", dtype=torch.int32), rnd(8, 1 << 16), rnd(m), rnd(n),
+                                                 rnd(m), rnd(n))
+    sides = [make(), make()]
+    x = torch.randn(12, n, generator=g, device="cuda").half()                  # nine rows and more: the same bits every time
+    want = [side(x) for side in sides]
+    layer = make()
+    names = [k for k, v in layer._buffers.items() if v is not None]
+    results = []
+    for i in range(100):
+        for name in names:
+            layer._buffers[name].copy_(sides[i & 1]._buffers[name])
+        results.append(layer(x))
+    for i, y in enumerate(results):
+        assert torch.equal(y, want[i & 1]), i
