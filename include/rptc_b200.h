@@ -344,12 +344,17 @@ int rptc_embed_mailbox(const void *table, const uint64_t *slots, uint32_t *steps
  * minimum (loss[rows]).  alphabet fp32 [2^L], 4 <= L <= 16.  First-minimum tie breaks and unfused fp32 arithmetic, as
  * in the reference.  workspace: rptc_viterbi_workspace_bytes(rows, n, L) bytes of device memory, 256-byte aligned
  * (two survivor bits per position, row and state prefix: 4 KiB per row and position at L = 16).
+ * rptc_viterbi_encode_rows: a range of consecutive rows of a matrix whose rows are in banks of rows_per_bank with an alphabet
+ * each; first_row is the number of the range's first row within its bank, alphabets that bank's and the following ones'.
  * rptc_viterbi_encode_banked: the rows are `banks` equal groups of consecutive rows with one alphabet each,
  * alphabets fp32 [banks][2^L] (quantize_hf.py:135-150), all of them in one launch. */
 int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L);
 int rptc_viterbi_encode(const float *alphabet, const float *pos_weight, const float *samples, int64_t ld_samples, int64_t rows,
                         int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss, void *workspace, int64_t workspace_bytes,
                         rptc_stream_t stream);
+int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per_bank, int64_t first_row, const float *pos_weight, const float *samples,
+                             int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
+                             void *workspace, int64_t workspace_bytes, rptc_stream_t stream);
 int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks, const float *pos_weight, const float *samples,
                                int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
                                void *workspace, int64_t workspace_bytes, rptc_stream_t stream);

@@ -32,7 +32,9 @@ struct ViterbiParams {
     int32_t *final_state;          // [rows]
     float *loss;                   // [rows]
     int32_t n, L;
-    int32_t rows_per_bank, items_per_bank, n_items;
+    // The rows at hand: rows_per_bank of each bank, of the first bank the last `first_rows`, of the last one what is left of `rows`.  An
+    // item is what a cluster takes at a time: R rows of a bank.
+    int32_t rows, first_rows, rows_per_bank, first_items, items_per_bank, n_items;
     unsigned int *status;
 };
 
@@ -114,9 +116,12 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
     auto wait = [] { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };
 
     for (int item = blockIdx.x / CL; item < p.n_items; item += gridDim.x / CL) {
-        const int bank = item / p.items_per_bank, j = item - bank * p.items_per_bank;
-        const int row0 = bank * p.rows_per_bank + j * R;
-        const int n_rows = R == 1 ? 1 : min(R, p.rows_per_bank - j * R);
+        // item number counted as if the first bank were whole
+        const int it = item + p.items_per_bank - p.first_items;
+        const int bank = item < p.first_items ? 0 : it / p.items_per_bank, j = item < p.first_items ? item : it - bank * p.items_per_bank;
+        const int bank0 = bank == 0 ? 0 : p.first_rows + (bank - 1) * p.rows_per_bank;
+        const int row0 = bank0 + j * R;
+        const int n_rows = R == 1 ? 1 : min(R, min(p.rows, p.first_rows + bank * p.rows_per_bank) - row0);
         f32x2 na[G][4][2];                                      // alphabet entries, negated: x - e = x + (-e)
         {
             const float4 *alpha = reinterpret_cast<const float4 *>(p.alphabets + (int64_t)bank * M);
@@ -356,12 +361,14 @@ extern "C" int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L) 
     return (back + 255) / 256 * 256 + rows * 4;
 }
 
-extern "C" int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks, const float *pos_weight, const float *samples,
-                                          int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
-                                          void *workspace, int64_t workspace_bytes, rptc_stream_t stream) {
+extern "C" int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per_bank, int64_t first_row, const float *pos_weight, const float *samples,
+                                        int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
+                                        void *workspace, int64_t workspace_bytes, rptc_stream_t stream) {
     if (!alphabets || !pos_weight || !samples || !symbols || !loss || !workspace) return RPTC_ERR_ARG;
     if (L < 4 || L > 16) return RPTC_ERR_UNSUPPORTED;
-    if (rows <= 0 || rows > 65535 || n <= 0 || banks <= 0 || rows % banks || ld_samples < n || ld_sym < n) return RPTC_ERR_SHAPE;
+    if (rows <= 0 || rows > 65535 || n <= 0 || rows_per_bank <= 0 || first_row < 0 || first_row >= rows_per_bank || ld_samples < n || ld_sym < n)
+        return RPTC_ERR_SHAPE;
+    if (rows_per_bank > (int64_t(1) << 30)) return RPTC_ERR_TOO_LARGE;
     if (n > (int64_t(1) << 30)) return RPTC_ERR_TOO_LARGE;
     if (workspace_bytes < rptc_viterbi_workspace_bytes(rows, n, L)) return RPTC_ERR_TOO_LARGE;
     if ((reinterpret_cast<uintptr_t>(alphabets) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255)) return RPTC_ERR_ALIGN;
@@ -378,39 +385,41 @@ extern "C" int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks,
     p.loss = loss;
     p.n = (int32_t)n;
     p.L = L;
-    p.rows_per_bank = (int32_t)(rows / banks);
+    p.rows = (int32_t)rows;
+    p.rows_per_bank = (int32_t)rows_per_bank;
+    p.first_rows = (int32_t)(rows < rows_per_bank - first_row ? rows : rows_per_bank - first_row);
     p.status = device_status_word();
     if (!p.status) return RPTC_ERR_CUDA;
     auto rows_at_once = [&](int r) {
+        const int left = p.rows - p.first_rows;
+        p.first_items = (p.first_rows + r - 1) / r;
         p.items_per_bank = (p.rows_per_bank + r - 1) / r;
-        p.n_items = (int32_t)(banks * p.items_per_bank);
+        p.n_items = p.first_items + left / p.rows_per_bank * p.items_per_bank + (left % p.rows_per_bank + r - 1) / r;
     };
     // Threads per CTA: a quarter of 2^(L-2) prefixes in groups of four, two groups a thread from L = 10 on (below, one warp
-    // has lanes to spare).  At L = 15 and 16 one CTA of 1024 threads fills an SM; two rows then alternate in it unless
-    // that would leave SMs idle (fewer pairs of rows than places for them).  Smaller L run one row per CTA and as many
-    // CTAs as fit (64 registers a thread).
-    const int groups = 1 << (L - 4), sms = num_sms();
+    // has lanes to spare).  At L = 15 and 16 one CTA of 1024 threads fills an SM; two rows then alternate in it, unless every
+    // row finds a place of its own: two at a time take less than one after the other (1024 samples, L = 16, 136 rows: 2.4
+    // against 4.4 ms).  Smaller L run one row per CTA and as many CTAs as fit (64 registers a thread).
+    const int groups = 1 << (L - 4), sms = num_sms(), places = L == 16 ? sms / 2 : sms;
+    const bool pairs = L >= 15 && rows > places;
+    rows_at_once(pairs ? 2 : 1);
     int e;
-    rows_at_once(2);
-    if (L == 16) {
-        const int places = sms / 2;
-        if (p.n_items >= places) {
-            e = launch_forward<2, 2, 2>(p, 1024, places, s);
-        } else {
-            rows_at_once(1);
-            e = launch_forward<2, 2, 1>(p, 1024, places, s);
-        }
-    } else if (L == 15 && p.n_items >= sms) {
-        e = launch_forward<1, 2, 2>(p, 1024, sms, s);
-    } else {
-        rows_at_once(1);
-        if (L >= 10) e = launch_forward<1, 2, 1>(p, groups / 2, sms * (L == 15 ? 1 : L == 10 ? 32 : 2048 / groups), s);
-        else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
-    }
+    if (L == 16) e = pairs ? launch_forward<2, 2, 2>(p, 1024, places, s) : launch_forward<2, 2, 1>(p, 1024, places, s);
+    else if (pairs) e = launch_forward<1, 2, 2>(p, 1024, places, s);
+    else if (L >= 10) e = launch_forward<1, 2, 1>(p, groups / 2, sms * (L == 15 ? 1 : L == 10 ? 32 : 2048 / groups), s);
+    else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
     if (e) return e;
     viterbi_backtrack_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym);
     RPTC_CUDA(cudaGetLastError());
     return RPTC_OK;
+}
+
+extern "C" int rptc_viterbi_encode_banked(const float *alphabets, int64_t banks, const float *pos_weight, const float *samples,
+                                          int64_t ld_samples, int64_t rows, int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss,
+                                          void *workspace, int64_t workspace_bytes, rptc_stream_t stream) {
+    if (rows <= 0 || banks <= 0 || rows % banks) return RPTC_ERR_SHAPE;
+    return rptc_viterbi_encode_rows(alphabets, rows / banks, 0, pos_weight, samples, ld_samples, rows, n, L, symbols, ld_sym, loss, workspace,
+                                    workspace_bytes, stream);
 }
 
 extern "C" int rptc_viterbi_encode(const float *alphabet, const float *pos_weight, const float *samples, int64_t ld_samples,

@@ -104,8 +104,9 @@ def round_weights(permute, weights: torch.Tensor, importance: torch.Tensor, shif
     quantiles = megabatch_alphabets(weights.reshape(num_banks, -1), shift_register_size)
     alphabets = torch.stack([permute(alphabet) for alphabet in quantiles])
     if weights.is_cuda and alphabets.dtype == torch.float32 and 4 <= shift_register_size <= 16:
-        # the CUDA encoder takes all banks at once: a bank has too few rows to fill the GPU
-        return ops.viterbi_encode_banked(alphabets, pos_weight, weights)[0], alphabets
+        # the CUDA encoder goes through the rows of all banks, as many at once as it has in flight (a bank has too few to fill the
+        # GPU), and with less memory batch_size of them
+        return ops.viterbi_encode_banked(alphabets, pos_weight, weights, least_rows=batch_size)[0], alphabets
     symbols = torch.empty((m, n), dtype=torch.int32, device=weights.device)
     for b, alphabet in enumerate(alphabets):
         rows = slice(b * per_bank, (b + 1) * per_bank)

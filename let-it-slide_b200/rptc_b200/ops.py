@@ -349,10 +349,22 @@ def viterbi_encode(alphabet: torch.Tensor, pos_weight: torch.Tensor, samples: to
     return viterbi_encode_banked(alphabet[None, :], pos_weight, samples, workspace_limit)
 
 
-def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, samples: torch.Tensor, workspace_limit: int = 12 << 30):
+def encoder_rows_at_once(L: int, n: int, sms: int, workspace_limit: int) -> int:
+    """How many rows of n samples go through the encoder at once.  More than the kernel has in flight (one row per SM at L = 16, two
+    at L = 15) only shorten the tail of the last ones, so beyond 4 GiB of survivor memory it is no more than those: 2.4 GB
+    at L = 16 and n = 4096.  Whole sets of them, so that no launch ends with idle SMs."""
+    fit = workspace_limit // lib().rptc_viterbi_workspace_bytes(1, n, L)
+    flight = sms // 2 * 2 if L == 16 else 2 * sms
+    most = max(flight, (4 << 30) // lib().rptc_viterbi_workspace_bytes(1, n, L))
+    rows = max(1, min(65535, fit, most))
+    return rows // flight * flight if rows >= flight else rows
+
+
+def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, samples: torch.Tensor, workspace_limit: int = 12 << 30,
+                          least_rows: int = 1):
     """The same for `alphabets` [banks, 2^L] whose banks own equal groups of consecutive rows of `samples`
-    (rptc_viterbi_encode_banked).  Rows go through in batches sized so that the survivor memory stays under
-    `workspace_limit`: whole banks while one fits, else parts of a bank."""
+    (rptc_viterbi_encode_rows).  Rows go through in batches whose survivor memory stays under `workspace_limit`
+    (encoder_rows_at_once), and in smaller ones, down to `least_rows`, where the device has no room for that."""
     banks, M = alphabets.shape
     L = M.bit_length() - 1
     if M != 1 << L:
@@ -365,23 +377,19 @@ def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, sam
         raise RuntimeError("the banks must hold equally many rows")
     symbols = torch.empty((rows, n), dtype=torch.int32, device=samples.device)
     loss = torch.empty(rows, dtype=torch.float32, device=samples.device)
-    fit = max(1, min(65535, workspace_limit // lib().rptc_viterbi_workspace_bytes(1, n, L)))      # rows at once
     per_bank = rows // banks
-    step = min(rows, fit // per_bank * per_bank if fit >= per_bank else fit)
-    with torch.cuda.device(samples.device):
+    step = min(rows, encoder_rows_at_once(L, n, torch.cuda.get_device_properties(samples.device).multi_processor_count, workspace_limit))
+    while True:
         need = lib().rptc_viterbi_workspace_bytes(step, n, L)
-        ws = torch.empty(need, dtype=torch.uint8, device=samples.device)
-        r0 = 0
-        while r0 < rows:
-            bank, inside = divmod(r0, per_bank)
-            r = min(step, rows - r0) if step >= per_bank else min(step, per_bank - inside)
-            check(lib().rptc_viterbi_encode_banked(ptr(alphabets[bank:]), max(1, r // per_bank), ptr(pos_weight), ptr(samples[r0:]), n, r, n, L,
-                                                   ptr(symbols[r0:]), n, ptr(loss[r0:]), ptr(ws), need, stream_ptr()),
-                  "rptc_viterbi_encode_banked")
-            r0 += r
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=samples.device)
+            break
+        except torch.OutOfMemoryError:
+            if step <= least_rows:
+                raise
+            step = max(least_rows, step // 2)
+    for r0 in range(0, rows, step):
+        bank, inside = divmod(r0, per_bank)
+        call("rptc_viterbi_encode_rows", samples.device, ptr(alphabets[bank:]), per_bank, inside, ptr(pos_weight), ptr(samples[r0:]), n,
+             min(step, rows - r0), n, L, ptr(symbols[r0:]), n, ptr(loss[r0:]), ptr(ws), need)
     return symbols, loss
-
-
-def device_status() -> None:
-    """Raises if a kernel reported a timed-out wait since the last call."""
-    check(lib().rptc_device_status(), "rptc_device_status")

@@ -103,3 +103,39 @@ def test_banked_encoder_at_the_edges_of_its_variants(L, n, banks, per_bank):
     again, _ = ops.viterbi_encode_banked(alphabets[:2].cuda(), weights.cuda(), samples[: min(banks, 2) * per_bank].cuda(),
                                          workspace_limit=2 * (n << (L - 4)) + 1024)
     assert torch.equal(again, sym[: again.shape[0]])
+
+
+@pytest.mark.parametrize("L,n,banks,per_bank", [(6, 20, 4, 5), (12, 30, 3, 7), (15, 9, 5, 3), (16, 7, 4, 5), (16, 5, 90, 2), (15, 4, 110, 3)])
+@pytest.mark.parametrize("at_once", [1, 2, 3, 8, 296])
+def test_encoder_takes_ranges_that_start_and_end_inside_banks(L, n, banks, per_bank, at_once):
+    from rptc_b200 import ops
+    from rptc_b200._lib import lib
+    g = torch.Generator(device="cuda").manual_seed(L * 100 + n)
+    alphabets = (torch.randn(banks, 1 << L, generator=g, device="cuda") * 64).round() / 64
+    samples = torch.randn(banks * per_bank, n, generator=g, device="cuda")
+    weights = 0.5 + torch.rand(n, generator=g, device="cuda")
+    want, want_loss = ops.viterbi_encode_banked(alphabets, weights, samples)
+    got, loss = ops.viterbi_encode_banked(alphabets, weights, samples, workspace_limit=at_once * lib().rptc_viterbi_workspace_bytes(1, n, L))
+    assert torch.equal(got, want) and torch.equal(loss, want_loss)
+
+
+def test_layer_quantisation_keeps_its_memory_bounded():
+    """At L = 16 and 4096 columns a row's survivors are 16 MiB: the rows of a whole layer at once would take 8.6 GB here.  With less memory
+    than the rows in flight need, batch_size rows at once are enough."""
+    import quantize_hf as q
+    g = torch.Generator(device="cuda").manual_seed(5)
+    weights, importance = torch.randn(512, 4096, generator=g, device="cuda"), 0.5 + torch.rand(4096, generator=g, device="cuda")
+    permute = q.seeded_permute(3)
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    symbols, alphabets = q.round_weights(permute, weights, importance, 16, 32, 8)
+    assert torch.cuda.max_memory_allocated() - before < 3 << 30
+    torch.cuda.empty_cache()
+    limit = (torch.cuda.memory_reserved() + (400 << 20)) / torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction(limit)
+    try:
+        again, _ = q.round_weights(permute, weights, importance, 16, 32, 8)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(again, symbols)

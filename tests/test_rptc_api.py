@@ -102,3 +102,11 @@ def test_dequantize_over_pieces_and_tails(rows, length, L, dtype):
         states[:, back:] |= sym[:, : length - back].long() << (2 * back)
     assert got.dtype == dtype and torch.equal(got, alphabet.half().to(dtype)[states & ((1 << L) - 1)])
     assert torch.equal(rptc.pack_symbols(sym, 2).cpu(), rptc.pack_symbols(sym.cpu(), 2))
+
+
+@pytest.mark.parametrize("L,n,limit,want", [(16, 4096, 12 << 30, 148), (16, 1024, 12 << 30, 888), (16, 4096, 1 << 30, 63), (16, 65536, 1 << 20, 1), (15, 4096, 12 << 30, 296),
+                                            (8, 4096, 12 << 30, 65416)])
+def test_encoder_rows_at_once_needs_no_gpu(L, n, limit, want):
+    """Survivor memory is 2^(L-4) bytes per row and position: whole sets of the rows in flight, 4 GiB beyond one set."""
+    from rptc_b200 import ops
+    assert ops.encoder_rows_at_once(L, n, 148, limit) == want
