@@ -109,7 +109,7 @@ int rptc_repack(const void *src, int src_layout, void *dst, int dst_layout, int6
 int rptc_decompress(const void *codes, const void *lut, const uint32_t *carry_in, void *out, int64_t ld_out,
                     int64_t m, int64_t n, const rptc_format *fmt, rptc_stream_t stream);
 
-/* Symbols (int32 [rows][length], 0..3) -> out[row][i] = alphabet[state_i] rounded to fp16, state = the last L <= 16 bits of
+/* Symbols (int32 [rows][length], 0..3) -> out[row][i] = alphabet[state_i] rounded to fp16, state = the last L bits (3 to 16) of
  * the row's symbols up to i, zero before the row (rptc.py:74-85).  alphabet [2^L] and out [rows][length] are both fp32
  * (is_f32 = 1) or both fp16. */
 int rptc_dequantize(const void *alphabet, const int32_t *symbols, void *out, int is_f32, int64_t rows, int64_t length, int L,

@@ -159,7 +159,7 @@ using namespace rptc;
 extern "C" int rptc_dequantize(const void *alphabet, const int32_t *symbols, void *out, int is_f32, int64_t rows, int64_t length, int L,
                                rptc_stream_t stream) {
     if (!alphabet || !symbols || !out) return RPTC_ERR_ARG;
-    if (L < 1 || L > 16) return RPTC_ERR_ARG;
+    if (L < 3 || L > 16) return RPTC_ERR_ARG;
     if (rows <= 0 || length <= 0) return RPTC_ERR_SHAPE;
     if (length > (int64_t(1) << 30) || rows > (int64_t(1) << 40) / length) return RPTC_ERR_TOO_LARGE;
     if (int e = rptc_check_device()) return e;

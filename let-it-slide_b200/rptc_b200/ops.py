@@ -78,6 +78,11 @@ def decompress(codes: torch.Tensor, lut: torch.Tensor, m: int, n: int, fmt: Form
     return out
 
 
+def check_alphabet(alphabet: torch.Tensor) -> None:
+    if alphabet.dim() != 1 or alphabet.shape[0] not in [1 << L for L in range(3, 17)]:
+        raise RuntimeError(f"the alphabet must be one row of 2^L entries, L = 3 to 16, got {tuple(alphabet.shape)}")
+
+
 def dequantize(alphabet: torch.Tensor, symbols: torch.Tensor) -> torch.Tensor:
     """2-bit symbols int32 [rows, length] -> alphabet[state], rounded to fp16, in the alphabet's dtype (fp16 or fp32)
     (rptc_dequantize)."""
@@ -85,6 +90,7 @@ def dequantize(alphabet: torch.Tensor, symbols: torch.Tensor) -> torch.Tensor:
     _cuda_contig(symbols, "symbols", torch.int32)
     if alphabet.dtype not in (torch.float16, torch.float32):
         raise RuntimeError("alphabet must be fp16 or fp32")
+    check_alphabet(alphabet)
     rows, length = symbols.shape
     out = torch.empty((rows, length), dtype=alphabet.dtype, device=symbols.device)
     if out.numel():

@@ -110,3 +110,24 @@ def test_encoder_rows_at_once_needs_no_gpu(L, n, limit, want):
     """Survivor memory is 2^(L-4) bytes per row and position: whole sets of the rows in flight, 4 GiB beyond one set."""
     from rptc_b200 import ops
     assert ops.encoder_rows_at_once(L, n, 148, limit) == want
+
+
+@pytest.mark.parametrize("shape", [(65535,), (100,), (4,), (1 << 17,), (2, 32768), (0,)])
+def test_dequantize_refuses_an_alphabet_that_is_not_a_table(shape):
+    """The state indexes 2^L entries: any other length would silently use its first ones."""
+    from rptc_b200 import lib, ops
+    with pytest.raises(RuntimeError, match="2\\^L entries"):
+        ops.check_alphabet(torch.zeros(shape))
+    for L in (3, 16):
+        ops.check_alphabet(torch.zeros(1 << L))
+    for L in (0, 2, 17):
+        assert lib().rptc_dequantize(1 << 8, 1 << 8, 1 << 8, 1, 1, 1, L, None) == -1
+
+
+@pytest.mark.gpu
+def test_dequantize_refuses_odd_alphabets_on_the_gpu():
+    import rptc
+    sym = torch.zeros(8, dtype=torch.int32, device="cuda")
+    for n in (100, 65535):
+        with pytest.raises(RuntimeError, match="2\\^L entries"):
+            rptc.dequantize(torch.zeros(n, device="cuda"), sym)
