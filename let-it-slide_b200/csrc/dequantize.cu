@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kDeqThreads, 1) dequantize_kernel(const T *__r
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const uint32_t mask = (1u << L) - 1u;
+    pdl_wait_prior_grids();                             // launched with the calling thread's rptc_set_pdl setting
     if (TABLE) {
         constexpr int kBatch = 8;                       // loads in flight per thread
         for (int i0 = threadIdx.x; i0 < (1 << L); i0 += kBatch * kDeqThreads) {

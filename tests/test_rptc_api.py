@@ -131,3 +131,32 @@ def test_dequantize_refuses_odd_alphabets_on_the_gpu():
     for n in (100, 65535):
         with pytest.raises(RuntimeError, match="2\\^L entries"):
             rptc.dequantize(torch.zeros(n, device="cuda"), sym)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,length", [(512, 4096), (4096, 4096)])
+def test_dequantize_keeps_stream_order_under_dependent_launch(rows, length):
+    """With rptc_set_pdl on, the kernel in front lets this one start early; it neither reads nor writes anything before that one is
+    done: here the memory that the decoder in front still reads its codes from becomes the result."""
+    import ctypes
+
+    from rptc_b200 import CODE_LUT, LAYOUT_TILED, Format, lib, ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    m, n, L = 4096, 8192, 16
+    fmt = Format(CODE_LUT, 2, L, 0, LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, 2, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(1 << L, generator=g, device="cuda").half()
+    symbols = torch.randint(0, 4, (rows, length), generator=g, device="cuda", dtype=torch.int32)
+    want_dense, want = ops.decompress(codes, lut, m, n, fmt), ops.dequantize(lut, symbols)
+    out, stream = torch.empty_like(want_dense), torch.cuda.current_stream().cuda_stream
+    shared = torch.empty(max(codes.numel(), want.numel() // 2), dtype=torch.int32, device="cuda")
+    lib().rptc_set_pdl(1)
+    try:
+        for _ in range(20):
+            shared[: codes.numel()].copy_(codes.reshape(-1))
+            assert lib().rptc_decompress(shared.data_ptr(), lut.data_ptr(), None, out.data_ptr(), n, m, n, ctypes.byref(fmt), stream) == 0
+            assert lib().rptc_dequantize(lut.data_ptr(), symbols.data_ptr(), shared.data_ptr(), 0, rows, length, L, stream) == 0
+            assert torch.equal(out, want_dense)
+            assert torch.equal(shared.view(torch.float16)[: want.numel()].view(want.shape), want)
+    finally:
+        lib().rptc_set_pdl(0)
