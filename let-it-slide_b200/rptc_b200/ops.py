@@ -7,7 +7,7 @@ import torch
 
 from . import _lib
 from ._lib import (CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_TILED, LAYOUT_UNITMAJOR, XORDER_NATURAL,
-                   Format, call, check, lib, ptr, stream_ptr)
+                   Format, call, check, lib, ptr)
 
 
 def _cuda_contig(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
@@ -399,3 +399,8 @@ def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, sam
         call("rptc_viterbi_encode_rows", samples.device, ptr(alphabets[bank:]), per_bank, inside, ptr(pos_weight), ptr(samples[r0:]), n,
              min(step, rows - r0), n, L, ptr(symbols[r0:]), n, ptr(loss[r0:]), ptr(ws), need)
     return symbols, loss
+
+
+def device_status() -> None:
+    """Raises if a kernel reported a timed-out wait since the last call."""
+    check(lib().rptc_device_status(), "rptc_device_status")
