@@ -237,7 +237,8 @@ int rptc_swiglu_hadamard_f16(const void *gate_up, int64_t ld_in, void *out, int6
  * of *_workspace_bytes for that number of rows; it holds nothing between calls. */
 /* y = s_out * H( scale * W( H( s_in * x ) ) ), Hadamard blocks block_in / block_out (rptc_hadamard's rules); without
  * signs (both NULL) y = scale * W x, where more than 64 rows leave the scale to the caller.  x fp16 [rows][n], y fp16 [rows][m].
- * TILED layout, K = 2 or 4, m % 32 == 0; more than 64 rows need n % 64 == 0. */
+ * TILED layout, K = 2 or 4, m % 32 == 0; more than 64 rows need n % 64 == 0.  At most 65535 rows with transforms,
+ * 2^24 without. */
 typedef struct rptc_linear {
     const void *codes, *lut;
     const uint32_t *carry_in;            /* or NULL */

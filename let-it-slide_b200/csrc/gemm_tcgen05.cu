@@ -593,7 +593,7 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks 
     for (int rows = 256; rows >= 128; rows >>= 1) {
         for (int halves = tokens > 128 ? 2 : 1; halves >= 1; --halves) {
             GemmParams probe;
-            if (!plan_gemm(probe, {rows, halves, 1}, f)) continue;
+            if (!plan_gemm(probe, {rows, halves, 1}, f) || tokens > 65535 * 128 * (int64_t)halves) continue;      // a grid row per tile of tokens
             const int64_t tiles = banks.banks * ((m + rows - 1) / rows) * ((tokens + halves * 128 - 1) / (halves * 128));
             for (int split = 1; split <= (banks.may_split ? rows / 64 : 1) && (split == 1 || steps >= 8 * split); split *= 2) {
                 const int64_t places = cluster_places(split);

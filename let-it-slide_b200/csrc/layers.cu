@@ -198,9 +198,11 @@ extern "C" int rptc_packed_forward(const rptc_packed *l, const void *x, int dtyp
 }
 
 // ---- the incoherent layer ----
+constexpr int64_t kFewRows = 65535;      // the transforms and the readers of an accumulator have a grid row per activation row
 // Whether the product goes through the fp32 accumulator: one or two rows, whatever the kernel for a few rows takes, and
 // up to 64 rows of a reduction that is not whole steps of 64 columns.  The others take the tiled product, whose last tile may be partial.
 static bool linear_few(const rptc_linear &l, int64_t rows) {
+    if (rows > kFewRows) return false;
     return rows <= 2 || gemv_few_takes(l.m, l.n, rows, Banks(), l.fmt, nullptr, l.n) || (rows <= 64 && l.n % 64);
 }
 
@@ -217,9 +219,10 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     if (l->fmt.layout != RPTC_LAYOUT_TILED || l->fmt.quirk != RPTC_QUIRK_NONE || (l->fmt.K != 2 && l->fmt.K != 4)) return RPTC_ERR_UNSUPPORTED;
     if (!l->signs_in != !l->signs_out) return RPTC_ERR_ARG;
     if (l->m <= 0 || l->n <= 0 || rows <= 0 || (l->m % 32) || (l->n % (128 / l->fmt.K)) || (l->m % 4)) return RPTC_ERR_SHAPE;
+    if (rows > (l->signs_in ? kFewRows : int64_t(1) << 24)) return RPTC_ERR_TOO_LARGE;
     const bool few = linear_few(*l, rows);
     if (!few && (l->n % 64)) return RPTC_ERR_SHAPE;
-    if (l->m > (int64_t(1) << 30) || l->n > (int64_t(1) << 30) || rows > 65535 || (l->m / 32) * (l->n / (128 / l->fmt.K)) >= (int64_t(1) << 31))
+    if (l->m > (int64_t(1) << 30) || l->n > (int64_t(1) << 30) || (l->m / 32) * (l->n / (128 / l->fmt.K)) >= (int64_t(1) << 31))
         return RPTC_ERR_TOO_LARGE;
     const int64_t need = rptc_linear_workspace_bytes(l, rows);
     if (need && (!workspace || workspace_bytes < need)) return RPTC_ERR_TOO_LARGE;

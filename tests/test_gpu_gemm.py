@@ -234,3 +234,16 @@ def test_layers_of_nine_rows_and_more_repeat_themselves(code, K, L, S, m, n, tok
     ref = x.float() @ layer.effective_weight().t()
     assert (first.float() - ref).abs().max() <= 1e-2 * ref.abs().max()
     ops.device_status()
+
+
+def test_layer_without_transforms_takes_more_rows_than_a_grid_has():
+    from rptc_b200 import Format
+    from rptc_b200._lib import RPTCError
+    from rptc_b200.linear import RPTCLinear
+    x = torch.randn((70001, 64), dtype=torch.float16, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    layer = RPTCLinear.random(64, 128, Format(), 0.5, 3, incoherent=False)
+    y = layer(x)
+    ref = x.float() @ layer.effective_weight().t()
+    assert (y.float() - ref).abs().max() <= 2e-3 * ref.abs().max()
+    with pytest.raises(RPTCError):
+        RPTCLinear.random(256, 256, Format(), 0.5, 3)(torch.zeros((70001, 256), dtype=torch.float16, device="cuda"))
