@@ -119,8 +119,9 @@ int rptc_dequantize(const void *alphabet, const int32_t *symbols, void *out, int
 int rptc_pack_symbols(const int32_t *symbols, void *words, int64_t rows, int64_t length, int64_t row_words, int bits,
                       rptc_stream_t stream);
 
-/* Fused decode + matvec, batch 1..64:  acc[b][row] += sum_c W[row][c] * x[b][c]   (fp32 acc).  One launch where x is
- * 16-byte aligned with ld_x % 8 == 0 and n % 64 == 0 (and for one or two rows), else one per two activation rows.
+/* Fused decode + matvec, batch 1..64:  acc[b][row] += sum_c W[row][c] * x[b][c]   (fp32 acc).  TILED layout without a
+ * quirk: one launch where x is 16-byte aligned with ld_x % 8 == 0 and n % 64 == 0 (and for one or two rows), else one per two
+ * activation rows; the other layouts and the quirks: one per row.
  * Replaces the kernels behind decompress_matvec_{16,20}_{6,8}_1 (inference.cu:189-277) and
  * decompress_matvec_t_{16,14} (inference_t.cu:68-175).  `acc` is fp32 SCRATCH of [batch][ld_acc]
  * that the caller zeroes (or pre-loads) and later converts with rptc_gemv_finish; partial sums

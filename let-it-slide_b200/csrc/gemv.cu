@@ -872,10 +872,12 @@ extern "C" int rptc_gemv(const void *codes, const void *lut, const uint32_t *car
     // Up to two rows the lane-per-row kernel is the faster one (28672 x 8192: 28.0 against 30.6 us).
     if (batch > 2 && x_order == RPTC_XORDER_NATURAL && gemv_few_takes(m, n, batch, Banks(), *fmt, x, ld_x))
         return gemv_few(codes, lut, carry_in, x, ld_x, acc, ld_acc, m, n, batch, Banks(), *fmt, static_cast<cudaStream_t>(stream));
-    // what the kernel for a few rows does not take (rows of x that are not 16-byte aligned, the legacy order): pairs of rows
+    // what the kernel for a few rows does not take (rows of x that are not 16-byte aligned, the legacy order): pairs of rows, and one at a
+    // time where the general kernels are the only ones (the reference's layouts and deviations)
+    const bool pairs = fmt->layout == RPTC_LAYOUT_TILED && fmt->quirk == RPTC_QUIRK_NONE;
     int done = 0;
     while (done < batch) {
-        const int b = batch - done >= 2 ? 2 : 1;
+        const int b = pairs && batch - done >= 2 ? 2 : 1;
         int e = gemv_one(codes, lut, carry_in, static_cast<const __half *>(x) + (int64_t)done * ld_x, ld_x,
                          acc + (int64_t)done * ld_acc, ld_acc, m, n, b, x_order, *fmt, static_cast<cudaStream_t>(stream));
         if (e) return e;

@@ -131,10 +131,11 @@ class RPTCLinear(nn.Module):
         return y
 
     def _forward_by_parts(self, x: torch.Tensor) -> torch.Tensor:
-        """The reference's layouts: one row at a time goes through the general matvec kernel."""
+        """The reference's layouts: one row at a time goes through the general matvec kernel (up to 64 to a call)."""
         x2 = x.reshape(-1, self.in_features).to(torch.float16).contiguous()
-        xt, acc = self.transform_in(x2), self.acc_buffer(x2.shape[0])
-        self.matvec_acc(xt, acc)
+        xt, acc = self.transform_in(x2), torch.zeros((x2.shape[0], self.out_features), dtype=torch.float32, device=x2.device)
+        for xb, ab in zip(xt.split(64), acc.split(64)):
+            self.matvec_acc(xb, ab)
         return self.finish(acc).reshape(*x.shape[:-1], self.out_features)
 
     # -- reference helpers ----------------------------------------------------------------------------

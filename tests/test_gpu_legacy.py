@@ -230,3 +230,19 @@ def test_dense_probes_matvec_and_rowsum():
     ms = rptc_kernels.rowsum(w, out)
     truth = w.float().sum(dim=-1)
     assert (out.float() - truth).abs().max() <= 1e-3 * truth.abs().max() + 2e-2
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 70])
+@pytest.mark.parametrize("layout,quirk", [(o.LAYOUT_ROWMAJOR, 0), (o.LAYOUT_CHUNKED, 0), (o.LAYOUT_UNITMAJOR, 0), (o.LAYOUT_TILED, 2)])
+@pytest.mark.parametrize("incoherent", [False, True])
+def test_layer_in_another_layout_takes_any_number_of_rows(rows, layout, quirk, incoherent):
+    """The general kernels have one activation row: a layer sends its rows through one by one."""
+    from rptc_b200 import Format
+    from rptc_b200.linear import RPTCLinear
+    m, n = 256, 2048
+    layer = RPTCLinear.random(n, m, Format(o.CODE_B, 2, 16, 8, layout, quirk), 0.02, 5, incoherent=incoherent)
+    x = torch.randn((rows, n), dtype=torch.float16, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows))
+    y = layer(x)
+    ref = x.float() @ layer.effective_weight().t()
+    assert y.shape == (rows, m)
+    assert (y.float() - ref).abs().max() <= 1e-2 * ref.abs().max()
