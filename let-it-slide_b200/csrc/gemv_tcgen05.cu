@@ -562,14 +562,16 @@ bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, co
     // a layer asks several times per call, and mostly the question of the call before
     struct Question {
         int64_t m, n, tokens;
-        int32_t banks, code, K, L, S;
+        int32_t banks, code, K, L, S, device;      // device: its SMs, and the clusters that fit on them
+        bool may_split;
         bool operator==(const Question &o) const {
-            return m == o.m && n == o.n && tokens == o.tokens && banks == o.banks && code == o.code && K == o.K && L == o.L && S == o.S;
+            return m == o.m && n == o.n && tokens == o.tokens && banks == o.banks && code == o.code && K == o.K && L == o.L && S == o.S && device == o.device &&
+                   may_split == o.may_split;
         }
     };
     static thread_local Question last = {};
     static thread_local bool last_answer = false;
-    const Question q = {m, n, tokens, banks.banks, f.code, f.K, f.L, f.S};
+    const Question q = {m, n, tokens, banks.banks, f.code, f.K, f.L, f.S, current_device(), banks.may_split};
     if (q == last) return last_answer;
     last_answer = few_is_faster(m, n, tokens, banks, f);
     last = q;
