@@ -383,6 +383,8 @@ def viterbi_encode_banked(alphabets: torch.Tensor, pos_weight: torch.Tensor, sam
         raise RuntimeError("the banks must hold equally many rows")
     symbols = torch.empty((rows, n), dtype=torch.int32, device=samples.device)
     loss = torch.empty(rows, dtype=torch.float32, device=samples.device)
+    if rows == 0:
+        return symbols, loss
     per_bank = rows // banks
     step = min(rows, encoder_rows_at_once(L, n, torch.cuda.get_device_properties(samples.device).multi_processor_count, workspace_limit))
     while True:

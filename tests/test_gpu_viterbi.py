@@ -139,3 +139,9 @@ def test_layer_quantisation_keeps_its_memory_bounded():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(again, symbols)
+
+
+def test_encoder_of_no_rows_returns_nothing():
+    import rptc
+    sym, loss = rptc.quantize_rows(torch.randn(256, device="cuda"), torch.ones(5, device="cuda"), torch.empty(0, 5, device="cuda"))
+    assert sym.shape == (0, 5) and sym.dtype == torch.int32 and loss.shape == (0,)
