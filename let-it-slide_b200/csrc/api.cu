@@ -135,6 +135,10 @@ extern "C" int rptc_device_status(void) {
 namespace rptc {
 struct TimerEvents {
     cudaEvent_t begin = nullptr, end = nullptr;
+    ~TimerEvents() {      // the thread ends (a runtime that has been shut down before refuses, and holds them no more)
+        if (begin) cudaEventDestroy(begin);
+        if (end) cudaEventDestroy(end);
+    }
 };
 static thread_local TimerEvents g_timers[kMaxDevices];      // kept: creating a pair costs as much as a launch
 static int timer_events(TimerEvents *&t) {

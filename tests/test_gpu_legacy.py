@@ -246,3 +246,31 @@ def test_layer_in_another_layout_takes_any_number_of_rows(rows, layout, quirk, i
     ref = x.float() @ layer.effective_weight().t()
     assert y.shape == (rows, m)
     assert (y.float() - ref).abs().max() <= 1e-2 * ref.abs().max()
+
+
+def test_drop_in_matvec_from_threads_that_come_and_go():
+    """Every thread has events of its own to time its calls with; they go with the thread."""
+    import threading
+
+    import rptc_kernels
+    g = torch.Generator(device="cuda").manual_seed(1)
+    codes = torch.randint(-2**31, 2**31 - 1, (1, 64, 128), dtype=torch.int32, device="cuda", generator=g)
+    lut, x = torch.randn(512, generator=g, device="cuda").half(), torch.randn(2048, generator=g, device="cuda").half()
+    want = torch.empty(64, dtype=torch.float16, device="cuda")
+    assert rptc_kernels.decompress_matvec_16_8_1(codes, lut, x, want) > 0
+    bad = []
+
+    def work():
+        out = torch.empty_like(want)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            ms = rptc_kernels.decompress_matvec_16_8_1(codes, lut, x, out)
+        if not ms > 0 or not torch.equal(out, want):
+            bad.append(ms)
+
+    for _ in range(20):
+        threads = [threading.Thread(target=work) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not bad
