@@ -96,6 +96,7 @@ int rptc_device_status(void);
 /* Launch kernels with programmatic dependent launch (1) or plainly (0, default).  The setting belongs to the
  * calling thread: launches made by other threads are not affected. */
 void rptc_set_pdl(int enable);
+int rptc_pdl(void);      /* the calling thread's setting */
 
 /* Re-tiles packed codes between layouts (a pure permutation of 128-bit units).
  * Replaces nothing in the reference: it connects the reference's three layouts.  m % 32 == 0. */

@@ -103,6 +103,7 @@ extern "C" int rptc_version(void) { return 100; }
 extern "C" int rptc_last_cuda_error(void) { return g_last_cuda_error; }
 
 extern "C" void rptc_set_pdl(int enable) { g_pdl = enable != 0; }
+extern "C" int rptc_pdl(void) { return g_pdl; }
 
 extern "C" int rptc_check_device(void) {
     const int dev = current_device();

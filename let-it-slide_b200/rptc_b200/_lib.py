@@ -86,6 +86,7 @@ _SIGS = {
     "rptc_check_device": (ctypes.c_int, []),
     "rptc_device_status": (ctypes.c_int, []),
     "rptc_set_pdl": (None, [ctypes.c_int]),
+    "rptc_pdl": (ctypes.c_int, []),
     "rptc_repack": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64,
                                    ctypes.c_int64, ctypes.c_void_p]),
     "rptc_decompress": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,

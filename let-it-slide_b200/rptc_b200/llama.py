@@ -538,11 +538,12 @@ class RPTCLlama:
         fused = b0.o.incoherent and R * T > 8 and self.tp_world == 1              # residuals, rotation and SwiGLU inside the glue kernels
         last = None
         if fused:
+            before = lib().rptc_pdl()
             lib().rptc_set_pdl(1)
             try:
                 last = self._prefill_blocks_fused(h, R, T)
             finally:
-                lib().rptc_set_pdl(0)
+                lib().rptc_set_pdl(before)
         else:
 
             def apply(lin, x):

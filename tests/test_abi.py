@@ -77,3 +77,19 @@ def test_status_strings_cover_every_code():
     from rptc_b200 import lib
     for code in range(-10, 1):
         assert lib().rptc_strerror(code) != b"unknown status"
+
+
+def test_dependent_launch_setting_belongs_to_the_thread():
+    import threading
+
+    from rptc_b200 import lib
+    assert lib().rptc_pdl() == 0
+    lib().rptc_set_pdl(1)
+    try:
+        seen = []
+        t = threading.Thread(target=lambda: seen.append(lib().rptc_pdl()))
+        t.start()
+        t.join()
+        assert lib().rptc_pdl() == 1 and seen == [0]
+    finally:
+        lib().rptc_set_pdl(0)

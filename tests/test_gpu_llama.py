@@ -427,3 +427,17 @@ def test_prefill_without_transforms_gives_a_position_the_same_bits_in_any_compan
     for T in (9, 40, 130, 300):
         model.prefill(tokens[:, :T])
         assert torch.equal(model.kcache[0][:, :T], k[:, :T]) and torch.equal(model.vcache[0][:, :T], v[:, :T]), T
+
+
+def test_prefill_leaves_the_threads_launch_setting_as_it_was():
+    from rptc_b200 import lib
+    from rptc_b200.llama import LlamaConfig, RPTCLlama
+    cfg = LlamaConfig(hidden=512, layers=1, heads=4, kv_heads=4, ffn=1024, vocab=64, max_pos=32)
+    model = RPTCLlama(cfg, rows=1, seed=3)
+    for setting in (0, 1):
+        lib().rptc_set_pdl(setting)
+        try:
+            model.prefill(torch.zeros((1, 16), dtype=torch.int64, device="cuda"))
+            assert lib().rptc_pdl() == setting
+        finally:
+            lib().rptc_set_pdl(0)
