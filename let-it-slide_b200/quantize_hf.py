@@ -65,9 +65,15 @@ def factorize(W: torch.Tensor):
     return biases_out, biases_in, scales_out, scales_in, normalized
 
 
+_SORT_AT_ONCE = 1 << 25      # values sorted at once: a sort takes about 20 bytes a value beside them, 0.6 GB
+
+
 def megabatch_alphabets(megabatches: torch.Tensor, shift_register_size: int) -> torch.Tensor:
     """2^L evenly spaced quantiles of each bank's values, megabatches [banks, values] -> fp32 [banks, 2^L], by linear
     interpolation of the sorted sample (quantize_hf.py:136-140).  Interpolated in float64 and rounded to fp32."""
+    at_once = max(1, _SORT_AT_ONCE // max(1, megabatches.shape[1]))
+    if megabatches.shape[0] > at_once:
+        return torch.cat([megabatch_alphabets(part, shift_register_size) for part in megabatches.split(at_once)])
     M = 1 << shift_register_size
     fp = torch.sort(megabatches, dim=1).values
     N = fp.shape[1]

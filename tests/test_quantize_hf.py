@@ -42,6 +42,15 @@ def test_quantize_layer_reconstruction_matches_reference(golden):
     np.testing.assert_allclose(recon, golden["ql_recon"], rtol=1e-3, atol=1e-4)
 
 
+@pytest.mark.parametrize("at_once", [1, 700, 1500, 1 << 25])
+def test_alphabets_of_banks_do_not_depend_on_how_many_are_sorted_at_once(monkeypatch, at_once):
+    import quantize_hf as q
+    banks = torch.randn(7, 700, generator=torch.Generator().manual_seed(1))
+    want = torch.stack([q.megabatch_alphabet(bank, 6) for bank in banks])
+    monkeypatch.setattr(q, "_SORT_AT_ONCE", at_once)
+    assert torch.equal(q.megabatch_alphabets(banks, 6), want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("tokens", [1, 5, 40])
 def test_packed_layer_forward_matches_its_reconstruction(tokens):
