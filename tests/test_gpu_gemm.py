@@ -119,21 +119,6 @@ def test_linear_prefill_path_matches_effective_weight():
     assert (y - ref).abs().max() <= 1e-2 * ref.abs().max()
 
 
-def test_two_sm_kernel_passes_the_identity_cases():
-    """The cta_group::2 kernel is chosen per process (RPTC_GEMM_PAIR=1 in the environment, read at the first call), so the
-    bit-exact identity cases above run once more in a child process with it switched on (identity activations are 4096 or
-    more tokens: every shape with m % 256 == 0 takes the two-SM kernel there)."""
-    import os
-    import subprocess
-    import sys
-    if os.environ.get("RPTC_GEMM_PAIR") == "1":
-        pytest.skip("already inside the child process")
-    env = dict(os.environ, RPTC_GEMM_PAIR="1")
-    r = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-x", "-k", "identity or llama_shapes"],
-                       env=env, capture_output=True, text=True, timeout=900)
-    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
-
-
 @pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_C, 4, 16, 8)])
 @pytest.mark.parametrize("m,n,tokens", [(128, 448, 9), (256, 1024, 128), (384, 2112, 129), (4096, 1088, 100), (256, 4160, 257), (1152, 4032, 640)])
 def test_gemm_tiles_and_splits(code, K, L, S, m, n, tokens):
