@@ -192,11 +192,6 @@ __device__ __forceinline__ uint4 ld_ordered_u128(const void *p) {
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ uint2 ld_ordered_u64(const void *p) {
-    uint2 v;
-    asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ uint32_t ld_ordered_u32(const void *p) {
     uint32_t v;
     asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -949,7 +949,7 @@ extern "C" int rptc_gemv_glued(const void *codes, const void *lut, const uint32_
         misaligned(in->clear) || (in->ld_acc % 4) || (in->clear_count % 4))
         return RPTC_ERR_ALIGN;
     if (in->clear_count < 0 || (in->clear_count && !in->clear)) return RPTC_ERR_ARG;
-    if (n != 4096 && n != 8192) return RPTC_ERR_UNSUPPORTED;                    // one or two 4096-point blocks, eight values a thread each
+    if (n != 4096 && n != 8192) return RPTC_ERR_UNSUPPORTED;                    // one or two 4096-point blocks, sixteen values a thread
     if (!in->h_in || !in->h_out || in->h_in == in->h_out || !in->w_norm) return RPTC_ERR_ARG;
     if (in->ld_h < n || (in->acc && in->ld_acc < n)) return RPTC_ERR_SHAPE;
     if (misaligned(in->h_in) || misaligned(in->h_out) || misaligned(in->w_norm) || (in->ld_h % 8)) return RPTC_ERR_ALIGN;

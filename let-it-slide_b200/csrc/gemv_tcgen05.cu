@@ -256,8 +256,8 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                     else if (again) __stcg(to, __ldcg(to) + v);
                     else __stcg(to, v);
                 };
-#pragma unroll 1
                 const int tokens = SHARED ? min(p.tokens - g.t0, p.n_cols) : p.tokens;
+#pragma unroll 1
                 for (int t0 = 8 * part; t0 < tokens; t0 += 8 * PARTS) {
                     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1

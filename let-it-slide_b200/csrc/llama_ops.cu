@@ -13,11 +13,6 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
 
 // out[r][:] = x[r][:] * rsqrt(mean(x^2) + eps) * w[:]      one CTA of 256 threads per row
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __half *__restrict__ x, int64_t ld_x, const __half *__restrict__ w,

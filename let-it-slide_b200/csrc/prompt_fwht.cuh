@@ -119,11 +119,5 @@ __device__ __forceinline__ void unpack8_at(const uint4 &a, float *v) {
         v[2 * i] = f.x, v[2 * i + 1] = f.y;
     }
 }
-__device__ __forceinline__ uint4 pack8_from(const float *v) {
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = half2_as_u32(__floats2half2_rn(v[2 * i], v[2 * i + 1]));
-    return make_uint4(o[0], o[1], o[2], o[3]);
-}
 
 }  // namespace rptc
