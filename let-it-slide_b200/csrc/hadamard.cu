@@ -24,12 +24,14 @@ struct HadParams {
     int64_t n;
     float *clear;               // optional fp32 range that this launch zeroes (its own, not the input)
     int64_t clear_count;        // a multiple of 4
+    int32_t late;               // the next kernel may start behind this one's wait only
 };
 
 __global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
     __shared__ __align__(16) float ex[4096];
-    pdl_allow_next_grid();
+    if (!p.late) pdl_allow_next_grid();
     pdl_wait_prior_grids();
+    if (p.late) pdl_allow_next_grid();
     const int t = threadIdx.x;
     const int64_t row = blockIdx.y;
     if (p.clear) {
@@ -168,7 +170,7 @@ namespace rptc {
 // many rows (prompt_ops.cu)
 int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int64_t ld_out, const __half *signs, const __half *residual,
                   int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
-                  cudaStream_t stream);
+                  cudaStream_t stream, bool late);
 // Which inputs go to the kernels that walk down the rows.  Blocks above 256 columns: from 32 rows on (2048 x 4096: 13.4 us
 // against 19.3; up to 128 rows both take 3.3).  Smaller blocks, with rows on 32-byte boundaries: from 2.5 million values on (512 x 11008:
 // 7.6 us against 8.9, 512 x 4096: 4.5 against 4.2).
@@ -182,7 +184,7 @@ static bool many_rows(int64_t rows, int64_t n, int block, const HadParams &p) {
 
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
-                       int64_t clear_count, cudaStream_t stream) {
+                       int64_t clear_count, cudaStream_t stream, bool late) {
     if (!in || !out) return RPTC_ERR_ARG;
     if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
     if (rows <= 0 || n <= 0 || (n % block) || ld_in < n || ld_out < n || (residual && ld_res < n)) return RPTC_ERR_SHAPE;
@@ -209,7 +211,8 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
     p.transpose = transpose;
     if (many_rows(rows, n, block, p))
         return hadamard_rows(in, in_is_f32, ld_in, static_cast<__half *>(out), ld_out, static_cast<const __half *>(signs),
-                             static_cast<const __half *>(residual), ld_res, rows, n, block, transpose, scale, clear_in, clear, clear_count, stream);
+                             static_cast<const __half *>(residual), ld_res, rows, n, block, transpose, scale, clear_in, clear, clear_count, stream, late);
+    p.late = late;
     p.clear_in = clear_in;
     p.scale = scale * hadamard_norm(block);
     p.n = n;
@@ -231,7 +234,7 @@ extern "C" int rptc_hadamard(const void *in, int in_is_f32, int64_t ld_in, void 
                              const void *residual, int64_t ld_res, int64_t rows, int64_t n, int block, int transpose,
                              float scale, int clear_in, rptc_stream_t stream) {
     return hadamard_and_clear(in, in_is_f32, ld_in, out, ld_out, signs, residual, ld_res, rows, n, block, transpose, scale, clear_in, nullptr, 0,
-                              static_cast<cudaStream_t>(stream));
+                              static_cast<cudaStream_t>(stream), false);
 }
 
 static int swiglu_launch(float *acc, const void *in16, int64_t ld_in, void *out, int64_t ld_out, const void *signs_out,

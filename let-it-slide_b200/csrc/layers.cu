@@ -13,16 +13,19 @@
 namespace rptc {
 
 int check_format(const rptc_format *f);   // api.cu
-// rptc_hadamard with a range to zero on the side (fp32, a multiple of 4 values, 16-byte aligned).   hadamard.cu
+// rptc_hadamard with a range to zero on the side (fp32, a multiple of 4 values, 16-byte aligned); `late`: the kernel behind may start
+// behind this one's wait only.                                                                    hadamard.cu
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
-                       int64_t clear_count, cudaStream_t stream);
+                       int64_t clear_count, cudaStream_t stream, bool late = false);
 
 // Programmatic dependent launch within a call, whatever the calling thread's setting.  The products read codes and tables before they
 // wait for the kernel in front.  They must not do so while an earlier kernel of the stream still writes a layer's buffers, so nothing
-// behind a call's first kernel may start before all work in front of the call is done.  The packed layer's first kernel lets the next one
-// start only behind its own wait (32.8 -> 31.3 us for one token against an ordinary launch); the transforms, which other paths want early,
-// are launched without the attribute when they come first (22016 x 4096, 8 rows: 24.0 -> 22.6).
+// behind a call's first kernel may start before all work in front of the call is done.  The first kernel of a call lets the next one
+// start only behind its own wait, and where the tiled product follows it is launched without the attribute.  Measured, calls one
+// after the other, an ordinary launch of the first kernel against this: packed layer of one token 32.8 and 31.3 us; transform in front
+// of 4096 x 4096, 1 row 12.4 and 11.9, 32 rows 21.9 and 19.0; 4096 x 11008, 256 rows 43.0 and 41.0; tiled product, 4096 x 4096 with
+// 2048 rows 83 and 87.6 (its CTAs wait for the early ones to leave).
 struct PdlScope {
     const bool before = pdl_enabled();
     explicit PdlScope(bool on) { set(on); }
@@ -230,7 +233,7 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     if (misaligned(l->codes) || misaligned(l->lut) || misaligned(x) || misaligned(y) || misaligned(workspace) || (l->n % 8) || (l->m % 8))
         return RPTC_ERR_ALIGN;
     if (int e = rptc_check_device()) return e;
-    PdlScope pdl(false);
+    PdlScope pdl(l->signs_in && few);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
     const int64_t m = l->m, n = l->n;
@@ -239,7 +242,7 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     float *partial = few && partials(m, n, rows, Banks(), l->fmt) ? acc + round_up(rows * m * 4) / 4 : nullptr;
     const int64_t clear = few && !partial ? rows * m : 0;
     if (l->signs_in) {
-        if (int e = hadamard_and_clear(x, 0, n, ws, n, l->signs_in, nullptr, 0, rows, n, l->block_in, 0, 1.f, 0, acc, clear, s)) return e;
+        if (int e = hadamard_and_clear(x, 0, n, ws, n, l->signs_in, nullptr, 0, rows, n, l->block_in, 0, 1.f, 0, acc, clear, s, true)) return e;
         pdl.set(true);
         xt = ws;
     } else if (clear) {

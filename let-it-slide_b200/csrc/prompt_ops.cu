@@ -32,6 +32,7 @@ struct HadRowsParams {
     float scale;
     float *clear;
     int64_t clear_count;
+    int32_t late;                    // the next kernel may start behind this one's wait only
 };
 
 __device__ __forceinline__ uint32_t ldcg_u32(const void *p) { return __ldcg(static_cast<const uint32_t *>(p)); }
@@ -45,8 +46,9 @@ __global__ void __launch_bounds__(128, 4) hadamard_rows_kernel(const HadRowsPara
     const SegThread th;
     const int segs = (int)((p.n + kSeg - 1) / kSeg);
     const int64_t worker = blockIdx.x, workers = (int64_t)gridDim.x / segs * segs;
-    pdl_allow_next_grid();
+    if (!p.late) pdl_allow_next_grid();
     pdl_wait_prior_grids();
+    if (p.late) pdl_allow_next_grid();
     if (p.clear) {
         float4 *z = reinterpret_cast<float4 *>(p.clear);
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < p.clear_count; i += (int64_t)gridDim.x * blockDim.x)
@@ -208,13 +210,14 @@ __global__ void __launch_bounds__(256, IN_F32 ? 2 : 3) hadamard_half_rows_kernel
     const Far16 far(buf, t);
     const int segs = (int)((p.n + 511) / 512);
     const int64_t worker = (int64_t)blockIdx.x * 8 + warp, workers = (int64_t)gridDim.x * 8 / segs * segs;
-    pdl_allow_next_grid();
+    if (!p.late) pdl_allow_next_grid();
     const int64_t col = (worker % segs) * 512 + 256 * half + 16 * t;
     const bool active = col < p.n;                           // a last segment of 256 columns leaves half of the warp without
     uint32_t sg[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) sg[i] = p.signs && active ? __ldg(reinterpret_cast<const uint32_t *>(p.signs + col) + i) : 0x3C003C00u;
     pdl_wait_prior_grids();
+    if (p.late) pdl_allow_next_grid();
     if (p.clear) {
         float4 *z = reinterpret_cast<float4 *>(p.clear);
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; 4 * i < p.clear_count; i += (int64_t)gridDim.x * blockDim.x)
@@ -292,7 +295,7 @@ static unsigned rows_grid(int64_t rows, int64_t segs, int units, int resident) {
 
 int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int64_t ld_out, const __half *signs, const __half *residual,
                   int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear, int64_t clear_count,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, bool late) {
     HadRowsParams p;
     p.in = in;
     p.ld_in = ld_in;
@@ -309,6 +312,7 @@ int hadamard_rows(const void *in, int in_is_f32, int64_t ld_in, __half *out, int
     p.scale = scale * norm_of(block);
     p.clear = clear_count > 0 ? clear : nullptr;
     p.clear_count = clear_count;
+    p.late = late;
     if (block <= 256) {
         const dim3 grid(rows_grid(rows, (n + 511) / 512, 8, in_is_f32 ? 2 : 3));
         return in_is_f32 ? launch(hadamard_half_rows_kernel<true>, grid, dim3(256), 0, stream, p)
