@@ -235,8 +235,9 @@ int rptc_swiglu_hadamard_f16(const void *gate_up, int64_t ld_in, void *out, int6
 /* --- whole layers in one call (no reference counterpart: the reference has no layer objects) ---
  * The kernels of a call follow one another by programmatic dependent launch whatever rptc_set_pdl says; everything that the
  * stream holds in front of the call, writes of codes, tables, scales and signs included, is complete before the call reads any
- * of it.  Workspace: caller-owned device memory, 256-byte aligned,
- * of *_workspace_bytes for that number of rows; it holds nothing between calls. */
+ * of it.  Nine rows and more: every sum is taken in a fixed order, equal calls give equal bits (the number of rows chooses the
+ * product and with it the order); fewer rows: sums meet by atomics, their last bits can differ between runs.  Workspace:
+ * caller-owned device memory, 256-byte aligned, of *_workspace_bytes for that number of rows; it holds nothing between calls. */
 /* y = s_out * H( scale * W( H( s_in * x ) ) ), Hadamard blocks block_in / block_out (rptc_hadamard's rules); without
  * signs (both NULL) y = scale * W x, where more than 64 rows leave the scale to the caller.  x fp16 [rows][n], y fp16 [rows][m].
  * TILED layout, K = 2 or 4, m % 32 == 0; more than 64 rows need n % 64 == 0.  At most 65535 rows with transforms,

@@ -27,7 +27,7 @@ def quantize_rows(permuted_alphabet: torch.Tensor, weights: torch.Tensor, sample
     B, length = samples.shape
     dev, dt = samples.device, permuted_alphabet.dtype
     if samples.is_cuda and dt == torch.float32 and 4 <= L <= 16:
-        # the CUDA encoder: same recurrence, ties and fp32 arithmetic, one launch per position for a batch of rows
+        # the CUDA encoder: same recurrence, ties and fp32 arithmetic, whole rows in one launch
         return ops.viterbi_encode(permuted_alphabet, weights, samples)
     rho = torch.full((B, M), float("inf"), dtype=dt, device=dev)
     rho[:, 0] = 0                                              # initial state is zero (rptc.py:57-58)

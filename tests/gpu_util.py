@@ -34,11 +34,11 @@ def lut_for_oracle(lut, code, S):
 
 # ---- tolerances derived from the kernels' arithmetic --------------------------------------------------------
 # |w|, |x| below are the Euclidean norms of a weight row and an activation row; y is the exact product.
-#  * batch 1 (HFMA2 kernels): four fp16 accumulators per 64-weight unit take eight fp16 products each, three fp16
+#  * batch 1 in the layouts of the general kernels (HFMA2; the TILED kernels keep the bound below): four fp16 accumulators per 64-weight unit take eight fp16 products each, three fp16
 #    adds join them, everything after that is fp32.  Each fp16 rounding is 2^-11 of a partial sum of at most 64
 #    terms, and the roundings of the n/64 units add in quadrature: about 4e-5 |w||x| at the worst row of a
 #    4096 x 4096 layer (0.147 absolute measured).  Bound: 1.5e-4 |w||x|.
-#  * batch >= 2 (mma.sync kernel) and the tcgen05 GEMM: fp16 products summed in fp32.  Bound: 2e-5 |w||x|.
+#  * TILED products (mma.sync for one or two rows, tcgen05 for more) and the tcgen05 GEMM: fp16 products summed in fp32.  Bound: 2e-5 |w||x|.
 #  * the fp16 rounding of the result itself: 2^-11 |y|.
 # One mis-decoded weight moves an output by |dw * x_c|, about 1 for N(0,1) weights and activations: at n = 4096 the
 # batch-1 bound is 0.6 absolute and the others 0.08, against 8.2 for the bound these tests used before.

@@ -1,10 +1,10 @@
 """GPU parity: the fused dequant-GEMV against the CPU oracle (fp64 product of bit-exact weights).
 
-Tolerance (derived in gpu_util.py from the kernels' arithmetic).  Batch 1 multiplies in fp16 pairs and adds eight
+Tolerance (derived in gpu_util.py from the kernels' arithmetic).  The general kernels multiply in fp16 pairs and add eight
 products per fp16 accumulator before widening to fp32: |y - exact| <= 1.5e-4 ||w_row|| ||x|| + 2^-11 |exact|, which is
 0.6 absolute at n = 4096 with N(0,1) data -- below the ~1 that ONE mis-decoded weight moves an output by (the
-reference's fully fp16-accumulated product, inference.cu:263,270-276, is about 200 times looser).  Batch 2-8 runs on
-mma.sync with fp32 accumulation: 2e-5 ||w_row|| ||x||.  Wrong weights are hunted exactly, column by column, in
+reference's fully fp16-accumulated product, inference.cu:263,270-276, is about 200 times looser).  The TILED
+layout's products are summed in fp32 (mma.sync up to two rows, tcgen05 above): 2e-5 ||w_row|| ||x||, checked for even batches.  Wrong weights are hunted exactly, column by column, in
 test_gpu_probe.py; this file checks the arithmetic on random inputs.
 """
 import numpy as np
@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _check(y, w16, x16, rel=None, what=""):
-    """rel defaults to the bound of the kernel that serves this batch size (1: HFMA2, 2-8: mma.sync)."""
+    """rel defaults to the bound of the kernel that serves this batch size (odd: the wider one of the general kernels)."""
     if rel is None:
         rel = GEMV_HFMA2_TOL if x16.shape[0] in (1, 3, 5, 7) else GEMV_FP32_TOL      # odd batches end in a batch-1 launch
     exact = o.matvec_exact(w16, x16)
@@ -124,7 +124,7 @@ def test_gemv_full_size_linearity(m, n):
     ref = (x.double() @ dense.double().T)
     scale = dense.double().norm(dim=1)[None, :] * x.double().norm(dim=1)[:, None]
     err = (y.double() - ref).abs()
-    tol = GEMV_FP32_TOL * scale + 2.0**-11 * ref.abs() + 1e-4                        # batch 2: the mma.sync kernel
+    tol = GEMV_FP32_TOL * scale + 2.0**-11 * ref.abs() + 1e-4                        # two rows: mma.sync
     assert bool((err <= tol).all()), f"max err/tol {(err / tol).max().item():.3f}"
     # batch 1 (HFMA2 kernel) on the fp16 sum of the two rows, against the same product
     xs = (x[0] + x[1]).unsqueeze(0)

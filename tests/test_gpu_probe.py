@@ -52,7 +52,7 @@ def _decoded(codes, lut, m, n, fmt, carry_in=None):
 @pytest.mark.parametrize("m,n", BASELINE_SHAPES + [(352, 11008), (96, 2048)])
 @pytest.mark.parametrize("batch", [1, 8])
 def test_every_column_of_the_headline_code(m, n, batch):
-    """HASH S=8 K=2, TILED: batch 1 is the HFMA2 pair kernel, batch 8 the mma.sync kernel (352 and 96 rows: an odd
+    """HASH S=8 K=2, TILED: batch 1 is the lane-per-row kernel, batch 8 the one with the weights in tensor memory (352 and 96 rows: an odd
     number of 32-row blocks, the last pair has no second block)."""
     from rptc_b200 import Format, ops
     fmt = Format()
