@@ -529,7 +529,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_rows_kernel(const GemvPa
                     z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             __half *x_sm = reinterpret_cast<__half *>(smem_raw + (xs - s0));
-            for (uint32_t b = cb_first + warp; b <= cb_last; b += kGemvWarps)
+            // (a CTA without granules would start behind the last block: the layer of a narrow model has fewer granules than there are SMs)
+            for (uint32_t b = cb_first + warp; cta_n && b <= cb_last; b += kGemvWarps)
 #pragma unroll 1
                 for (int r = 0; r < BATCH; ++r)
                     swiglu_chunk(p.sw, r, (int64_t)b * 256 + 8 * lane, nullptr, false,
