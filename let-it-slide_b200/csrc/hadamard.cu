@@ -7,6 +7,9 @@
 // shared-memory exchange.  Sign flips, the 1/sqrt(block) scale and the fp16 conversion are fused in.
 #include "common.cuh"
 #include "fwht.cuh"
+#include "matmul.cuh"
+
+#include <type_traits>
 
 namespace rptc {
 
@@ -26,10 +29,16 @@ struct HadParams {
     int64_t clear_count;        // a multiple of 4
     int32_t late;               // the next kernel may start behind this one's wait only
 };
+struct HadSumsParams : HadParams {
+    GemvSums sums;              // the input is a product's sums, to be added up
+};
 
-__global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
+template <bool SUMS>
+__global__ void __launch_bounds__(512) hadamard_kernel(const std::conditional_t<SUMS, HadSumsParams, HadParams> p) {
     __shared__ __align__(16) float ex[4096];
     if (!p.late) pdl_allow_next_grid();
+    int n_sums = 0;
+    if constexpr (SUMS) n_sums = p.sums.count((uint32_t)(blockIdx.x * p.chunk + 8 * threadIdx.x), blockIdx.y);      // eight columns lie in one tile
     pdl_wait_prior_grids();
     if (p.late) pdl_allow_next_grid();
     const int t = threadIdx.x;
@@ -43,8 +52,24 @@ __global__ void __launch_bounds__(512) hadamard_kernel(const HadParams p) {
     const int64_t col = (int64_t)blockIdx.x * p.chunk + 8 * t;
     if (col >= p.n) return;     // only with blocks <= 256 (whole warps leave; such blocks need no CTA barrier)
     float v[8];
-    if (p.in_is_f32) load8_f32(const_cast<float *>(static_cast<const float *>(p.in)) + row * p.ld_in + col, v, p.clear_in != 0);
-    else load8_f16(static_cast<const __half *>(p.in) + row * p.ld_in + col, v);
+    if constexpr (SUMS) {
+        constexpr int kAhead = 4;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = 0.f;
+        const float *src = static_cast<const float *>(p.in) + row * p.ld_in + col;
+        for (int s = 0; s < n_sums; s += kAhead, src += kAhead * p.sums.plane) {
+            float w[kAhead][8] = {};
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                if (s + k < n_sums) load8_f32_cg(src + k * p.sums.plane, w[k]);
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] += w[k][i];
+        }
+    } else if (p.in_is_f32) {
+        load8_f32(const_cast<float *>(static_cast<const float *>(p.in)) + row * p.ld_in + col, v, p.clear_in != 0);
+    } else load8_f16(static_cast<const __half *>(p.in) + row * p.ld_in + col, v);
     float sg[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) sg[i] = 1.f;
@@ -222,11 +247,29 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
         // small blocks: a warp per 256 columns, eight warps per CTA, so that many-row inputs do not become
         // hundreds of thousands of one-warp CTAs
         p.chunk = 2048;
-        return launch(hadamard_kernel, dim3((unsigned)((n + 2047) / 2048), (unsigned)rows), dim3(256), 0,
-                      stream, p);
+        return launch(hadamard_kernel<false>, dim3((unsigned)((n + 2047) / 2048), (unsigned)rows), dim3(256), 0, stream, p);
     }
-    return launch(hadamard_kernel, dim3((unsigned)(n / chunk), (unsigned)rows), dim3(chunk / 8), 0,
-                  stream, p);
+    return launch(hadamard_kernel<false>, dim3((unsigned)(n / chunk), (unsigned)rows), dim3(chunk / 8), 0, stream, p);
+}
+
+int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
+                     int block, float scale, cudaStream_t stream) {
+    if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
+    const int chunk = block < 256 ? 256 : block;
+    if (n % chunk) return RPTC_ERR_SHAPE;
+    HadSumsParams p = {};
+    p.in = partial;
+    p.ld_in = ld;
+    p.out = static_cast<__half *>(out);
+    p.ld_out = ld_out;
+    p.signs = static_cast<const __half *>(signs);
+    p.block = block;
+    p.chunk = block <= 256 && n > 256 ? 2048 : chunk;
+    p.transpose = 1;
+    p.scale = scale * hadamard_norm(block);
+    p.n = n;
+    p.sums = sums;
+    return launch(hadamard_kernel<true>, dim3((unsigned)((n + p.chunk - 1) / p.chunk), (unsigned)rows), dim3(p.chunk / 8), 0, stream, p);
 }
 }  // namespace rptc
 

@@ -10,6 +10,9 @@
 #include "common.cuh"
 #include "matmul.cuh"
 
+#include <math.h>
+#include <type_traits>
+
 namespace rptc {
 
 int check_format(const rptc_format *f);   // api.cu
@@ -18,6 +21,9 @@ int check_format(const rptc_format *f);   // api.cu
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late = false);
+// out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]
+int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
+                     int block, float scale, cudaStream_t stream);
 
 // Programmatic dependent launch within a call, whatever the calling thread's setting.  The products read codes and tables before they
 // wait for the kernel in front.  They must not do so while an earlier kernel of the stream still writes a layer's buffers, so nothing
@@ -98,22 +104,39 @@ __global__ void __launch_bounds__(kPackedThreads) packed_input_kernel(const T *_
 }
 
 // y[token][row] from the product's fp32 accumulator (`acc`) or fp16 result (`prod`), whose columns are banks of
-// `bank_cols` of which the first `bank_rows` hold rows of the layer.
-template <typename T>
+// `bank_cols` of which the first `bank_rows` hold rows of the layer.  SUMS: the accumulator is to be added up first.
+template <typename T, bool SUMS>
 __global__ void __launch_bounds__(256) packed_output_kernel(const float *__restrict__ acc, const __half *__restrict__ prod, int64_t ld,
                                                             const float2 *__restrict__ sums, const float *__restrict__ scales_out,
                                                             const float *__restrict__ biases_out, const float *__restrict__ bias,
-                                                            T *__restrict__ y, int m, int bank_rows, int bank_cols) {
+                                                            T *__restrict__ y, int m, int bank_rows, int bank_cols, const GemvSums parts) {
     pdl_allow_next_grid();
     const int row = blockIdx.x * 256 + threadIdx.x;
     const int64_t token = blockIdx.y;
     float so = 0.f, bo = 0.f, bb = 0.f;
     if (row < m) so = __ldg(scales_out + row), bo = __ldg(biases_out + row), bb = bias ? __ldg(bias + row) : 0.f;
+    const int n_parts = SUMS ? parts.count((uint32_t)(row % bank_rows), (uint32_t)token) : 1;
     pdl_wait_prior_grids();
     if (row >= m) return;
     const int bank = row / bank_rows, col = bank * bank_cols + row - bank * bank_rows;
-    const float2 s = sums[token];
-    const float v = acc ? acc[token * ld + col] : __half2float(prod[token * ld + col]);
+    float v;
+    float2 s;
+    if (SUMS) {
+        constexpr int kAhead = 4;                    // loads under way at a time
+        const float *src = acc + token * ld + col;
+        s = __ldcg(sums + token);
+        v = 0.f;
+        for (int i = 0; i < n_parts; i += kAhead) {
+            float w[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) w[k] = i + k < n_parts ? __ldcg(src + (i + k) * parts.plane) : 0.f;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) v += w[k];
+        }
+    } else {
+        s = sums[token];
+        v = acc ? acc[token * ld + col] : __half2float(prod[token * ld + col]);
+    }
     y[token * m + row] = from_float<T>(v * so + s.x * bo + s.y + bb);
 }
 
@@ -125,6 +148,11 @@ static Banks packed_banks(const rptc_packed &l) {
     return banks;
 }
 
+// One or two tokens: no kernel in front of the product.
+static bool packed_alone(const rptc_packed &l, int64_t tokens) {
+    return gemv_alone_takes((int64_t)l.bank_blocks * 32, l.n, tokens, 0, packed_banks(l), packed_format(l));
+}
+
 template <typename T>
 static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t tokens, char *ws, bool few, int64_t cols, cudaStream_t s) {
     PdlScope pdl(true);
@@ -134,6 +162,22 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
     float2 *sums = reinterpret_cast<float2 *>(ws);
     __half *xs = reinterpret_cast<__half *>(ws + round_up(tokens * 8));
     char *prod = reinterpret_cast<char *>(xs) + round_up(tokens * l.n * 2);
+    auto output = [&](const float *acc, const GemvSums &parts) {
+        return launch(parts.per ? packed_output_kernel<T, true> : packed_output_kernel<T, false>, dim3((unsigned)((l.m + 255) / 256), (unsigned)tokens), dim3(256),
+                      0, s, acc, acc ? nullptr : reinterpret_cast<const __half *>(prod), ld, sums, l.scales_out, l.biases_out, l.bias, static_cast<T *>(y),
+                      (int)l.m, (int)(l.m / l.banks), (int)cols, parts);
+    };
+    if (packed_alone(l, tokens)) {
+        GemvInput in = {};
+        in.x = x;
+        in.dtype = std::is_same<T, __half>::value ? 0 : std::is_same<T, float>::value ? 2 : 1;
+        in.scales_in = l.scales_in;
+        in.biases_in = l.biases_in;
+        in.sums = sums;
+        GemvSums parts;
+        if (int e = gemv_alone(l.codes, l.alphabets, nullptr, in, reinterpret_cast<float *>(prod), stored, l.n, tokens, banks, f, s, &parts)) return e;
+        return output(reinterpret_cast<const float *>(prod), parts);
+    }
     float *partial = few && partials(stored, l.n, tokens, banks, f) ? reinterpret_cast<float *>(prod + round_up(tokens * ld * 4)) : nullptr;
     if (int e = launch(packed_input_kernel<T>, dim3((unsigned)tokens), dim3(kPackedThreads), 0, s, static_cast<const T *>(x), l.scales_in, l.biases_in,
                        xs, sums, few && !partial ? reinterpret_cast<float *>(prod) : nullptr, ld, (int)l.n))
@@ -141,9 +185,7 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
     const int e = few ? gemv_banked(l.codes, l.alphabets, xs, l.n, reinterpret_cast<float *>(prod), ld, stored, l.n, tokens, banks, f, s, tokens >= kOrderedRows, partial)
                       : gemm_banked(l.codes, l.alphabets, nullptr, xs, l.n, prod, ld, stored, l.n, tokens, banks, f, s);
     if (e) return e;
-    return launch(packed_output_kernel<T>, dim3((unsigned)((l.m + 255) / 256), (unsigned)tokens), dim3(256), 0, s,
-                  few ? reinterpret_cast<const float *>(prod) : nullptr, few ? nullptr : reinterpret_cast<const __half *>(prod), ld, sums, l.scales_out,
-                  l.biases_out, l.bias, static_cast<T *>(y), (int)l.m, (int)(l.m / l.banks), (int)cols);
+    return output(few ? reinterpret_cast<const float *>(prod) : nullptr, GemvSums{});
 }
 
 // Which product a packed layer takes, and how many columns it gives per bank.
@@ -173,6 +215,8 @@ extern "C" int64_t rptc_packed_workspace_bytes(const rptc_packed *l, int64_t tok
     if (check_packed(l, tokens)) return -1;
     int64_t cols;
     const bool few = packed_plan(*l, tokens, cols);
+    if (packed_alone(*l, tokens))
+        return round_up(tokens * 8) + round_up(tokens * l->n * 2) + 4 * gemv_alone_partials((int64_t)l->bank_blocks * 32, l->n, tokens, packed_banks(*l), packed_format(*l));
     const int64_t partial = few ? partials((int64_t)l->bank_blocks * 32, l->n, tokens, packed_banks(*l), packed_format(*l)) : 0;
     return round_up(tokens * 8) + round_up(tokens * l->n * 2) + round_up(tokens * l->banks * cols * (few ? 4 : 2)) + partial * 4;
 }
@@ -209,8 +253,14 @@ static bool linear_few(const rptc_linear &l, int64_t rows) {
     return rows <= 2 || gemv_few_takes(l.m, l.n, rows, Banks(), l.fmt, nullptr, l.n) || (rows <= 64 && l.n % 64);
 }
 
+// A single row: no kernel in front of the product.
+static bool linear_alone(const rptc_linear &l, int64_t rows) {
+    return l.signs_in && rows == 1 && gemv_alone_takes(l.m, l.n, rows, l.block_in, Banks(), l.fmt);
+}
+
 extern "C" int64_t rptc_linear_workspace_bytes(const rptc_linear *l, int64_t rows) {
     if (!l || rows <= 0) return -1;
+    if (linear_alone(*l, rows)) return 4 * gemv_alone_partials(l->m, l->n, rows, Banks(), l->fmt);
     const int64_t xt = l->signs_in ? round_up(rows * l->n * 2) : 0;
     return xt + (linear_few(*l, rows) ? round_up(rows * l->m * 4) + 4 * partials(l->m, l->n, rows, Banks(), l->fmt) : 0);
 }
@@ -237,6 +287,19 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
     const int64_t m = l->m, n = l->n;
+    if (linear_alone(*l, rows)) {
+        if (misaligned(l->signs_in) || misaligned(l->signs_out)) return RPTC_ERR_ALIGN;
+        pdl.set(true);
+        GemvInput in = {};
+        in.x = x;
+        in.signs = static_cast<const __half *>(l->signs_in);
+        in.block = l->block_in;
+        in.norm = 1.f / sqrtf((float)l->block_in);
+        GemvSums sums;
+        float *partial = static_cast<float *>(workspace);
+        if (int e = gemv_alone(l->codes, l->lut, l->carry_in, in, partial, m, n, rows, Banks(), l->fmt, s, &sums)) return e;
+        return hadamard_of_sums(partial, m, sums, y, m, l->signs_out, rows, m, l->block_out, l->scale, s);
+    }
     const void *xt = x;
     float *acc = few ? reinterpret_cast<float *>(ws + (l->signs_in ? round_up(rows * n * 2) : 0)) : nullptr;
     float *partial = few && partials(m, n, rows, Banks(), l->fmt) ? acc + round_up(rows * m * 4) / 4 : nullptr;

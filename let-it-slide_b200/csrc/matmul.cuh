@@ -37,4 +37,43 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
                 const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr);
 
+// ---- one or two activation rows, as the first kernel of a layer's call (gemv.cu) ----
+// The input side that the product makes in its CTAs.
+struct GemvInput {
+    const void *x;                       // [batch][n]: fp16, or with scales_in fp16, bf16, fp32 (dtype 0, 1, 2)
+    const float *scales_in, *biases_in;  // fp32 [n]: x * scales_in goes in, and sums[row] = (sum of x, <biases_in, x>) comes out
+    float2 *sums;
+    const __half *signs;                 // [n]: H(signs * x) * norm over blocks of `block` goes in
+    int32_t dtype, block;
+    float norm;
+};
+// Where a product's sums are: a value's as many as there are CTAs that meet in its tile, `plane` values apart, in order.  The tiles' granules
+// (steps along the rows), laid end to end, are cut into ranges of equal weight.  gemv_alone: a tile is a pair of 32-row blocks, a granule
+// of which counts two, that of an odd last block one.  gemv_few: tiles of rows x tokens, all granules count one.
+struct GemvSums {
+    int64_t plane;
+    uint32_t per, extra;                 // weight of a CTA's range, and how many CTAs have one more
+    uint32_t paired, units;              // how many granules count two; granules of a tile
+    int32_t tile_rows, token_tiles, n_cols;      // tiles of the same rows, n_cols tokens each
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t begin(uint32_t cta) const { return cta * per + min(cta, extra); }
+    __device__ __forceinline__ uint32_t weight(uint32_t granule) const { return granule + min(granule, paired); }
+    __device__ __forceinline__ uint32_t granule_at(uint32_t w) const { return w >= 2 * paired ? w - paired : (w + 1) >> 1; }
+    __device__ __forceinline__ uint32_t cta_of(uint32_t w) const {
+        return w < extra * (per + 1) ? w / (per + 1) : extra + (w - extra * (per + 1)) / per;
+    }
+    // how many there are of a bank's row and a token
+    __device__ __forceinline__ int count(uint32_t row, uint32_t token) const {
+        const uint32_t g = (row / (uint32_t)tile_rows * (uint32_t)token_tiles + (token_tiles > 1 ? token / (uint32_t)n_cols : 0u)) * units;
+        return (int)(cta_of(weight(g + units - 1)) - cta_of(weight(g))) + 1;
+    }
+#endif
+};
+// Whether gemv_alone takes the layer (`block`: of the Hadamard transform, 0 with scales_in), and the fp32 values of room for its sums.
+bool gemv_alone_takes(int64_t m, int64_t n, int64_t rows, int block, const Banks &banks, const rptc_format &f);
+int64_t gemv_alone_partials(int64_t m, int64_t n, int64_t rows, const Banks &banks, const rptc_format &f);
+// partial[slot][row of x][bank * m + row] for slot < sums.count(row)
+int gemv_alone(const void *codes, const void *lut, const uint32_t *carry_in, const GemvInput &in, float *partial, int64_t m, int64_t n, int64_t rows,
+               const Banks &banks, const rptc_format &f, cudaStream_t stream, GemvSums *sums);
+
 }  // namespace rptc

@@ -183,3 +183,22 @@ def test_gemv_of_layouts_with_a_row_together(code, K, L, S, layout, m, n):
     ops.device_status()
     check_product(y.float().cpu().numpy(), (x.double() @ dense.t()).cpu().numpy(), dense.norm(dim=1).cpu().numpy(), x.double().norm(dim=1).cpu().numpy(),
                   GEMV_HFMA2_TOL * (4096 / min(n, 4096)) ** 0.5)
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 2, 16, 8), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("m,n", [(256, 256), (512, 1536), (1280, 2304), (4096, 4096), (768, 3072), (22016, 1024), (9984, 2048), (1024, 5120)])
+def test_layer_of_one_row(code, K, L, S, m, n):
+    """The product makes the input transform (blocks of 256 to 4096, spans that the row ends inside) and puts down sums that the output
+    transform adds up: few and many CTAs in a row block; the last size has a kernel in front.  Activations and results are rounded to fp16,
+    2^-11 of each value at most."""
+    from rptc_b200 import Format, ops
+    from rptc_b200.linear import RPTCLinear
+    layer = RPTCLinear.random(n, m, Format(code, K, L, S, o.LAYOUT_TILED), 0.02, m + n)
+    g = torch.Generator(device="cuda").manual_seed(m * 3 + n)
+    x = torch.randn(1, n, generator=g, device="cuda").half()
+    y = layer(x)
+    want = x.double() @ layer.effective_weight().double().t()
+    assert (y.double() - want).norm() <= 2.0**-10 * want.norm()
+    for _ in range(5 if n <= 4096 else 0):                     # sums in a fixed order
+        assert torch.equal(layer(x), y)
+    ops.device_status()

@@ -207,3 +207,24 @@ def test_packed_layers_of_nine_tokens_and_more_repeat_themselves(m, n, banks, L,
     want = ((x * layer.scales_in).half().double() @ layer.decoded().double().t()) * layer.scales_out.double() \
         + x.double().sum(1, keepdim=True) * layer.biases_out.double() + (x.double() @ layer.biases_in.double())[:, None]
     assert (first.double() - want).norm() <= 6e-4 * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,n,banks,L,tokens", [(24, 64, 1, 8, 1), (96, 1024, 1, 16, 2), (11008, 4096, 32, 16, 1), (1376, 2112, 4, 16, 2), (480, 9216, 4, 12, 1),
+                                                (320, 11008, 8, 16, 2), (8192, 128, 16, 14, 1)])
+def test_packed_layer_of_one_or_two_tokens(m, n, banks, L, tokens, dtype):
+    """The product scales the input itself; banks of one block of rows, odd numbers of them, many CTAs in one, rows too short for two runs a
+    warp, two rows of activations that do not fit beside the table."""
+    import quantize_hf as q
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    symbols = torch.randint(0, 4, (m, n), generator=g, device="cuda", dtype=torch.int32)
+    layer = q.FactorizedRPTCLinear.from_parts(symbols, rnd(banks, 1 << L), 0.1 * rnd(m), 0.1 * rnd(n), 0.5 + rnd(m).abs(), 0.5 + rnd(n).abs(), rnd(m))
+    x = rnd(tokens, n).to(dtype)
+    xs = (x.float() * layer.scales_in).half()
+    want = (xs.double() @ layer.decoded().double().t()) * layer.scales_out.double() + x.double().sum(1, keepdim=True) * layer.biases_out.double() \
+        + (x.double() @ layer.biases_in.double())[:, None] + layer.bias.double()
+    got = layer(x)
+    assert got.dtype == dtype
+    assert (got.double() - want).norm() <= (4e-3 if dtype == torch.bfloat16 else 6e-4) * want.norm()
