@@ -1,5 +1,6 @@
 // Host-side plumbing of the C ABI: status strings, device checks, the device status word.
 #include "common.cuh"
+#include "matmul.cuh"
 
 namespace rptc {
 
@@ -171,9 +172,62 @@ extern "C" int rptc_timer_end(float *ms, rptc_stream_t stream) {
     return RPTC_OK;
 }
 
+// ---- a matvec whose caller waits for it ----
+namespace rptc {
+// A thread's timer on a device; kept, and given back when the thread ends.
+struct WaitedTimer {
+    HostTime *host = nullptr;
+    DeviceTime *device = nullptr;
+    unsigned int ticket = 0;
+    ~WaitedTimer() { release(); }
+    void release() {
+        if (device) cudaFree(device);      // waits for a kernel that may still write
+        if (host) cudaFreeHost(host);
+        device = nullptr, host = nullptr;
+    }
+    int ready() {
+        if (device) return RPTC_OK;
+        const DeviceTime none = {~0ull, 0u};
+        RPTC_CUDA(cudaHostAlloc(&host, sizeof(HostTime), cudaHostAllocMapped));
+        host->ticket = ticket;
+        DeviceTime *d = nullptr;
+        RPTC_CUDA(cudaMalloc(&d, sizeof(DeviceTime)));
+        device = d;
+        RPTC_CUDA(cudaMemcpy(device, &none, sizeof(none), cudaMemcpyHostToDevice));
+        return RPTC_OK;
+    }
+};
+static thread_local WaitedTimer g_waited[kMaxDevices];
+// Until the kernel with `ticket` has left its time.  The stream is asked now and then: work that failed leaves none.
+static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
+    volatile HostTime *h = t.host;
+    for (unsigned int spin = 1;; ++spin) {
+        if (h->ticket == t.ticket) break;
+        if (spin % 4096) continue;
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e == cudaSuccess && h->ticket == t.ticket) break;
+        t.release();
+        return e == cudaSuccess ? RPTC_ERR_TIMEOUT : cuda_fail(e);      // the kernel gave up, or the stream failed
+    }
+    __atomic_thread_fence(__ATOMIC_ACQUIRE);
+    *ms = (float)((double)h->ns * 1e-6);
+    return RPTC_OK;
+}
+}  // namespace rptc
+
 extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x, float *acc, void *y, int64_t m, int64_t n, int x_order,
                                int accumulate, const rptc_format *fmt, float *ms, rptc_stream_t stream) {
     if (!y || !ms) return RPTC_ERR_ARG;
+    if (int e = validate_gemv_args(codes, lut, x, n, acc, m, m, n, 1, x_order, fmt)) return e;
+    if (int e = rptc_check_device()) return e;
+    const int dev = current_device();
+    if (dev < 0) return cuda_fail(cudaErrorNoDevice);
+    if (int e = g_waited[dev].ready()) return e;
+    WaitedTimer &t = g_waited[dev];
+    const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
+    if (e == RPTC_OK) return wait_for(t, static_cast<cudaStream_t>(stream), ms);
+    if (e != RPTC_ERR_UNSUPPORTED) return e;
     if (int e = rptc_timer_begin(stream)) return e;
     if (int e = rptc_gemv(codes, lut, nullptr, x, n, acc, m, m, n, 1, x_order, fmt, stream)) return e;
     {

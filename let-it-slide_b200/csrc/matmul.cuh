@@ -76,4 +76,46 @@ int64_t gemv_alone_partials(int64_t m, int64_t n, int64_t rows, const Banks &ban
 int gemv_alone(const void *codes, const void *lut, const uint32_t *carry_in, const GemvInput &in, float *partial, int64_t m, int64_t n, int64_t rows,
                const Banks &banks, const rptc_format &f, cudaStream_t stream, GemvSums *sums);
 
+// ---- a matvec whose caller waits for it ----
+// The device time of a kernel, left in host memory by the last of its CTAs together with `ticket`, which tells the waiting thread that
+// the kernel's results are there.
+struct HostTime {
+    unsigned long long ns;
+    unsigned int ticket;
+};
+struct DeviceTime {
+    unsigned long long begin;            // earliest start; all ones between kernels
+    unsigned int ended;                  // CTAs that have; 0 between kernels
+};
+struct DeviceTimer {
+    DeviceTime *device;
+    HostTime *host;                      // pinned, as the device sees it
+    unsigned int ticket;
+#ifdef __CUDACC__
+    static __device__ __forceinline__ unsigned long long now() {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)::"memory");
+        return t;
+    }
+    __device__ __forceinline__ void begin() const { atomicMin(&device->begin, now()); }
+    // by one thread of each of `ctas` CTAs, behind a barrier behind its last result
+    __device__ __forceinline__ void end(unsigned int ctas) const {
+        __threadfence();
+        if (atomicAdd(&device->ended, 1u) + 1u != ctas) return;
+        __threadfence();
+        const unsigned long long from = atomicExch(&device->begin, ~0ull);
+        device->ended = 0u;
+        *reinterpret_cast<volatile unsigned long long *>(&host->ns) = now() - from;
+        __threadfence_system();
+        *reinterpret_cast<volatile unsigned int *>(&host->ticket) = ticket;
+    }
+#endif
+};
+int validate_gemv_args(const void *codes, const void *lut, const void *x, int64_t ld_x, const float *acc, int64_t ld_acc, int64_t m, int64_t n, int batch,
+                       int x_order, const rptc_format *fmt);
+// y = (or +=) W x, one row, codes whose units of a row lie together (ROWMAJOR, CHUNKED); RPTC_ERR_UNSUPPORTED, and nothing is launched, for others
+// and for rows that do not fit into shared memory.  The arguments have been checked.
+int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64_t m, int64_t n, int x_order, int accumulate, const rptc_format &f,
+               const DeviceTimer &timer, cudaStream_t stream);
+
 }  // namespace rptc

@@ -202,3 +202,34 @@ def test_layer_of_one_row(code, K, L, S, m, n):
     for _ in range(5 if n <= 4096 else 0):                     # sums in a fixed order
         assert torch.equal(layer(x), y)
     ops.device_status()
+
+
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_B, 2, 16, 6), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 4, 16, 8)])
+@pytest.mark.parametrize("layout,x_order,quirk", [(o.LAYOUT_ROWMAJOR, 0, 0), (o.LAYOUT_CHUNKED, 0, 0), (o.LAYOUT_CHUNKED, 1, o.QUIRK_K2_LANE0_CARRY)])
+@pytest.mark.parametrize("m,n", [(32, 2048), (32, 16384), (160, 6144), (1056, 8192), (4128, 4096), (22016, 2048), (64, 51200)])
+def test_timed_matvec_stores_and_adds(code, K, L, S, layout, x_order, quirk, m, n):
+    """rptc_gemv_timed: a warp and several per row, one and many rows a warp, the last size beyond shared memory (a kernel and one behind it).
+    The same product as rptc_gemv's, a store and an addition in fp16, a positive time."""
+    from rptc_b200 import Format, ops
+    from rptc_b200._lib import native
+    if quirk and K != 2 or layout == o.LAYOUT_CHUNKED and (n * K // 128) % 32:
+        pytest.skip("not defined")
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    fmt = Format(code, K, L, S, layout, quirk)
+    codes = torch.randint(-2**31, 2**31 - 1, (m * n * K // 32,), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    x = torch.randn(n, dtype=torch.float16, device="cuda", generator=g)
+    acc = torch.zeros((1, m), device="cuda")
+    ops.gemv_acc(codes, lut, x, acc, m, n, fmt, x_order=x_order)
+    want = acc[0].clone()
+    acc.zero_()
+    y = torch.full((m,), 7.0, dtype=torch.float16, device="cuda")
+    assert native().gemv_timed(codes, lut, x, acc, y, m, n, x_order, 0, fmt) > 0
+    # the same fp16 products, summed in another order in fp32, then one rounding
+    scale = want.abs().max().item()
+    assert (y.float() - want).abs().max().item() <= 2e-5 * scale * 16 + 2.0**-11 * scale
+    first = y.clone()
+    assert native().gemv_timed(codes, lut, x, acc, y, m, n, x_order, 1, fmt) > 0
+    assert (y.float() - 2 * first.float()).abs().max().item() <= (2e-5 * 16 + 2.0**-9) * scale
+    assert not acc.any()
+    ops.device_status()
