@@ -10,12 +10,15 @@
 // row is ONE piece of work of a persistent launch instead of one launch per position.  A thread owns G groups of four
 // consecutive p', so a group needs four values of best and gives four, and its 16 alphabet entries, which no position
 // changes, stay in registers.  At L = 16 the 65,536 entries are as large as a register file, so a cluster of two CTAs
-// shares a row: each CTA makes half of the p' and sends the half of its results that its partner reads by one bulk copy.  Two rows alternate in a CTA there, so that a row's values travel under the other's work.
+// shares a row: each CTA makes half of the p' and sends the half of its results that its partner reads by bulk copies.  Two rows
+// alternate in a CTA there, so that a row's values travel under the other's work.
 // Bound: instruction issue (four unfused operations per state and the minima; pairs of fp32 values take half the issue
-// slots for the former).  1024 x 1024 samples, L = 16: 603 ms with one launch per position and batch of eight rows and
-// the costs in L2; 23.1 ms with cluster barriers between positions (their release waits for the winners' stores); 30.8 ms
-// with st.async into the partner; 16.3 ms as it is (issue slots 76 % used).  L = 15: 7.2 ms.
-// The winners d leave as two bits each, four to a byte, and a warp per row walks them backwards (rptc.py:62-68), three
+// slots for the former), then, at L = 16, the exchange.  1024 x 1024 samples, L = 16: 603 ms with one launch per position and batch of eight
+// rows and the costs in L2; 23.1 ms with cluster barriers between positions (their release waits for the winners' stores); 30.8 ms
+// with st.async into the partner; 16.5 ms with two groups a thread and 1024 threads, the last warp sending; 15.3 ms with four groups a
+// thread, whose steps' fixed part (a fifth of 211 instructions per 32 states) counts half (13.4 ms without
+// winners).
+// The winners d leave as two bits each, four to a byte; and a warp per row walks them backwards (rptc.py:62-68), three
 // positions per trip to memory.
 // The arithmetic is spelled with round-to-nearest instructions so that no multiply-add is contracted: costs, and
 // therefore ties and paths, are those of the fp32 reference.
@@ -69,7 +72,7 @@ __device__ __forceinline__ unsigned long long cost_key(float v, uint32_t state) 
 
 // CL CTAs share a row, a thread owns G groups of four prefixes, R rows alternate in a CTA.
 template <int CL, int G, int R>
-__global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiParams p) {
+__global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel(const ViterbiParams p) {
     extern __shared__ __align__(128) float best_sm[];           // per row and buffer: P / CL values, and with CL == 2 half as many to send
     __shared__ unsigned long long red[33];
     __shared__ __align__(8) unsigned long long full_bar[R][2];  // CL == 2
@@ -86,11 +89,16 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
     // Where this thread's 4 G results go: prefix i = 4 k is read as best[d Q + k'] with d = i / Q, k' = i % Q, by the CTA
     // that owns group k'.  4 G results never straddle two readers (CL == 2 has QC = 2048).  What the partner reads is
     // put down behind this CTA's own values, in the order in which the partner holds it (quarters 2 rank, 2 rank + 1).
-    uint32_t out_off = 16u * (uint32_t)k;
+    uint32_t out_off = 16u * (uint32_t)k;                       // 16-byte piece k
     if (CL == 2) {
         const int d = 4 * k / Q, o = 4 * k - d * Q, reader = o / QC;
         out_off = 4u * (uint32_t)((reader == (int)rank ? d * QC : PC + (d - 2 * (int)rank) * QC) + o - reader * QC);
     }
+    // Pieces of 16 bytes change places within groups of G, piece c is at c ^ (c >> 3 & (G - 1)): a thread stores G of them side by side, and
+    // eight lanes that store theirs at once meet all banks.  (Of 42 wavefronts per warp and step 8 were such conflicts with G = 2.)
+    constexpr uint32_t kSwap = G - 1;                           // these bits of a piece are bits of kk: QC is 64 at least, with G == 4 128
+    const uint32_t swap = ((uint32_t)k >> 3) & kSwap;           // of piece k
+    const int load_at = kk ^ (int)(4u * (((uint32_t)kk >> 5) & kSwap));      // float kk is in piece kk / 4
     const uint32_t s0 = smem_addr(best_sm);
     // CL == 2, per row: `full` of a buffer completes when this CTA's warps have all put down their values of a position
     // and the partner's half has landed.  The warp that finishes a position last sends this CTA's half.  So a completed
@@ -159,10 +167,13 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
 
         // the four predecessors' values of this thread's groups
         auto load_best = [&](int r, int cur, float (&b)[4][G]) {
-            const float *src = best_sm + (2 * r + cur) * slab + kk;
+            const float *src = best_sm + (2 * r + cur) * slab + load_at;
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
-                if (G == 2) {
+                if (G == 4) {
+                    const float4 v = *reinterpret_cast<const float4 *>(src + d * QC);
+                    b[d][0] = v.x, b[d][1 % G] = v.y, b[d][2 % G] = v.z, b[d][3 % G] = v.w;
+                } else if (G == 2) {
                     const float2 v = *reinterpret_cast<const float2 *>(src + d * QC);
                     b[d][0] = v.x, b[d][G - 1] = v.y;
                 } else {
@@ -189,7 +200,9 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
             load_best(r, cur, b);
             const f32x2 x2 = pack2(x, x), w2 = pack2(w, w);
             const uint32_t to = 4u * (uint32_t)((2 * r + nxt) * slab), dst = s0 + to + out_off;
-            float bits = 8388608.f;                             // 2^23
+            float bits[(G + 1) / 2];                            // sixteen bits each
+#pragma unroll
+            for (int i = 0; i < (G + 1) / 2; ++i) bits[i] = 8388608.f;      // 2^23
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 float m[4];
@@ -197,11 +210,11 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
                 for (int h = 0; h < 2; ++h) {
                     float lo[4], hi[4];
                     costs(b, g, h, x2, w2, lo, hi);
-                    m[2 * h] = first_min(lo[0], lo[1], lo[2], lo[3], bits, 8 * g + 4 * h);
-                    m[2 * h + 1] = first_min(hi[0], hi[1], hi[2], hi[3], bits, 8 * g + 4 * h + 2);
+                    m[2 * h] = first_min(lo[0], lo[1], lo[2], lo[3], bits[g / 2], 8 * (g % 2) + 4 * h);
+                    m[2 * h + 1] = first_min(hi[0], hi[1], hi[2], hi[3], bits[g / 2], 8 * (g % 2) + 4 * h + 2);
                 }
                 if (active)
-                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16u * g), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst ^ (16u * ((uint32_t)g ^ swap))), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
             }
             if (CL == 2) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the copy engine reads what was put down
@@ -209,7 +222,8 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
                 if ((t & 31) == 0) {
                     uint32_t before;
                     asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_addr(&warps_done[r])) : "memory");
-                    if ((before & 31u) == 31u) {                // 32 warps: this was the last one
+                    constexpr uint32_t kWarps = G == 4 ? 16 : 32;
+                    if ((before & (kWarps - 1)) == kWarps - 1) {      // this was the last one
                         const uint32_t half = 2u * (uint32_t)PC;
                         mbar_expect_tx(full0 + 8 * (2 * r + nxt), half);
                         bulk_s2s(peer_s0 + to + rank * half, s0 + to + 2u * half, half, peer_full0 + 8u * (uint32_t)(2 * r + nxt));
@@ -219,8 +233,9 @@ __global__ void __launch_bounds__(1024, 1) viterbi_forward_kernel(const ViterbiP
             }
             bp[r] += Q;
             if (active) {
-                if (G == 2) *reinterpret_cast<uint16_t *>(bp[r]) = (uint16_t)__float_as_uint(bits);
-                else *bp[r] = (uint8_t)__float_as_uint(bits);
+                if (G == 4) *reinterpret_cast<uint32_t *>(bp[r]) = __byte_perm(__float_as_uint(bits[0]), __float_as_uint(bits[(G - 1) / 2]), 0x5410);
+                else if (G == 2) *reinterpret_cast<uint16_t *>(bp[r]) = (uint16_t)__float_as_uint(bits[0]);
+                else *bp[r] = (uint8_t)__float_as_uint(bits[0]);
             }
         };
         int cur = 0;
@@ -396,17 +411,19 @@ extern "C" int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per
         p.items_per_bank = (p.rows_per_bank + r - 1) / r;
         p.n_items = p.first_items + left / p.rows_per_bank * p.items_per_bank + (left % p.rows_per_bank + r - 1) / r;
     };
-    // Threads per CTA: a quarter of 2^(L-2) prefixes in groups of four, two groups a thread from L = 10 on (below, one warp
-    // has lanes to spare).  At L = 15 and 16 one CTA of 1024 threads fills an SM; two rows then alternate in it, unless every
+    // Threads per CTA: a quarter of 2^(L-2) prefixes in groups of four, four groups a thread from L = 11 on (512 x 512 samples, L = 14, with
+    // two: 1250 us, with four 1026; 1024 x 512, L = 12: 630 and 566), two at L = 10, one below, where a warp has lanes to spare.  At
+    // L = 15 and 16 one CTA of 512 threads fills an SM; two rows then alternate in it, unless every
     // row finds a place of its own: two at a time take less than one after the other (1024 samples, L = 16, 136 rows: 2.4
-    // against 4.4 ms).  Smaller L run one row per CTA and as many CTAs as fit (64 registers a thread).
+    // against 4.4 ms).  Smaller L run one row per CTA and as many CTAs as fit (128 registers a thread).
     const int groups = 1 << (L - 4), sms = num_sms(), places = L == 16 ? sms / 2 : sms;
     const bool pairs = L >= 15 && rows > places;
     rows_at_once(pairs ? 2 : 1);
     int e;
-    if (L == 16) e = pairs ? launch_forward<2, 2, 2>(p, 1024, places, s) : launch_forward<2, 2, 1>(p, 1024, places, s);
-    else if (pairs) e = launch_forward<1, 2, 2>(p, 1024, places, s);
-    else if (L >= 10) e = launch_forward<1, 2, 1>(p, groups / 2, sms * (L == 15 ? 1 : L == 10 ? 32 : 2048 / groups), s);
+    if (L == 16) e = pairs ? launch_forward<2, 4, 2>(p, 512, places, s) : launch_forward<2, 4, 1>(p, 512, places, s);
+    else if (pairs) e = launch_forward<1, 4, 2>(p, 512, places, s);
+    else if (L >= 11) e = launch_forward<1, 4, 1>(p, groups / 4, sms * (2048 / groups), s);
+    else if (L == 10) e = launch_forward<1, 2, 1>(p, 32, sms * 32, s);
     else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
     if (e) return e;
     viterbi_backtrack_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym);
