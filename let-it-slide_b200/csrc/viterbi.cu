@@ -17,7 +17,7 @@
 // rows and the costs in L2; 23.1 ms with cluster barriers between positions (their release waits for the winners' stores); 30.8 ms
 // with st.async into the partner; 16.5 ms with two groups a thread and 1024 threads, the last warp sending; 15.3 ms with four groups a
 // thread, whose steps' fixed part (a fifth of 211 instructions per 32 states) counts half (13.4 ms without
-// winners).
+// winners); 14.1 ms with every warp sending for itself.
 // The winners d leave as two bits each, four to a byte; and a warp per row walks them backwards (rptc.py:62-68), three
 // positions per trip to memory.
 // The arithmetic is spelled with round-to-nearest instructions so that no multiply-add is contracted: costs, and
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
     extern __shared__ __align__(128) float best_sm[];           // per row and buffer: P / CL values, and with CL == 2 half as many to send
     __shared__ unsigned long long red[33];
     __shared__ __align__(8) unsigned long long full_bar[R][2];  // CL == 2
-    __shared__ uint32_t warps_done[R];
+    __shared__ __align__(16) uint32_t word_sent[2][4];          // CL == 2: what a warp with nothing to send does send, and where that lands
     const int t = threadIdx.x;
     const int M = 1 << p.L, P = M >> 2, Q = M >> 4;
     const int QC = Q / CL, PC = P / CL;                         // this CTA's share of a quarter, of all prefixes
@@ -100,22 +100,24 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
     const uint32_t swap = ((uint32_t)k >> 3) & kSwap;           // of piece k
     const int load_at = kk ^ (int)(4u * (((uint32_t)kk >> 5) & kSwap));      // float kk is in piece kk / 4
     const uint32_t s0 = smem_addr(best_sm);
-    // CL == 2, per row: `full` of a buffer completes when this CTA's warps have all put down their values of a position
-    // and the partner's half has landed.  The warp that finishes a position last sends this CTA's half.  So a completed
-    // `full` also says that both CTAs have finished with the buffer that the next results go to, and that what was sent
+    // CL == 2, per row: `full` of a buffer completes when this CTA's warps have all put down their values of a position and every warp of
+    // the partner has sent what it has: half of them 2 KiB that this CTA reads, the others sixteen bytes that nobody does.  So a
+    // completed `full` also says that both CTAs have finished with the buffer that the next results go to, and that what was sent
     // from the other buffer has arrived.  Nothing here needs a fence at cluster scope, which would wait for the winners
-    // on their way to global memory.  Once a wait has run out no other is tried: the kernel goes on to its end with
-    // what it has.
+    // on their way to global memory.  Once a wait has run
+    // out no other is tried: the kernel goes on to its end with what it has.
+    constexpr uint32_t kWarps = G == 4 ? 16 : 32, kWarpBytes = 32 * G * 16;      // warps of a CTA, what one puts down per position
     const uint32_t full0 = smem_addr(full_bar);
-    uint32_t peer_s0 = s0, peer_full0 = full0;
+    uint32_t peer_s0 = s0, peer_full0 = full0, peer_word = 0;
+    const bool sends = out_off >= 4u * (uint32_t)PC;            // of a whole warp: 32 G pieces lie with one reader
     uint32_t full_phase = 0;                                    // bit 2 r + buffer
     bool ok = true;
     if (CL == 2) {
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer_full0) : "r"(full0), "r"(rank ^ 1u));
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer_s0) : "r"(s0), "r"(rank ^ 1u));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer_word) : "r"(smem_addr(word_sent[1])), "r"(rank ^ 1u));
         if (t == 0) {
-            for (int i = 0; i < 2 * R; ++i) mbar_init(full0 + 8 * i, 1);
-            for (int i = 0; i < R; ++i) warps_done[i] = 0;
+            for (int i = 0; i < 2 * R; ++i) mbar_init(full0 + 8 * i, kWarps);
             mbar_fence_init();
         }
     }
@@ -220,14 +222,12 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the copy engine reads what was put down
                 __syncwarp();
                 if ((t & 31) == 0) {
-                    uint32_t before;
-                    asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_addr(&warps_done[r])) : "memory");
-                    constexpr uint32_t kWarps = G == 4 ? 16 : 32;
-                    if ((before & (kWarps - 1)) == kWarps - 1) {      // this was the last one
-                        const uint32_t half = 2u * (uint32_t)PC;
-                        mbar_expect_tx(full0 + 8 * (2 * r + nxt), half);
-                        bulk_s2s(peer_s0 + to + rank * half, s0 + to + 2u * half, half, peer_full0 + 8u * (uint32_t)(2 * r + nxt));
-                    }
+                    const uint32_t mine = full0 + 8 * (2 * r + nxt), theirs = peer_full0 + 8u * (uint32_t)(2 * r + nxt);
+                    if (t == 0)
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mine), "r"(kWarps / 2 * (kWarpBytes + 16u)) : "memory");
+                    else mbar_arrive(mine);
+                    if (sends) bulk_s2s(peer_s0 + to + out_off - 4u * (uint32_t)PC + rank * 2u * (uint32_t)PC, s0 + to + out_off, kWarpBytes, theirs);
+                    else bulk_s2s(peer_word, smem_addr(word_sent[0]), 16u, theirs);
                 }
                 __syncwarp();
             }
