@@ -18,8 +18,7 @@
 // with st.async into the partner; 16.5 ms with two groups a thread and 1024 threads, the last warp sending; 15.3 ms with four groups a
 // thread, whose steps' fixed part (a fifth of 211 instructions per 32 states) counts half (13.4 ms without
 // winners); 14.1 ms with every warp sending for itself.
-// The winners d leave as two bits each, four to a byte; and a warp per row walks them backwards (rptc.py:62-68), three
-// positions per trip to memory.
+// The winners d leave as two bits each, four to a byte; a second kernel walks them backwards (rptc.py:62-68).
 // The arithmetic is spelled with round-to-nearest instructions so that no multiply-add is contracted: costs, and
 // therefore ties and paths, are those of the fp32 reference.
 #include "common.cuh"
@@ -311,35 +310,72 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
     }
 }
 
-// One warp per row walks the winners from the last position to the first.  A position's winner is needed to know which
-// winner of the position before it to read, but with two bits each there are only four (sixteen) candidates one (two)
-// positions on: lanes 0, 1-4 and 5-20 fetch all of them at once, and the walk takes three positions per trip to memory.
-__global__ void __launch_bounds__(128) viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state,
-                                                                int64_t rows, int64_t n, int L, int32_t *__restrict__ symbols,
-                                                                int64_t ld_sym) {
-    const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const int64_t Q = int64_t(1) << (L - 4);
-    const uint8_t *b = back + row * n * Q;
-    const int level = lane == 0 ? 0 : lane < 5 ? 1 : 2;
-    const uint32_t d1 = level == 0 ? 0u : level == 1 ? (uint32_t)lane - 1u : (uint32_t)(lane - 5) >> 2, d2 = (uint32_t)(lane - 5) & 3u;
-    auto before = [&](uint32_t s, uint32_t d) { return (d << (L - 2)) | (s >> 2); };      // the state that reached s by winner d
-    uint32_t state = (uint32_t)final_state[row];
-    for (int64_t i = n - 1; i >= 0; i -= 3) {
-        uint32_t s = state;
-        if (level >= 1) s = before(s, d1);
-        if (level >= 2) s = before(s, d2);
-        const int64_t at = i - level;
-        uint32_t d = 0;                                         // before position 1 there is only the start state
-        if (lane < 21 && at >= 1) d = ((uint32_t)__ldg(b + at * Q + (s >> 4)) >> (2 * ((s >> 2) & 3u))) & 3u;
-        const uint32_t w0 = __shfl_sync(0xFFFFFFFFu, d, 0);
-        const uint32_t w1 = __shfl_sync(0xFFFFFFFFu, d, 1 + (int)w0);
-        const uint32_t w2 = __shfl_sync(0xFFFFFFFFu, d, 5 + 4 * (int)w0 + (int)w1);
-        const uint32_t s1 = before(state, w0), s2 = before(s1, w1);
-        const uint32_t mine = lane == 0 ? state : lane == 1 ? s1 : s2;
-        if (lane < 3 && i - lane >= 0) symbols[row * ld_sym + i - lane] = (int32_t)(mine & 3u);
-        state = before(s2, w2);
+// Walks a row's winners from position `hi` down to `lo`; returns the state at position lo - 1, and with WRITE sets the symbols on the
+// way.  A position's winner is needed to know which winner of the position before it to read, but with two bits each there are only
+// four (sixteen) candidates one (two) positions on: lanes 0, 1-4 and 5-20 fetch all of them at once, and the walk takes three
+// positions per trip to memory.
+struct TracedRow {
+    const uint8_t *back;
+    int32_t *symbols;
+    int64_t Q;
+    int L;
+    template <bool WRITE>
+    __device__ __forceinline__ uint32_t walk(uint32_t state, int64_t hi, int64_t lo) const {
+        const int lane = threadIdx.x & 31;
+        const int level = lane == 0 ? 0 : lane < 5 ? 1 : 2;
+        const uint32_t d1 = level == 0 ? 0u : level == 1 ? (uint32_t)lane - 1u : (uint32_t)(lane - 5) >> 2, d2 = (uint32_t)(lane - 5) & 3u;
+        auto before = [&](uint32_t s, uint32_t d) { return (d << (L - 2)) | (s >> 2); };      // the state that reached s by winner d
+        for (int64_t i = hi; i >= lo; i -= 3) {
+            uint32_t s = state;
+            if (level >= 1) s = before(s, d1);
+            if (level >= 2) s = before(s, d2);
+            const int64_t at = i - level;
+            uint32_t d = 0;                                     // before position 1 there is only the start state
+            if (lane < 21 && at >= 1) d = ((uint32_t)__ldg(back + at * Q + (s >> 4)) >> (2 * ((s >> 2) & 3u))) & 3u;
+            const uint32_t w0 = __shfl_sync(0xFFFFFFFFu, d, 0);
+            const uint32_t w1 = __shfl_sync(0xFFFFFFFFu, d, 1 + (int)w0);
+            const uint32_t w2 = __shfl_sync(0xFFFFFFFFu, d, 5 + 4 * (int)w0 + (int)w1);
+            const uint32_t s1 = before(state, w0), s2 = before(s1, w1);
+            if (WRITE) {
+                const uint32_t mine = lane == 0 ? state : lane == 1 ? s1 : s2;
+                if (lane < 3 && i - lane >= lo) symbols[i - lane] = (int32_t)(mine & 3u);
+            }
+            state = i - lo >= 2 ? before(s2, w2) : i == lo ? s1 : s2;
+        }
+        return state;
+    }
+};
+
+// A CTA per row, its positions in equal pieces, a warp each.  The last piece starts from the row's final state.  Which state the path
+// passes at the end of another piece is not known yet, but walks from different states meet after some times the L / 2 positions that a
+// state remembers: such a warp starts kMeet * L positions further on from any state, and writes symbols from its own piece on.  Pieces whose
+// state is not the one that the piece behind was left with are walked again from that one, all of them at once, until all fit (at
+// L = 16 most of them once).
+// Bound by the trips to memory one after the other: with a warp per row 256 rows of 1024 samples took 0.1 ms at L = 12.
+constexpr int kTraceWarps = 16, kMeet = 4;
+__global__ void __launch_bounds__(32 * kTraceWarps) viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state,
+                                                                             int64_t n, int L, int32_t *__restrict__ symbols, int64_t ld_sym,
+                                                                             int64_t piece, int pieces) {
+    __shared__ uint32_t left[kTraceWarps];                      // state in front of a piece's first position
+    const int64_t row = blockIdx.x;
+    const int c = threadIdx.x >> 5;
+    TracedRow r;
+    r.Q = int64_t(1) << (L - 4);
+    r.L = L;
+    r.back = back + row * n * r.Q;
+    r.symbols = symbols + row * ld_sym;
+    const int64_t lo = c * piece, hi = c + 1 < pieces ? lo + piece - 1 : n - 1;
+    const int64_t from = min(n - 1, hi + kMeet * L);
+    uint32_t state = from == n - 1 ? (uint32_t)final_state[row] : 0u;
+    state = r.walk<false>(state, from, hi + 1);
+    uint32_t out = r.walk<true>(state, hi, lo);
+    for (;;) {
+        if ((threadIdx.x & 31) == 0) left[c] = out;
+        __syncthreads();
+        const uint32_t want = c + 1 < pieces ? left[c + 1] : state;
+        // at the latest when the pieces have been set right one by one from the last on, all fit
+        if (!__syncthreads_or(want != state)) break;
+        if (want != state) state = want, out = r.walk<true>(state, hi, lo);
     }
 }
 
@@ -426,7 +462,14 @@ extern "C" int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per
     else if (L == 10) e = launch_forward<1, 2, 1>(p, 32, sms * 32, s);
     else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
     if (e) return e;
-    viterbi_backtrack_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym);
+    // Pieces at least as long as the way to them, and only of rows too few to keep enough loads under way by themselves: pieces walk up to
+    // twice the positions.  Encoder with a warp a row / in pieces (us): L = 9 1024 rows 359 / 308, 4096 rows 1002 / 1067; L = 12 256 rows
+    // 473 / 391, 2048 rows 3243 / 3200; L = 14 128 rows 724 / 634, 1024 rows 1615 / 1669; L = 15 512 rows 1782 / 1832; L = 16 64 rows
+    // 1605 / 1532, 256 rows 4190 / 4154, 1024 rows 14126 / 14250.
+    const bool in_pieces = rows <= (L <= 12 ? 2048 : 256);
+    const int64_t most = !in_pieces || n < kMeet * L ? 1 : n / (kMeet * L) < kTraceWarps ? n / (kMeet * L) : kTraceWarps;
+    const int64_t piece = (n + most - 1) / most, pieces = (n + piece - 1) / piece;
+    viterbi_backtrack_kernel<<<(unsigned)rows, (unsigned)(32 * pieces), 0, s>>>(p.back, p.final_state, n, L, symbols, ld_sym, piece, (int)pieces);
     RPTC_CUDA(cudaGetLastError());
     return RPTC_OK;
 }

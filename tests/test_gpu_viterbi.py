@@ -145,3 +145,26 @@ def test_encoder_of_no_rows_returns_nothing():
     import rptc
     sym, loss = rptc.quantize_rows(torch.randn(256, device="cuda"), torch.ones(5, device="cuda"), torch.empty(0, 5, device="cuda"))
     assert sym.shape == (0, 5) and sym.dtype == torch.int32 and loss.shape == (0,)
+
+
+@pytest.mark.parametrize("L,n", [(4, 33), (6, 47), (6, 48), (6, 49), (8, 700), (11, 1000), (16, 64), (16, 127), (16, 1100)])
+@pytest.mark.parametrize("parted", [False, True])
+def test_trace_back_in_pieces(L, n, parted):
+    """Pieces of a row are walked from guessed states.  `parted`: two cheap paths that stay apart for good, the states 0 and M - 1 -- the
+    guess follows the one, the cheapest path is the other, and every piece has to be walked again."""
+    import rptc
+    M = 1 << L
+    g = torch.Generator().manual_seed(L * 1000 + n)
+    weights = 0.5 + torch.rand(n, generator=g)
+    if parted:
+        alphabet = torch.full((M,), 100.0)
+        alphabet[0], alphabet[-1] = 1.0, -1.0
+        samples = torch.zeros(2, n)
+        samples[0, 0], samples[1, -1] = 1e4, -1e4             # cheapest: 0 throughout; M - 1 in the end, and so all the way to it
+    else:
+        alphabet = torch.randn(M, generator=g)
+        samples = torch.randn(2, n, generator=g)
+    want, want_loss = rptc.quantize_rows(alphabet, weights, samples)
+    got, loss = rptc.quantize_rows(alphabet.cuda(), weights.cuda(), samples.cuda())
+    assert torch.equal(got.cpu(), want)
+    torch.testing.assert_close(loss.cpu(), want_loss, rtol=1e-6, atol=0)
