@@ -353,6 +353,9 @@ int rptc_embed_mailbox(const void *table, const uint64_t *slots, uint32_t *steps
  * rptc_viterbi_encode_banked: the rows are `banks` equal groups of consecutive rows with one alphabet each,
  * alphabets fp32 [banks][2^L] (quantize_hf.py:135-150), all of them in one launch. */
 int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L);
+/* The encoder's alphabets (quantize_hf.py:136-140): out[bank][i], i < 2^L, is the quantile (2 i + 1) / 2^(L + 1) of the bank's `values` values,
+ * sorted fp32 [banks][values], by linear interpolation in double precision; out fp32 [banks][2^L], at most 65535 banks, L <= 16. */
+int rptc_quantiles(const float *sorted, int64_t banks, int64_t values, int L, float *out, rptc_stream_t stream);
 int rptc_viterbi_encode(const float *alphabet, const float *pos_weight, const float *samples, int64_t ld_samples, int64_t rows,
                         int64_t n, int L, int32_t *symbols, int64_t ld_sym, float *loss, void *workspace, int64_t workspace_bytes,
                         rptc_stream_t stream);

@@ -379,6 +379,21 @@ __global__ void __launch_bounds__(32 * kTraceWarps) viterbi_backtrack_kernel(con
     }
 }
 
+// out[bank][i] = quantile (2 i + 1) / 2^(L+1) of the bank's sorted values, linear between the neighbours on their grid (2 j + 1) / (2 N)
+// (quantize_hf.py:136-140), in double precision and unfused, as the tensor operations round that it stands for (fourteen launches).
+__global__ void __launch_bounds__(256) quantiles_kernel(const float *__restrict__ sorted, int64_t n, int L, float *__restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= int64_t(1) << L) return;
+    const double x = (double)(2 * i + 1) * 0.5 / (double)(int64_t(1) << L);
+    const double pos = __dadd_rn(__dmul_rn(x, (double)n), -0.5);
+    const double floor_pos = floor(pos);
+    const int64_t lo = floor_pos < 0.0 ? 0 : floor_pos > (double)(n - 1) ? n - 1 : (int64_t)floor_pos, hi = lo + 1 < n ? lo + 1 : n - 1;
+    const double frac = fmin(fmax(__dadd_rn(pos, -(double)lo), 0.0), 1.0);
+    const float *row = sorted + blockIdx.y * n;
+    const double a = row[lo], b = row[hi];
+    out[((int64_t)blockIdx.y << L) + i] = (float)__dadd_rn(a, __dmul_rn(__dadd_rn(b, -a), frac));
+}
+
 template <int CL, int G, int R>
 static int launch_forward(const ViterbiParams &p, int threads, int slots, cudaStream_t stream) {
     static SmemOptIn opted;
@@ -410,6 +425,16 @@ extern "C" int64_t rptc_viterbi_workspace_bytes(int64_t rows, int64_t n, int L) 
     if (rows <= 0 || n <= 0 || L < 4 || L > 16) return -1;
     const int64_t back = rows * n * (int64_t(1) << (L - 4));
     return (back + 255) / 256 * 256 + rows * 4;
+}
+
+extern "C" int rptc_quantiles(const float *sorted, int64_t banks, int64_t values, int L, float *out, rptc_stream_t stream) {
+    if (!sorted || !out) return RPTC_ERR_ARG;
+    if (L < 1 || L > 16) return RPTC_ERR_ARG;
+    if (banks <= 0 || banks > 65535 || values <= 0) return RPTC_ERR_SHAPE;
+    if (int e = rptc_check_device()) return e;
+    quantiles_kernel<<<dim3(((1u << L) + 255) / 256, (unsigned)banks), 256, 0, static_cast<cudaStream_t>(stream)>>>(sorted, values, L, out);
+    RPTC_CUDA(cudaGetLastError());
+    return RPTC_OK;
 }
 
 extern "C" int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per_bank, int64_t first_row, const float *pos_weight, const float *samples,

@@ -77,6 +77,8 @@ def megabatch_alphabets(megabatches: torch.Tensor, shift_register_size: int) -> 
     M = 1 << shift_register_size
     fp = torch.sort(megabatches, dim=1).values
     N = fp.shape[1]
+    if fp.is_cuda and fp.dtype == torch.float32 and fp.numel() and fp.shape[0] <= 65535 and 1 <= shift_register_size <= 16:
+        return ops.quantiles(fp.contiguous(), shift_register_size)
     x = (2 * torch.arange(M, dtype=torch.float64, device=fp.device) + 1) / 2 / M
     pos = x * N - 0.5                                  # position of x on the sample grid xp[j] = (2j+1)/(2N)
     lo = pos.floor().clamp(0, N - 1).to(torch.int64)

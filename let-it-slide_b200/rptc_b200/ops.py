@@ -355,6 +355,14 @@ def viterbi_encode(alphabet: torch.Tensor, pos_weight: torch.Tensor, samples: to
     return viterbi_encode_banked(alphabet[None, :], pos_weight, samples, workspace_limit)
 
 
+def quantiles(sorted_values: torch.Tensor, L: int) -> torch.Tensor:
+    """2^L evenly spaced quantiles of each row of sorted fp32 values [banks, n] -> fp32 [banks, 2^L] (rptc_quantiles)."""
+    _cuda_contig(sorted_values, "sorted_values", torch.float32)
+    out = torch.empty((sorted_values.shape[0], 1 << L), dtype=torch.float32, device=sorted_values.device)
+    call("rptc_quantiles", out.device, ptr(sorted_values), sorted_values.shape[0], sorted_values.shape[1], L, ptr(out))
+    return out
+
+
 def encoder_rows_at_once(L: int, n: int, sms: int, workspace_limit: int) -> int:
     """How many rows of n samples go through the encoder at once.  More than the kernel has in flight (one row per SM at L = 16, two
     at L = 15) only shorten the tail of the last ones, so beyond 4 GiB of survivor memory it is no more than those: 2.4 GB

@@ -228,3 +228,12 @@ def test_packed_layer_of_one_or_two_tokens(m, n, banks, L, tokens, dtype):
     got = layer(x)
     assert got.dtype == dtype
     assert (got.double() - want).norm() <= (4e-3 if dtype == torch.bfloat16 else 6e-4) * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("banks,values,L", [(1, 1, 4), (3, 7, 8), (32, 32768, 16), (5, 100003, 3), (2, 65536, 16)])
+def test_alphabets_on_the_gpu_are_those_of_the_tensor_operations(banks, values, L):
+    import quantize_hf as q
+    g = torch.Generator().manual_seed(values)
+    x = torch.randn(banks, values, generator=g)
+    assert torch.equal(q.megabatch_alphabets(x.cuda(), L).cpu(), q.megabatch_alphabets(x, L))
