@@ -403,27 +403,23 @@ static int launch_few_sums(int rb, const FewParams &p, const CUtensorMap &map, u
 struct SumParams {
     const float *partial;                            // [CTA within the tile][token][ld]
     float *acc;
-    int64_t plane, ld;
-    uint32_t per, extra, n_steps;                    // the CTAs' ranges of steps: `per`, the first `extra` one more; steps of a tile
-    int32_t columns, m, tile_rows, token_tiles, n_cols;
-    __device__ __forceinline__ uint32_t cta_of(uint32_t pos) const {
-        return pos < extra * (per + 1) ? pos / (per + 1) : extra + (pos - extra * (per + 1)) / per;
-    }
+    int64_t ld;
+    GemvSums sums;
+    int32_t columns, m;
 };
 __global__ void __launch_bounds__(128) ordered_sum_kernel(const SumParams p) {
     constexpr int kAhead = 8;
     pdl_allow_next_grid();
     const int col = 4 * (blockIdx.x * 128 + threadIdx.x), token = blockIdx.y;
-    const uint32_t from = (uint32_t)(col % p.m / p.tile_rows * p.token_tiles + token / p.n_cols) * p.n_steps;
-    const int slots = (int)(p.cta_of(from + p.n_steps - 1) - p.cta_of(from)) + 1;
+    const int slots = p.sums.count((uint32_t)(col % p.m), (uint32_t)token);
     const float *src = p.partial + (int64_t)token * p.ld + col;
     pdl_wait_prior_grids();
     if (col >= p.columns) return;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < slots; s += kAhead, src += kAhead * p.plane) {
+    for (int s = 0; s < slots; s += kAhead, src += kAhead * p.sums.plane) {
         float4 v[kAhead];
 #pragma unroll
-        for (int i = 0; i < kAhead; ++i) v[i] = s + i < slots ? __ldcg(reinterpret_cast<const float4 *>(src + i * p.plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < kAhead; ++i) v[i] = s + i < slots ? __ldcg(reinterpret_cast<const float4 *>(src + i * p.sums.plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) sum.x += v[i].x, sum.y += v[i].y, sum.z += v[i].z, sum.w += v[i].w;
     }
@@ -579,7 +575,7 @@ bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, co
 }
 
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
-             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s, bool ordered, float *partial) {
+             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s, bool ordered, float *partial, GemvSums *parts) {
     FewParams p;
     const int rb = few_choose(p, f, m, tokens, ordered);
     if (!rb) return RPTC_ERR_UNSUPPORTED;
@@ -614,19 +610,25 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
     }
     if (e || !apart) return e;
     const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps;
+    GemvSums sums = {};
+    sums.plane = tokens * ld_acc;
+    sums.per = (uint32_t)(steps / p.ctas);
+    sums.extra = (uint32_t)(steps % p.ctas);
+    sums.units = (uint32_t)p.n_steps;
+    sums.tile_rows = rb * 128;
+    sums.token_tiles = p.token_tiles;
+    sums.n_cols = p.n_cols;
+    if (parts) {
+        *parts = sums;
+        return RPTC_OK;
+    }
     SumParams q;
     q.partial = partial;
     q.acc = acc;
-    q.plane = tokens * ld_acc;
     q.ld = ld_acc;
-    q.per = (uint32_t)(steps / p.ctas);
-    q.extra = (uint32_t)(steps % p.ctas);
-    q.n_steps = (uint32_t)p.n_steps;
+    q.sums = sums;
     q.columns = (int32_t)(banks.banks * m);
     q.m = (int32_t)m;
-    q.tile_rows = rb * 128;
-    q.token_tiles = p.token_tiles;
-    q.n_cols = p.n_cols;
     return launch(ordered_sum_kernel, dim3((unsigned)((q.columns + 511) / 512), (unsigned)tokens), dim3(128), 0, s, q);
 }
 

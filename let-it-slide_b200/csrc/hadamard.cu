@@ -252,6 +252,7 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
     return launch(hadamard_kernel<false>, dim3((unsigned)(n / chunk), (unsigned)rows), dim3(chunk / 8), 0, stream, p);
 }
 
+bool hadamard_takes_sums(int64_t rows, int64_t n, int block) { return block > 256 ? rows < 32 && block < 4096 : rows <= 96 && rows * n < (int64_t(5) << 19); }
 int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
                      int block, float scale, cudaStream_t stream) {
     if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;

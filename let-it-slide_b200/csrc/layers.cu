@@ -21,7 +21,9 @@ int check_format(const rptc_format *f);   // api.cu
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late = false);
-// out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]
+// out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]; for how many rows that is as fast as adding them up in a
+// kernel in front
+bool hadamard_takes_sums(int64_t rows, int64_t n, int block);
 int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
                      int block, float scale, cudaStream_t stream);
 
@@ -182,6 +184,11 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
     if (int e = launch(packed_input_kernel<T>, dim3((unsigned)tokens), dim3(kPackedThreads), 0, s, static_cast<const T *>(x), l.scales_in, l.biases_in,
                        xs, sums, few && !partial ? reinterpret_cast<float *>(prod) : nullptr, ld, (int)l.n))
         return e;
+    if (partial && tokens <= kFewOwnTokens) {        // the output side adds them up: 896 x 704, 34 tokens 11.9 -> 9.3 us; 2048 x 2560, 235 tokens 21.8 -> 22.2
+        GemvSums parts;
+        if (int e = gemv_few(l.codes, l.alphabets, nullptr, xs, l.n, nullptr, ld, stored, l.n, tokens, banks, f, s, true, partial, &parts)) return e;
+        return output(partial, parts);
+    }
     const int e = few ? gemv_banked(l.codes, l.alphabets, xs, l.n, reinterpret_cast<float *>(prod), ld, stored, l.n, tokens, banks, f, s, tokens >= kOrderedRows, partial)
                       : gemm_banked(l.codes, l.alphabets, nullptr, xs, l.n, prod, ld, stored, l.n, tokens, banks, f, s);
     if (e) return e;
@@ -314,8 +321,12 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     if (few) {
         if (rows < kOrderedRows || !gemv_few_takes(m, n, rows, Banks(), l->fmt, xt, n)) {
             if (int e = rptc_gemv(l->codes, l->lut, l->carry_in, xt, n, acc, m, m, n, (int)rows, RPTC_XORDER_NATURAL, &l->fmt, stream)) return e;
-        } else if (int e = gemv_few(l->codes, l->lut, l->carry_in, xt, n, acc, m, m, n, rows, Banks(), l->fmt, s, true, partial)) {
-            return e;
+        } else {
+            GemvSums parts;
+            const bool added_up = partial && l->signs_out && hadamard_takes_sums(rows, m, l->block_out);
+            if (int e = gemv_few(l->codes, l->lut, l->carry_in, xt, n, acc, m, m, n, rows, Banks(), l->fmt, s, true, partial, added_up ? &parts : nullptr)) return e;
+            pdl.set(true);
+            if (added_up) return hadamard_of_sums(partial, m, parts, y, m, l->signs_out, rows, m, l->block_out, l->scale, s);
         }
         pdl.set(true);
         if (l->signs_out)

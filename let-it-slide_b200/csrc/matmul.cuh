@@ -30,8 +30,11 @@ bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, co
 // gemv_few_partials fp32 values (16-byte aligned; ld_acc a multiple of 4), and acc = instead of +=.  Where that is 0 the sums meet in acc as
 // they do without (+=, from zeros): there are two of them at most, and a + b is b + a.
 int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f);
+// With `parts` the caller adds them up: partial[slot][token][ld_acc] for slot < parts->count(row, token), nothing in acc.
+struct GemvSums;
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
-             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr);
+             int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr,
+             GemvSums *parts = nullptr);
 // The same for any number of activation rows (TILED codes, no quirk, no carry): gemv_few where it takes them, else the
 // lane-per-row kernel for one or two rows at a time.
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
