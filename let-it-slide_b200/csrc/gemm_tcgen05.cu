@@ -16,8 +16,11 @@
 //              K-major layout the tensor core reads.  After the last step the same warps run the epilogue.
 //   warp 8     one lane issues the 2-D TMA loads of the activation tile (128 tokens each), as far ahead as the
 //              activation ring allows.
-//   warp 9     owns the TMEM allocation; one lane issues tcgen05.mma (M = 128, N = NROWS, K = 16, fp32 accumulators
-//              in TMEM, one or two token halves) and commits each stage of either ring back to its producer.
+//   warp 9     owns the TMEM allocation; the whole warp waits, and an elected lane issues tcgen05.mma (M = 128, N = NROWS,
+//              K = 16, fp32 accumulators in TMEM, one or two token halves) and commits each stage back to its producer.
+//              Small tiles were bound by this one thread: a step of a 128 x 128 tile 0.48 us with a lane that waits and
+//              issues by itself (its operands are then not known to be uniform); 0.39 with one ring instead of two, one wait and one
+//              commit less; 0.36 with the elected lane, where decoding and shared memory bound it.
 // Where there are fewer tiles than SMs, a cluster of two or four CTAs shares a tile and each takes a part of the
 // reduction; the partial sums meet in fp32 through distributed shared memory (`exchange_partials`) and each CTA stores
 // its share of the tile's rows.
@@ -78,6 +81,10 @@ __device__ __forceinline__ GemmBars gemm_bars(uint32_t base) {
 
 // The HASH code is looked up in the packed table (128-byte rows) here: 32 KiB instead of 64 KiB leaves room for one more
 // ring stage, and the extra shift per lookup is hidden behind the tensor pipe.
+// Tiles of up to 128 x 128: activations and weights of a step share a stage and its barriers.  Wide ones have a ring each, the
+// activations' a deeper one (22016 x 4096, 22 tokens in tiles of 256 rows: 45.7 us, 47.5 with one ring).
+constexpr bool one_ring(int rows, int halves) { return rows <= 128 && halves == 1; }
+
 template <int CODE>
 struct GemmDecode {
     static constexpr int kCode = CODE == RPTC_CODE_HASH ? kCodeHashPacked : CODE;
@@ -150,13 +157,13 @@ __device__ __forceinline__ bool produce_weights(const GemmParams &p, uint32_t wi
 }
 
 // ---- activation loads (one thread) ----------------------------------------------------------------------------------
-template <int HALVES>
+template <int HALVES, bool ONE_RING>
 __device__ __forceinline__ bool load_activations(const GemmParams &p, uint32_t window, const GemmBars &bars, const CUtensorMap *x_map, int tok0,
                                                  int step0, int n_steps) {
     RingPos pos = {0, 1u};
     for (int it = 0; it < n_steps; ++it) {
-        if (!mbar_wait(bars.empty_x + 8 * pos.s, pos.phase, p.status)) return false;
-        const uint32_t bar = bars.full_x + 8 * pos.s;
+        if (!mbar_wait((ONE_RING ? bars.empty_w : bars.empty_x) + 8 * pos.s, pos.phase, p.status)) return false;
+        const uint32_t bar = (ONE_RING ? bars.full_w : bars.full_x) + 8 * pos.s;
         mbar_expect_tx(bar, HALVES * kXHalfBytes);
         tma_load_2d(p.xa_addr[pos.s] | window, x_map, (step0 + it) * kStepCols, tok0, bar);
         if (HALVES == 2) tma_load_2d(p.xb_addr[pos.s] | window, x_map, (step0 + it) * kStepCols, tok0 + 128, bar);
@@ -311,6 +318,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     constexpr uint32_t kTmemCols = HALVES * NROWS;       // NROWS fp32 columns per 128 tokens
     constexpr uint32_t kInstrDesc = instr_desc(NROWS);
     constexpr int kGroups = NROWS == 256 ? 1 : 2;        // producer groups taking alternate steps
+    constexpr bool kOneRing = one_ring(NROWS, HALVES);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // In a cluster every CTA's shared-memory window sits at its own place in the cluster's window: shared addresses of
@@ -334,7 +342,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int64_t tile_row = (int64_t)(blockIdx.x - bank * p.tiles_per_bank) * NROWS;
     const uint4 *codes = p.codes + (int64_t)bank * p.m * p.n_units;
 
-    if (tid == 0) init_ring_barriers(bars, 256 / kGroups);
+    if (tid == 0) init_ring_barriers(bars, NROWS + (kOneRing ? 1 : 0));
     if (warp == kMmaWarp) {                     // TMEM: fp32 accumulators of NROWS columns per 128 tokens
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars.tmem_slot), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -363,27 +371,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         ok = produce_weights<CODE, K, kGroups>(p, window, bars, codes, row < p.m ? row : p.m - 1, step0, n_steps);
     } else if (warp == kTmaWarp) {
         pdl_wait_prior_grids();
-        if (lane == 0) load_activations<HALVES>(p, window, bars, &x_map, tok0, step0, n_steps);
-    } else if (lane == 0) {
+        if (lane == 0) load_activations<HALVES, kOneRing>(p, window, bars, &x_map, tok0, step0, n_steps);
+    } else {
         // ================= MMA issue =================
         RingPos px = {0, 0u}, pw = {0, 0u};
         for (int it = 0; it < n_steps && ok; ++it) {
-            ok = mbar_wait(bars.full_x + 8 * px.s, px.phase, p.status) && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
+            ok = (kOneRing || mbar_wait(bars.full_x + 8 * px.s, px.phase, p.status)) && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t xa = p.xa_addr[px.s], xb = p.xb_addr[px.s], wa = p.w_addr[pw.s];
+            const uint64_t xa = umma_desc_sw128(p.xa_addr[px.s]), xb = umma_desc_sw128(p.xb_addr[px.s]), wd = umma_desc_sw128(p.w_addr[pw.s]);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kStepCols / 16; ++k) {
-                const uint64_t bdesc = umma_desc_sw128(wa + 32u * k);
-                tc_mma_f16(tmem_base, umma_desc_sw128(xa + 32u * k), bdesc, kInstrDesc, (it | k) != 0);
-                if (HALVES == 2) tc_mma_f16(tmem_base + (uint32_t)NROWS, umma_desc_sw128(xb + 32u * k), bdesc, kInstrDesc, (it | k) != 0);
+                for (uint32_t k = 0; k < kStepCols / 16; ++k) {           // + 32 bytes per K = 16
+                    tc_mma_f16(tmem_base, xa + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
+                    if (HALVES == 2) tc_mma_f16(tmem_base + (uint32_t)NROWS, xb + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
+                }
+                if (!kOneRing) tc_commit(bars.empty_x + 8 * px.s);      // each arrives when the MMAs above have read the stage
+                tc_commit(bars.empty_w + 8 * pw.s);
             }
-            tc_commit(bars.empty_x + 8 * px.s);       // each arrives when the MMAs above have read the stage
-            tc_commit(bars.empty_w + 8 * pw.s);
+            __syncwarp();
             px.advance(p.n_xstages);
             pw.advance(p.n_wstages);
         }
-        if (ok) tc_commit(bars.accum);              // arrives when every MMA has written its accumulator
+        if (ok && elect_one()) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
     }
     __syncwarp();
 
@@ -508,8 +518,10 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
         return 0;
     };
     int xs = 0, ws = 0;
+    const bool one = one_ring(g.rows, g.halves);
+    const int most_x = kMaxGemmStages, most_w = one ? most_x : 3;
     auto add_x = [&]() -> bool {
-        if (xs == kMaxGemmStages) return false;
+        if (xs == most_x) return false;
         const uint32_t save0 = free_lo[0], save1 = free_lo[1];
         const uint32_t xa = take(kXHalfBytes), xb = g.halves == 2 ? take(kXHalfBytes) : xa;
         if (!xa || !xb) {
@@ -521,7 +533,7 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
         return true;
     };
     auto add_w = [&]() -> bool {
-        if (ws == kMaxGemmStages) return false;
+        if (ws == most_w) return false;
         const uint32_t w = take((uint32_t)g.rows * 128u);
         if (!w) return false;
         p.w_addr[ws++] = w;
@@ -531,12 +543,12 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
     if (xs < 2 || ws < 2) return false;
     for (bool grew = true; grew;) {
         grew = add_x();
-        if (ws < 3) grew = add_w() || grew;
+        grew = add_w() || grew;
     }
     for (int s = xs; s < kMaxGemmStages; ++s) p.xa_addr[s] = p.xb_addr[s] = 0;
     for (int s = ws; s < kMaxGemmStages; ++s) p.w_addr[s] = 0;
-    p.n_xstages = xs;
-    p.n_wstages = ws;
+    p.n_xstages = one && ws < xs ? ws : xs;
+    p.n_wstages = one && xs < ws ? xs : ws;
     return true;
 }
 
@@ -545,7 +557,7 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
 static double step_us(int rows, int halves, int code) {
     if (code == RPTC_CODE_LUT) return rows == 256 ? 1.43 : halves == 2 ? 0.92 : 0.77;
     if (halves == 2) return rows == 256 ? 0.61 : 0.56;
-    return rows == 256 ? 0.58 : 0.44;
+    return rows == 256 ? 0.58 : 0.36;
 }
 static double around_us(int rows, int halves, int split) {
     const double tile = rows / 256.0 * halves;               // in wide tiles of one half
