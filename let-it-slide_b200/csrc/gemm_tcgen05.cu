@@ -2,14 +2,14 @@
 //
 //   y[t][row] = sum_c x[t][c] * W[row][c]        x: [tokens][n] fp16,  W decoded on the fly
 //
-// One CTA owns an output tile of TOKENS (128 or 256) x NROWS (128 or 256) and walks the reduction dimension in steps of 64
+// One CTA owns an output tile of TOKENS (128 or 256) x NROWS (256, 128, or with 128 tokens 64 or 32) and walks the reduction dimension in steps of 64
 // columns.  With both operands read from shared memory a 128 x 128 x 16 MMA needs 8 KiB of operand reads per 64
 // tensor-core cycles -- exactly the 128 B/clk a SM's shared memory delivers -- so the wide tile (N = 256, 12 KiB per 128
 // cycles) is what lets the tensor pipe run ahead of shared memory.  The two operands travel through separate
 // shared-memory rings (activations: up to four stages of 16 KiB per 128 tokens; decoded weights: two or three stages of
 // 128 bytes per tile row), each with its own full/empty barriers.  Warp roles:
 //   warps 0-7  decode producers: thread r owns weight row r of the tile (256-row tiles: every thread takes every step;
-//              128-row tiles: two groups of four warps take alternate steps).  Per step a thread takes its row's next
+//              narrower ones: two, four or eight groups of threads take the steps in turn).  Per step a thread takes its row's next
 //              128 * K / 2 code bits with 128-bit loads (coalesced per 32-row block of the TILED layout), rebuilds the
 //              shift-register windows with funnel shifts and looks the 64 weights up INTO REGISTERS; only then does it
 //              wait for the stage, and writes its 128-byte row of the B operand straight into the 128-byte-swizzled
@@ -21,6 +21,10 @@
 //              Small tiles were bound by this one thread: a step of a 128 x 128 tile 0.48 us with a lane that waits and
 //              issues by itself (its operands are then not known to be uniform); 0.39 with one ring instead of two, one wait and one
 //              commit less; 0.36 with the elected lane, where decoding and shared memory bound it.
+// Narrow tiles are for few tokens, whose wide tiles leave most SMs idle, where the order of additions must stay the wide ones'
+// (invariant products, so the prompts of a model) or splitting gives less: 4096 x 11008, 22 tokens, 32 tiles of 128 rows 65.6 us, 64 of 64
+// rows 45.5, 128 of 32 rows 43.5; of tables without bank conflicts 64 rows take a step in 0.24 us and 32 in 0.21.  Their ring
+// is up to eight stages deep, and one copy of activations has the tokens that there are instead of 128.
 // Where there are fewer tiles than SMs, a cluster of two or four CTAs shares a tile and each takes a part of the
 // reduction; the partial sums meet in fp32 through distributed shared memory (`exchange_partials`) and each CTA stores
 // its share of the tile's rows.
@@ -37,7 +41,7 @@ namespace rptc {
 
 constexpr int kStepCols = 64;          // one 128-byte swizzle atom of fp16
 constexpr uint32_t kXHalfBytes = 128 * kStepCols * 2;          // 16 KiB: 128 tokens of a step
-constexpr int kMaxGemmStages = 4;      // per ring
+constexpr int kMaxGemmStages = 8;      // per ring
 constexpr int kGemmThreads = 320;
 constexpr int kProducerWarps = 8, kTmaWarp = 8, kMmaWarp = 9;
 
@@ -56,6 +60,7 @@ struct GemmParams {
     int32_t tiles_per_bank, n_split;  // tiles that a bank's rows are rounded up to; CTAs that share a tile's reduction
     int64_t lut_stride;               // fp16 elements from one bank's table to the next
     int32_t n_xstages, n_wstages;
+    uint32_t x_bytes;                 // of one copy of activations
     uint32_t bar_addr, lut_addr;      // offsets in the CTA's shared window
     uint32_t xa_addr[kMaxGemmStages], xb_addr[kMaxGemmStages];   // activation ring: two 128-token halves per stage
     uint32_t w_addr[kMaxGemmStages];                             // decoded-weight ring
@@ -93,7 +98,7 @@ struct GemmDecode {
 // `window` in the functions below: bits to OR onto every planned shared-memory offset (0 outside a cluster; inside one,
 // the upper address bits that select this CTA's window in the cluster's).
 // ---- decode producers ------------------------------------------------------------------------------------------------
-// GROUPS groups of 256 / GROUPS threads take alternate steps; thread r of a group owns row `row` of the bank whose codes
+// GROUPS groups of 256 / GROUPS threads take the steps in turn; thread r of a group owns row `row` of the bank whose codes
 // start at `codes`.  A step's 64 weights are decoded into registers BEFORE the wait for the stage, so that between the
 // tensor cores handing a stage back and its next contents being announced lie only eight 128-bit stores and a fence.
 template <int CODE, int K, int GROUPS>
@@ -103,10 +108,10 @@ __device__ __forceinline__ bool produce_weights(const GemmParams &p, uint32_t wi
     constexpr int UPS = K / 2;                 // 128-bit units per 64-column step
     constexpr int kPairs = GroupShape<K>::kPairs;
     static_assert(UPS * kPairs == 32, "a step is 32 weight pairs per row");
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const Lut<DC> lut = lut_view<DC>(p.lut_addr | window, p.L, p.S);
-    const int group = GROUPS == 2 ? warp >> 2 : 0;      // takes steps it = group, group + GROUPS, ...
-    const int r = GROUPS == 2 ? (tid & 127) : tid;      // row of the tile
+    const int group = tid / (256 / GROUPS);              // takes steps it = group, group + GROUPS, ...
+    const int r = tid % (256 / GROUPS);                  // row of the tile
     // TILED layout: unit u of row -> ((row >> 5) * n_units + u) * 32 + (row & 31)
     const uint4 *src = codes + ((row >> 5) * (int64_t)p.n_units + (int64_t)step0 * UPS) * 32 + (row & 31);
     auto history = [&](int it) -> uint32_t {             // last word before step `it` of this CTA's part
@@ -128,11 +133,11 @@ __device__ __forceinline__ bool produce_weights(const GemmParams &p, uint32_t wi
         uint4 cur[UPS];
 #pragma unroll
         for (int q = 0; q < UPS; ++q) cur[q] = nxt[q];
-        uint32_t prevw = (GROUPS == 2 || it == 0) ? nxt_prev : carry;
+        uint32_t prevw = (GROUPS > 1 || it == 0) ? nxt_prev : carry;
         if (it + GROUPS < n_steps) {
 #pragma unroll
             for (int q = 0; q < UPS; ++q) nxt[q] = ldg128_stream(src + ((int64_t)(it + GROUPS) * UPS + q) * 32);
-            nxt_prev = GROUPS == 2 ? history(it + GROUPS) : 0u;
+            nxt_prev = GROUPS > 1 ? history(it + GROUPS) : 0u;
         }
         uint32_t out[32];
 #pragma unroll
@@ -164,7 +169,7 @@ __device__ __forceinline__ bool load_activations(const GemmParams &p, uint32_t w
     for (int it = 0; it < n_steps; ++it) {
         if (!mbar_wait((ONE_RING ? bars.empty_w : bars.empty_x) + 8 * pos.s, pos.phase, p.status)) return false;
         const uint32_t bar = (ONE_RING ? bars.full_w : bars.full_x) + 8 * pos.s;
-        mbar_expect_tx(bar, HALVES * kXHalfBytes);
+        mbar_expect_tx(bar, HALVES * p.x_bytes);
         tma_load_2d(p.xa_addr[pos.s] | window, x_map, (step0 + it) * kStepCols, tok0, bar);
         if (HALVES == 2) tma_load_2d(p.xb_addr[pos.s] | window, x_map, (step0 + it) * kStepCols, tok0 + 128, bar);
         pos.advance(p.n_xstages);
@@ -260,15 +265,16 @@ __device__ __forceinline__ void drain_accumulators(const GemmParams &p, uint32_t
                 v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + __uint_as_float(o.w));
             }
         }
-        const uint32_t prow = panels + (uint32_t)(me.half * (C / 64) + (c >> 1)) * kXHalfBytes + t * 128u;
+        // tiles of 32 rows: a panel of 32 columns, 64-byte rows with the 64-byte swizzle
+        const uint32_t prow = NROWS == 32 ? panels + t * 64u : panels + (uint32_t)(me.half * (C / 64) + (c >> 1)) * kXHalfBytes + t * 128u;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             uint32_t o[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 o[e] = half2_as_u32(__floats2half2_rn(__uint_as_float(v[8 * j + 2 * e]), __uint_as_float(v[8 * j + 2 * e + 1])));
-            const uint32_t chunk = (uint32_t)((c & 1) * 4 + j);
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + 16u * (chunk ^ (t & 7u))), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
+            const uint32_t chunk = (uint32_t)((c & 1) * 4 + j) ^ (NROWS == 32 ? t >> 1 & 3u : t & 7u);
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(prow + 16u * chunk), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
                          : "memory");
         }
     }
@@ -287,7 +293,7 @@ __device__ __forceinline__ void drain_accumulators(const GemmParams &p, uint32_t
         for (int hh = 0; hh < HALVES; ++hh) {
             if ((int64_t)tok0 + hh * 128 >= p.tokens) break;  // a half with no tokens at all (rows beyond `tokens` inside a half are clipped)
 #pragma unroll 1
-            for (int q = 0; q < C / 64 && row0 + q * 64 < col_end; ++q)
+            for (int q = 0; q < (NROWS == 32 ? 1 : C / 64) && row0 + q * 64 < col_end; ++q)
                 tma_store_2d(y_map, (int)row0 + q * 64, tok0 + hh * 128, panels + (uint32_t)(hh * (C / 64) + q) * kXHalfBytes);
         }
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -317,7 +323,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     constexpr int DC = GemmDecode<CODE>::kCode;
     constexpr uint32_t kTmemCols = HALVES * NROWS;       // NROWS fp32 columns per 128 tokens
     constexpr uint32_t kInstrDesc = instr_desc(NROWS);
-    constexpr int kGroups = NROWS == 256 ? 1 : 2;        // producer groups taking alternate steps
+    constexpr int kGroups = 256 / NROWS;                 // producer groups taking the steps in turn
     constexpr bool kOneRing = one_ring(NROWS, HALVES);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -367,7 +373,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
     if (warp < kProducerWarps) {
         // rows beyond the bank's end decode its last row; their columns of the output hold no result
-        const int64_t row = tile_row + (kGroups == 2 ? (tid & 127) : tid);
+        const int64_t row = tile_row + tid % NROWS;
         ok = produce_weights<CODE, K, kGroups>(p, window, bars, codes, row < p.m ? row : p.m - 1, step0, n_steps);
     } else if (warp == kTmaWarp) {
         pdl_wait_prior_grids();
@@ -483,6 +489,8 @@ static int launch_gemm_shape(const GemmShape &g, const GemmParams &p, const CUte
                              cudaStream_t stream) {
     if (g.rows == 256)
         return g.halves == 2 ? launch_gemm<CODE, K, 256, 2>(p, map, ymap, smem, grid, stream) : launch_gemm<CODE, K, 256, 1>(p, map, ymap, smem, grid, stream);
+    if (g.rows == 64) return launch_gemm<CODE, K, 64, 1>(p, map, ymap, smem, grid, stream);
+    if (g.rows == 32) return launch_gemm<CODE, K, 32, 1>(p, map, ymap, smem, grid, stream);
     return g.halves == 2 ? launch_gemm<CODE, K, 128, 2>(p, map, ymap, smem, grid, stream) : launch_gemm<CODE, K, 128, 1>(p, map, ymap, smem, grid, stream);
 }
 
@@ -519,7 +527,7 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
     };
     int xs = 0, ws = 0;
     const bool one = one_ring(g.rows, g.halves);
-    const int most_x = kMaxGemmStages, most_w = one ? most_x : 3;
+    const int most_x = g.rows < 128 ? kMaxGemmStages : 4, most_w = one ? most_x : 3;
     auto add_x = [&]() -> bool {
         if (xs == most_x) return false;
         const uint32_t save0 = free_lo[0], save1 = free_lo[1];
@@ -549,12 +557,15 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
     for (int s = ws; s < kMaxGemmStages; ++s) p.w_addr[s] = 0;
     p.n_xstages = one && ws < xs ? ws : xs;
     p.n_wstages = one && xs < ws ? xs : ws;
-    return true;
+    // A group must find no stage two uses behind: a wait tells the uses' parity only.
+    return p.n_wstages >= 256 / g.rows;
 }
 
 // Microseconds of one 64-column step of a tile, and of a CTA around its steps (start, table, epilogue, and where a tile is
 // shared the exchange of partial sums).  Measured on 4096 rows x 4096 and 11008 columns; what matters is their ratio.
 static double step_us(int rows, int halves, int code) {
+    if (rows == 64) return code == RPTC_CODE_LUT ? 0.42 : 0.235;
+    if (rows == 32) return code == RPTC_CODE_LUT ? 0.25 : 0.21;
     if (code == RPTC_CODE_LUT) return rows == 256 ? 1.43 : halves == 2 ? 0.92 : 0.77;
     if (halves == 2) return rows == 256 ? 0.61 : 0.56;
     return rows == 256 ? 0.58 : 0.36;
@@ -602,12 +613,12 @@ static GemmShape choose_shape(int64_t m, int64_t n, int64_t tokens, const Banks 
     GemmShape best = {0, 0, 0};
     double best_us = 0;
     const int64_t steps = n / kStepCols;
-    for (int rows = 256; rows >= 128; rows >>= 1) {
-        for (int halves = tokens > 128 ? 2 : 1; halves >= 1; --halves) {
+    for (int rows = 256; rows >= 32; rows >>= 1) {
+        for (int halves = tokens > 128 && rows >= 128 ? 2 : 1; halves >= 1; --halves) {
             GemmParams probe;
             if (!plan_gemm(probe, {rows, halves, 1}, f) || tokens > 65535 * 128 * (int64_t)halves) continue;      // a grid row per tile of tokens
             const int64_t tiles = banks.banks * ((m + rows - 1) / rows) * ((tokens + halves * 128 - 1) / (halves * 128));
-            for (int split = 1; split <= (banks.may_split ? rows / 64 : 1) && (split == 1 || steps >= 8 * split); split *= 2) {
+            for (int split = 1; split <= (banks.may_split && rows >= 128 ? rows / 64 : 1) && (split == 1 || steps >= 8 * split); split *= 2) {
                 const int64_t places = cluster_places(split);
                 const int64_t waves = (tiles + places - 1) / places;
                 const double us = waves * ((double)((steps + split - 1) / split) * step_us(rows, halves, f.code) + around_us(rows, halves, split));
@@ -637,8 +648,10 @@ int gemm_banked(const void *codes, const void *lut, const uint32_t *carry_in, co
     if (!g.rows || !plan_gemm(p, g, f)) return RPTC_ERR_UNSUPPORTED;
     p.tiles_per_bank = (int32_t)((m + g.rows - 1) / g.rows);
     CUtensorMap map, ymap;
-    if (int e = encode_map(map, x, n, tokens, ld_x, 128)) return e;
-    if (int e = encode_map(ymap, y, banks.banks == 1 ? m : (int64_t)banks.banks * p.tiles_per_bank * g.rows, tokens, ld_y, 128)) return e;
+    const int x_rows = g.halves == 1 && tokens < 128 ? (int)((tokens + 7) / 8 * 8) : 128;      // what lies in a stage's other rows does not mix with these
+    p.x_bytes = (uint32_t)x_rows * kStepCols * 2;
+    if (int e = encode_map(map, x, n, tokens, ld_x, x_rows)) return e;
+    if (int e = encode_map(ymap, y, banks.banks == 1 ? m : (int64_t)banks.banks * p.tiles_per_bank * g.rows, tokens, ld_y, 128, g.rows == 32 ? 32 : 64)) return e;
     p.codes = static_cast<const uint4 *>(codes);
     p.lut = static_cast<const __half *>(lut);
     p.carry_in = carry_in;

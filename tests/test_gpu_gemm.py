@@ -138,6 +138,24 @@ def test_gemm_invariant_gives_a_token_the_same_bits_in_any_company():
         assert torch.equal(ops.gemm(codes, lut, x[:tokens], m, n, fmt, invariant=True), full[:tokens]), tokens
 
 
+@pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 4, 16, 9)])
+@pytest.mark.parametrize("m,n", [(128, 64), (1152, 576), (4096, 2048), (7168, 1024)])
+def test_gemm_of_few_tokens_in_narrow_tiles(code, K, L, S, m, n):
+    """Tiles of 32 and 64 rows against the wide ones, whose order of additions they keep: the same bits."""
+    from rptc_b200 import Format, ops
+    rng = np.random.default_rng(m + n)
+    w, lut, fmt = rand_words(rng, m, n, K), to_dev(rand_lut(rng, code, L, S)), Format(code, K, L, S, o.LAYOUT_TILED)
+    codes = to_dev(o.from_rowmajor(w, o.LAYOUT_TILED))
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((2048, n), dtype=torch.float16, device="cuda", generator=g)
+    wide = ops.gemm(codes, lut, x, m, n, fmt, invariant=True)
+    for tokens in (1, 8, 31, 100, 127, 128, 129, 300):
+        y = torch.full((tokens + 1, m), 7.0, dtype=torch.float16, device="cuda")
+        ops.gemm(codes, lut, x[:tokens], m, n, fmt, invariant=True, out=y[:tokens])
+        assert torch.equal(y[:tokens], wide[:tokens]) and (y[tokens] == 7.0).all(), tokens
+    _run(code, K, L, S, m, n, 30, seed=m)
+
+
 @pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 16, 0), (o.CODE_C, 4, 16, 8)])
 @pytest.mark.parametrize("m,n,tokens", [(64, 4096, 80), (32, 8192, 97), (160, 11008, 112), (1056, 8256, 193), (288, 4160, 385), (4096, 4096, 160)])
 def test_layer_of_some_hundred_tokens(code, K, L, S, m, n, tokens):
