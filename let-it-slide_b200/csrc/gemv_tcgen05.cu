@@ -32,7 +32,11 @@ namespace rptc {
 
 static_assert(4 * kFewOwnTokens <= 512 - 128 && 4 * 2 * 48 <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
 constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * (kFewMmaWarp + 4);
-constexpr int kFewAhead = 4;                         // steps of a thread's code bits in flight
+// Steps of a thread's code bits in flight.  Two where a 128 KiB table leaves little room: a group takes more than two microseconds for a step's
+// look-ups, and 16 KiB more hold two stages of 256 tokens.  With one stage fewer tokens fit into a tile, and every weight is looked up once
+// per tile: layers of 4096 x 4096 in 32 banks, 256 tokens (two tiles of 128, now one) 32.1 -> 29.4 us, 384 tokens 47.2 -> 36.7; 4096 x 11008 in
+// eight, 256 tokens 68.9 -> 50.1; up to 144 tokens the same time.
+constexpr int few_ahead(int code, bool shared) { return shared && code == RPTC_CODE_LUT ? 2 : 4; }
 constexpr uint32_t kFewBars = 0x400, kFewHistory = 0x800, kFewCodes = 0x2800, kFewTop = 0x38800;
 constexpr int kFewMaxXStages = 8;
 constexpr int kFewACols = 32 * 4;                    // tensor-memory columns of the decoded weights: 64 fp16 per group and lane
@@ -92,7 +96,7 @@ template <int CODE, int K, int RB, bool SHARED, bool ORDERED>
 __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const FewParams p, const __grid_constant__ CUtensorMap x_map) {
     constexpr int UPS = K / 2;                       // 128-bit units per step
     constexpr int PARTS = 4 / RB, RINGS = SHARED ? 1 : PARTS;
-    constexpr int NW = 4 * UPS;
+    constexpr int NW = 4 * UPS, kAhead = few_ahead(CODE, SHARED);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (smem_addr(smem_raw) > kFewBars) {            // the dynamic area starts later than the plan says
@@ -133,7 +137,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
     // ---- a producer's code bits: private ring of copies ----
     const int group = warp >> 2, block = group % RB, part = group / RB;
     const int32_t lane_row = block * 128 + (warp & 3) * 32 + lane;       // row inside the tile
-    const uint32_t ring = kFewCodes + (uint32_t)warp * (kFewAhead * UPS * 512) + 16u * lane, hist = kFewHistory + 4u * tid;
+    const uint32_t ring = kFewCodes + (uint32_t)warp * (kAhead * UPS * 512) + 16u * lane, hist = kFewHistory + 4u * tid;
     const uint4 *bank_codes = p.codes + (int64_t)bank * p.m * p.n_units;
     // rows past the bank's end decode its last block of 32 rows; their sums are not used
     auto row_in_bank = [&](int32_t tile) { return min((int64_t)tile * (RB * 128) + lane_row, p.m - 32 + lane); };
@@ -175,11 +179,11 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         if (f_left > 0) copy_step();
         else fetch_any();
         cp_async_commit();                                                // an empty group when nothing is left keeps the count constant
-        slot = (slot + 1) % kFewAhead;
+        slot = (slot + 1) % kAhead;
     };
     if (warp < kFewWarps) {
 #pragma unroll 1
-        for (int i = 0; i < kFewAhead; ++i) fetch();
+        for (int i = 0; i < kAhead; ++i) fetch();
     }
     // ---- table filled
     if (CODE != RPTC_CODE_LUT) lut_fill_end<CODE>(p.lut_addr, entries, p.S);
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
             uint32_t prevw = 0;
 #pragma unroll 1
             for (int32_t i = 0; i < len && ok; ++i) {
-                cp_async_wait<kFewAhead - 1>();      // this step's words have landed
+                cp_async_wait<kAhead - 1>();      // this step's words have landed
                 uint32_t R[2 * NW], out[16];
                 if (i == 0) prevw = lds32(hist + 2048u * slot);
 #pragma unroll
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                         prevw = w[k];
                     }
                 }
-                fetch();                             // the words are in registers: the slot takes the step kFewAhead further on
+                fetch();                             // the words are in registers: the slot takes the step kAhead further on
 #pragma unroll
                 for (int pi = 0; pi < 32; pi += 4) {
                     uint32_t four[4];
@@ -455,7 +459,8 @@ static double shared_step_us(int rb, int n_cols, int code) {
 
 // Tile of `rb` row blocks, where the table and the activation ring go; false when they do not fit.
 static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb) {
-    const uint32_t codes_end = kFewCodes + kFewWarps * kFewAhead * (f.K / 2) * 512;
+    p.shared = tokens > kFewOwnTokens;
+    const uint32_t codes_end = kFewCodes + kFewWarps * few_ahead(f.code, p.shared) * (f.K / 2) * 512;
     uint32_t free;
     if (f.code == RPTC_CODE_HASH) {
         p.lut_addr = kHashLutWindow;
@@ -466,10 +471,9 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
     }
     if (free >= kFewTop) return false;
     p.x_addr = free;
-    p.shared = tokens > kFewOwnTokens;
     p.token_tiles = 1;
-    if (p.shared) {      // three stages of activations, and the accumulators beside the decoded weights, bound the tile
-        const int64_t fit = (kFewTop - free) / (3 * 128) / 16 * 16, most = rb == 1 ? 256 : 192, cols = fit < most ? fit : most;
+    if (p.shared) {      // three stages of activations (two under a table's slower look-ups), and the accumulators beside the decoded weights, bound the tile
+        const int64_t fit = (kFewTop - free) / ((f.code == RPTC_CODE_LUT ? 2 : 3) * 128) / 16 * 16, most = rb == 1 ? 256 : 192, cols = fit < most ? fit : most;
         if (cols < 16) return false;
         p.token_tiles = (int32_t)((tokens + cols - 1) / cols);
     }

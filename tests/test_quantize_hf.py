@@ -237,3 +237,21 @@ def test_alphabets_on_the_gpu_are_those_of_the_tensor_operations(banks, values, 
     g = torch.Generator().manual_seed(values)
     x = torch.randn(banks, values, generator=g)
     assert torch.equal(q.megabatch_alphabets(x.cuda(), L).cpu(), q.megabatch_alphabets(x, L))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,banks", [(128, 64, 1), (352, 1088, 4), (4096, 2048, 32)])
+@pytest.mark.parametrize("tokens", [145, 192, 193, 256, 257, 520])
+def test_packed_layer_whose_table_leaves_two_stages_of_tokens(m, n, banks, tokens):
+    """L = 16: tiles of up to 256 tokens beside a table of 128 KiB, their last one partly filled; sums of one and of several CTAs."""
+    import quantize_hf as q
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    symbols = torch.randint(0, 4, (m, n), generator=g, device="cuda", dtype=torch.int32)
+    layer = q.FactorizedRPTCLinear.from_parts(symbols, rnd(banks, 1 << 16), 0.1 * rnd(m), 0.1 * rnd(n), 0.5 + rnd(m).abs(), 0.5 + rnd(n).abs(), None)
+    x = rnd(tokens, n).half()
+    want = ((x.float() * layer.scales_in).half().double() @ layer.decoded().double().t()) * layer.scales_out.double() \
+        + x.double().sum(1, keepdim=True) * layer.biases_out.double() + (x.double() @ layer.biases_in.double())[:, None]
+    got = layer(x)
+    assert (got.double() - want).norm() <= 6e-4 * want.norm()
+    assert torch.equal(layer(x), got)
