@@ -284,8 +284,8 @@ int rptc_rope_cache(void *qkv, int64_t ld_qkv, const int32_t *pos, void *kcache,
 int rptc_rope_cache_prompt(void *qkv, int64_t ld_qkv, int64_t rows, int64_t tokens, void *kcache, void *vcache, int hq, int hkv,
                            int d, int max_pos, float theta, rptc_stream_t stream);
 /* The glue of a prompt's forward pass around the matrix products (fp16 products in, before their output transform).
- * rptc_prompt_norm: h += s_out * H(y) * scale_out (y NULL: h as it is); out = H(s_in * rmsnorm(h) * w_norm), rows of n =
- * 4096 or 8192 in Hadamard blocks of 4096; h in place.
+ * rptc_prompt_norm: h += s_out * H(y) * scale_out (y NULL: h as it is); out = H(s_in * rmsnorm(h) * w_norm), rows of n, a
+ * power of two from 256 to 8192, in one Hadamard block or two of 4096; h in place.
  * rptc_prompt_qkv: qkv fp16 [rows * tokens][ld] = [q | k | v heads of 128], y = s_out * H(qkv) * scale in blocks of 128; q rotated in
  * place, rotated k and v to cache positions 0 .. tokens-1.  angles: fp32 [tokens][64][2], cosines and sines
  * (rptc_rope_angles). */

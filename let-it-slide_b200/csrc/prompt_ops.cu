@@ -534,6 +534,108 @@ __global__ void __launch_bounds__(128 * NH, 4 / NH) norm_rows_kernel(const NormR
     }
 }
 
+// The same for rows of 2^BITS = 256 to 2048 elements, one Hadamard block each: a segment of 4096 elements is 4096 / 2^BITS rows.  Bound as
+// above by the trips through shared memory and their barriers.  2048 rows of 2048 14.8 us, a row per CTA with eight values a thread and
+// shuffles 31.1, as three kernels 38; a prompt of 1024 tokens through 24 layers of hidden 2048 5.62 -> 4.96 ms, of 64 tokens 3.83 -> 3.03.
+template <int BITS>
+__global__ void __launch_bounds__(128, 4) norm_short_rows_kernel(const NormRowsParams p, float hn) {
+    constexpr int n = 1 << BITS, R = 4096 >> BITS, KR = n / 256;      // rows of a segment, pairs of a thread in each
+    __shared__ __align__(16) float smem[kCtaSegFloats];
+    __shared__ float red[R][8];
+    const SegThread th;
+    uint32_t so[KR], ws[KR];
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+        const int c = th.pair(k);
+        so[k] = p.signs_out ? __ldg(reinterpret_cast<const uint32_t *>(p.signs_out + c)) : 0x3C003C00u;
+        const float2 w = __half22float2(u32_as_half2(__ldg(reinterpret_cast<const uint32_t *>(p.w_norm + c))));
+        const float2 si = p.signs_in ? __half22float2(u32_as_half2(__ldg(reinterpret_cast<const uint32_t *>(p.signs_in + c)))) : make_float2(1.f, 1.f);
+        ws[k] = half2_as_u32(__floats2half2_rn(w.x * si.x, w.y * si.y));
+    }
+    pdl_allow_next_grid();
+    pdl_wait_prior_grids();
+    for (int64_t row0 = (int64_t)blockIdx.x * R; row0 < p.rows; row0 += (int64_t)gridDim.x * R) {
+        // rows past the end read the last one and store nothing
+        auto row_of = [&](int e) { return min(row0 + (e >> BITS), p.rows - 1); };
+        auto inside = [&](int k) { return row0 + k / KR < p.rows; };
+        uint32_t hr[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) hr[k] = ldcg_u32(p.h + row_of(256 * k) * p.ld_h + th.pair(k % KR));
+        float v[32];
+        if (p.y) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                unpack8_at(__ldcg(reinterpret_cast<const uint4 *>(p.y + row_of(th.piece(j)) * p.ld_y + (th.piece(j) & (n - 1)))), v + 8 * j);
+            piece_stages(v);
+            th.put_pieces(smem, v);
+            __syncthreads();
+            th.get_columns(smem, v);
+            column_stages(v, BITS);
+            th.put_columns(smem, v);
+            __syncthreads();
+            th.get_pairs(smem, v);
+            far_stages(v, BITS);
+            const float sc = p.scale_out * hn;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const float2 s = __half22float2(u32_as_half2(so[k % KR])), r = __half22float2(u32_as_half2(hr[k]));
+                const float a = __fadd_rn(__fmul_rn(v[2 * k], sc * s.x), r.x), b = __fadd_rn(__fmul_rn(v[2 * k + 1], sc * s.y), r.y);
+                hr[k] = half2_as_u32(__floats2half2_rn(a, b));
+                if (inside(k)) *reinterpret_cast<uint32_t *>(p.h + row_of(256 * k) * p.ld_h + th.pair(k % KR)) = hr[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float2 f = __half22float2(u32_as_half2(hr[k]));
+            v[2 * k] = f.x, v[2 * k + 1] = f.y;
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            float ss[2] = {0.f, 0.f};
+#pragma unroll
+            for (int k = q * KR; k < (q + 1) * KR; ++k) ss[(k - q * KR) & 1] += v[2 * k] * v[2 * k] + v[2 * k + 1] * v[2 * k + 1];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ss[i] += __shfl_xor_sync(0xFFFFFFFFu, ss[i], o);
+                if (th.lane == 0) red[q][4 * i + th.warp] = ss[i];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            float tot = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tot += red[q][i];
+            const float inv = rsqrtf(tot / n + p.eps);
+#pragma unroll
+            for (int k = q * KR; k < (q + 1) * KR; ++k) {
+                const float2 w = __half22float2(u32_as_half2(ws[k % KR]));
+                const float2 f = __half22float2(__floats2half2_rn(v[2 * k] * inv * w.x, v[2 * k + 1] * inv * w.y));
+                v[2 * k] = f.x, v[2 * k + 1] = f.y;
+            }
+        }
+        th.put_pairs(smem, v);
+        __syncthreads();
+        th.get_pieces(smem, v);
+        piece_stages(v);
+        th.put_pieces(smem, v);
+        __syncthreads();
+        th.get_columns(smem, v);
+        column_stages(v, BITS);
+        th.put_columns(smem, v);
+        __syncthreads();
+        th.get_pairs(smem, v);
+        far_stages(v, BITS);
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (inside(k))
+                *reinterpret_cast<uint32_t *>(p.out + row_of(256 * k) * p.ld_out + th.pair(k % KR)) =
+                    half2_as_u32(__floats2half2_rn(v[2 * k] * hn, v[2 * k + 1] * hn));
+        __syncthreads();                                      // the buffer is free for the next rows
+    }
+}
+
 // ---- output side of the fused qkv layer for a prompt -------------------------------------------------------------------
 struct QkvRowsParams {
     __half *qkv;                     // [rows * tokens][ld]: the product; q comes back in place
@@ -646,7 +748,7 @@ using namespace rptc;
 extern "C" int rptc_prompt_norm(const void *y, int64_t ld_y, const void *signs_out, float scale_out, void *h, int64_t ld_h, const void *w_norm,
                                 float eps, const void *signs_in, void *out, int64_t ld_out, int64_t rows, int64_t n, rptc_stream_t stream) {
     if (!h || !w_norm || !out) return RPTC_ERR_ARG;
-    if (n != 4096 && n != 8192) return RPTC_ERR_UNSUPPORTED;
+    if (n < 256 || n > 8192 || (n & (n - 1))) return RPTC_ERR_UNSUPPORTED;
     if (rows <= 0 || ld_h < n || ld_out < n || (y && ld_y < n)) return RPTC_ERR_SHAPE;
     auto misaligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
     if (misaligned(y) || misaligned(h) || misaligned(w_norm) || misaligned(out) || misaligned(signs_out) || misaligned(signs_in) || (ld_h % 8) ||
@@ -667,6 +769,14 @@ extern "C" int rptc_prompt_norm(const void *y, int64_t ld_y, const void *signs_o
     p.ld_out = ld_out;
     p.rows = rows;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (n < 4096) {
+        const dim3 grid(rows_grid((rows * n + 4095) / 4096, 1, 1, 4));
+        const float hn = norm_of((int)n);
+        if (n == 2048) return launch(norm_short_rows_kernel<11>, grid, dim3(128), 0, s, p, hn);
+        if (n == 1024) return launch(norm_short_rows_kernel<10>, grid, dim3(128), 0, s, p, hn);
+        if (n == 512) return launch(norm_short_rows_kernel<9>, grid, dim3(128), 0, s, p, hn);
+        return launch(norm_short_rows_kernel<8>, grid, dim3(128), 0, s, p, hn);
+    }
     if (n == 4096) return launch(norm_rows_kernel<1>, dim3(rows_grid(rows, 1, 1, 4)), dim3(128), 0, s, p);
     return launch(norm_rows_kernel<2>, dim3(rows_grid(rows, 1, 1, 2)), dim3(256), 0, s, p);
 }

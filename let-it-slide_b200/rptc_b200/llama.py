@@ -584,7 +584,7 @@ class RPTCLlama:
         matrix products in one kernel each; returns the residual stream of every row's last position."""
         cfg = self.cfg
         heads_of_128 = cfg.head_dim == 128 and self.blocks[0].qkv.block_out == 128
-        whole_rows = cfg.hidden in (4096, 8192)                      # the norm kernel's rows: one or two 4096-point blocks
+        whole_rows = 256 <= cfg.hidden <= 8192 and cfg.hidden & (cfg.hidden - 1) == 0      # the norm kernel's rows: a block, or two of 4096
         xt, mlp = torch.empty_like(h), torch.empty((R * T, self.ffn_l), dtype=torch.float16, device=h.device)
         angles = ops.rope_angles(T, cfg.rope_theta, h.device) if heads_of_128 else None
         y, prev = None, None                                         # product whose output side is still to be added to h, its layer

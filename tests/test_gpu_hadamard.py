@@ -250,3 +250,18 @@ def test_prompt_qkv_off_32_byte_boundaries():
         ops.prompt_qkv(qkv, signs, 0.5, 1, tokens, *kv, hq, hkv, ops.rope_angles(tokens, 10000.0, "cuda:0"))
     assert off.data_ptr() % 32 == 16 and torch.equal(x, off)
     assert all(torch.equal(a, b) for a, b in zip(*caches))
+
+
+@pytest.mark.parametrize("n", [256, 512, 1024, 2048])
+@pytest.mark.parametrize("rows", [9, 1500])
+@pytest.mark.parametrize("with_y", [False, True])
+def test_prompt_norm_of_short_rows_matches_its_parts(n, rows, with_y):
+    from rptc_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n + rows)
+    f16 = lambda *s: torch.randn(*s, generator=g, device="cuda").half()
+    h, y, w = f16(rows, n), f16(rows, n), (1 + 0.1 * f16(n))
+    so, si = [(torch.randint(0, 2, (n,), generator=g, device="cuda") * 2 - 1).half() for _ in range(2)]
+    h_want = ops.hadamard(y, so, n, transpose=True, scale=0.3, residual=h) if with_y else h.clone()
+    want = ops.hadamard(ops.rmsnorm(h_want, w, torch.empty_like(h), 1e-5), si, n)
+    got = ops.prompt_norm(y if with_y else None, so, 0.3, h, w, 1e-5, si, torch.empty_like(h))
+    assert torch.equal(h, h_want) and torch.equal(got, want)
