@@ -27,6 +27,8 @@ struct {
     decltype(&rptc_packed_workspace_bytes) packed_workspace_bytes;
     decltype(&rptc_packed_forward) packed_forward;
     decltype(&rptc_gemv_timed) gemv_timed;
+    decltype(&rptc_dequantize) dequantize;
+    decltype(&rptc_decompress) decompress;
 } g_lib;
 
 #define RPTC_NAMES(X) X(in_features) X(out_features) X(block_in) X(block_out) X(scale) X(fmt) X(_buffers) X(codes) X(lut) X(carry_in) \
@@ -262,12 +264,63 @@ PyObject *gemv_timed(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     });
 }
 
-// bind(linear_workspace_bytes, linear_forward, packed_workspace_bytes, packed_forward, gemv_timed): addresses
+bool plain(const at::Tensor &t, at::ScalarType type) { return t.is_cuda() && t.scalar_type() == type && t.is_contiguous(); }
+
+// dequantize(alphabet, symbols): symbols to weights, or None for what is not as the kernel reads it (the caller converts it, or refuses it)
+PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 2) fail("dequantize(alphabet, symbols)");
+        if (!THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) Py_RETURN_NONE;
+        const at::Tensor &alphabet = THPVariable_Unpack(args[0]), &symbols = THPVariable_Unpack(args[1]);
+        const bool f32 = alphabet.scalar_type() == at::kFloat;
+        const int64_t entries = alphabet.numel(), dims = symbols.dim();
+        if (!plain(alphabet, f32 ? at::kFloat : at::kHalf) || !plain(symbols, at::kInt) || alphabet.device() != symbols.device() || alphabet.dim() != 1 ||
+            entries < 8 || entries > 65536 || (entries & (entries - 1)) || dims < 1 || dims > 2 || symbols.numel() == 0)
+            Py_RETURN_NONE;
+        const c10::cuda::OptionalCUDAGuard guard(symbols.device());
+        at::Tensor out = at::empty(symbols.sizes(), alphabet.options().requires_grad(false));
+        int L = 0;
+        while ((int64_t(1) << L) < entries) ++L;
+        const cudaStream_t s = current_stream(symbols);
+        int status;
+        Py_BEGIN_ALLOW_THREADS
+        status = g_lib.dequantize(alphabet.data_ptr(), static_cast<const int32_t *>(symbols.data_ptr()), out.data_ptr(), f32, dims == 2 ? symbols.size(0) : 1,
+                                  symbols.size(-1), L, s);
+        Py_END_ALLOW_THREADS
+        return status == RPTC_OK ? THPVariable_Wrap(std::move(out)) : PyLong_FromLong(status);
+    });
+}
+
+// decompress(codes, lut, m, n, fmt, out): 0 when done, None for what is not as the kernel reads it (the caller refuses it)
+PyObject *decompress(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject * {
+        if (nargs != 6) fail("decompress(codes, lut, m, n, fmt, out)");
+        if (!THPVariable_Check(args[0]) || !THPVariable_Check(args[1]) || !THPVariable_Check(args[5])) Py_RETURN_NONE;
+        const at::Tensor &codes = THPVariable_Unpack(args[0]), &lut = THPVariable_Unpack(args[1]), &out = THPVariable_Unpack(args[5]);
+        const long long m = PyLong_AsLongLong(args[2]), n = PyLong_AsLongLong(args[3]);
+        if (PyErr_Occurred()) throw PyError();
+        const rptc_format fmt = format_of(args[4]);
+        if (fmt.L < 1 || fmt.L > 16 || fmt.S < 0 || fmt.S > 16 || m <= 0 || n <= 0 || m > (1 << 30) || n > (1 << 30)) Py_RETURN_NONE;
+        if (!plain(codes, at::kInt) || !plain(lut, at::kHalf) || codes.device() != lut.device() || codes.device() != out.device() ||
+            lut.numel() != (fmt.code == RPTC_CODE_LUT ? int64_t(1) << fmt.L : int64_t(2) << fmt.S) || codes.numel() * 32 != m * n * fmt.K ||
+            out.scalar_type() != at::kHalf || out.dim() != 2 || out.size(0) != m || out.size(1) != n || out.stride(1) != 1)
+            Py_RETURN_NONE;
+        const c10::cuda::OptionalCUDAGuard guard(codes.device());
+        const cudaStream_t s = current_stream(codes);
+        int status;
+        Py_BEGIN_ALLOW_THREADS
+        status = g_lib.decompress(codes.data_ptr(), lut.data_ptr(), nullptr, out.data_ptr(), out.stride(0), m, n, &fmt, s);
+        Py_END_ALLOW_THREADS
+        return PyLong_FromLong(status);
+    });
+}
+
+// bind(linear_workspace_bytes, linear_forward, packed_workspace_bytes, packed_forward, gemv_timed, dequantize, decompress): addresses
 PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject * {
-        if (nargs != 5) fail("bind(five addresses)");
-        void *p[5];
-        for (int i = 0; i < 5; ++i) {
+        if (nargs != 7) fail("bind(seven addresses)");
+        void *p[7];
+        for (int i = 0; i < 7; ++i) {
             p[i] = PyLong_AsVoidPtr(args[i]);
             if (!p[i]) {
                 if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "null address");
@@ -279,13 +332,15 @@ PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         g_lib.packed_workspace_bytes = reinterpret_cast<decltype(g_lib.packed_workspace_bytes)>(p[2]);
         g_lib.packed_forward = reinterpret_cast<decltype(g_lib.packed_forward)>(p[3]);
         g_lib.gemv_timed = reinterpret_cast<decltype(g_lib.gemv_timed)>(p[4]);
+        g_lib.dequantize = reinterpret_cast<decltype(g_lib.dequantize)>(p[5]);
+        g_lib.decompress = reinterpret_cast<decltype(g_lib.decompress)>(p[6]);
         Py_RETURN_NONE;
     });
 }
 
 #define RPTC_METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {RPTC_METHOD(bind), RPTC_METHOD(linear_forward), RPTC_METHOD(packed_forward), RPTC_METHOD(gemv_timed),
-                           {nullptr, nullptr, 0, nullptr}};
+                           RPTC_METHOD(dequantize), RPTC_METHOD(decompress), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

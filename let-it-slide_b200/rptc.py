@@ -17,6 +17,7 @@ from __future__ import annotations
 import torch
 
 from rptc_b200 import ops
+from rptc_b200._lib import RPTCError, native
 
 
 def quantize_rows(permuted_alphabet: torch.Tensor, weights: torch.Tensor, samples: torch.Tensor):
@@ -80,6 +81,11 @@ def dequantize(permuted_alphabet: torch.Tensor, quantized: torch.Tensor) -> torc
     """rptc.py:74-85 on the GPU: `quantized` [length] or [rows, length] symbols in 0..3."""
     if not quantized.is_cuda:
         raise RuntimeError("dequantize runs on the CUDA kernels: pass CUDA tensors")
+    out = native().dequantize(permuted_alphabet, quantized)      # None: something is not as the kernel reads it
+    if out is not None:
+        if type(out) is int:
+            raise RPTCError(out, "rptc_dequantize")
+        return out
     single = quantized.dim() == 1
     q = (quantized[None, :] if single else quantized).to(torch.int32).contiguous()
     # fp32 alphabets are rounded to fp16 on the way into the kernel's table; other types here

@@ -223,7 +223,8 @@ def native():
         from . import _native as ext
         L = lib()
         ext.bind(*[ctypes.cast(getattr(L, "rptc_" + name), ctypes.c_void_p).value for name in (
-            "linear_workspace_bytes", "linear_forward", "packed_workspace_bytes", "packed_forward", "gemv_timed")])
+            "linear_workspace_bytes", "linear_forward", "packed_workspace_bytes", "packed_forward", "gemv_timed",
+            "dequantize", "decompress")])
         _native = ext
     return _native
 

@@ -6,8 +6,8 @@ import ctypes
 import torch
 
 from . import _lib
-from ._lib import (CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_TILED, LAYOUT_UNITMAJOR, XORDER_NATURAL,
-                   Format, call, check, lib, ptr)
+from ._lib import (CODE_HASH, CODE_LITE, CODE_LUT, LAYOUT_CHUNKED, LAYOUT_ROWMAJOR, LAYOUT_TILED, LAYOUT_UNITMAJOR,
+                  XORDER_NATURAL, Format, call, check, lib, ptr, native)
 
 
 def _cuda_contig(t: torch.Tensor, name: str, dtype: torch.dtype | None = None) -> None:
@@ -61,6 +61,11 @@ def repack(codes: torch.Tensor, src_layout: int, dst_layout: int, m: int, n_unit
 def decompress(codes: torch.Tensor, lut: torch.Tensor, m: int, n: int, fmt: Format, out: torch.Tensor | None = None,
                carry_in: torch.Tensor | None = None) -> torch.Tensor:
     """Packed codes -> dense fp16 [m, n] (rptc_decompress)."""
+    if out is not None and carry_in is None:
+        status = native().decompress(codes, lut, m, n, fmt, out)      # None: something is not as the kernel reads it
+        if status is not None:
+            check(status, "rptc_decompress")
+            return out
     _cuda_contig(codes, "codes", torch.int32)
     _cuda_contig(lut, "lut", torch.float16)
     if lut.numel() != fmt.lut_numel():

@@ -160,3 +160,31 @@ def test_dequantize_keeps_stream_order_under_dependent_launch(rows, length):
             assert torch.equal(shared.view(torch.float16)[: want.numel()].view(want.shape), want)
     finally:
         lib().rptc_set_pdl(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("L", [3, 4, 9])
+def test_dequantize_and_decompress_by_either_route(L, dtype):
+    """What the native call takes and what it leaves to the converting path: 64-bit and strided symbols, other types, a
+    single row; outputs with a stride, and those that are refused."""
+    import rptc
+    from rptc_b200 import CODE_LUT, LAYOUT_TILED, Format, ops
+    g = torch.Generator(device="cuda").manual_seed(L)
+    alphabet = torch.randn(1 << L, generator=g, device="cuda").to(dtype)
+    wide = torch.randint(0, 4, (6, 300), generator=g, device="cuda")
+    want = rptc.dequantize(alphabet, wide)
+    assert torch.equal(rptc.dequantize(alphabet, wide.int()), want) and torch.equal(rptc.dequantize(alphabet, wide[2].int()), want[2])
+    strided = torch.zeros((6, 600), dtype=torch.int32, device="cuda")[:, ::2]
+    strided.copy_(wide)
+    assert torch.equal(rptc.dequantize(alphabet, strided), want)
+    m, n = 64, 256
+    fmt = Format(CODE_LUT, 2, max(L, 8), 0, LAYOUT_TILED)
+    codes = torch.randint(-2**31, 2**31 - 1, ops.codes_shape(m, n, 2, fmt.layout), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), generator=g, device="cuda").half()
+    dense = ops.decompress(codes, lut, m, n, fmt)
+    out = torch.empty((m, n + 16), dtype=torch.float16, device="cuda")
+    assert torch.equal(ops.decompress(codes, lut, m, n, fmt, out=out[:, :n]), dense)
+    for refused in (out, out[:, :n].float(), out[: m // 2, :n], torch.empty((n, m), dtype=torch.float16, device="cuda").t()):
+        with pytest.raises(Exception):
+            ops.decompress(codes, lut, m, n, fmt, out=refused)
