@@ -16,11 +16,12 @@
 //              K-major layout the tensor core reads.  After the last step the same warps run the epilogue.
 //   warp 8     one lane issues the 2-D TMA loads of the activation tile (128 tokens each), as far ahead as the
 //              activation ring allows.
-//   warp 9     owns the TMEM allocation; the whole warp waits, and an elected lane issues tcgen05.mma (M = 128, N = NROWS,
+//   warp 9     owns the TMEM allocation; one lane (small tiles: an elected one of a warp that waits) issues tcgen05.mma (M = 128, N = NROWS,
 //              K = 16, fp32 accumulators in TMEM, one or two token halves) and commits each stage back to its producer.
 //              Small tiles were bound by this one thread: a step of a 128 x 128 tile 0.48 us with a lane that waits and
 //              issues by itself (its operands are then not known to be uniform); 0.39 with one ring instead of two, one wait and one
 //              commit less; 0.36 with the elected lane, where decoding and shared memory bound it.
+//              Wide tiles, bound by the tensor core, lose by 31 more lanes that wait: prefill of 2048 tokens 29.25 -> 29.66 ms.
 // Narrow tiles are for few tokens, whose wide tiles leave most SMs idle, where the order of additions must stay the wide ones'
 // (invariant products, so the prompts of a model) or splitting gives less: 4096 x 11008, 22 tokens, 32 tiles of 128 rows 65.6 us, 64 of 64
 // rows 45.5, 128 of 32 rows 43.5; of tables without bank conflicts 64 rows take a step in 0.24 us and 32 in 0.21.  Their ring
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     } else if (warp == kTmaWarp) {
         pdl_wait_prior_grids();
         if (lane == 0) load_activations<HALVES, kOneRing>(p, window, bars, &x_map, tok0, step0, n_steps);
-    } else {
+    } else if (kOneRing || lane == 0) {
         // ================= MMA issue =================
         RingPos px = {0, 0u}, pw = {0, 0u};
         for (int it = 0; it < n_steps && ok; ++it) {
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             if (!ok) break;
             tc_fence_after();
             const uint64_t xa = umma_desc_sw128(p.xa_addr[px.s]), xb = umma_desc_sw128(p.xb_addr[px.s]), wd = umma_desc_sw128(p.w_addr[pw.s]);
-            if (elect_one()) {
+            if (!kOneRing || elect_one()) {
 #pragma unroll
                 for (uint32_t k = 0; k < kStepCols / 16; ++k) {           // + 32 bytes per K = 16
                     tc_mma_f16(tmem_base, xa + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
@@ -395,11 +396,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 if (!kOneRing) tc_commit(bars.empty_x + 8 * px.s);      // each arrives when the MMAs above have read the stage
                 tc_commit(bars.empty_w + 8 * pw.s);
             }
-            __syncwarp();
+            if (kOneRing) __syncwarp();
             px.advance(p.n_xstages);
             pw.advance(p.n_wstages);
         }
-        if (ok && elect_one()) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
+        if (ok && (!kOneRing || elect_one())) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
     }
     __syncwarp();
 
