@@ -9,7 +9,7 @@ constexpr uint32_t kUnitsRing = kGemvWarps * kUnitsAhead * 512, kUnitsHist = kGe
 // sixteenth of its rows chunk by chunk (the activations of a chunk are read into registers once for up to eight rows), or, of fewer rows
 // than warps, a part of the chunks.  All activations are staged at once; a lane's running sums are kept in shared memory.  The last CTA to
 // finish leaves the device time in host memory (DeviceTimer), where the calling thread waits for it: 4096 x 4096 HASH, a drop-in call
-// 31.3 us with a kernel behind and events around.
+// 31.3 us with a kernel behind and events around, 23.4 so.
 constexpr int kWholeRows = 8;
 constexpr uint32_t kWholeSums = kGemvWarps * kWholeRows * 32 * 4, kWholeParts = 256;
 static_assert(kBarBytes + kUnitsRing + kUnitsHist + kWholeSums + kWholeParts + 1024 <= kHashLutWindow, "in front of the HASH table window");
