@@ -207,6 +207,8 @@ static bool many_rows(int64_t rows, int64_t n, int block, const HadParams &p) {
            (!p.residual || on_32_bytes(p.residual, p.ld_res * 2));
 }
 
+int check_signs(const void *signs) { return reinterpret_cast<uintptr_t>(signs) & 15 ? RPTC_ERR_ALIGN : RPTC_OK; }      // read sixteen bytes at a time
+
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late) {
@@ -217,7 +219,7 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
     const int chunk = block < 256 ? 256 : block;
     if (n % chunk) return RPTC_ERR_SHAPE;
     if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15) ||
-        (signs && (reinterpret_cast<uintptr_t>(signs) & 15)) || (residual && (reinterpret_cast<uintptr_t>(residual) & 15)) ||
+        check_signs(signs) || (residual && (reinterpret_cast<uintptr_t>(residual) & 15)) ||
         (ld_in % 8) || (ld_out % 8) || (residual && (ld_res % 8)))
         return RPTC_ERR_ALIGN;
     if (clear_in && !in_is_f32) return RPTC_ERR_ARG;
@@ -258,6 +260,7 @@ int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, voi
     if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
     const int chunk = block < 256 ? 256 : block;
     if (n % chunk) return RPTC_ERR_SHAPE;
+    if (int e = check_signs(signs)) return e;
     HadSumsParams p = {};
     p.in = partial;
     p.ld_in = ld;

@@ -21,6 +21,7 @@ int check_format(const rptc_format *f);   // api.cu
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late = false);
+int check_signs(const void *signs);
 // out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]; for how many rows that is as fast as adding them up in a
 // kernel in front
 bool hadamard_takes_sums(int64_t rows, int64_t n, int block);
@@ -289,13 +290,14 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     auto misaligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
     if (misaligned(l->codes) || misaligned(l->lut) || misaligned(x) || misaligned(y) || misaligned(workspace) || (l->n % 8) || (l->m % 8))
         return RPTC_ERR_ALIGN;
+    if (int e = check_signs(l->signs_in)) return e;
+    if (int e = check_signs(l->signs_out)) return e;
     if (int e = rptc_check_device()) return e;
     PdlScope pdl(l->signs_in && few);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(workspace);
     const int64_t m = l->m, n = l->n;
     if (linear_alone(*l, rows)) {
-        if (misaligned(l->signs_in) || misaligned(l->signs_out)) return RPTC_ERR_ALIGN;
         pdl.set(true);
         GemvInput in = {};
         in.x = x;

@@ -3,6 +3,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -71,6 +73,27 @@ def test_entry_point_without_scratch_rejects_bad_calls_before_it_touches_its_arr
     assert status(ld_x=32) == -2                                # ld_x < n
     assert status(m=262144 // 8 + 32, ld_y=1 << 20, batch=8) == -7      # beyond the fixed accumulator
     assert status(batch=9) == -1
+
+
+def _linear_status(rows, fmt=None, **kw):
+    """rptc_linear_forward's answer for a 1024 x 512 layer whose addresses are made up: for calls that are refused before a CUDA call."""
+    import torch
+
+    from rptc_b200 import Format, lib
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses stay off a GPU")
+    from rptc_b200._lib import Linear
+    layer = Linear(**{**dict(codes=1 << 12, lut=1 << 12, signs_in=1 << 12, signs_out=1 << 12, m=1024, n=512, block_in=512, block_out=1024, scale=1.0), **kw})
+    layer.fmt = fmt or Format(1, 2, 16, 8, 3)
+    return lib().rptc_linear_forward(ctypes.byref(layer), 1 << 12, 1 << 16, rows, 1 << 20, 1 << 40, None)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 9, 40, 97, 512])
+@pytest.mark.parametrize("name", ["signs_in", "signs_out"])
+def test_layers_refuse_signs_off_16_byte_boundaries(rows, name):
+    """Whichever kernels the number of rows leads to: they read signs sixteen bytes at a time."""
+    assert _linear_status(rows, **{name: (1 << 12) + 2}) == -3
+    assert _linear_status(rows, **{name: (1 << 12) + 8}) == -3
 
 
 def test_status_strings_cover_every_code():
