@@ -15,7 +15,7 @@ static bool alone_plan(AlonePlan &a, int64_t m, int64_t n, int64_t rows, int blo
     // The transform in every CTA pays for one short row, whose call is bound by the host's launches: 11.0 us a call with a kernel in front, 9.1
     // (3072 x 2304) and 10.8 (4096 x 4096, from 12.8) without; on the device alone 7.2 and 8.6, 8.9 and 9.2, since nothing but the
     // wait may lie in front of the first loads.  Two rows of 4096: 11.1 against 12.0; 4096 x 5120: 11.0 and 12.7.
-    if (block && (rows > 1 || n > 4096 || block < 8 || block > 4096 || (block & (block - 1)) || n % (block < 256 ? 256 : block))) return false;
+    if (block != kNoTransform && (rows > 1 || n > 4096 || block < 8 || block > 4096 || (block & (block - 1)) || n % (block < 256 ? 256 : block))) return false;
     const int64_t units = n / (128 / f.K), blocks = m / 32, total = blocks * units;
     if (total >= (int64_t(1) << 31)) return false;
     int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
@@ -43,12 +43,12 @@ bool gemv_alone_takes(int64_t m, int64_t n, int64_t rows, int block, const Banks
 }
 int64_t gemv_alone_partials(int64_t m, int64_t n, int64_t rows, const Banks &banks, const rptc_format &f) {
     AlonePlan a;
-    return alone_plan(a, m, n, rows, 0, banks, f) ? a.slots * rows * banks.banks * m : 0;
+    return alone_plan(a, m, n, rows, kNoTransform, banks, f) ? a.slots * rows * banks.banks * m : 0;
 }
 int gemv_alone(const void *codes, const void *lut, const uint32_t *carry_in, const GemvInput &in, float *partial, int64_t m, int64_t n, int64_t rows,
                const Banks &banks, const rptc_format &f, cudaStream_t stream, GemvSums *sums) {
     AlonePlan a;
-    if (!alone_plan(a, m, n, rows, in.scales_in ? 0 : in.block, banks, f)) return RPTC_ERR_UNSUPPORTED;
+    if (!alone_plan(a, m, n, rows, in.scales_in ? kNoTransform : in.block, banks, f)) return RPTC_ERR_UNSUPPORTED;
     GemvAlone p = {};
     p.codes = static_cast<const uint4 *>(codes);
     p.lut = static_cast<const __half *>(lut);

@@ -207,17 +207,21 @@ static bool many_rows(int64_t rows, int64_t n, int block, const HadParams &p) {
            (!p.residual || on_32_bytes(p.residual, p.ld_res * 2));
 }
 
+// Blocks of 8 to 4096 columns, a power of two, in rows of whole warps of them.
+int check_blocks(int64_t n, int block) {
+    if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
+    return n <= 0 || n % (block < 256 ? 256 : block) ? RPTC_ERR_SHAPE : RPTC_OK;
+}
 int check_signs(const void *signs) { return reinterpret_cast<uintptr_t>(signs) & 15 ? RPTC_ERR_ALIGN : RPTC_OK; }      // read sixteen bytes at a time
 
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late) {
     if (!in || !out) return RPTC_ERR_ARG;
-    if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
-    if (rows <= 0 || n <= 0 || (n % block) || ld_in < n || ld_out < n || (residual && ld_res < n)) return RPTC_ERR_SHAPE;
+    if (int e = check_blocks(n, block)) return e;
+    if (rows <= 0 || ld_in < n || ld_out < n || (residual && ld_res < n)) return RPTC_ERR_SHAPE;
     if (rows > 65535) return RPTC_ERR_TOO_LARGE;
     const int chunk = block < 256 ? 256 : block;
-    if (n % chunk) return RPTC_ERR_SHAPE;
     if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15) ||
         check_signs(signs) || (residual && (reinterpret_cast<uintptr_t>(residual) & 15)) ||
         (ld_in % 8) || (ld_out % 8) || (residual && (ld_res % 8)))
@@ -257,10 +261,9 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
 bool hadamard_takes_sums(int64_t rows, int64_t n, int block) { return block > 256 ? rows < 32 && block < 4096 : rows <= 96 && rows * n < (int64_t(5) << 19); }
 int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
                      int block, float scale, cudaStream_t stream) {
-    if (block < 8 || block > 4096 || (block & (block - 1))) return RPTC_ERR_ARG;
-    const int chunk = block < 256 ? 256 : block;
-    if (n % chunk) return RPTC_ERR_SHAPE;
+    if (int e = check_blocks(n, block)) return e;
     if (int e = check_signs(signs)) return e;
+    const int chunk = block < 256 ? 256 : block;
     HadSumsParams p = {};
     p.in = partial;
     p.ld_in = ld;

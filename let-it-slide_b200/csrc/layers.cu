@@ -21,6 +21,7 @@ int check_format(const rptc_format *f);   // api.cu
 int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, int64_t ld_out, const void *signs, const void *residual,
                        int64_t ld_res, int64_t rows, int64_t n, int block, int transpose, float scale, int clear_in, float *clear,
                        int64_t clear_count, cudaStream_t stream, bool late = false);
+int check_blocks(int64_t n, int block);
 int check_signs(const void *signs);
 // out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]; for how many rows that is as fast as adding them up in a
 // kernel in front
@@ -153,7 +154,7 @@ static Banks packed_banks(const rptc_packed &l) {
 
 // One or two tokens: no kernel in front of the product.
 static bool packed_alone(const rptc_packed &l, int64_t tokens) {
-    return gemv_alone_takes((int64_t)l.bank_blocks * 32, l.n, tokens, 0, packed_banks(l), packed_format(l));
+    return gemv_alone_takes((int64_t)l.bank_blocks * 32, l.n, tokens, kNoTransform, packed_banks(l), packed_format(l));
 }
 
 template <typename T>
@@ -290,6 +291,10 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
     auto misaligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
     if (misaligned(l->codes) || misaligned(l->lut) || misaligned(x) || misaligned(y) || misaligned(workspace) || (l->n % 8) || (l->m % 8))
         return RPTC_ERR_ALIGN;
+    if (l->signs_in) {
+        if (int e = check_blocks(l->n, l->block_in)) return e;
+        if (int e = check_blocks(l->m, l->block_out)) return e;
+    }
     if (int e = check_signs(l->signs_in)) return e;
     if (int e = check_signs(l->signs_out)) return e;
     if (int e = rptc_check_device()) return e;

@@ -72,7 +72,8 @@ struct GemvSums {
     }
 #endif
 };
-// Whether gemv_alone takes the layer (`block`: of the Hadamard transform, 0 with scales_in), and the fp32 values of room for its sums.
+// Whether gemv_alone takes the layer (`block`: of the Hadamard transform, kNoTransform with scales_in), and the fp32 values of room for its sums.
+constexpr int kNoTransform = -1;
 bool gemv_alone_takes(int64_t m, int64_t n, int64_t rows, int block, const Banks &banks, const rptc_format &f);
 int64_t gemv_alone_partials(int64_t m, int64_t n, int64_t rows, const Banks &banks, const rptc_format &f);
 // partial[slot][row of x][bank * m + row] for slot < sums.count(row)

@@ -96,6 +96,14 @@ def test_layers_refuse_signs_off_16_byte_boundaries(rows, name):
     assert _linear_status(rows, **{name: (1 << 12) + 8}) == -3
 
 
+@pytest.mark.parametrize("rows", [1, 2, 9, 40, 97, 512])
+@pytest.mark.parametrize("name", ["block_in", "block_out"])
+def test_layers_refuse_blocks_that_no_transform_has(rows, name):
+    """Whichever kernels the number of rows leads to, and before any of them is launched."""
+    for block, status in ((0, -1), (-1, -1), (-8, -1), (4, -1), (8192, -1), (768, -1), (1024 if name == "block_in" else 2048, -2)):
+        assert _linear_status(rows, **{name: block}) == status, block
+
+
 def test_status_strings_cover_every_code():
     from rptc_b200 import lib
     for code in range(-10, 1):
