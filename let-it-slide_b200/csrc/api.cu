@@ -216,6 +216,19 @@ static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
 }
 }  // namespace rptc
 
+namespace rptc {
+static bool overlap(const void *a, int64_t a_bytes, const void *b, int64_t b_bytes) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + (uintptr_t)b_bytes && q < p + (uintptr_t)a_bytes;
+}
+// Whether y may be written while the product is under way: a CTA of gemv_whole stores its rows when others still read (x == y with m == n is
+// a call that the product with a kernel behind it answers).
+static bool written_apart(const void *y, const void *codes, const void *lut, const void *x, int64_t m, int64_t n, const rptc_format &f) {
+    const int64_t lut_bytes = f.code == RPTC_CODE_LUT ? int64_t(2) << f.L : int64_t(4) << f.S;
+    return !overlap(y, 2 * m, x, 2 * n) && !overlap(y, 2 * m, lut, lut_bytes) && !overlap(y, 2 * m, codes, m * n / 8 * f.K);
+}
+}  // namespace rptc
+
 extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x, float *acc, void *y, int64_t m, int64_t n, int x_order,
                                int accumulate, const rptc_format *fmt, float *ms, rptc_stream_t stream) {
     if (!y || !ms) return RPTC_ERR_ARG;
@@ -223,11 +236,13 @@ extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x
     if (int e = rptc_check_device()) return e;
     const int dev = current_device();
     if (dev < 0) return cuda_fail(cudaErrorNoDevice);
-    if (int e = g_waited[dev].ready()) return e;
-    WaitedTimer &t = g_waited[dev];
-    const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
-    if (e == RPTC_OK) return wait_for(t, static_cast<cudaStream_t>(stream), ms);
-    if (e != RPTC_ERR_UNSUPPORTED) return e;
+    if (written_apart(y, codes, lut, x, m, n, *fmt)) {
+        if (int e = g_waited[dev].ready()) return e;
+        WaitedTimer &t = g_waited[dev];
+        const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
+        if (e == RPTC_OK) return wait_for(t, static_cast<cudaStream_t>(stream), ms);
+        if (e != RPTC_ERR_UNSUPPORTED) return e;
+    }
     if (int e = rptc_timer_begin(stream)) return e;
     if (int e = rptc_gemv(codes, lut, nullptr, x, n, acc, m, m, n, 1, x_order, fmt, stream)) return e;
     {

@@ -233,3 +233,29 @@ def test_timed_matvec_stores_and_adds(code, K, L, S, layout, x_order, quirk, m, 
     assert (y.float() - 2 * first.float()).abs().max().item() <= (2e-5 * 16 + 2.0**-9) * scale
     assert not acc.any()
     ops.device_status()
+
+
+@pytest.mark.parametrize("layout", [o.LAYOUT_ROWMAJOR, o.LAYOUT_CHUNKED])
+@pytest.mark.parametrize("m,n,at", [(2048, 2048, 0), (8192, 8192, 0), (4096, 4096, 1024), (1024, 6144, 5120), (6144, 2048, 2046)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_timed_matvec_whose_result_replaces_its_activations(layout, m, n, at, accumulate):
+    """y lies over x, all of it or a part: the product reads x as it was before the call."""
+    from rptc_b200 import Format, ops
+    from rptc_b200._lib import native
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    fmt = Format(o.CODE_B, 2, 16, 8, layout)
+    codes = torch.randint(-2**31, 2**31 - 1, (m * n * 2 // 32,), dtype=torch.int32, device="cuda", generator=g)
+    lut = torch.randn(fmt.lut_numel(), dtype=torch.float16, device="cuda", generator=g)
+    room = torch.randn(max(n, at + m), dtype=torch.float16, device="cuda", generator=g)
+    x, y = room[:n], room[at:at + m]
+    before = room.clone()
+    acc = torch.zeros((1, m), device="cuda")
+    ops.gemv_acc(codes, lut, x, acc, m, n, fmt)
+    want = acc[0] + (y.float() if accumulate else 0.0)
+    acc.zero_()
+    assert native().gemv_timed(codes, lut, x, acc, y, m, n, 0, accumulate, fmt) > 0
+    scale = want.abs().max().item()
+    # the same fp16 products, summed in another order in fp32, rounded to fp16 (twice where the result is added to y)
+    assert (y.float() - want).abs().max().item() <= (2e-5 * 16 + 2.0**-10) * scale
+    before[at:at + m] = y
+    assert torch.equal(room, before)
