@@ -174,29 +174,6 @@ extern "C" int rptc_timer_end(float *ms, rptc_stream_t stream) {
 
 // ---- a matvec whose caller waits for it ----
 namespace rptc {
-// A thread's timer on a device; kept, and given back when the thread ends.
-struct WaitedTimer {
-    HostTime *host = nullptr;
-    DeviceTime *device = nullptr;
-    unsigned int ticket = 0;
-    ~WaitedTimer() { release(); }
-    void release() {
-        if (device) cudaFree(device);      // waits for a kernel that may still write
-        if (host) cudaFreeHost(host);
-        device = nullptr, host = nullptr;
-    }
-    int ready() {
-        if (device) return RPTC_OK;
-        const DeviceTime none = {~0ull, 0u};
-        RPTC_CUDA(cudaHostAlloc(&host, sizeof(HostTime), cudaHostAllocMapped));
-        host->ticket = ticket;
-        DeviceTime *d = nullptr;
-        RPTC_CUDA(cudaMalloc(&d, sizeof(DeviceTime)));
-        device = d;
-        RPTC_CUDA(cudaMemcpy(device, &none, sizeof(none), cudaMemcpyHostToDevice));
-        return RPTC_OK;
-    }
-};
 static thread_local WaitedTimer g_waited[kMaxDevices];
 // Until the kernel with `ticket` has left its time.  The stream is asked now and then: work that failed leaves none.
 static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
@@ -214,9 +191,6 @@ static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
     *ms = (float)((double)h->ns * 1e-6);
     return RPTC_OK;
 }
-}  // namespace rptc
-
-namespace rptc {
 static bool overlap(const void *a, int64_t a_bytes, const void *b, int64_t b_bytes) {
     const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
     return p < q + (uintptr_t)b_bytes && q < p + (uintptr_t)a_bytes;
@@ -236,12 +210,11 @@ extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x
     if (int e = rptc_check_device()) return e;
     const int dev = current_device();
     if (dev < 0) return cuda_fail(cudaErrorNoDevice);
-    if (written_apart(y, codes, lut, x, m, n, *fmt)) {
-        if (int e = g_waited[dev].ready()) return e;
+    if (gemv_whole_takes(m, n, *fmt) && written_apart(y, codes, lut, x, m, n, *fmt)) {
         WaitedTimer &t = g_waited[dev];
+        RPTC_CUDA(t.ready());
         const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
-        if (e == RPTC_OK) return wait_for(t, static_cast<cudaStream_t>(stream), ms);
-        if (e != RPTC_ERR_UNSUPPORTED) return e;
+        return e == RPTC_OK ? wait_for(t, static_cast<cudaStream_t>(stream), ms) : e;
     }
     if (int e = rptc_timer_begin(stream)) return e;
     if (int e = rptc_gemv(codes, lut, nullptr, x, n, acc, m, m, n, 1, x_order, fmt, stream)) return e;

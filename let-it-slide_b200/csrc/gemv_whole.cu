@@ -174,9 +174,16 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_whole_kernel(const GemvW
     if (threadIdx.x == 0) p.timer.end(gridDim.x);
 }
 
+static size_t whole_smem(int64_t n, const rptc_format &f) {
+    const int64_t chunks = (n / (128 / f.K) + 31) / 32;
+    return fixed_smem(f, kUnitsRing + kUnitsHist + kWholeSums + kWholeParts) + (size_t)chunks * 32 * (128 / f.K) * 2;
+}
+bool gemv_whole_takes(int64_t m, int64_t n, const rptc_format &f) {
+    return (f.layout == RPTC_LAYOUT_ROWMAJOR || f.layout == RPTC_LAYOUT_CHUNKED) && (f.K == 2 || f.K == 4) && whole_smem(n, f) <= kMaxSmem;
+}
 int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64_t m, int64_t n, int x_order, int accumulate, const rptc_format &f,
                const DeviceTimer &timer, cudaStream_t stream) {
-    if ((f.layout != RPTC_LAYOUT_ROWMAJOR && f.layout != RPTC_LAYOUT_CHUNKED) || (f.K != 2 && f.K != 4)) return RPTC_ERR_UNSUPPORTED;
+    if (!gemv_whole_takes(m, n, f)) return RPTC_ERR_UNSUPPORTED;
     GemvWhole p = {};
     p.codes = static_cast<const uint4 *>(codes);
     p.lut = static_cast<const __half *>(lut);
@@ -195,8 +202,7 @@ int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64
     p.accumulate = accumulate;
     p.timer = timer;
     const int64_t chunks = (p.n_units + 31) / 32;
-    const size_t smem = fixed_smem(f, kUnitsRing + kUnitsHist + kWholeSums + kWholeParts) + (size_t)chunks * 32 * (128 / f.K) * 2;
-    if (smem > kMaxSmem) return RPTC_ERR_UNSUPPORTED;
+    const size_t smem = whole_smem(n, f);
     const int ctas = (int)(m < num_sms() ? m : num_sms());
     // warps that share a row's chunks: as many as leave no warp without one (kWholeParts holds 16 x 4 sums)
     const int64_t rows = (m + ctas - 1) / ctas;

@@ -2,6 +2,7 @@
 // and the rows of W may come in banks that each have a lookup table of their own.
 #pragma once
 #include "common.cuh"
+#include "waited_timer.cuh"
 
 namespace rptc {
 
@@ -40,7 +41,7 @@ int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const
 int gemv_banked(const void *codes, const void *lut, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m, int64_t n, int64_t tokens,
                 const Banks &banks, const rptc_format &f, cudaStream_t stream, bool ordered = false, float *partial = nullptr);
 
-// ---- one or two activation rows, as the first kernel of a layer's call (gemv.cu) ----
+// ---- one or two activation rows, as the first kernel of a layer's call (gemv_alone.cu) ----
 // The input side that the product makes in its CTAs.
 struct GemvInput {
     const void *x;                       // [batch][n]: fp16, or with scales_in fp16, bf16, fp32 (dtype 0, 1, 2)
@@ -80,45 +81,12 @@ int64_t gemv_alone_partials(int64_t m, int64_t n, int64_t rows, const Banks &ban
 int gemv_alone(const void *codes, const void *lut, const uint32_t *carry_in, const GemvInput &in, float *partial, int64_t m, int64_t n, int64_t rows,
                const Banks &banks, const rptc_format &f, cudaStream_t stream, GemvSums *sums);
 
-// ---- a matvec whose caller waits for it ----
-// The device time of a kernel, left in host memory by the last of its CTAs together with `ticket`, which tells the waiting thread that
-// the kernel's results are there.
-struct HostTime {
-    unsigned long long ns;
-    unsigned int ticket;
-};
-struct DeviceTime {
-    unsigned long long begin;            // earliest start; all ones between kernels
-    unsigned int ended;                  // CTAs that have; 0 between kernels
-};
-struct DeviceTimer {
-    DeviceTime *device;
-    HostTime *host;                      // pinned, as the device sees it
-    unsigned int ticket;
-#ifdef __CUDACC__
-    static __device__ __forceinline__ unsigned long long now() {
-        unsigned long long t;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)::"memory");
-        return t;
-    }
-    __device__ __forceinline__ void begin() const { atomicMin(&device->begin, now()); }
-    // by one thread of each of `ctas` CTAs, behind a barrier behind its last result
-    __device__ __forceinline__ void end(unsigned int ctas) const {
-        __threadfence();
-        if (atomicAdd(&device->ended, 1u) + 1u != ctas) return;
-        __threadfence();
-        const unsigned long long from = atomicExch(&device->begin, ~0ull);
-        device->ended = 0u;
-        *reinterpret_cast<volatile unsigned long long *>(&host->ns) = now() - from;
-        __threadfence_system();
-        *reinterpret_cast<volatile unsigned int *>(&host->ticket) = ticket;
-    }
-#endif
-};
+// ---- a matvec whose caller waits for it (gemv_whole.cu) ----
 int validate_gemv_args(const void *codes, const void *lut, const void *x, int64_t ld_x, const float *acc, int64_t ld_acc, int64_t m, int64_t n, int batch,
                        int x_order, const rptc_format *fmt);
-// y = (or +=) W x, one row, codes whose units of a row lie together (ROWMAJOR, CHUNKED); RPTC_ERR_UNSUPPORTED, and nothing is launched, for others
-// and for rows that do not fit into shared memory.  The arguments have been checked.
+// y = (or +=) W x, one row, for codes whose units of a row lie together (ROWMAJOR, CHUNKED) and rows that fit into shared memory
+// (gemv_whole_takes).  The arguments have been checked, and y lies over none of them.
+bool gemv_whole_takes(int64_t m, int64_t n, const rptc_format &f);
 int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64_t m, int64_t n, int x_order, int accumulate, const rptc_format &f,
                const DeviceTimer &timer, cudaStream_t stream);
 
