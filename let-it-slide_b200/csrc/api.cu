@@ -167,6 +167,7 @@ extern "C" int rptc_timer_end(float *ms, rptc_stream_t stream) {
     if (int e = rptc_check_device()) return e;
     if (int e = timer_events(t)) return e;
     RPTC_CUDA(cudaEventRecord(t->end, static_cast<cudaStream_t>(stream)));
+    BesideCaptures mode;
     RPTC_CUDA(cudaEventSynchronize(t->end));
     RPTC_CUDA(cudaEventElapsedTime(ms, t->begin, t->end));
     return RPTC_OK;
@@ -181,6 +182,7 @@ static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
     for (unsigned int spin = 1;; ++spin) {
         if (h->ticket == t.ticket) break;
         if (spin % 4096) continue;
+        BesideCaptures mode;
         const cudaError_t e = cudaStreamQuery(stream);
         if (e == cudaErrorNotReady) continue;
         if (e == cudaSuccess && h->ticket == t.ticket) break;
@@ -212,6 +214,9 @@ extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x
     if (dev < 0) return cuda_fail(cudaErrorNoDevice);
     if (gemv_whole_takes(m, n, *fmt) && written_apart(y, codes, lut, x, m, n, *fmt)) {
         WaitedTimer &t = g_waited[dev];
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        RPTC_CUDA(cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture));
+        if (capture != cudaStreamCaptureStatusNone) return cuda_fail(cudaErrorStreamCaptureUnsupported);      // nothing to wait for
         RPTC_CUDA(t.ready());
         const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
         return e == RPTC_OK ? wait_for(t, static_cast<cudaStream_t>(stream), ms) : e;

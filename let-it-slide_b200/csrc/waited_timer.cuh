@@ -41,6 +41,18 @@ struct DeviceTimer {
 #endif
 };
 
+// While a thread captures a graph in the default mode, calls that allocate or wait are refused to every thread, and spoil the capture
+// (cudaMalloc, cudaEventSynchronize and cudaStreamQuery do).  Those here touch no captured stream, which this tells the runtime.
+class BesideCaptures {
+public:
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    BesideCaptures(const BesideCaptures &) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;      // the thread's own meanwhile
+};
+
 // A thread's timer on a device; kept, and given back when the thread ends.
 struct WaitedTimer {
     HostTime *host = nullptr;
@@ -49,6 +61,7 @@ struct WaitedTimer {
     ~WaitedTimer() { release(); }
     void release() {
         if (!device) return;
+        BesideCaptures mode;
         cudaFree(device);                  // waits for a kernel that may still write
         cudaFreeHost(host);
         device = nullptr, host = nullptr;
@@ -56,6 +69,7 @@ struct WaitedTimer {
     // All of it or nothing: a timer that could not be set up is set up by the next call.
     cudaError_t ready() {
         if (device) return cudaSuccess;
+        BesideCaptures mode;
         HostTime *h = nullptr;
         DeviceTime *d = nullptr;
         cudaStream_t s = nullptr;
