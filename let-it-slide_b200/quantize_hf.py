@@ -68,6 +68,11 @@ def factorize(W: torch.Tensor):
 _SORT_AT_ONCE = 1 << 25      # values sorted at once: a sort takes about 20 bytes a value beside them, 0.6 GB
 
 
+def _values_only(t: torch.Tensor) -> bool:
+    """Whether nothing follows what is done with t (autograd, forward mode, vmap), so that a kernel may take its values."""
+    return not t.requires_grad and not torch._C._functorch.is_functorch_wrapped_tensor(t) and torch.autograd.forward_ad.unpack_dual(t).tangent is None
+
+
 def megabatch_alphabets(megabatches: torch.Tensor, shift_register_size: int) -> torch.Tensor:
     """2^L evenly spaced quantiles of each bank's values, megabatches [banks, values] -> fp32 [banks, 2^L], by linear
     interpolation of the sorted sample (quantize_hf.py:136-140).  Interpolated in float64 and rounded to fp32."""
@@ -77,7 +82,7 @@ def megabatch_alphabets(megabatches: torch.Tensor, shift_register_size: int) -> 
     M = 1 << shift_register_size
     fp = torch.sort(megabatches, dim=1).values
     N = fp.shape[1]
-    if fp.is_cuda and fp.dtype == torch.float32 and fp.numel() and fp.shape[0] <= 65535 and 1 <= shift_register_size <= 16:
+    if fp.is_cuda and fp.dtype == torch.float32 and fp.numel() and fp.shape[0] <= 65535 and 1 <= shift_register_size <= 16 and _values_only(fp):
         return ops.quantiles(fp.contiguous(), shift_register_size)
     x = (2 * torch.arange(M, dtype=torch.float64, device=fp.device) + 1) / 2 / M
     pos = x * N - 0.5                                  # position of x on the sample grid xp[j] = (2j+1)/(2N)

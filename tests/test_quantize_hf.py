@@ -240,6 +240,26 @@ def test_alphabets_on_the_gpu_are_those_of_the_tensor_operations(banks, values, 
 
 
 @pytest.mark.gpu
+def test_alphabets_on_the_gpu_can_be_differentiated():
+    """Reverse mode, forward mode and vmap, as on the CPU: a kernel that takes values only stands aside."""
+    import quantize_hf as q
+    g = torch.Generator().manual_seed(5)
+    x, t, up = torch.randn(3, 1000, generator=g), torch.randn(3, 1000, generator=g), torch.randn(3, 256, generator=g)
+    f = lambda a: q.megabatch_alphabets(a, 8)
+    grads = []
+    for dev in ("cpu", "cuda"):
+        a = x.clone().to(dev).requires_grad_()
+        y = f(a)
+        y.backward(up.to(dev))
+        grads.append((y.detach().cpu(), a.grad.cpu(), torch.func.jvp(f, (x.to(dev),), (t.to(dev),))[1].cpu(),
+                      torch.func.vmap(f)(x.to(dev).reshape(3, 1, 1000)).cpu().reshape(3, 256)))
+    for a, b in zip(*grads):
+        torch.testing.assert_close(b, a, rtol=1e-6, atol=1e-7)       # the sums of a gradient meet in any order
+    with torch.no_grad():
+        assert torch.equal(f(x.cuda().requires_grad_()).cpu(), grads[0][0])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,banks", [(128, 64, 1), (352, 1088, 4), (4096, 2048, 32)])
 @pytest.mark.parametrize("tokens", [145, 192, 193, 256, 257, 520])
 def test_packed_layer_whose_table_leaves_two_stages_of_tokens(m, n, banks, tokens):
