@@ -382,12 +382,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     } else if (kOneRing || lane == 0) {
         // ================= MMA issue =================
         RingPos px = {0, 0u}, pw = {0, 0u};
-        for (int it = 0; it < n_steps && ok; ++it) {
-            ok = (kOneRing || mbar_wait(bars.full_x + 8 * px.s, px.phase, p.status)) && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
-            if (!ok) break;
+        for (int it = 0; it < n_steps; ++it) {
+            const bool issues = !kOneRing || elect_one();
+            if (kOneRing) {
+                ok = ok && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
+            } else {
+                ok = mbar_wait(bars.full_x + 8 * px.s, px.phase, p.status) && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
+                if (!ok) break;
+            }
             tc_fence_after();
             const uint64_t xa = umma_desc_sw128(p.xa_addr[px.s]), xb = umma_desc_sw128(p.xb_addr[px.s]), wd = umma_desc_sw128(p.w_addr[pw.s]);
-            if (!kOneRing || elect_one()) {
+            if (issues && ok) {
 #pragma unroll
                 for (uint32_t k = 0; k < kStepCols / 16; ++k) {           // + 32 bytes per K = 16
                     tc_mma_f16(tmem_base, xa + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
@@ -400,7 +405,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             px.advance(p.n_xstages);
             pw.advance(p.n_wstages);
         }
-        if (ok && (!kOneRing || elect_one())) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
+        if ((!kOneRing || elect_one()) && ok) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
     }
     __syncwarp();
 

@@ -298,18 +298,19 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
 #pragma unroll
         for (int q = 0; q < RINGS; ++q) px[q] = {0, 1u};
         const uint32_t bytes = 128u * (uint32_t)p.n_cols;
-        for (uint32_t pos = c0; pos < c1 && ok;) {
+        for (uint32_t pos = c0; pos < c1;) {
             const FewSegment<SHARED> g(pos, c1, p);
             pos = g.end;
             const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
-            for (int32_t j = 0; j < rounds && ok; ++j)
+            for (int32_t j = 0; j < rounds; ++j)
 #pragma unroll
                 for (int q = 0; q < PARTS; ++q) {
                     const int32_t s = g.part_begin<PARTS>(q) + j;
-                    if (s >= g.part_begin<PARTS>(q + 1) || !ok) continue;
+                    if (s >= g.part_begin<PARTS>(q + 1)) continue;
                     const int ring = SHARED ? 0 : q, stage = ring * p.n_xstages + px[ring].s;
-                    ok = mbar_wait(empty_x + 8 * stage, px[ring].phase, p.status);
-                    if (ok && elect_one()) {
+                    const bool issues = elect_one();
+                    ok = ok && mbar_wait(empty_x + 8 * stage, px[ring].phase, p.status);
+                    if (issues && ok) {
                         mbar_expect_tx(full_x + 8 * stage, bytes);
                         tma_load_2d(p.x_addr + (uint32_t)stage * bytes, &x_map, s * 64, g.t0, full_x + 8 * stage);
                     }
@@ -326,48 +327,43 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
         const uint32_t d_tmem = tmem + (uint32_t)(grp * p.n_sums * p.n_cols), a_first = a_cols + 32u * (uint32_t)grp;
         // the four MMAs of a step go round the accumulators
         const uint32_t d1 = p.n_sums == 2 ? (uint32_t)p.n_cols : 0u;
-        for (uint32_t pos = c0; pos < c1 && ok; ++seg) {
+        for (uint32_t pos = c0; pos < c1; ++seg) {
             const FewSegment<SHARED> g(pos, c1, p);
             pos = g.end;
-            if (seg > 0) ok = mbar_wait(drained, (seg - 1) & 1u, p.status);      // the last segment's sums have been taken
+            if (seg > 0) ok = ok && mbar_wait(drained, (seg - 1) & 1u, p.status);      // the last segment's sums have been taken
             tc_fence_after();
             const int32_t rounds = (g.s1 - g.s0 + PARTS - 1) / PARTS;
             uint32_t accumulate = 0u;
-            for (int32_t j = 0; j < rounds && ok; ++j)
+            for (int32_t j = 0; j < rounds; ++j)
 #pragma unroll
                 for (int q = 0; q < PARTS; ++q) {
                     if (!(SHARED || q == mine) || g.part_begin<PARTS>(q) + j >= g.part_begin<PARTS>(q + 1)) continue;
-                    if (ok) {
-                        const int from = SHARED ? q * RB : 0;                // + grp: the group whose step it is
-                        const int stage = ring + px.s;
-                        ok = mbar_wait(full_x + 8 * stage, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), SHARED ? (a_phase >> q) & 1u : a_phase, p.status);
-                        a_phase ^= SHARED ? 1u << q : 1u;
-                        if (ok) {
-                            tc_fence_after();
-                            const uint32_t a_tmem = a_first + 32u * (uint32_t)from;
-                            const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)stage * bytes);
-                            if (elect_one()) {
-                                // + 32 bytes of shared memory, + 8 columns of tensor memory per K = 16
-                                tc_mma_f16_ta(d_tmem, a_tmem, xb, idesc, accumulate);
-                                tc_mma_f16_ta(d_tmem + d1, a_tmem + 8u, xb + 2u, idesc, accumulate | (uint32_t)(p.n_sums == 1));
-                                tc_mma_f16_ta(d_tmem, a_tmem + 16u, xb + 4u, idesc, 1u);
-                                tc_mma_f16_ta(d_tmem + d1, a_tmem + 24u, xb + 6u, idesc, 1u);
-                                tc_commit(empty_a + 8 * (grp + from));
-                                tc_commit(empty_x + 8 * stage);
-                            }
-                            __syncwarp();
-                            accumulate = 1u;
-                        }
+                    const int from = SHARED ? q * RB : 0;                // + grp: the group whose step it is
+                    const int stage = ring + px.s;
+                    const bool issues = elect_one();
+                    ok = ok && mbar_wait(full_x + 8 * stage, px.phase, p.status) && mbar_wait(full_a + 8 * (grp + from), SHARED ? (a_phase >> q) & 1u : a_phase, p.status);
+                    a_phase ^= SHARED ? 1u << q : 1u;
+                    tc_fence_after();
+                    const uint32_t a_tmem = a_first + 32u * (uint32_t)from;
+                    const uint64_t xb = umma_desc_sw128(p.x_addr + (uint32_t)stage * bytes);
+                    if (issues && ok) {
+                        // + 32 bytes of shared memory, + 8 columns of tensor memory per K = 16
+                        tc_mma_f16_ta(d_tmem, a_tmem, xb, idesc, accumulate);
+                        tc_mma_f16_ta(d_tmem + d1, a_tmem + 8u, xb + 2u, idesc, accumulate | (uint32_t)(p.n_sums == 1));
+                        tc_mma_f16_ta(d_tmem, a_tmem + 16u, xb + 4u, idesc, 1u);
+                        tc_mma_f16_ta(d_tmem + d1, a_tmem + 24u, xb + 6u, idesc, 1u);
+                        tc_commit(empty_a + 8 * (grp + from));
+                        tc_commit(empty_x + 8 * stage);
                     }
+                    __syncwarp();
+                    accumulate = 1u;
                     px.advance(p.n_xstages);
                 }
-            if (ok) {
-                if (elect_one()) {
-                    if (accumulate) tc_commit(sums);
-                    else mbar_arrive(sums);          // no step of this segment
-                }
-                __syncwarp();
+            if (elect_one() && ok) {
+                if (accumulate) tc_commit(sums);
+                else mbar_arrive(sums);          // no step of this segment
             }
+            __syncwarp();
         }
     }
     tc_fence_before();

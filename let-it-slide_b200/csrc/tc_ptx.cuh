@@ -81,7 +81,10 @@ __device__ __forceinline__ void tma_prefetch_map(const void *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
-// True in one lane of a converged warp.
+// True in one lane of a warp, all of whose lanes have to come here.  Lanes of a warp that waits as a whole may run out of tries one by one (the
+// barrier completes at the others' last), so a lane whose wait gave up goes on with its warp to the end of the loop: it waits no more,
+// and issues nothing if it is the elected one.  Elected in front of the wait: behind it 1 % more time (4096 x 11008 HASH, 400 tokens in
+// tiles of 128 x 128 69.4 us against 68.3).
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
