@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
     }
 }
 
-// Walks a row's winners from position `hi` down to `lo`; returns the state at position lo - 1, and with WRITE sets the symbols on the
-// way.  A position's winner is needed to know which winner of the position before it to read, but with two bits each there are only
+// Walks a row's winners from position `hi` down to `lo`; returns the state at position lo - 1 (TO_START: lo is 0 and nothing is in front), and
+// with WRITE sets the symbols on the way.  A position's winner is needed to know which winner of the position before it to read, but with two bits each there are only
 // four (sixteen) candidates one (two) positions on: lanes 0, 1-4 and 5-20 fetch all of them at once, and the walk takes three
 // positions per trip to memory.
 struct TracedRow {
@@ -319,7 +319,7 @@ struct TracedRow {
     int32_t *symbols;
     int64_t Q;
     int L;
-    template <bool WRITE>
+    template <bool WRITE, bool TO_START = false>
     __device__ __forceinline__ uint32_t walk(uint32_t state, int64_t hi, int64_t lo) const {
         const int lane = threadIdx.x & 31;
         const int level = lane == 0 ? 0 : lane < 5 ? 1 : 2;
@@ -340,30 +340,36 @@ struct TracedRow {
                 const uint32_t mine = lane == 0 ? state : lane == 1 ? s1 : s2;
                 if (lane < 3 && i - lane >= lo) symbols[i - lane] = (int32_t)(mine & 3u);
             }
-            state = i - lo >= 2 ? before(s2, w2) : i == lo ? s1 : s2;
+            state = TO_START || i - lo >= 2 ? before(s2, w2) : i == lo ? s1 : s2;
         }
         return state;
     }
 };
 
-// A CTA per row, its positions in equal pieces, a warp each.  The last piece starts from the row's final state.  Which state the path
+// PIECES: a CTA per row, its positions in equal pieces, a warp each.  Without, four rows per CTA, a warp each.  The last piece starts from the row's final state.  Which state the path
 // passes at the end of another piece is not known yet, but walks from different states meet after some times the L / 2 positions that a
 // state remembers: such a warp starts kMeet * L positions further on from any state, and writes symbols from its own piece on.  Pieces whose
 // state is not the one that the piece behind was left with are walked again from that one, all of them at once, until all fit (at
 // L = 16 most of them once).
 // Bound by the trips to memory one after the other: with a warp per row 256 rows of 1024 samples took 0.1 ms at L = 12.
-constexpr int kTraceWarps = 16, kMeet = 4;
-__global__ void __launch_bounds__(32 * kTraceWarps) viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state,
-                                                                             int64_t n, int L, int32_t *__restrict__ symbols, int64_t ld_sym,
-                                                                             int64_t piece, int pieces) {
+constexpr int kTraceWarps = 16, kTraceRows = 4, kMeet = 4;
+template <bool PIECES>
+__global__ void __launch_bounds__(32 * (PIECES ? kTraceWarps : kTraceRows))
+    viterbi_backtrack_kernel(const uint8_t *__restrict__ back, const int32_t *__restrict__ final_state, int64_t rows, int64_t n, int L,
+                             int32_t *__restrict__ symbols, int64_t ld_sym, int64_t piece, int pieces) {
     __shared__ uint32_t left[kTraceWarps];                      // state in front of a piece's first position
-    const int64_t row = blockIdx.x;
     const int c = threadIdx.x >> 5;
+    const int64_t row = PIECES ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kTraceRows + c;
+    if (!PIECES && row >= rows) return;
     TracedRow r;
     r.Q = int64_t(1) << (L - 4);
     r.L = L;
     r.back = back + row * n * r.Q;
     r.symbols = symbols + row * ld_sym;
+    if constexpr (!PIECES) {
+        r.walk<true, true>((uint32_t)final_state[row], n - 1, 0);
+        return;
+    }
     const int64_t lo = c * piece, hi = c + 1 < pieces ? lo + piece - 1 : n - 1;
     const int64_t from = min(n - 1, hi + kMeet * L);
     uint32_t state = from == n - 1 ? (uint32_t)final_state[row] : 0u;
@@ -487,14 +493,17 @@ extern "C" int rptc_viterbi_encode_rows(const float *alphabets, int64_t rows_per
     else if (L == 10) e = launch_forward<1, 2, 1>(p, 32, sms * 32, s);
     else e = launch_forward<1, 1, 1>(p, 32, sms * 32, s);
     if (e) return e;
-    // Pieces at least as long as the way to them, and only of rows too few to keep enough loads under way by themselves: pieces walk up to
-    // twice the positions.  Encoder with a warp a row / in pieces (us): L = 9 1024 rows 359 / 308, 4096 rows 1002 / 1067; L = 12 256 rows
-    // 473 / 391, 2048 rows 3243 / 3200; L = 14 128 rows 724 / 634, 1024 rows 1615 / 1669; L = 15 512 rows 1782 / 1832; L = 16 64 rows
-    // 1605 / 1532, 256 rows 4190 / 4154, 1024 rows 14126 / 14250.
-    const bool in_pieces = rows <= (L <= 12 ? 2048 : 256);
-    const int64_t most = !in_pieces || n < kMeet * L ? 1 : n / (kMeet * L) < kTraceWarps ? n / (kMeet * L) : kTraceWarps;
-    const int64_t piece = (n + most - 1) / most, pieces = (n + piece - 1) / piece;
-    viterbi_backtrack_kernel<<<(unsigned)rows, (unsigned)(32 * pieces), 0, s>>>(p.back, p.final_state, n, L, symbols, ld_sym, piece, (int)pieces);
+    // In pieces, at least as long as the way to them, where there are five of them or more and rows too few to keep enough loads under way
+    // by themselves: pieces walk up to twice the positions.  Whole encoder, a warp per row / in pieces (us): 512 x 1024 samples, L = 8 299 / 205,
+    // L = 12 658 / 542; 128 x 1024, L = 16 2233 / 2126; 1024 x 256, L = 9 93 / 85; 2048 x 4096, L = 9 2397 / 2071.  On the other side of the line
+    // 2048 x 256, L = 9 144 / 153; 4096 x 1024, L = 10 1550 / 1650; 1024 x 256, L = 15 1723 / 1763; 256 x 96, L = 11 49.6 / 53.7.
+    const int64_t most = n / (kMeet * L) < kTraceWarps ? n / (kMeet * L) : kTraceWarps;
+    if (most >= 5 && rows <= (L > 12 ? 256 : n >= 1024 ? 2048 : 1024)) {
+        const int64_t piece = (n + most - 1) / most, pieces = (n + piece - 1) / piece;
+        viterbi_backtrack_kernel<true><<<(unsigned)rows, (unsigned)(32 * pieces), 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym, piece, (int)pieces);
+    } else {
+        viterbi_backtrack_kernel<false><<<(unsigned)((rows + kTraceRows - 1) / kTraceRows), 32 * kTraceRows, 0, s>>>(p.back, p.final_state, rows, n, L, symbols, ld_sym, n, 1);
+    }
     RPTC_CUDA(cudaGetLastError());
     return RPTC_OK;
 }

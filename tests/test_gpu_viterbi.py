@@ -168,3 +168,19 @@ def test_trace_back_in_pieces(L, n, parted):
     got, loss = rptc.quantize_rows(alphabet.cuda(), weights.cuda(), samples.cuda())
     assert torch.equal(got.cpu(), want)
     torch.testing.assert_close(loss.cpu(), want_loss, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("L,n,rows", [(8, 159, 3), (8, 160, 3), (12, 239, 5), (12, 240, 5), (6, 1023, 1025), (6, 1024, 1025), (6, 130, 2049), (16, 320, 6)])
+def test_trace_back_by_a_warp_and_in_pieces(L, n, rows):
+    """Both sides of the lines between them (pieces of a row, rows), and rows that do not fill the last CTA of four."""
+    import rptc
+    g = torch.Generator().manual_seed(L + n + rows)
+    alphabet, weights, samples = torch.randn(1 << L, generator=g), 0.5 + torch.rand(n, generator=g), torch.randn(rows, n, generator=g)
+    got, loss = rptc.quantize_rows(alphabet.cuda(), weights.cuda(), samples.cuda())
+    some = slice(None) if rows < 8 else torch.cat([torch.arange(3), torch.arange(rows - 5, rows)])
+    want, want_loss = rptc.quantize_rows(alphabet, weights, samples[some])
+    assert torch.equal(got[some].cpu(), want)
+    torch.testing.assert_close(loss[some].cpu(), want_loss, rtol=1e-6, atol=0)
+    # the rest against itself: rows encoded by eights take a few CTAs
+    for r0 in range(0, rows, 512):
+        assert torch.equal(rptc.quantize_rows(alphabet.cuda(), weights.cuda(), samples[r0:r0 + 8].cuda())[0], got[r0:r0 + 8])
