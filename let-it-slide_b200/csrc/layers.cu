@@ -23,9 +23,9 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
                        int64_t clear_count, cudaStream_t stream, bool late = false);
 int check_blocks(int64_t n, int block);
 int check_signs(const void *signs);
-// out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]; for how many rows that is as fast as adding them up in a
-// kernel in front
-bool hadamard_takes_sums(int64_t rows, int64_t n, int block);
+// out = signs * H(the product's sums) * scale over blocks, fp16 [rows][ld_out]; whether that is as fast as adding them up, `sums` a value at
+// most, in a kernel in front
+bool hadamard_takes_sums(int64_t rows, int64_t n, int block, int64_t sums);
 int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
                      int block, float scale, cudaStream_t stream);
 
@@ -186,7 +186,11 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
     if (int e = launch(packed_input_kernel<T>, dim3((unsigned)tokens), dim3(kPackedThreads), 0, s, static_cast<const T *>(x), l.scales_in, l.biases_in,
                        xs, sums, few && !partial ? reinterpret_cast<float *>(prod) : nullptr, ld, (int)l.n))
         return e;
-    if (partial && tokens <= kFewOwnTokens) {        // the output side adds them up: 896 x 704, 34 tokens 11.9 -> 9.3 us; 2048 x 2560, 235 tokens 21.8 -> 22.2
+    // The output side adds the sums up by itself, a value per thread, where there are few of them (in front / there, us): 1792 x 1536 in 32 banks, 9
+    // tokens 15.8 / 13.2, 96 20.6 / 19.4; 5504 x 1088 in 16, 48 tokens (264 thousand values) 15.9 / 15.0; 7296 x 7104 in 16, 48 (350) 41.7 / 40.4;
+    // 8832 x 4288 in 8, 48 (424) 32.6 / 32.5; 10240 x 576 in 16, 48 (492) 16.3 / 16.7; 96 tokens: 3072 x 512 in 16 (295) 18.7 / 18.3, 3712 x 832 in 16
+    // (356) 19.8 / 20.2, 4480 x 640 in 8 (430) 20.2 / 20.9.
+    if (partial && tokens <= kFewOwnTokens && tokens * l.m <= (tokens <= 48 ? 420 : 310) << 10) {
         GemvSums parts;
         if (int e = gemv_few(l.codes, l.alphabets, nullptr, xs, l.n, nullptr, ld, stored, l.n, tokens, banks, f, s, true, partial, &parts)) return e;
         return output(partial, parts);
@@ -330,7 +334,7 @@ extern "C" int rptc_linear_forward(const rptc_linear *l, const void *x, void *y,
             if (int e = rptc_gemv(l->codes, l->lut, l->carry_in, xt, n, acc, m, m, n, (int)rows, RPTC_XORDER_NATURAL, &l->fmt, stream)) return e;
         } else {
             GemvSums parts;
-            const bool added_up = partial && l->signs_out && hadamard_takes_sums(rows, m, l->block_out);
+            const bool added_up = partial && l->signs_out && hadamard_takes_sums(rows, m, l->block_out, partials(m, n, rows, Banks(), l->fmt) / (rows * m));
             if (int e = gemv_few(l->codes, l->lut, l->carry_in, xt, n, acc, m, m, n, rows, Banks(), l->fmt, s, true, partial, added_up ? &parts : nullptr)) return e;
             pdl.set(true);
             if (added_up) return hadamard_of_sums(partial, m, parts, y, m, l->signs_out, rows, m, l->block_out, l->scale, s);
