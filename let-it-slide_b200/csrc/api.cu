@@ -212,7 +212,7 @@ extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x
     if (int e = rptc_check_device()) return e;
     const int dev = current_device();
     if (dev < 0) return cuda_fail(cudaErrorNoDevice);
-    if (gemv_whole_takes(m, n, *fmt) && written_apart(y, codes, lut, x, m, n, *fmt)) {
+    if (gemv_whole_takes(n, x_order, *fmt) && written_apart(y, codes, lut, x, m, n, *fmt)) {
         WaitedTimer &t = g_waited[dev];
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         RPTC_CUDA(cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture));

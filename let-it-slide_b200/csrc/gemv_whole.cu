@@ -178,12 +178,17 @@ static size_t whole_smem(int64_t n, const rptc_format &f) {
     const int64_t chunks = (n / (128 / f.K) + 31) / 32;
     return fixed_smem(f, kUnitsRing + kUnitsHist + kWholeSums + kWholeParts) + (size_t)chunks * 32 * (128 / f.K) * 2;
 }
-bool gemv_whole_takes(int64_t m, int64_t n, const rptc_format &f) {
-    return (f.layout == RPTC_LAYOUT_ROWMAJOR || f.layout == RPTC_LAYOUT_CHUNKED) && (f.K == 2 || f.K == 4) && whole_smem(n, f) <= kMaxSmem;
+// In the legacy order every CTA gathers all activations, 4 bytes here and there, with a division each: from some number of columns on that is more
+// than the product with a kernel behind it costs (calls, us, that / this): 4096 rows HASH, 4096 columns 30.3 / 22.7, 8192 34.7 / 34.2, 10240 35.7 / 35.8,
+// 12288 36.2 / 37.2, 16384 38.2 / 40.4, 24576 42.8 / 51.6; 1024 rows, 10240 29.9 / 26.1, 16384 30.2 / 35.6.  In the natural order what fits into shared
+// memory pays: 8192 x 24576 LITE 61.5 / 57.1, 2048 x 32768 table code 54.0 / 53.8.
+bool gemv_whole_takes(int64_t n, int x_order, const rptc_format &f) {
+    return (f.layout == RPTC_LAYOUT_ROWMAJOR || f.layout == RPTC_LAYOUT_CHUNKED) && (f.K == 2 || f.K == 4) && whole_smem(n, f) <= kMaxSmem &&
+           (x_order == RPTC_XORDER_NATURAL || n <= 10240);
 }
 int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64_t m, int64_t n, int x_order, int accumulate, const rptc_format &f,
                const DeviceTimer &timer, cudaStream_t stream) {
-    if (!gemv_whole_takes(m, n, f)) return RPTC_ERR_UNSUPPORTED;
+    if (!gemv_whole_takes(n, x_order, f)) return RPTC_ERR_UNSUPPORTED;
     GemvWhole p = {};
     p.codes = static_cast<const uint4 *>(codes);
     p.lut = static_cast<const __half *>(lut);

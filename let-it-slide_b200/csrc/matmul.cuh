@@ -84,9 +84,9 @@ int gemv_alone(const void *codes, const void *lut, const uint32_t *carry_in, con
 // ---- a matvec whose caller waits for it (gemv_whole.cu) ----
 int validate_gemv_args(const void *codes, const void *lut, const void *x, int64_t ld_x, const float *acc, int64_t ld_acc, int64_t m, int64_t n, int batch,
                        int x_order, const rptc_format *fmt);
-// y = (or +=) W x, one row, for codes whose units of a row lie together (ROWMAJOR, CHUNKED) and rows that fit into shared memory
-// (gemv_whole_takes).  The arguments have been checked, and y lies over none of them.
-bool gemv_whole_takes(int64_t m, int64_t n, const rptc_format &f);
+// y = (or +=) W x, one row, for codes whose units of a row lie together (ROWMAJOR, CHUNKED) and rows that fit into shared memory and are gathered
+// cheaply enough (gemv_whole_takes).  The arguments have been checked, and y lies over none of them.
+bool gemv_whole_takes(int64_t n, int x_order, const rptc_format &f);
 int gemv_whole(const void *codes, const void *lut, const void *x, void *y, int64_t m, int64_t n, int x_order, int accumulate, const rptc_format &f,
                const DeviceTimer &timer, cudaStream_t stream);
 

@@ -206,9 +206,10 @@ def test_layer_of_one_row(code, K, L, S, m, n):
 
 @pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_B, 2, 16, 6), (o.CODE_A, 2, 16, 0), (o.CODE_A, 4, 14, 0), (o.CODE_C, 4, 16, 8)])
 @pytest.mark.parametrize("layout,x_order,quirk", [(o.LAYOUT_ROWMAJOR, 0, 0), (o.LAYOUT_CHUNKED, 0, 0), (o.LAYOUT_CHUNKED, 1, o.QUIRK_K2_LANE0_CARRY)])
-@pytest.mark.parametrize("m,n", [(32, 2048), (32, 16384), (160, 6144), (1056, 8192), (4128, 4096), (22016, 2048), (64, 51200)])
+@pytest.mark.parametrize("m,n", [(32, 2048), (32, 16384), (160, 6144), (1056, 8192), (96, 10240), (96, 12288), (4128, 4096), (22016, 2048), (64, 51200), (64, 81920)])
 def test_timed_matvec_stores_and_adds(code, K, L, S, layout, x_order, quirk, m, n):
-    """rptc_gemv_timed: a warp and several per row, one and many rows a warp, the last size beyond shared memory (a kernel and one behind it).
+    """rptc_gemv_timed: a warp and several per row, one and many rows a warp, the last sizes beyond the shared memory that the HASH code and all codes
+    leave, and both sides of the line in the legacy order (beyond either a kernel and one behind it).
     The same product as rptc_gemv's, a store and an addition in fp16, a positive time."""
     from rptc_b200 import Format, ops
     from rptc_b200._lib import native
