@@ -85,12 +85,13 @@ __device__ __forceinline__ GemmBars gemm_bars(uint32_t base) {
     return b;
 }
 
+// Tiles of up to 128 x 128: activations and weights of a step share a stage and its barriers.  Wide ones have a ring each, the
+// activations' a deeper one (22016 x 4096, 22 tokens in tiles of 256 rows: 45.7 us, 47.5 with one ring), and so have tiles of 128 rows beside a
+// table of 128 KiB, which leaves three stages: 15616 x 1536, 100 tokens 25.5 us, 26.1 with one ring (32 KiB and K = 4, 128 tokens: 25.1 and 24.6).
+constexpr bool one_ring(int rows, int halves, int table_bytes) { return halves == 1 && rows <= (table_bytes > 64 << 10 ? 64 : 128); }
+
 // The HASH code is looked up in the packed table (128-byte rows) here: 32 KiB instead of 64 KiB leaves room for one more
 // ring stage, and the extra shift per lookup is hidden behind the tensor pipe.
-// Tiles of up to 128 x 128: activations and weights of a step share a stage and its barriers.  Wide ones have a ring each, the
-// activations' a deeper one (22016 x 4096, 22 tokens in tiles of 256 rows: 45.7 us, 47.5 with one ring).
-constexpr bool one_ring(int rows, int halves) { return rows <= 128 && halves == 1; }
-
 template <int CODE>
 struct GemmDecode {
     static constexpr int kCode = CODE == RPTC_CODE_HASH ? kCodeHashPacked : CODE;
@@ -302,11 +303,14 @@ __device__ __forceinline__ void drain_accumulators(const GemmParams &p, uint32_t
     }
 }
 
-__device__ __forceinline__ void init_ring_barriers(const GemmBars &bars, uint32_t w_arrivals) {
-    for (int s = 0; s < kMaxGemmStages; ++s) {
+// Of the stages in use: one thread does it, in front of everything.
+__device__ __forceinline__ void init_ring_barriers(const GemmBars &bars, int x_stages, int w_stages, uint32_t w_arrivals) {
+    for (int s = 0; s < w_stages; ++s) {
         mbar_init(bars.full_w + 8 * s, w_arrivals);
-        mbar_init(bars.full_x + 8 * s, 1);
         mbar_init(bars.empty_w + 8 * s, 1);
+    }
+    for (int s = 0; s < x_stages; ++s) {
+        mbar_init(bars.full_x + 8 * s, 1);
         mbar_init(bars.empty_x + 8 * s, 1);
     }
     mbar_init(bars.accum, 1);
@@ -318,14 +322,13 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int CODE, int K, int NROWS, int HALVES>
+template <int CODE, int K, int NROWS, int HALVES, bool ONE_RING>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap y_map) {
     constexpr int DC = GemmDecode<CODE>::kCode;
     constexpr uint32_t kTmemCols = HALVES * NROWS;       // NROWS fp32 columns per 128 tokens
     constexpr uint32_t kInstrDesc = instr_desc(NROWS);
     constexpr int kGroups = 256 / NROWS;                 // producer groups taking the steps in turn
-    constexpr bool kOneRing = one_ring(NROWS, HALVES);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // In a cluster every CTA's shared-memory window sits at its own place in the cluster's window: shared addresses of
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int64_t tile_row = (int64_t)(blockIdx.x - bank * p.tiles_per_bank) * NROWS;
     const uint4 *codes = p.codes + (int64_t)bank * p.m * p.n_units;
 
-    if (tid == 0) init_ring_barriers(bars, NROWS + (kOneRing ? 1 : 0));
+    if (tid == 0) init_ring_barriers(bars, ONE_RING ? 0 : p.n_xstages, p.n_wstages, NROWS + (ONE_RING ? 1 : 0));
     if (warp == kMmaWarp) {                     // TMEM: fp32 accumulators of NROWS columns per 128 tokens
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(bars.tmem_slot), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -378,13 +381,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         ok = produce_weights<CODE, K, kGroups>(p, window, bars, codes, row < p.m ? row : p.m - 1, step0, n_steps);
     } else if (warp == kTmaWarp) {
         pdl_wait_prior_grids();
-        if (lane == 0) load_activations<HALVES, kOneRing>(p, window, bars, &x_map, tok0, step0, n_steps);
-    } else if (kOneRing || lane == 0) {
+        if (lane == 0) load_activations<HALVES, ONE_RING>(p, window, bars, &x_map, tok0, step0, n_steps);
+    } else if (ONE_RING || lane == 0) {
         // ================= MMA issue =================
         RingPos px = {0, 0u}, pw = {0, 0u};
         for (int it = 0; it < n_steps; ++it) {
-            const bool issues = !kOneRing || elect_one();
-            if (kOneRing) {
+            const bool issues = !ONE_RING || elect_one();
+            if (ONE_RING) {
                 ok = ok && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
             } else {
                 ok = mbar_wait(bars.full_x + 8 * px.s, px.phase, p.status) && mbar_wait(bars.full_w + 8 * pw.s, pw.phase, p.status);
@@ -392,20 +395,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             }
             tc_fence_after();
             const uint64_t xa = umma_desc_sw128(p.xa_addr[px.s]), xb = umma_desc_sw128(p.xb_addr[px.s]), wd = umma_desc_sw128(p.w_addr[pw.s]);
-            if (issues && ok) {
+            if (!ONE_RING && CODE == RPTC_CODE_LUT) {
+                // Descriptors made MMA by MMA: look-ups bind these tiles, and with the additions below they take 1 to 2 % more time (4096 x 11008, L = 16,
+                // 900 tokens 165.7 and 168.2 us); the other codes' 0.6 % less (HASH, 22016 x 4096, 2048 tokens 271.6 and 270.1).
+#pragma unroll
+                for (uint32_t k = 0; k < kStepCols / 16; ++k) {
+                    const uint64_t w_desc = umma_desc_sw128(p.w_addr[pw.s] + 32u * k);
+                    tc_mma_f16(tmem_base, umma_desc_sw128(p.xa_addr[px.s] + 32u * k), w_desc, kInstrDesc, (it | k) != 0);
+                    if (HALVES == 2) tc_mma_f16(tmem_base + (uint32_t)NROWS, umma_desc_sw128(p.xb_addr[px.s] + 32u * k), w_desc, kInstrDesc, (it | k) != 0);
+                }
+                tc_commit(bars.empty_x + 8 * px.s);
+                tc_commit(bars.empty_w + 8 * pw.s);
+            } else if (issues && ok) {
 #pragma unroll
                 for (uint32_t k = 0; k < kStepCols / 16; ++k) {           // + 32 bytes per K = 16
                     tc_mma_f16(tmem_base, xa + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
                     if (HALVES == 2) tc_mma_f16(tmem_base + (uint32_t)NROWS, xb + 2u * k, wd + 2u * k, kInstrDesc, (it | k) != 0);
                 }
-                if (!kOneRing) tc_commit(bars.empty_x + 8 * px.s);      // each arrives when the MMAs above have read the stage
+                if (!ONE_RING) tc_commit(bars.empty_x + 8 * px.s);      // each arrives when the MMAs above have read the stage
                 tc_commit(bars.empty_w + 8 * pw.s);
             }
-            if (kOneRing) __syncwarp();
+            if (ONE_RING) __syncwarp();
             px.advance(p.n_xstages);
             pw.advance(p.n_wstages);
         }
-        if ((!kOneRing || elect_one()) && ok) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
+        if ((!ONE_RING || elect_one()) && ok) tc_commit(bars.accum);   // arrives when every MMA has written its accumulator
     }
     __syncwarp();
 
@@ -462,10 +476,10 @@ struct GemmShape {
     int rows, halves, split;      // weight rows and 128-token halves of a tile, CTAs that share a tile's reduction
 };
 
-template <int CODE, int K, int NROWS, int HALVES>
+template <int CODE, int K, int NROWS, int HALVES, bool ONE_RING>
 static int launch_gemm(const GemmParams &p, const CUtensorMap &map, const CUtensorMap &ymap, size_t smem, dim3 grid, cudaStream_t stream) {
     static SmemOptIn opted;
-    auto kern = gemm_kernel<CODE, K, NROWS, HALVES>;
+    auto kern = gemm_kernel<CODE, K, NROWS, HALVES, ONE_RING>;
     if (int e = allow_max_smem(kern, opted)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -494,10 +508,13 @@ template <int CODE, int K>
 static int launch_gemm_shape(const GemmShape &g, const GemmParams &p, const CUtensorMap &map, const CUtensorMap &ymap, size_t smem, dim3 grid,
                              cudaStream_t stream) {
     if (g.rows == 256)
-        return g.halves == 2 ? launch_gemm<CODE, K, 256, 2>(p, map, ymap, smem, grid, stream) : launch_gemm<CODE, K, 256, 1>(p, map, ymap, smem, grid, stream);
-    if (g.rows == 64) return launch_gemm<CODE, K, 64, 1>(p, map, ymap, smem, grid, stream);
-    if (g.rows == 32) return launch_gemm<CODE, K, 32, 1>(p, map, ymap, smem, grid, stream);
-    return g.halves == 2 ? launch_gemm<CODE, K, 128, 2>(p, map, ymap, smem, grid, stream) : launch_gemm<CODE, K, 128, 1>(p, map, ymap, smem, grid, stream);
+        return g.halves == 2 ? launch_gemm<CODE, K, 256, 2, false>(p, map, ymap, smem, grid, stream) : launch_gemm<CODE, K, 256, 1, false>(p, map, ymap, smem, grid, stream);
+    if (g.rows == 64) return launch_gemm<CODE, K, 64, 1, true>(p, map, ymap, smem, grid, stream);
+    if (g.rows == 32) return launch_gemm<CODE, K, 32, 1, true>(p, map, ymap, smem, grid, stream);
+    if (g.halves == 2) return launch_gemm<CODE, K, 128, 2, false>(p, map, ymap, smem, grid, stream);
+    if constexpr (CODE == RPTC_CODE_LUT)
+        if (!one_ring(128, 1, 2 << p.L)) return launch_gemm<CODE, K, 128, 1, false>(p, map, ymap, smem, grid, stream);
+    return launch_gemm<CODE, K, 128, 1, true>(p, map, ymap, smem, grid, stream);
 }
 
 // Shared-window plan (offsets in the CTA's window; the dynamic area is expected to start at or below 0x400).  The packed
@@ -532,7 +549,7 @@ static bool plan_gemm(GemmParams &p, const GemmShape &g, const rptc_format &f) {
         return 0;
     };
     int xs = 0, ws = 0;
-    const bool one = one_ring(g.rows, g.halves);
+    const bool one = one_ring(g.rows, g.halves, f.code == RPTC_CODE_LUT ? 2 << f.L : 0);
     const int most_x = g.rows < 128 ? kMaxGemmStages : 4, most_w = one ? most_x : 3;
     auto add_x = [&]() -> bool {
         if (xs == most_x) return false;
@@ -589,7 +606,7 @@ static int64_t cluster_places(int split) {
     if (split == 1 || dev < 0) return num_sms() / split;
     int &places = cached[dev][split == 4];
     if (!places) {
-        auto kern = gemm_kernel<RPTC_CODE_HASH, 2, 256, 2>;
+        auto kern = gemm_kernel<RPTC_CODE_HASH, 2, 256, 2, false>;
         SmemOptIn first;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, 1, (unsigned)split);

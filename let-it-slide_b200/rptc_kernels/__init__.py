@@ -11,7 +11,7 @@ instead of the reference's kernels.  Differences, all deliberate:
     `set_reference_quirks(True)` reproduces those deviations bit for bit;
   * `decompress_matvec_t_*` computes the intended product; the reference kernel's inner loop does
     not advance its shift registers (inference_t.cu:125-134) and is not reproduced;
-  * `decompress_matvec_*` of more than 10240 columns and `decompress_matvec_t_*` add partial sums into an fp32 accumulator
+  * `decompress_matvec_t_*`, and `decompress_matvec_*` of more than 10240 columns or with an `out` over its inputs, add partial sums into an fp32 accumulator
     that this module keeps per (device, stream, m): two calls on the same stream are ordered by the stream; calls from two host
     threads that share one stream must be serialised by the caller;
   * shape rules are relaxed: n needs to be a multiple of 64 only, except for the chunked layout of
