@@ -446,10 +446,10 @@ static int few_row_blocks(int64_t m) {
 static int ordered_row_blocks(int64_t m, int64_t tokens, int code) {
     return code == RPTC_CODE_LUT || m <= 32 * 128 || tokens > 48 ? 1 : 2;
 }
-// SHARED: microseconds of a 64-column step of a tile.  The decode (a 65,536-entry table: bank conflicts), the tensor core (four
-// clocks per token and pair of row blocks), or one thread's issue of the step.
-static double shared_step_us(int rb, int n_cols, int code) {
-    const double decode = rb * (code == RPTC_CODE_LUT ? 0.60 : 0.14), mma = rb * n_cols * 2 / 1900.0, issue = 0.34;
+// SHARED: microseconds of a 64-column step of a tile.  The decode (tables: bank conflicts, of 65,536 entries a little more), the tensor
+// core (four clocks per token and pair of row blocks), or one thread's issue of the step.
+static double shared_step_us(int rb, int n_cols, const rptc_format &f) {
+    const double decode = rb * (f.code != RPTC_CODE_LUT ? 0.14 : f.L == 16 ? 0.60 : 0.55), mma = rb * n_cols * 2 / 1900.0, issue = 0.34;
     return decode > mma ? (decode > issue ? decode : issue) : (mma > issue ? mma : issue);
 }
 
@@ -487,8 +487,8 @@ static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tok
         FewParams one, two;
         const bool has_one = few_plan(one, f, tokens, 1), has_two = few_plan(two, f, tokens, 2);
         if (!has_one && !has_two) return 0;
-        rb = !has_two || (has_one && few_tiles(m, 1) * one.token_tiles * shared_step_us(1, one.n_cols, f.code) <
-                                         few_tiles(m, 2) * two.token_tiles * shared_step_us(2, two.n_cols, f.code))
+        rb = !has_two || (has_one && few_tiles(m, 1) * one.token_tiles * shared_step_us(1, one.n_cols, f) <
+                                         few_tiles(m, 2) * two.token_tiles * shared_step_us(2, two.n_cols, f))
                  ? 1
                  : 2;
     }
@@ -534,11 +534,14 @@ int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &ban
 // Up to kFewOwnTokens activation rows always (a step costs its decode), beyond that where it is estimated to finish before
 // the fused GEMM: a GEMM tile of 256 x 256 feeds the tensor core better and its result is fp16, but its decode goes through
 // shared memory and half of its SMs are idle for a few hundred tokens.  Here a CTA has its equal share of the steps, takes
-// its tiles' sums to memory (0.021 us per token and pair of row blocks), where more than two of them for a tile cost about 2.5 us
-// (they are added up in order by a second kernel), and the fp32 result is read behind.  The time around the steps is fitted to
-// whole layers of both codes.  Measured, whole layers, GEMM against this: 4096 x 11008 HASH, 128 tokens 44.5 and 31.6 us, 512 57.1 and
-// 58.6; 22016 x 4096, 192 tokens 67.4 and 57.6; 1024 x 14336, 256 tokens 53.8 and 34; 4096 x 4096 in 32 banks, 112 tokens 36.9 and
-// 23; on the other side of the line 14336 x 1024, 512 tokens 38.7 and 51.7, 22016 x 4096, 2048 tokens 350 and 406.
+// its tiles' sums to memory (0.021 us per token and pair of row blocks, 1 us for every further tile of tokens), where more than two of them for a
+// tile cost about 2.5 us and 0.3 per million values (they are added up in order by a second kernel), and the fp32 result is read behind.  The time
+// around the steps is fitted to whole layers of both codes, and so is what a layer takes around the tiled product beyond that product's
+// estimate: 1.7 us with a table, 4 with the others, whose layers have transforms on both sides that do not run under the start of this product.
+// 2301 layers of 256 to 18176 rows and 512 to 14336 columns, 97 to 512 tokens, all codes, by both products: the choice costs 0.6 % over the better
+// one; without the last three terms 1.2 (1280 x 3584 in 32 banks, L = 14, 158 tokens 17.0 here and 22.8; 4096 x 4096 in 32, L = 10, 128 21.8 and 24.6;
+// 1024 x 3840 LITE, 512 25.2 and 28.7; on the other side 640 x 2752 in 8, L = 8, 500 23.0 and 18.7; 1024 x 2048 in 8, L = 10, 256 17.3 and 15.8).  Measured, whole layers, GEMM against this: 4096 x 11008 HASH, 128 tokens 44.5 and 31.6 us, 512
+// 57.1 and 58.6; 22016 x 4096, 192 tokens 67.4 and 57.6; 1024 x 14336, 256 tokens 53.8 and 34; on the other side of the line 14336 x 1024, 512 tokens 38.7 and 51.7, 22016 x 4096, 2048 tokens 350 and 406.
 static bool few_is_faster(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     FewParams p;
     const int rb = few_choose(p, f, m, tokens, true);
@@ -546,10 +549,11 @@ static bool few_is_faster(int64_t m, int64_t n, int64_t tokens, const Banks &ban
     const int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1, waves = (banks.banks * ctas + num_sms() - 1) / num_sms();
     const int64_t n_steps = n / 64, steps = (few_tiles(m, rb) * p.token_tiles * n_steps + ctas - 1) / ctas;
     const double drains = 1 + steps / n_steps;
-    const double us = waves * ((f.code == RPTC_CODE_LUT ? 8.0 : 12.0) + steps * shared_step_us(rb, p.n_cols, f.code) + drains * 0.0105 * rb * p.n_cols) +
-                      (double)banks.banks * m * tokens * 8 / 4.5e6 + (gemv_few_partials(m, n, tokens, banks, f) ? 2.5 : 0.0);
+    const int64_t partials = gemv_few_partials(m, n, tokens, banks, f);
+    const double us = waves * ((f.code == RPTC_CODE_LUT ? 8.0 : 12.0) + steps * shared_step_us(rb, p.n_cols, f) + drains * 0.0105 * rb * p.n_cols) +
+                      (double)banks.banks * m * tokens * 8 / 4.5e6 + (partials ? 2.5 + 0.3e-6 * (double)partials : 0.0) + (p.token_tiles - 1);
     const double gemm = gemm_us(m, n, tokens, banks, f);
-    return gemm == 0 || us < gemm;
+    return gemm == 0 || us < gemm + (f.code == RPTC_CODE_LUT ? 1.7 : 4.0);
 }
 
 bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, const void *x, int64_t ld_x) {
