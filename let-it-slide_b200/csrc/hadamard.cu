@@ -262,10 +262,11 @@ int hadamard_and_clear(const void *in, int in_is_f32, int64_t ld_in, void *out, 
 // few threads take in turn: HASH, 9 and 31 rows, 1536 x 2048 (17 sums) 16.3 / 14.2 and 15.6 / 15.8, 1024 x 8192 (23) 15.5 / 16.4 and 16.5 / 17.7,
 // 1024 x 2048 (32) 16.1 / 18.8 and 15.8 / 19.3.  Blocks above 256 up to 31 rows, behind which the transform that walks down the rows takes over, and
 // below 4096, whose CTA has a whole row to add up: 2048 x 2048 15.4 / 13.3 and 16.1 / 13.3, 22016 x 4096 26.3 / 23.4 and 29.1 / 27.9, 4096 x 4096
-// 15.9 / 16.5 and 17.3 / 17.9.  Smaller blocks: 11008 x 4096, 9 rows 18.0 / 17.4, 72 33.3 / 32.7, 96 34.7 / 35.0; 3840 x 3584, 9 rows 16.2 / 13.2, 72
-// 25.3 / 24.9, 96 28.2 / 28.8.
+// 15.9 / 16.5 and 17.3 / 17.9.  Smaller blocks: 11008 x 4096, 9 rows 18.0 / 17.4, 72 33.3 / 32.7; 3840 x 3584, 9 rows 16.2 / 13.2, 72 25.3 / 24.9; 96 rows
+// of few values 28.2 / 28.8 there, of many 24320 x 2560 61.4 / 57.8, 12544 x 7168 46.2 / 44.6, 7936 x 1280 25.3 / 24.6.
 bool hadamard_takes_sums(int64_t rows, int64_t n, int block, int64_t sums) {
-    return sums <= 20 && (block > 256 ? rows < 32 && block < 4096 : rows <= 72 && rows * n < (int64_t(5) << 19));
+    if (block > 256) return sums <= 20 && rows < 32 && block < 4096;
+    return sums <= 20 && (rows <= 72 || (rows <= 96 && rows * n >= 700000)) && rows * n < (int64_t(5) << 19);
 }
 int hadamard_of_sums(const float *partial, int64_t ld, const GemvSums &sums, void *out, int64_t ld_out, const void *signs, int64_t rows, int64_t n,
                      int block, float scale, cudaStream_t stream) {

@@ -263,7 +263,7 @@ def test_timed_matvec_whose_result_replaces_its_activations(layout, m, n, at, ac
 
 
 @pytest.mark.parametrize("code,K,L,S", [(o.CODE_B, 2, 16, 8), (o.CODE_A, 2, 16, 0), (o.CODE_C, 4, 16, 8)])
-@pytest.mark.parametrize("m,n", [(512, 4096), (768, 2048), (1536, 2048), (2048, 2048), (4096, 1024), (3840, 3584)])
+@pytest.mark.parametrize("m,n", [(512, 4096), (768, 2048), (1536, 2048), (2048, 2048), (4096, 1024), (3840, 3584), (7936, 1280)])
 @pytest.mark.parametrize("rows", [9, 31, 32, 72, 73, 96])
 def test_layer_whose_sums_are_added_up_in_front_of_or_in_its_output_transform(code, K, L, S, m, n, rows):
     """Blocks of 256 to 4096, many and few sums a value, both sides of the lines in rows.  Activations and results are rounded to fp16, 2^-11 of
