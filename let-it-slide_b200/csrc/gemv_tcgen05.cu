@@ -24,6 +24,8 @@
 // clocks and its decode about 430 issue slots per scheduler, so that decoding again for the next 192 tokens is free.
 // ORDERED: segments' sums are put down side by side instead, and a second kernel adds them up in their order.
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status word and the CTA drains and returns.
+#include <algorithm>
+
 #include "common.cuh"
 #include "matmul.cuh"
 #include "tc_ptx.cuh"
@@ -454,7 +456,7 @@ static double shared_step_us(int rb, int n_cols, const rptc_format &f) {
 }
 
 // Tile of `rb` row blocks, where the table and the activation ring go; false when they do not fit.
-static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb) {
+static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb, int64_t most_cols) {
     p.shared = tokens > kFewOwnTokens;
     const uint32_t codes_end = kFewCodes + kFewWarps * few_ahead(f.code, p.shared) * (f.K / 2) * 512;
     uint32_t free;
@@ -469,7 +471,7 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
     p.x_addr = free;
     p.token_tiles = 1;
     if (p.shared) {      // three stages of activations (two under a table's slower look-ups), and the accumulators beside the decoded weights, bound the tile
-        const int64_t fit = (kFewTop - free) / ((f.code == RPTC_CODE_LUT ? 2 : 3) * 128) / 16 * 16, most = rb == 1 ? 256 : 192, cols = fit < most ? fit : most;
+        const int64_t fit = (kFewTop - free) / ((f.code == RPTC_CODE_LUT ? 2 : 3) * 128) / 16 * 16, most = rb == 1 ? most_cols : std::min<int64_t>(most_cols, 192), cols = fit < most ? fit : most;
         if (cols < 16) return false;
         p.token_tiles = (int32_t)((tokens + cols - 1) / cols);
     }
@@ -481,11 +483,15 @@ static bool few_plan(FewParams &p, const rptc_format &f, int64_t tokens, int rb)
 }
 static int64_t few_tiles(int64_t m, int rb) { return (m + rb * 128 - 1) / (rb * 128); }
 // The plan for `tokens` activation rows: row blocks per tile, or 0 where there is none.
-static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tokens, bool ordered) {
+static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t n, int64_t tokens, const Banks &banks, bool ordered) {
+    // Beside a table of 128 KiB a weight is looked up once per tile of tokens, but a CTA of two steps looks up little, and tiles of more tokens leave
+    // more CTAs to put down sums of a value: 1024 x 2048 in 8 banks, 192 and 256 tokens in two tiles 16.8 and 16.7 us, in one 17.5 and 17.6.
+    const int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1;
+    const int64_t most_cols = f.code == RPTC_CODE_LUT && f.L == 16 && few_tiles(m, 1) * (n / 64) < 3 * ctas ? 144 : 256;
     int rb = ordered ? ordered_row_blocks(m, tokens, f.code) : few_row_blocks(m);
     if (tokens > kFewOwnTokens) {
         FewParams one, two;
-        const bool has_one = few_plan(one, f, tokens, 1), has_two = few_plan(two, f, tokens, 2);
+        const bool has_one = few_plan(one, f, tokens, 1, most_cols), has_two = few_plan(two, f, tokens, 2, most_cols);
         if (!has_one && !has_two) return 0;
         rb = !has_two || (has_one && few_tiles(m, 1) * one.token_tiles * shared_step_us(1, one.n_cols, f) <
                                          few_tiles(m, 2) * two.token_tiles * shared_step_us(2, two.n_cols, f))
@@ -494,7 +500,7 @@ static int few_choose(FewParams &p, const rptc_format &f, int64_t m, int64_t tok
     }
     // a table and tokens that leave no stage for each of the parts take tiles of more row blocks, which have fewer of them
     for (; rb <= 4; rb *= 2) {
-        if (few_plan(p, f, tokens, rb)) return rb;
+        if (few_plan(p, f, tokens, rb, most_cols)) return rb;
         if (p.shared) break;
     }
     return 0;
@@ -521,7 +527,7 @@ static int few_ranges(FewParams &p, int rb, int64_t m, int64_t n, const Banks &b
 
 int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     FewParams p;
-    const int rb = few_choose(p, f, m, tokens, true);
+    const int rb = few_choose(p, f, m, n, tokens, banks, true);
     if (!rb || few_ranges(p, rb, m, n, banks)) return 0;
     // CTAs that meet in a tile: its first step may be a range's last, unless whole ranges make up a tile; those behind are full ones
     const int64_t steps = (int64_t)p.tiles * p.token_tiles * p.n_steps, per = steps / p.ctas;
@@ -544,7 +550,7 @@ int64_t gemv_few_partials(int64_t m, int64_t n, int64_t tokens, const Banks &ban
 // 57.1 and 58.6; 22016 x 4096, 192 tokens 67.4 and 57.6; 1024 x 14336, 256 tokens 53.8 and 34; on the other side of the line 14336 x 1024, 512 tokens 38.7 and 51.7, 22016 x 4096, 2048 tokens 350 and 406.
 static bool few_is_faster(int64_t m, int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f) {
     FewParams p;
-    const int rb = few_choose(p, f, m, tokens, true);
+    const int rb = few_choose(p, f, m, n, tokens, banks, true);
     if (!rb || !p.shared) return rb != 0;
     const int64_t ctas = num_sms() / banks.banks > 0 ? num_sms() / banks.banks : 1, waves = (banks.banks * ctas + num_sms() - 1) / num_sms();
     const int64_t n_steps = n / 64, steps = (few_tiles(m, rb) * p.token_tiles * n_steps + ctas - 1) / ctas;
@@ -581,7 +587,7 @@ bool gemv_few_takes(int64_t m, int64_t n, int64_t tokens, const Banks &banks, co
 int gemv_few(const void *codes, const void *lut, const uint32_t *carry_in, const void *x, int64_t ld_x, float *acc, int64_t ld_acc, int64_t m,
              int64_t n, int64_t tokens, const Banks &banks, const rptc_format &f, cudaStream_t s, bool ordered, float *partial, GemvSums *parts) {
     FewParams p;
-    const int rb = few_choose(p, f, m, tokens, ordered);
+    const int rb = few_choose(p, f, m, n, tokens, banks, ordered);
     if (!rb) return RPTC_ERR_UNSUPPORTED;
     if (int e = few_ranges(p, rb, m, n, banks)) return e;
     CUtensorMap map;

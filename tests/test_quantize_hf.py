@@ -260,10 +260,11 @@ def test_alphabets_on_the_gpu_can_be_differentiated():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m,n,banks", [(128, 64, 1), (352, 1088, 4), (4096, 2048, 32)])
-@pytest.mark.parametrize("tokens", [145, 192, 193, 256, 257, 520])
+@pytest.mark.parametrize("m,n,banks", [(128, 64, 1), (352, 1088, 4), (1024, 2048, 8), (4096, 2048, 32)])
+@pytest.mark.parametrize("tokens", [144, 145, 192, 193, 256, 257, 520])
 def test_packed_layer_whose_table_leaves_two_stages_of_tokens(m, n, banks, tokens):
-    """L = 16: tiles of up to 256 tokens beside a table of 128 KiB, their last one partly filled; sums of one and of several CTAs."""
+    """L = 16: tiles of up to 256 tokens beside a table of 128 KiB, their last one partly filled (of 144 where a CTA has few
+    steps); sums of one and of several CTAs."""
     import quantize_hf as q
     g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
