@@ -34,10 +34,11 @@ namespace rptc {
 
 static_assert(4 * kFewOwnTokens <= 512 - 128 && 4 * 2 * 48 <= 512 - 128, "an accumulator per group beside the decoded weights in tensor memory");
 constexpr int kFewWarps = 16, kFewTmaWarp = 16, kFewMmaWarp = 17, kFewThreads = 32 * (kFewMmaWarp + 4);
-// Steps of a thread's code bits in flight.  Two where a 128 KiB table leaves little room: a group takes more than two microseconds for a step's
-// look-ups, and 16 KiB more hold two stages of 256 tokens.  With one stage fewer tokens fit into a tile, and every weight is looked up once
-// per tile: layers of 4096 x 4096 in 32 banks, 256 tokens (two tiles of 128, now one) 32.1 -> 29.4 us, 384 tokens 47.2 -> 36.7; 4096 x 11008 in
-// eight, 256 tokens 68.9 -> 50.1; up to 144 tokens the same time.
+// Steps of a thread's code bits in flight.  Two beside a table, whose look-ups take a group more than two microseconds a step: at L = 16 the table
+// leaves little room, and 16 KiB more hold two stages of 256 tokens.  With one stage fewer tokens fit into a tile, and every weight is looked up
+// once per tile: layers of 4096 x 4096 in 32 banks, 256 tokens (two tiles of 128, now one) 32.1 -> 29.4 us, 384 tokens 47.2 -> 36.7; 4096 x 11008 in
+// eight, 256 tokens 68.9 -> 50.1; up to 144 tokens the same time.  Smaller tables have the room for four as well, which is within 1 % either way (four /
+// two: 4096 x 4096 in 32, L = 8, 256 tokens 26.5 / 26.2, 400 32.1 / 32.3; 11008 x 4096 in 8, L = 12, 320 74.5 / 75.1), so one form serves all.
 constexpr int few_ahead(int code, bool shared) { return shared && code == RPTC_CODE_LUT ? 2 : 4; }
 constexpr uint32_t kFewBars = 0x400, kFewHistory = 0x800, kFewCodes = 0x2800, kFewTop = 0x38800;
 constexpr int kFewMaxXStages = 8;

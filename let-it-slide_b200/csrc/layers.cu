@@ -165,13 +165,14 @@ static int packed_forward(const rptc_packed &l, const void *x, void *y, int64_t 
     const int64_t stored = (int64_t)l.bank_blocks * 32, ld = (int64_t)l.banks * cols;
     float2 *sums = reinterpret_cast<float2 *>(ws);
     __half *xs = reinterpret_cast<__half *>(ws + round_up(tokens * 8));
-    char *prod = reinterpret_cast<char *>(xs) + round_up(tokens * l.n * 2);
+    const bool alone = packed_alone(l, tokens);      // nothing in xs
+    char *prod = reinterpret_cast<char *>(xs) + (alone ? 0 : round_up(tokens * l.n * 2));
     auto output = [&](const float *acc, const GemvSums &parts) {
         return launch(parts.per ? packed_output_kernel<T, true> : packed_output_kernel<T, false>, dim3((unsigned)((l.m + 255) / 256), (unsigned)tokens), dim3(256),
                       0, s, acc, acc ? nullptr : reinterpret_cast<const __half *>(prod), ld, sums, l.scales_out, l.biases_out, l.bias, static_cast<T *>(y),
                       (int)l.m, (int)(l.m / l.banks), (int)cols, parts);
     };
-    if (packed_alone(l, tokens)) {
+    if (alone) {
         GemvInput in = {};
         in.x = x;
         in.dtype = std::is_same<T, __half>::value ? 0 : std::is_same<T, float>::value ? 2 : 1;
@@ -229,7 +230,7 @@ extern "C" int64_t rptc_packed_workspace_bytes(const rptc_packed *l, int64_t tok
     int64_t cols;
     const bool few = packed_plan(*l, tokens, cols);
     if (packed_alone(*l, tokens))
-        return round_up(tokens * 8) + round_up(tokens * l->n * 2) + 4 * gemv_alone_partials((int64_t)l->bank_blocks * 32, l->n, tokens, packed_banks(*l), packed_format(*l));
+        return round_up(tokens * 8) + 4 * gemv_alone_partials((int64_t)l->bank_blocks * 32, l->n, tokens, packed_banks(*l), packed_format(*l));
     const int64_t partial = few ? partials((int64_t)l->bank_blocks * 32, l->n, tokens, packed_banks(*l), packed_format(*l)) : 0;
     return round_up(tokens * 8) + round_up(tokens * l->n * 2) + round_up(tokens * l->banks * cols * (few ? 4 : 2)) + partial * 4;
 }

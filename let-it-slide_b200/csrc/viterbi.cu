@@ -71,7 +71,8 @@ __device__ __forceinline__ unsigned long long cost_key(float v, uint32_t state) 
 
 // CL CTAs share a row, a thread owns G groups of four prefixes, R rows alternate in a CTA.
 template <int CL, int G, int R>
-__global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel(const ViterbiParams p) {
+__global__ void __launch_bounds__(G == 4 ? 512 : 32, G == 4 ? 1 : 32) viterbi_forward_kernel(const ViterbiParams p) {
+    static_assert(G == 4 || (CL == 1 && R == 1), "fewer groups a thread only where a warp is a row");
     extern __shared__ __align__(128) float best_sm[];           // per row and buffer: P / CL values, and with CL == 2 half as many to send
     __shared__ unsigned long long red[33];
     __shared__ __align__(8) unsigned long long full_bar[R][2];  // CL == 2
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(G == 4 ? 512 : 1024, 1) viterbi_forward_kernel
     // from the other buffer has arrived.  Nothing here needs a fence at cluster scope, which would wait for the winners
     // on their way to global memory.  Once a wait has run
     // out no other is tried: the kernel goes on to its end with what it has.
-    constexpr uint32_t kWarps = G == 4 ? 16 : 32, kWarpBytes = 32 * G * 16;      // warps of a CTA, what one puts down per position
+    constexpr uint32_t kWarps = 16, kWarpBytes = 32 * G * 16;   // warps of a CTA, what one puts down per position
     const uint32_t full0 = smem_addr(full_bar);
     uint32_t peer_s0 = s0, peer_full0 = full0, peer_word = 0;
     const bool sends = out_off >= 4u * (uint32_t)PC;            // of a whole warp: 32 G pieces lie with one reader

@@ -201,6 +201,11 @@ def test_layer_of_one_row(code, K, L, S, m, n):
     assert (y.double() - want).norm() <= 2.0**-10 * want.norm()
     for _ in range(5 if n <= 4096 else 0):                     # sums in a fixed order
         assert torch.equal(layer(x), y)
+    # history in front of the rows (a shard of a layer whose reduction is cut)
+    layer.carry_in = torch.randint(-2**31, 2**31 - 1, (m,), dtype=torch.int32, device="cuda", generator=g)
+    want = x.double() @ layer.effective_weight().double().t()
+    carried = layer(x)
+    assert (carried.double() - want).norm() <= 2.0**-10 * want.norm() and not torch.equal(carried, y)
     ops.device_status()
 
 
