@@ -317,7 +317,6 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                         mbar_expect_tx(full_x + 8 * stage, bytes);
                         tma_load_2d(p.x_addr + (uint32_t)stage * bytes, &x_map, s * 64, g.t0, full_x + 8 * stage);
                     }
-                    __syncwarp();
                     px[ring].advance(p.n_xstages);
                 }
         }
@@ -358,7 +357,6 @@ __global__ void __launch_bounds__(kFewRegisterThreads, 1) gemv_few_kernel(const 
                         tc_commit(empty_a + 8 * (grp + from));
                         tc_commit(empty_x + 8 * stage);
                     }
-                    __syncwarp();
                     accumulate = 1u;
                     px.advance(p.n_xstages);
                 }
