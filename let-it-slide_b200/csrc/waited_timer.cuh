@@ -34,7 +34,8 @@ struct DeviceTimer {
         __threadfence();
         const unsigned long long from = atomicExch(&device->begin, ~0ull);
         device->ended = 0u;
-        *reinterpret_cast<volatile unsigned long long *>(&host->ns) = now() - from;
+        const unsigned long long to = now();      // another SM's reading than `from`
+        *reinterpret_cast<volatile unsigned long long *>(&host->ns) = to > from ? to - from : 0ull;
         __threadfence_system();
         *reinterpret_cast<volatile unsigned int *>(&host->ticket) = ticket;
     }
