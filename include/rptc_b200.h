@@ -179,7 +179,8 @@ int rptc_gemv_finish(float *acc, int64_t ld_acc, void *y, int64_t ld_y, int64_t 
  * result.  *ms: milliseconds on the device, from the first start to the last end of the kernel's blocks where one kernel does it all
  * (ROWMAJOR, CHUNKED; acc is not touched then), else between events on the stream around the work.  A thread's first call on a device
  * allocates for the former (48 bytes of pinned and 16 of device memory, given back when the thread ends) and creates two events for the latter; a thread that captures
- * a graph meanwhile is not disturbed.  Refused on a stream that is being captured. */
+ * a graph meanwhile is not disturbed.  Refused on a stream that is being captured, whose
+ * capture it ends with an error. */
 int rptc_gemv_timed(const void *codes, const void *lut, const void *x, float *acc, void *y, int64_t m, int64_t n, int x_order,
                     int accumulate, const rptc_format *fmt, float *ms, rptc_stream_t stream);
 /* Device time of whatever is launched between the two on the stream, by the calling thread (one pair of events per thread

@@ -178,6 +178,14 @@ namespace rptc {
 static thread_local WaitedTimer g_waited[kMaxDevices];
 // Until the kernel with `ticket` has left its time.  The stream is asked now and then: work that failed leaves none.
 static int wait_for(WaitedTimer &t, cudaStream_t stream, float *ms) {
+    // Asked behind the launch, under the kernel's time: in front of it the question is 0.2 us of a call.  A capture now holds a kernel that writes to
+    // this thread's timer, and must not become a graph: asking for the stream's state ends it.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    RPTC_CUDA(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        cudaStreamQuery(stream);
+        return cuda_fail(cudaErrorStreamCaptureUnsupported);      // nothing to wait for
+    }
     volatile HostTime *h = t.host;
     for (unsigned int spin = 1;; ++spin) {
         if (h->ticket == t.ticket) break;
@@ -214,9 +222,6 @@ extern "C" int rptc_gemv_timed(const void *codes, const void *lut, const void *x
     if (dev < 0) return cuda_fail(cudaErrorNoDevice);
     if (gemv_whole_takes(n, x_order, *fmt) && written_apart(y, codes, lut, x, m, n, *fmt)) {
         WaitedTimer &t = g_waited[dev];
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        RPTC_CUDA(cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture));
-        if (capture != cudaStreamCaptureStatusNone) return cuda_fail(cudaErrorStreamCaptureUnsupported);      // nothing to wait for
         RPTC_CUDA(t.ready());
         const int e = gemv_whole(codes, lut, x, y, m, n, x_order, accumulate, *fmt, {t.device, t.host, ++t.ticket}, static_cast<cudaStream_t>(stream));
         return e == RPTC_OK ? wait_for(t, static_cast<cudaStream_t>(stream), ms) : e;

@@ -1,6 +1,7 @@
 """The memory behind a matvec that its caller waits for: set up whole or not at all, and beside another thread's capture."""
 import os
 import subprocess
+import sys
 import threading
 
 import pytest
@@ -59,21 +60,34 @@ def test_first_timed_matvec_of_a_thread_while_another_captures():
     ops.device_status()
 
 
-@pytest.mark.gpu
-def test_timed_matvec_is_refused_on_a_stream_under_capture():
-    """There is no result to wait for; the capture itself goes on."""
-    from rptc_b200 import CODE_HASH, LAYOUT_CHUNKED, Format
-    from rptc_b200._lib import native
-    m = n = 2048
-    fmt = Format(CODE_HASH, 2, 16, 8, LAYOUT_CHUNKED)
-    codes, lut = torch.zeros(m * n // 16, dtype=torch.int32, device="cuda"), torch.ones(fmt.lut_numel(), dtype=torch.float16, device="cuda")
-    x, y, acc, a = torch.ones(n, device="cuda").half(), torch.zeros(m, device="cuda").half(), torch.zeros((1, m), device="cuda"), torch.zeros(1, device="cuda")
-    graph = torch.cuda.CUDAGraph()
-    torch.cuda.synchronize()
+_UNDER_CAPTURE = """
+import torch
+from rptc_b200 import CODE_HASH, LAYOUT_CHUNKED, Format
+from rptc_b200._lib import native
+m = n = 2048
+fmt = Format(CODE_HASH, 2, 16, 8, LAYOUT_CHUNKED)
+codes, lut = torch.zeros(m * n // 16, dtype=torch.int32, device="cuda"), torch.ones(fmt.lut_numel(), dtype=torch.float16, device="cuda")
+x, y, acc, a = torch.ones(n, device="cuda").half(), torch.zeros(m, device="cuda").half(), torch.zeros((1, m), device="cuda"), torch.zeros(1, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+try:
     with torch.cuda.graph(graph):
         a += 1
         status = native().gemv_timed(codes, lut, x, acc, y, m, n, 0, 0, fmt)
-    graph.replay()
-    torch.cuda.synchronize()
-    assert status == -5 and (a == 1).all() and not y.any()
-    assert native().gemv_timed(codes, lut, x, acc, y, m, n, 0, 0, fmt) > 0 and y.any()
+    ended = False
+except RuntimeError as e:
+    ended = "capture" in str(e)
+torch.cuda.synchronize()
+assert ended and status == -5 and not a.any() and not y.any(), (ended, status)
+assert native().gemv_timed(codes, lut, x, acc, y, m, n, 0, 0, fmt) > 0 and y.any()
+print("refused")
+"""
+
+
+@pytest.mark.gpu
+def test_timed_matvec_is_refused_on_a_stream_under_capture():
+    """There is no result to wait for, and no graph may come of a capture that holds the kernel.  In a process of its own: torch's generators stay
+    in the state of a capture that ended with an error."""
+    env = dict(os.environ, PYTHONPATH=os.path.join(os.path.dirname(HERE), "let-it-slide_b200"))
+    r = subprocess.run([sys.executable, "-c", _UNDER_CAPTURE], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "refused", r.stdout + r.stderr
